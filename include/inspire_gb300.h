@@ -466,7 +466,7 @@ int ig_response_encode_rims_device(ig_ctx* ctx, uint32_t count, const uint64_t* 
 int ig_profile_enable(ig_ctx* ctx, int on);
 int ig_profile_read(ig_ctx* ctx, double* ms, uint64_t* counts, int regions, int reset);
 /* Integer roofline probe: runs blocks_per_sm x SMs CTAs of 256 threads, each thread iters
- * rounds of eight lazy butterflies (one Shoup product mod q each) on register-resident
+ * rounds of eight lazy butterflies (one product mod q each) on register-resident
  * words, and stores the measured butterflies per second. The respond kernels' transform
  * and product rates are reported against it. */
 int ig_butterfly_peak(ig_ctx* ctx, int blocks_per_sm, int iters, double* per_s);

@@ -288,7 +288,7 @@ class Context:
         self.check(self._lib.ig_ctx_join(self.h))
 
     def butterfly_peak(self, blocks_per_sm=4, iters=4096):
-        """Measured rate of lazy mod-q butterflies (one Shoup product each) in registers, per
+        """Measured rate of lazy mod-q butterflies (one product each) in registers, per
         second: the integer ceiling of the transform work."""
         v = ctypes.c_double()
         self.check(self._lib.ig_butterfly_peak(self.h, blocks_per_sm, iters, ctypes.byref(v)))

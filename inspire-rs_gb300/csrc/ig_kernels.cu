@@ -29,60 +29,75 @@ using namespace ig;
 // inverse ladder (math/ntt.rs:626-654) without the final n^-1, which consumers fold into
 // their first use. Both are linear in standard form.
 //
-// Radix-4 transforms: each thread carries one 4-element unit through two
-// consecutive stages in registers (N/4 threads), halving shared-memory round trips and
-// barriers against a stage-per-barrier radix-2 schedule. Odd log n adds one radix-2 stage
-// (first in the forward, last in the inverse). The butterflies are Harvey's lazy ones: the
-// forward keeps words in [0, 4q) and the inverse in [0, 2q) (inputs canonical), reducing
-// only where the bound requires; results agree with the reference transform mod q. The
-// recursion kernels' per-link transforms use bf_fwd8 / bf_inv4 instead, whose products
-// take one 32-bit multiply fewer and whose words stay below 8q and 4q.
+// Radix-4 transforms: each thread carries one 4-element unit through two consecutive stages in
+// registers (N/4 threads), halving shared-memory round trips and barriers against a
+// stage-per-barrier radix-2 schedule. Odd log n adds one radix-2 stage (first in the forward,
+// last in the inverse). Words are lazy: a product by a twiddle (mulw) lands in [0, 2q + 2^47) for
+// any 64-bit operand, so a 64-bit word has room for 16q of sums and a word is brought back to
+// just above q (red60) only where the next sums could pass that. Bounds are written beside each
+// pass in units of q; "2+" is a little above 2q.
 
-// Forward CT butterfly on lazy words: X, Y < 4q in, both outputs < 4q.
-__device__ __forceinline__ void bf_fwd(u64& X, u64& Y, u64 w, u64 wp) {
-  const u64 x = csub2(X);
-  const u64 t = shoup_lazy(Y, w, wp);
-  X = x + t;
-  Y = x - t + 2 * Q;
+// Forward butterfly (Cooley-Tukey): X grows by at most 3q, Y is any 64-bit word.
+__device__ __forceinline__ void bf_fwd(u64& X, u64& Y, const Tw& w) {
+  const u64 t = mulw(Y, w);
+  Y = X - t + 3 * Q;
+  X += t;
 }
 
-// Inverse GS butterfly: X, Y < 2q in, both outputs < 2q.
-__device__ __forceinline__ void bf_inv(u64& X, u64& Y, u64 w, u64 wp) {
-  const u64 u = csub2(X + Y);
-  Y = shoup_lazy(X - Y + 2 * Q, w, wp);
-  X = u;
+// Inverse butterfly (Gentleman-Sande), X, Y -> X + Y, (X - Y) w^-1, with the forward ladder's
+// entry f of the mirrored index: w^-1 = psi^-brv(m) = -f, so (X - Y) w^-1 = (Y - X) f, and
+// f = ladder[3 2^s - 1 - m] for m in [2^s, 2^(s+1)). X must be at most C q.
+template <int C>
+__device__ __forceinline__ void bf_inv(u64& X, u64& Y, const Tw& f) {
+  const u64 d = Y - X + C * Q;
+  X += Y;
+  Y = mulw(d, f);
 }
 
-// The same butterflies on shoup_lazy4 (one 32-bit multiply fewer per product), with the
-// bounds doubled: the forward keeps words below 8q, the inverse below 4q.
-__device__ __forceinline__ void bf_fwd8(u64& X, u64& Y, u64 w, u64 wp) {
-  const u64 x = csub4(X);
-  const u64 t = shoup_lazy4(Y, w, wp);
-  X = x + t;
-  Y = x - t + 4 * Q;
-}
-__device__ __forceinline__ void bf_inv4(u64& X, u64& Y, u64 w, u64 wp) {
-  const u64 u = csub4(X + Y);
-  Y = shoup_lazy4(X - Y + 4 * Q, w, wp);
-  X = u;
+// Two forward stages on a unit; out <= in + 6. RED brings the two words that are not multiplied
+// first down to 1, and the outputs are then at most 7.
+template <bool RED>
+__device__ __forceinline__ void fwd_unit(u64& a0, u64& a1, u64& a2, u64& a3, const Tw& wa, const Tw& wb,
+                                         const Tw& wc) {
+  if (RED) {
+    a0 = red60(a0);
+    a1 = red60(a1);
+  }
+  bf_fwd(a0, a2, wa);
+  bf_fwd(a1, a3, wa);
+  bf_fwd(a0, a1, wb);
+  bf_fwd(a2, a3, wc);
 }
 
+// Two inverse stages on a unit of words up to 2+: sums up to 8+ and 4+ come back to 1, products
+// are 2+.
+__device__ __forceinline__ void inv_unit(u64& a0, u64& a1, u64& a2, u64& a3, const Tw& f0, const Tw& f1,
+                                         const Tw& f2) {
+  bf_inv<3>(a0, a1, f0);
+  bf_inv<3>(a2, a3, f1);
+  bf_inv<5>(a0, a2, f2);
+  bf_inv<3>(a1, a3, f2);
+  a0 = red60(a0);
+  a1 = red60(a1);
+}
+
+// In: at most 2. Out: at most 7.
 template <int LOGN, int NT, int NB>
-__device__ __forceinline__ void ntt_fwd_r4(u64* const (&x)[NB], const u64* tw, const u64* twp) {
+__device__ __forceinline__ void ntt_fwd_r4(u64* const (&x)[NB], const Tw* tw) {
   constexpr int N = 1 << LOGN, UPT = N / 4 / NT;
   static_assert(UPT >= 1 && (N / 4) % NT == 0, "whole radix-4 units per thread");
   const int tid = threadIdx.x;
   int s = 0;
   if (LOGN & 1) {
     constexpr int t = N / 2;
-    const u64 w = tw[1], wp = twp[1];
+    const Tw w = tw[1];
 #pragma unroll
     for (int r = 0; r < 2 * UPT; r++) {
       const int b = tid + r * NT;
 #pragma unroll
       for (int k = 0; k < NB; k++) {
         u64 a = x[k][b], c = x[k][b + t];
-        bf_fwd(a, c, w, wp);
+        bf_fwd(a, c, w);
         x[k][b] = a;
         x[k][b + t] = c;
       }
@@ -98,16 +113,11 @@ __device__ __forceinline__ void ntt_fwd_r4(u64* const (&x)[NB], const u64* tw, c
       const int u = tid + uu * NT;
       const int i = u / h, o = u - i * h;
       const int e0 = i * 2 * t + o;
-      const u64 wa = tw[m + i], wap = twp[m + i];
-      const u64 wb = tw[2 * m + 2 * i], wbp = twp[2 * m + 2 * i];
-      const u64 wc = tw[2 * m + 2 * i + 1], wcp = twp[2 * m + 2 * i + 1];
+      const Tw wa = tw[m + i], wb = tw[2 * m + 2 * i], wc = tw[2 * m + 2 * i + 1];
 #pragma unroll
       for (int k = 0; k < NB; k++) {
         u64 a0 = x[k][e0], a1 = x[k][e0 + h], a2 = x[k][e0 + t], a3 = x[k][e0 + t + h];
-        bf_fwd(a0, a2, wa, wap);
-        bf_fwd(a1, a3, wa, wap);
-        bf_fwd(a0, a1, wb, wbp);
-        bf_fwd(a2, a3, wc, wcp);
+        fwd_unit<true>(a0, a1, a2, a3, wa, wb, wc);
         x[k][e0] = a0;
         x[k][e0 + h] = a1;
         x[k][e0 + t] = a2;
@@ -118,17 +128,9 @@ __device__ __forceinline__ void ntt_fwd_r4(u64* const (&x)[NB], const u64* tw, c
   }
 }
 
-// Inverse ladder entry m from the forward one: psi^-brv(m) = q - f[3*2^s - 1 - m] for m in
-// [2^s, 2^(s+1)), and the Shoup companion of q - w is the bitwise complement of w's.
-__device__ __forceinline__ void inv_twiddle(const u64* tw, const u64* twp, int m, u64& w, u64& wp) {
-  const int s = 31 - __clz(m);
-  const int mp = 3 * (1 << s) - 1 - m;
-  w = Q - tw[mp];
-  wp = ~twp[mp];
-}
-
+// In: at most 2+. Out: at most 4+, without n^-1.
 template <int LOGN, int NT, int NB>
-__device__ __forceinline__ void ntt_inv_r4(u64* const (&x)[NB], const u64* tw, const u64* twp) {
+__device__ __forceinline__ void ntt_inv_r4(u64* const (&x)[NB], const Tw* tw) {
   constexpr int N = 1 << LOGN, UPT = N / 4 / NT;
   static_assert(UPT >= 1 && (N / 4) % NT == 0, "whole radix-4 units per thread");
   const int tid = threadIdx.x;
@@ -141,17 +143,11 @@ __device__ __forceinline__ void ntt_inv_r4(u64* const (&x)[NB], const u64* tw, c
       const int u = tid + uu * NT;
       const int B = u >> s, o = u & (t - 1);
       const int e0 = B * 4 * t + o;
-      u64 w0, w0p, w1, w1p, w2, w2p;
-      inv_twiddle(tw, twp, m + 2 * B, w0, w0p);
-      inv_twiddle(tw, twp, m + 2 * B + 1, w1, w1p);
-      inv_twiddle(tw, twp, (m >> 1) + B, w2, w2p);
+      const Tw f0 = tw[2 * m - 1 - 2 * B], f1 = tw[2 * m - 2 - 2 * B], f2 = tw[m - 1 - B];
 #pragma unroll
       for (int k = 0; k < NB; k++) {
         u64 a0 = x[k][e0], a1 = x[k][e0 + t], a2 = x[k][e0 + 2 * t], a3 = x[k][e0 + 3 * t];
-        bf_inv(a0, a1, w0, w0p);
-        bf_inv(a2, a3, w1, w1p);
-        bf_inv(a0, a2, w2, w2p);
-        bf_inv(a1, a3, w2, w2p);
+        inv_unit(a0, a1, a2, a3, f0, f1, f2);
         x[k][e0] = a0;
         x[k][e0 + t] = a1;
         x[k][e0 + 2 * t] = a2;
@@ -162,15 +158,14 @@ __device__ __forceinline__ void ntt_inv_r4(u64* const (&x)[NB], const u64* tw, c
   }
   if (LOGN & 1) {
     constexpr int t = N / 2;
-    u64 w, wp;
-    inv_twiddle(tw, twp, 1, w, wp);
+    const Tw f = tw[1];
 #pragma unroll
     for (int r = 0; r < 2 * UPT; r++) {
       const int b = tid + r * NT;
 #pragma unroll
       for (int k = 0; k < NB; k++) {
         u64 a = x[k][b], c = x[k][b + t];
-        bf_inv(a, c, w, wp);
+        bf_inv<3>(a, c, f);
         x[k][b] = a;
         x[k][b + t] = c;
       }
@@ -182,26 +177,23 @@ __device__ __forceinline__ void ntt_inv_r4(u64* const (&x)[NB], const u64* tw, c
 // ------------------------------------------------------------------------------------
 // Batched forward NTT: one CTA per row.
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 4) k_ntt_rows(CrsDev c, const u64* in, u64* out, u64 scale,
-                                                              u64 scalep) {
+__global__ void __launch_bounds__((1 << LOGN) / 4) k_ntt_rows(CrsDev c, const u64* in, u64* out, Tw scale) {
   constexpr int N = 1 << LOGN, NT = N / 4;
   extern __shared__ __align__(16) u64 sm[];
-  u64* x = sm;
-  u64* tw = sm + N;
-  u64* twp = sm + 2 * N;
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* x = sm + 2 * N;
   const u64* row = in + (size_t)blockIdx.x * N;
   for (int k = threadIdx.x; k < N; k += NT) {
     x[k] = reduce128(row[k]);
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
   }
   __syncthreads();
   {
     u64* const bufs[1] = {x};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
   u64* o = out + (size_t)blockIdx.x * N;
-  for (int k = threadIdx.x; k < N; k += NT) o[k] = shoup(x[k], scale, scalep);
+  for (int k = threadIdx.x; k < N; k += NT) o[k] = canon(mulw(x[k], scale));
 }
 
 // ------------------------------------------------------------------------------------
@@ -592,56 +584,99 @@ __device__ __forceinline__ u64 mod_switch_word(u64 cv, u64 qn) {
   return quo % qn;
 }
 
-// Rows X_0, X_1, X_2 (R-form, `stride` words apart) of a 3-digit gadget key, folded for
+// Rows X_0, X_1, X_2 (R-form, `stride` words apart, `dst_stride` in dst) of a 3-digit gadget key, folded for
 // digits whose third transform is derived, D_2 = base^-2 (R - D_0 - base D_1):
 //   sum_k X_k D_k = D_0 (X_0 - base^-2 X_2) + D_1 (X_1 - base^-1 X_2) + R base^-2 X_2.
 // The folded rows are R-form too; a consumer then needs neither D_2 nor its reduction.
 // Every read precedes every write, so src may equal dst.
 __device__ __forceinline__ void fold_gadget3(u64 ld_inv_R, u64 ld_c0_R, u64 ld_c1_R, const u64* src, u64* dst,
-                                             int stride) {
+                                             int stride, int dst_stride) {
   const u64 x0 = src[0], x1 = src[stride], x2 = src[2 * stride];
   const u64 f0 = addq(x0, mont(x2, ld_c0_R));
   const u64 f1 = addq(x1, mont(x2, ld_c1_R));
   const u64 f2 = mont(x2, ld_inv_R);
   dst[0] = f0;
-  dst[stride] = f1;
-  dst[2 * stride] = f2;
+  dst[dst_stride] = f1;
+  dst[2 * dst_stride] = f2;
 }
 
-// The Galois keys ([key][digit][part][n], R-form NTT) folded in place by fold_gadget3.
+// The Galois keys ([key][digit][part][n], R-form NTT) folded in place by fold_gadget3 and brought
+// to standard form. The tree holds n^-1 times each node, so a digit's product is scaled by n^-1
+// and the node's own stays.
 __global__ void k_fold_gadget_keys(CrsDev c, u64* keys, u32 count) {
   const u32 n = c.n;
   const u32 i = blockIdx.x * blockDim.x + threadIdx.x;  // (key, part, coefficient)
   if (i >= count * 2 * n) return;
   const u32 key = i / (2 * n), r = i - key * 2 * n;
   u64* x = keys + (size_t)key * 6 * n + r;
-  fold_gadget3(c.ld_inv_R, c.ld_c0_R, c.ld_c1_R, x, x, (int)(2 * n));
+  fold_gadget3(c.ld_inv_R, c.ld_c0_R, c.ld_c1_R, x, x, (int)(2 * n), (int)(2 * n));
+  x[0] = canon(mulw(x[0], c.s_ninv_rinv));
+  x[2 * n] = canon(mulw(x[2 * n], c.s_ninv_rinv));
+  x[4 * n] = canon(mulw(x[4 * n], c.s_rinv));
 }
 
-// Per-query constants into shared memory: forward ladder and slot tables of the ring (c),
-// the mask rows of the query's parameter set (v) and the seat's key rows (both R-form NTT;
-// with the exact gadget, folded by fold_gadget3).
+// Key rows of one query in shared memory, standard form: the rows of digits 0 and 1 side by side
+// for the mask (W01) and the seat (Y01), the rows of the derived digit 2 of both (WY2). The
+// pointwise step gathers them with three 16-byte loads a slot.
+struct KeyRows {
+  ulonglong2 *W01, *Y01, *WY2;
+};
+
+// Per-query constants into shared memory: forward ladder and slot tables of the ring (c), the mask
+// rows of the query's parameter set (v) and the seat's key rows (R-form NTT in global memory). The
+// recursion holds c_i = n^-1 R_i, so the inverse transform of a link needs no n^-1:
+//   c_i = (n^-1 a)[tau] S + sum_k (n^-1 W_k)[tau] D_k,   sum_b += sum_k Y_k[tau] D_k,
+// and with the exact gadget (rows folded by fold_gadget3), where R_{i+1} = n c_{i+1} takes the third
+// digit's place, W_2 stays and Y_2 is scaled by n.
 template <int N, int NT>
-__device__ __forceinline__ void stage_constants(const CrsDev& c, const SetView& v, const u64* yR, u64* tw, u64* twp,
-                                                u64* Wm, u64* Y, uint16_t* e_tab, uint16_t* s_tab) {
+__device__ __forceinline__ void stage_constants(const CrsDev& c, const SetView& v, const u64* yR, Tw* tw,
+                                                const KeyRows& K, uint16_t* e_tab, uint16_t* s_tab) {
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
     e_tab[k] = c.slot_exp[k];
     s_tab[k] = c.exp_slot[k];
-  }
-  if (v.approx == 0) {
-    for (int k = threadIdx.x; k < N; k += NT) {
-      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, v.wmask_R + k, Wm + k, N);
-      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, yR + k, Y + k, N);
+    u64 w[3] = {v.wmask_R[k], v.wmask_R[N + k], 0}, y[3] = {yR[k], yR[N + k], 0};
+    if (v.approx == 0) {
+      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, v.wmask_R + k, w, N, 1);
+      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, yR + k, y, N, 1);
     }
-  } else {
-    for (u32 k = threadIdx.x; k < v.rows * N; k += NT) {
-      Wm[k] = v.wmask_R[k];
-      Y[k] = yR[k];
-    }
+    K.W01[k] = make_ulonglong2(canon(mulw(w[0], c.s_ninv_rinv)), canon(mulw(w[1], c.s_ninv_rinv)));
+    K.Y01[k] = make_ulonglong2(canon(mulw(y[0], c.s_rinv)), canon(mulw(y[1], c.s_rinv)));
+    K.WY2[k] = make_ulonglong2(canon(mulw(w[2], c.s_rinv)), canon(mulw(y[2], c.s_n_rinv)));
   }
 }
+
+// The query's `a` (coefficient form, in place) to n^-1 2^-64 NTT(a): the factor that takes an R-form
+// store word to c_i's scale. Ends with a barrier.
+template <int LOGN, int NT>
+__device__ __forceinline__ void transform_a(const CrsDev& c, u64* a, const Tw* tw) {
+  u64* const bufs[1] = {a};
+  ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
+#pragma unroll
+  for (int k = threadIdx.x; k < (1 << LOGN); k += NT) a[k] = canon(mulw(a[k], c.s_ninv_rinv));
+  __syncthreads();
+}
+
+// The pointwise step of one slot at the gathered position tb: adds sum_k Y_k D_k to sb and returns
+// c_i. d0, d1 at most 15q, cur at most 1+: sb takes at most 31 q^2 < 2^125 a call.
+__device__ __forceinline__ u64 link_slot(Acc& sb, u64 d0, u64 d1, u64 cur, u64 s_R, const u64* a_ntt,
+                                         const KeyRows& K, u32 tb, bool exact) {
+  const ulonglong2 w = K.W01[tb], y = K.Y01[tb];
+  Acc r{0, 0, 0, 0};
+  mac(r, a_ntt[tb], s_R);
+  mac(r, d0, w.x);
+  mac(sb, d0, y.x);
+  mac(r, d1, w.y);
+  mac(sb, d1, y.y);
+  if (exact) {  // the rows are folded: c_{i+1} stands in for digit 2
+    const ulonglong2 z = K.WY2[tb];
+    mac(r, cur, z.x);
+    mac(sb, cur, z.y);
+  }
+  return acc_fold(r);
+}
+// The links whose slot sums go without a fold: 4 x 2^125 and what is carried in stay below 2^128.
+constexpr int SB_FOLD_LINKS = 4;
 
 // The query's `a` in coefficient form: the ChaCha20 keystream of its seed as u64 words
 // in order, each accepted by rand's gen_range(0..q) rule (math/poly.rs:657-671). Block b
@@ -692,12 +727,14 @@ __device__ __forceinline__ void expand_a(const QueryDev& qd, u64* a, u32* status
   }
 }
 
-__device__ __forceinline__ u64 finish_a(const CrsDev& c, u64 x, u64 ms) {
-  const u64 v = shoup(x, c.ninv, c.ninvp);
+// Coefficients of the response from the unscaled inverse transforms of c_0 = n^-1 R_0 (a) and of
+// the online sum (b).
+__device__ __forceinline__ u64 finish_a(u64 x, u64 ms) {
+  const u64 v = canon(x);
   return ms ? mod_switch_word(v, ms) : v;
 }
 __device__ __forceinline__ u64 finish_b(const CrsDev& c, u64 x, u32 t, u32 gamma, const u64* fold, u64 ms) {
-  u64 v = shoup(x, c.ninv, c.ninvp);
+  u64 v = canon(mulw(x, c.ninv));
   if (t < gamma) v = addq(v, fold[t]);
   return ms ? mod_switch_word(v, ms) : v;
 }
@@ -711,18 +748,165 @@ __device__ __forceinline__ u64 finish_b(const CrsDev& c, u64 x, u32 t, u32 gamma
 __device__ __forceinline__ int sw(int e) { return e ^ (((e >> 4) & 3) << 2); }
 
 // ------------------------------------------------------------------------------------
+// The digits 0 and 1 of a canonical coefficient: base 2^20, of the coefficient itself (exact) or of
+// its rounding to a multiple of 2^20 with the lowest digit dropped (the top carry is kept).
+__device__ __forceinline__ void split_digits(u64 r, bool exact, u32& g0, u32& g1) {
+  constexpr u32 DMASK = (1u << 20) - 1;
+  if (exact) {
+    g0 = (u32)r & DMASK;
+    g1 = (u32)(r >> 20) & DMASK;
+  } else {
+    const u64 rr = (r + (1ULL << 19)) >> 20;
+    g0 = (u32)rr & DMASK;
+    g1 = (u32)(rr >> 20);
+  }
+}
+
+// Inverse stages S .. logn-2 in shared memory, words up to 2+ (radix-4 pairs; a radix-2 stage last
+// when logn is even, its sums up to 4+). Each pass ends with a barrier.
+template <int LOGN, int S>
+__device__ __forceinline__ void inv_middle(u64* X, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 4;
+  const int tid = threadIdx.x;
+  if constexpr (S + 1 <= LOGN - 2) {
+    constexpr int t = 1 << S, m = N >> (S + 1);
+    const int B = tid >> S, o = tid & (t - 1);
+    const int e0 = B * 4 * t + o;
+    const int i0 = sw(e0), i1 = sw(e0 + t), i2 = sw(e0 + 2 * t), i3 = sw(e0 + 3 * t);
+    u64 a0 = X[i0], a1 = X[i1], a2 = X[i2], a3 = X[i3];
+    inv_unit(a0, a1, a2, a3, tw[2 * m - 1 - 2 * B], tw[2 * m - 2 - 2 * B], tw[m - 1 - B]);
+    X[i0] = a0;
+    X[i1] = a1;
+    X[i2] = a2;
+    X[i3] = a3;
+    __syncthreads();
+    inv_middle<LOGN, S + 2>(X, tw);
+  } else if constexpr (S == LOGN - 2) {
+    constexpr int t = 1 << S, m = N >> (S + 1);
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int v = tid + r * NT;
+      const int B = v >> S, o = v & (t - 1);
+      const int e = sw(B * 2 * t + o), f = sw(B * 2 * t + o + t);
+      u64 a = X[e], b = X[f];
+      bf_inv<3>(a, b, tw[2 * m - 1 - B]);
+      X[e] = a;
+      X[f] = b;
+    }
+    __syncthreads();
+  }
+}
+
+// Forward stages S .. logn-3 of digits 0 and 1 (x and x + N) in shared memory, words up to BIN in
+// (a radix-2 stage first when their count is odd), up to fwd_bound out. Each pass ends with a barrier.
+constexpr int FWD_FREE = 9;  // a unit whose words are at most this needs no reduction: 9 + 6 < 16
+__host__ __device__ constexpr int fwd_bound(int logn, int s, int b) {
+  if ((logn - 2 - s) & 1) b += 3, s++;
+  for (; s < logn - 2; s += 2) b = (b > FWD_FREE ? 1 : b) + 6;
+  return b;
+}
+template <int LOGN, int S, int BIN>
+__device__ __forceinline__ void fwd_middle(u64* D, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 4;
+  const int tid = threadIdx.x;
+  if constexpr (S < LOGN - 2 && ((LOGN - 2 - S) & 1)) {
+    constexpr int lt = LOGN - S - 1, t = 1 << lt;
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int v = tid + r * NT;
+      const int ib = v >> lt, o = v & (t - 1);
+      const int e = sw(ib * 2 * t + o), f = sw(ib * 2 * t + o + t);
+      const Tw w = tw[(1 << S) + ib];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        u64* x = D + k * N;
+        u64 a = x[e], b = x[f];
+        bf_fwd(a, b, w);
+        x[e] = a;
+        x[f] = b;
+      }
+    }
+    __syncthreads();
+    fwd_middle<LOGN, S + 1, BIN + 3>(D, tw);
+  } else if constexpr (S < LOGN - 2) {
+    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S, h = t >> 1;
+    constexpr bool RED = BIN > FWD_FREE;
+    const int ib = tid >> (lt - 1), o = tid & (h - 1);
+    const int e0 = ib * 2 * t + o;
+    const Tw wa = tw[m + ib], wb = tw[2 * m + 2 * ib], wc = tw[2 * m + 2 * ib + 1];
+    const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + t), i3 = sw(e0 + t + h);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      u64* x = D + k * N;
+      u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
+      fwd_unit<RED>(a0, a1, a2, a3, wa, wb, wc);
+      x[i0] = a0;
+      x[i1] = a1;
+      x[i2] = a2;
+      x[i3] = a3;
+    }
+    __syncthreads();
+    fwd_middle<LOGN, S + 2, (RED ? 1 : BIN) + 6>(D, tw);
+  }
+}
+
+// One link's transforms on one CTA of N/4 threads: thread tid holds the NTT-domain words cur of its
+// unit (slots 4 tid .. 4 tid + 3, at most 1+, scaled by n^-1) and gets the transforms d0, d1 of digits
+// 0 and 1 of their inverse transform at the same slots, at most 15. The inverse's first two stages and
+// the forward's last two act within a unit and run in registers; the inverse's last stage, the digit
+// split and the forward's first stage are one pass over the pairs (b, b + N/2). X: N words, D: 2N.
+template <int LOGN>
+__device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4], u64 (&d1)[4], u64* X, u64* D,
+                                                const Tw* tw, bool exact) {
+  constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2, MF = 1 << (LOGN - 2);
+  const int tid = threadIdx.x, l0 = 4 * tid;
+  {
+    u64 a0 = cur[0], a1 = cur[1], a2 = cur[2], a3 = cur[3];
+    inv_unit(a0, a1, a2, a3, tw[N - 1 - 2 * tid], tw[N - 2 - 2 * tid], tw[H - 1 - tid]);
+    *reinterpret_cast<ulonglong2*>(X + sw(l0)) = make_ulonglong2(a0, a1);
+    *reinterpret_cast<ulonglong2*>(X + sw(l0 + 2)) = make_ulonglong2(a2, a3);
+  }
+  __syncthreads();
+  inv_middle<LOGN, 2>(X, tw);
+  const Tw wf = tw[1];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int b = sw(tid + j * NT), b2 = sw(tid + j * NT + H);
+    const u64 x0 = X[b], x1 = X[b2];
+    u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + N/2
+    split_digits(canon(x0 + x1), exact, p0, p1);
+    split_digits(canon(mulw(x1 - x0 + 5 * Q, wf)), exact, q0, q1);
+    const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
+    D[b] = p0 + t0;
+    D[b2] = p0 + 3 * Q - t0;
+    D[N + b] = p1 + t1;
+    D[N + b2] = p1 + 3 * Q - t1;
+  }
+  __syncthreads();
+  fwd_middle<LOGN, 1, 3>(D, tw);
+  {
+    constexpr bool RED = fwd_bound(LOGN, 1, 3) > FWD_FREE;
+    const Tw fa = tw[MF + tid], fb = tw[2 * MF + 2 * tid], fc = tw[2 * MF + 2 * tid + 1];
+    const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(D + sw(l0));
+    const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(D + sw(l0 + 2));
+    const ulonglong2 g01 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0));
+    const ulonglong2 g23 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0 + 2));
+    d0[0] = v01.x, d0[1] = v01.y, d0[2] = v23.x, d0[3] = v23.y;
+    d1[0] = g01.x, d1[1] = g01.y, d1[2] = g23.x, d1[3] = g23.y;
+    fwd_unit<RED>(d0[0], d0[1], d0[2], d0[3], fa, fb, fc);
+    fwd_unit<RED>(d1[0], d1[1], d1[2], d1[3], fa, fb, fc);
+  }
+}
+
 // One CTA per query (batches that fill the GPU). Thread u owns slots 4u..4u+3 of every
 // NTT-domain vector (one transform unit). Each link of the recursion (i from gamma-2 down
-// to 0) holds R_{i+1} in NTT form (`cur`, in registers):
+// to 0) holds n^-1 R_{i+1} in NTT form (`cur`, in registers):
 //   r = INTT(R_{i+1});  d_k = base-2^20 digits of r (rounded, top carry kept, when the
 //   lowest digit is dropped);  D_k = NTT(d_k);
 //   sum_b += sum_k Y_k[tau_i(t)] D_k[t];
 //   R_i[t] = a_ntt[tau_i(t)] S_i[t] + sum_k W_k[tau_i(t)] D_k[t]
 // with tau_i the slot permutation of the automorphism X -> X^(g^i), S the packing store,
-// W the mask rows and Y the seat. Each sum of products takes one Montgomery reduction.
-// The inverse's first two stages and the forward's last two act within each thread's unit
-// and run in registers; the inverse's last stage, n^-1, the digit split and the forward's
-// first stage fuse into one pass. Digits 0 and 1 are transformed; with the exact gadget
+// W the mask rows and Y the seat. Digits 0 and 1 are transformed; with the exact gadget
 // digit 2's transform is D_2 = base^-2 (R_{i+1} - D_0 - base D_1) (inspiring2.rs:1094-1161),
 // a fixed linear combination, so the key rows are folded at staging (fold_gadget3) and
 // R_{i+1} takes digit 2's place in the sums.
@@ -730,20 +914,18 @@ template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
     k_respond(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out, u64* b_out,
               u32* status, int force_serial) {
-  constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2;
+  constexpr int N = 1 << LOGN, NT = N / 4;
   constexpr u32 M2N = 2 * N - 1;
-  constexpr u64 DMASK = (1ULL << 20) - 1;
   extern __shared__ __align__(16) u64 sm[];
   u64* X = sm;       // N: the inverse in progress
   u64* D = sm + N;   // 2N: digits 0 and 1 (forward in progress)
   u64* a_ntt = D + 2 * N;
-  u64* tw = a_ntt + N;
-  u64* twp = tw + N;
+  Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
   // Room for three key rows whatever the query's gadget, so queries of different sets
   // share a launch.
-  u64* Wm = twp + N;
-  u64* Y = Wm + 3 * N;
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(Y + 3 * N);
+  ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);
+  const KeyRows K{rows, rows + N, rows + 2 * N};
+  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
   uint16_t* s_tab = e_tab + N;
 
   const int tid = threadIdx.x;
@@ -755,14 +937,12 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
   const bool exact = ps.approx == 0;
   const int l0 = 4 * tid;
 
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, twp, Wm, Y, e_tab, s_tab);
+  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
   expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  {
-    u64* const bufs[1] = {a_ntt};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
-  }
+  transform_a<LOGN, NT>(c, a_ntt, tw);
 
-  u64 cur[4], sb[4];
+  u64 cur[4];
+  Acc sb[4];
   u32 et[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) et[k] = e_tab[l0 + k];
@@ -772,202 +952,44 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = mont(a_ntt[tb], Srow[l0 + k]);
-      sb[k] = 0;
+      cur[k] = mulq(a_ntt[tb], Srow[l0 + k]);
+      sb[k] = Acc{0, 0, 0, 0};
     }
   }
-  constexpr int MF = 1 << (LOGN - 2);
-  const u64 wf = tw[1], wfp = twp[1];
 #pragma unroll 1
   for (int i = (int)gamma - 2; i >= 0; i--) {
     const u64* Srow = sh.sums_R + (size_t)i * N + l0;
     const ulonglong2 sv01 = *reinterpret_cast<const ulonglong2*>(Srow);
     const ulonglong2 sv23 = *reinterpret_cast<const ulonglong2*>(Srow + 2);
     const u32 gp = ps.gpow[i];
-    {
-      // Inverse stages 0-1 of unit tid (block B = tid, m = N/2).
-      u64 w0, w0p, w1, w1p, w2, w2p;
-      inv_twiddle(tw, twp, H + 2 * tid, w0, w0p);
-      inv_twiddle(tw, twp, H + 2 * tid + 1, w1, w1p);
-      inv_twiddle(tw, twp, H / 2 + tid, w2, w2p);
-      u64 a0 = cur[0], a1 = cur[1], a2 = cur[2], a3 = cur[3];
-      bf_inv4(a0, a1, w0, w0p);
-      bf_inv4(a2, a3, w1, w1p);
-      bf_inv4(a0, a2, w2, w2p);
-      bf_inv4(a1, a3, w2, w2p);
-      *reinterpret_cast<ulonglong2*>(X + sw(l0)) = make_ulonglong2(a0, a1);
-      *reinterpret_cast<ulonglong2*>(X + sw(l0 + 2)) = make_ulonglong2(a2, a3);
-    }
-    __syncthreads();
-    // Inverse stages 2 .. logn-2 (radix-4 pairs, a radix-2 stage last when logn is even).
-    int s = 2;
-#pragma unroll 1
-    for (; s + 1 <= LOGN - 2; s += 2) {
-      const int t = 1 << s, m = N >> (s + 1);
-      const int B = tid >> s, o = tid & (t - 1);
-      const int e0 = B * 4 * t + o;
-      u64 w0, w0p, w1, w1p, w2, w2p;
-      inv_twiddle(tw, twp, m + 2 * B, w0, w0p);
-      inv_twiddle(tw, twp, m + 2 * B + 1, w1, w1p);
-      inv_twiddle(tw, twp, (m >> 1) + B, w2, w2p);
-      u64 a0 = X[sw(e0)], a1 = X[sw(e0 + t)], a2 = X[sw(e0 + 2 * t)], a3 = X[sw(e0 + 3 * t)];
-      bf_inv4(a0, a1, w0, w0p);
-      bf_inv4(a2, a3, w1, w1p);
-      bf_inv4(a0, a2, w2, w2p);
-      bf_inv4(a1, a3, w2, w2p);
-      X[sw(e0)] = a0;
-      X[sw(e0 + t)] = a1;
-      X[sw(e0 + 2 * t)] = a2;
-      X[sw(e0 + 3 * t)] = a3;
-      __syncthreads();
-    }
-    if (s == LOGN - 2) {
-      const int t = 1 << s, m = N >> (s + 1);
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int v = tid + r * NT;
-        const int B = v >> s, o = v & (t - 1);
-        const int e = B * 2 * t + o;
-        u64 w, wp;
-        inv_twiddle(tw, twp, m + B, w, wp);
-        u64 a = X[sw(e)], b = X[sw(e + t)];
-        bf_inv4(a, b, w, wp);
-        X[sw(e)] = a;
-        X[sw(e + t)] = b;
-      }
-      __syncthreads();
-    }
-    // Inverse stage logn-1, n^-1, digit split and forward stage 0, per pair (b, b + N/2).
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int b = tid + j * NT;
-      const u64 x0 = X[sw(b)], x1 = X[sw(b + H)];
-      // The inverse's last stage and n^-1 as one product per output: n^-1 on the sum,
-      // n^-1 times the stage's twiddle on the difference.
-      const u64 r0 = shoup(x0 + x1, c.ninv, c.ninvp), r1 = shoup(x0 - x1 + 4 * Q, c.nlast, c.nlastp);
-      u64 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + N/2
-      if (exact) {
-        p0 = r0 & DMASK;
-        p1 = (r0 >> 20) & DMASK;
-        q0 = r1 & DMASK;
-        q1 = (r1 >> 20) & DMASK;
-      } else {
-        const u64 rr0 = (r0 + (1ULL << 19)) >> 20, rr1 = (r1 + (1ULL << 19)) >> 20;
-        p0 = rr0 & DMASK;
-        p1 = rr0 >> 20;
-        q0 = rr1 & DMASK;
-        q1 = rr1 >> 20;
-      }
-      const u64 t0 = shoup_digit((u32)q0, wf, wfp), t1 = shoup_digit((u32)q1, wf, wfp);
-      D[sw(b)] = p0 + t0;
-      D[sw(b + H)] = p0 + 4 * Q - t0;
-      D[N + sw(b)] = p1 + t1;
-      D[N + sw(b + H)] = p1 + 4 * Q - t1;
-    }
-    __syncthreads();
-    // Forward stages 1 .. logn-3 (a radix-2 stage first when logn is even), both digits.
-    s = 1;
-    if (!(LOGN & 1)) {
-      const int lt = LOGN - 2, t = 1 << lt;
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int v = tid + r * NT;
-        const int ib = v >> lt, o = v & (t - 1);
-        const int e = ib * 2 * t + o;
-        const u64 w = tw[2 + ib], wp = twp[2 + ib];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-          u64* x = D + k * N;
-          u64 a = x[sw(e)], b = x[sw(e + t)];
-          bf_fwd8(a, b, w, wp);
-          x[sw(e)] = a;
-          x[sw(e + t)] = b;
-        }
-      }
-      __syncthreads();
-      s = 2;
-    }
-#pragma unroll 1
-    for (; s < LOGN - 2; s += 2) {
-      const int t = N >> (s + 1), m = 1 << s, h = t >> 1;
-      const int ib = tid / h, o = tid - ib * h;
-      const int e0 = ib * 2 * t + o;
-      const u64 wa = tw[m + ib], wap = twp[m + ib];
-      const u64 wb = tw[2 * m + 2 * ib], wbp = twp[2 * m + 2 * ib];
-      const u64 wc = tw[2 * m + 2 * ib + 1], wcp = twp[2 * m + 2 * ib + 1];
-      const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + t), i3 = sw(e0 + t + h);
-      u64* x0 = D;
-      u64* x1 = D + N;
-      u64 a0 = x0[i0], a1 = x0[i1], a2 = x0[i2], a3 = x0[i3];
-      u64 c0 = x1[i0], c1 = x1[i1], c2 = x1[i2], c3 = x1[i3];
-      bf_fwd8(a0, a2, wa, wap);
-      bf_fwd8(c0, c2, wa, wap);
-      bf_fwd8(a1, a3, wa, wap);
-      bf_fwd8(c1, c3, wa, wap);
-      bf_fwd8(a0, a1, wb, wbp);
-      bf_fwd8(c0, c1, wb, wbp);
-      bf_fwd8(a2, a3, wc, wcp);
-      bf_fwd8(c2, c3, wc, wcp);
-      x0[i0] = a0;
-      x0[i1] = a1;
-      x0[i2] = a2;
-      x0[i3] = a3;
-      x1[i0] = c0;
-      x1[i1] = c1;
-      x1[i2] = c2;
-      x1[i3] = c3;
-      __syncthreads();
-    }
-    // Forward stages logn-2, logn-1 of unit tid, both digits, in registers.
     u64 d0[4], d1[4];
-    {
-      const u64 fa = tw[MF + tid], fap = twp[MF + tid];
-      const u64 fb = tw[2 * MF + 2 * tid], fbp = twp[2 * MF + 2 * tid];
-      const u64 fc = tw[2 * MF + 2 * tid + 1], fcp = twp[2 * MF + 2 * tid + 1];
-      const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(D + sw(l0));
-      const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(D + sw(l0 + 2));
-      const ulonglong2 g01 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0));
-      const ulonglong2 g23 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0 + 2));
-      d0[0] = v01.x, d0[1] = v01.y, d0[2] = v23.x, d0[3] = v23.y;
-      d1[0] = g01.x, d1[1] = g01.y, d1[2] = g23.x, d1[3] = g23.y;
-      bf_fwd8(d0[0], d0[2], fa, fap);
-      bf_fwd8(d1[0], d1[2], fa, fap);
-      bf_fwd8(d0[1], d0[3], fa, fap);
-      bf_fwd8(d1[1], d1[3], fa, fap);
-      bf_fwd8(d0[0], d0[1], fb, fbp);
-      bf_fwd8(d1[0], d1[1], fb, fbp);
-      bf_fwd8(d0[2], d0[3], fc, fcp);
-      bf_fwd8(d1[2], d1[3], fc, fcp);
-    }
+    link_transforms<LOGN>(cur, d0, d1, X, D, tw, exact);
     const u64 sv[4] = {sv01.x, sv01.y, sv23.x, sv23.y};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      u128 nb = wide(d0[k], Y[tb]) + wide(d1[k], Y[N + tb]);
-      u128 nc = wide(a_ntt[tb], sv[k]) + wide(d0[k], Wm[tb]) + wide(d1[k], Wm[N + tb]);
-      if (exact) {  // the rows are folded: R_{i+1} stands in for digit 2
-        nb += wide(cur[k], Y[2 * N + tb]);
-        nc += wide(cur[k], Wm[2 * N + tb]);
-      }
-      sb[k] = addq(sb[k], redc_wide(nb));
-      cur[k] = redc_wide(nc);
+      cur[k] = link_slot(sb[k], d0[k], d1[k], cur[k], sv[k], a_ntt, K, tb, exact);
+    }
+    if (i % SB_FOLD_LINKS == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) sb[k] = acc_from(acc_fold(sb[k]));
     }
   }
   __syncthreads();  // every thread is past its last read of D
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     D[l0 + k] = cur[k];
-    D[N + l0 + k] = sb[k];
+    D[N + l0 + k] = acc_fold(sb[k]);
   }
   __syncthreads();
   {
     u64* const bufs[2] = {D, D + N};
-    ntt_inv_r4<LOGN, NT, 2>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 2>(bufs, tw);
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int t = tid + k * NT;
-    a_out[(size_t)qi * N + t] = finish_a(c, D[t], qd.ms);
+    a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
     b_out[(size_t)qi * N + t] = finish_b(c, D[N + t], t, gamma, b_fold + qd.fold_off, qd.ms);
   }
 }
@@ -985,105 +1007,88 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
 // the forward's stages log R .. logn-1 stay inside a part. The helpers below run a local
 // pass on the part of rank `rank` of a cluster of R CTAs (R = 2 or 4).
 
-// Inverse radix-4 pass (stages s, s+1) over this CTA's part xp (N/R words, local index);
-// threads below N/(4R) carry one unit each. Ends with a barrier.
-template <int LOGN, int R>
-__device__ __forceinline__ void inv_part_r4(u64* xp, int s, int rank, const u64* tw, const u64* twp) {
-  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4;
+// Inverse stages S .. logn-1-log R over this CTA's part xp (N/R words, local index), words up to 2+:
+// radix-4 passes, one unit per thread below N/(4R), then a radix-2 stage when the count is odd
+// (its sums up to 4+). Each pass ends with a barrier.
+template <int LOGN, int R, int S>
+__device__ __forceinline__ void inv_part(u64* xp, int rank, const Tw* tw) {
+  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4, LR = R == 4 ? 2 : 1;
   const int tid = threadIdx.x;
-  if (tid < PU) {
-    const int u = rank * PU + tid;
-    const int t = 1 << s, m = N >> (s + 1);
-    const int B = u >> s, o = u & (t - 1);
-    const int e0 = B * 4 * t + o - rank * P;
-    u64 w0, w0p, w1, w1p, w2, w2p;
-    inv_twiddle(tw, twp, m + 2 * B, w0, w0p);
-    inv_twiddle(tw, twp, m + 2 * B + 1, w1, w1p);
-    inv_twiddle(tw, twp, (m >> 1) + B, w2, w2p);
-    u64 a0 = xp[sw(e0)], a1 = xp[sw(e0 + t)], a2 = xp[sw(e0 + 2 * t)], a3 = xp[sw(e0 + 3 * t)];
-    bf_inv4(a0, a1, w0, w0p);
-    bf_inv4(a2, a3, w1, w1p);
-    bf_inv4(a0, a2, w2, w2p);
-    bf_inv4(a1, a3, w2, w2p);
-    xp[sw(e0)] = a0;
-    xp[sw(e0 + t)] = a1;
-    xp[sw(e0 + 2 * t)] = a2;
-    xp[sw(e0 + 3 * t)] = a3;
-  }
-  __syncthreads();
-}
-
-// Inverse radix-2 stage s over this CTA's part (the last local stage when their count is
-// odd); one butterfly per thread below N/(2R). Ends with a barrier.
-template <int LOGN, int R>
-__device__ __forceinline__ void inv_part_r2(u64* xp, int s, int rank, const u64* tw, const u64* twp) {
-  constexpr int N = 1 << LOGN, P = N / R;
-  if ((int)threadIdx.x < P / 2) {
-    const int v = rank * (P / 2) + (int)threadIdx.x;
-    const int t = 1 << s, m = N >> (s + 1);
-    const int B = v >> s, o = v & (t - 1);
-    const int e = B * 2 * t + o - rank * P;
-    u64 w, wp;
-    inv_twiddle(tw, twp, m + B, w, wp);
-    u64 a = xp[sw(e)], b = xp[sw(e + t)];
-    bf_inv4(a, b, w, wp);
-    xp[sw(e)] = a;
-    xp[sw(e + t)] = b;
-  }
-  __syncthreads();
-}
-
-// Forward radix-4 pass (stages s, s+1; s >= log R) over this CTA's part of two buffers
-// D[0..P) and D[P..2P), P = N/R; one unit per thread below N/(2R). Ends with a barrier.
-template <int LOGN, int R>
-__device__ __forceinline__ void fwd_part_r4(u64* D, int s, int rank, const u64* tw, const u64* twp) {
-  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4;
-  const int tid = threadIdx.x;
-  if (tid < 2 * PU) {
-    u64* x = D + (tid >= PU ? P : 0);
-    const int u = rank * PU + (tid & (PU - 1));
-    const int lt = LOGN - s - 1;  // log2 t
-    const int t = 1 << lt, m = 1 << s, h = t >> 1;
-    const int i = u >> (lt - 1), o = u & (h - 1);
-    const int e0 = i * 2 * t + o - rank * P;
-    const u64 wa = tw[m + i], wap = twp[m + i];
-    const u64 wb = tw[2 * m + 2 * i], wbp = twp[2 * m + 2 * i];
-    const u64 wc = tw[2 * m + 2 * i + 1], wcp = twp[2 * m + 2 * i + 1];
-    u64 a0 = x[sw(e0)], a1 = x[sw(e0 + h)], a2 = x[sw(e0 + t)], a3 = x[sw(e0 + t + h)];
-    bf_fwd8(a0, a2, wa, wap);
-    bf_fwd8(a1, a3, wa, wap);
-    bf_fwd8(a0, a1, wb, wbp);
-    bf_fwd8(a2, a3, wc, wcp);
-    x[sw(e0)] = a0;
-    x[sw(e0 + h)] = a1;
-    x[sw(e0 + t)] = a2;
-    x[sw(e0 + t + h)] = a3;
-  }
-  __syncthreads();
-}
-
-// Forward radix-2 stage s over this CTA's part of both buffers (when the local stages are
-// odd in number); one butterfly per buffer per thread below N/(2R). Ends with a barrier.
-template <int LOGN, int R>
-__device__ __forceinline__ void fwd_part_r2(u64* D, int s, int rank, const u64* tw, const u64* twp) {
-  constexpr int N = 1 << LOGN, P = N / R;
-  if ((int)threadIdx.x < P / 2) {
-    const int v = rank * (P / 2) + (int)threadIdx.x;
-    const int lt = LOGN - s - 1;
-    const int t = 1 << lt, m = 1 << s;
-    const int i = v >> lt, o = v & (t - 1);
-    const int e = i * 2 * t + o - rank * P;
-    const u64 w = tw[m + i], wp = twp[m + i];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      u64* x = D + k * P;
-      u64 a = x[sw(e)], b = x[sw(e + t)];
-      bf_fwd8(a, b, w, wp);
-      x[sw(e)] = a;
-      x[sw(e + t)] = b;
+  if constexpr (S + 1 <= LOGN - 1 - LR) {
+    constexpr int t = 1 << S, m = N >> (S + 1);
+    if (tid < PU) {
+      const int u = rank * PU + tid;
+      const int B = u >> S, o = u & (t - 1);
+      const int e0 = B * 4 * t + o - rank * P;
+      const int i0 = sw(e0), i1 = sw(e0 + t), i2 = sw(e0 + 2 * t), i3 = sw(e0 + 3 * t);
+      u64 a0 = xp[i0], a1 = xp[i1], a2 = xp[i2], a3 = xp[i3];
+      inv_unit(a0, a1, a2, a3, tw[2 * m - 1 - 2 * B], tw[2 * m - 2 - 2 * B], tw[m - 1 - B]);
+      xp[i0] = a0;
+      xp[i1] = a1;
+      xp[i2] = a2;
+      xp[i3] = a3;
     }
+    __syncthreads();
+    inv_part<LOGN, R, S + 2>(xp, rank, tw);
+  } else if constexpr (S == LOGN - 1 - LR) {
+    constexpr int t = 1 << S, m = N >> (S + 1);
+    for (int v0 = tid; v0 < P / 2; v0 += blockDim.x) {
+      const int v = rank * (P / 2) + v0;
+      const int B = v >> S, o = v & (t - 1);
+      const int e = sw(B * 2 * t + o - rank * P), f = sw(B * 2 * t + o - rank * P + t);
+      u64 a = xp[e], b = xp[f];
+      bf_inv<3>(a, b, tw[2 * m - 1 - B]);
+      xp[e] = a;
+      xp[f] = b;
+    }
+    __syncthreads();
   }
-  __syncthreads();
+}
+
+// Forward stages S .. END-1 (S >= log R) over this CTA's part of two buffers D[0..P) and D[P..2P),
+// P = N/R, words up to BIN in and fwd_bound out: a radix-2 stage first when the count is odd, then
+// radix-4 passes, one unit per thread below N/(2R). Each pass ends with a barrier.
+template <int LOGN, int R, int S, int END, int BIN>
+__device__ __forceinline__ void fwd_part(u64* D, int rank, const Tw* tw) {
+  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4;
+  const int tid = threadIdx.x;
+  if constexpr (S < END && ((END - S) & 1)) {
+    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S;
+    for (int v0 = tid; v0 < P / 2; v0 += blockDim.x) {
+      const int v = rank * (P / 2) + v0;
+      const int i = v >> lt, o = v & (t - 1);
+      const int e = sw(i * 2 * t + o - rank * P), f = sw(i * 2 * t + o - rank * P + t);
+      const Tw w = tw[m + i];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        u64* x = D + k * P;
+        u64 a = x[e], b = x[f];
+        bf_fwd(a, b, w);
+        x[e] = a;
+        x[f] = b;
+      }
+    }
+    __syncthreads();
+    fwd_part<LOGN, R, S + 1, END, BIN + 3>(D, rank, tw);
+  } else if constexpr (S < END) {
+    constexpr bool RED = BIN > FWD_FREE;
+    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S, h = t >> 1;
+    if (tid < 2 * PU) {
+      u64* x = D + (tid >= PU ? P : 0);
+      const int u = rank * PU + (tid & (PU - 1));
+      const int i = u >> (lt - 1), o = u & (h - 1);
+      const int e0 = i * 2 * t + o - rank * P;
+      const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + t), i3 = sw(e0 + t + h);
+      u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
+      fwd_unit<RED>(a0, a1, a2, a3, tw[m + i], tw[2 * m + 2 * i], tw[2 * m + 2 * i + 1]);
+      x[i0] = a0;
+      x[i1] = a1;
+      x[i2] = a2;
+      x[i3] = a3;
+    }
+    __syncthreads();
+    fwd_part<LOGN, R, S + 2, END, (RED ? 1 : BIN) + 6>(D, rank, tw);
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -1108,16 +1113,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
   namespace cg = cooperative_groups;
   constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2, HU = N / 8;
   constexpr u32 M2N = 2 * N - 1;
-  constexpr u64 DMASK = (1ULL << 20) - 1;
   extern __shared__ __align__(16) u64 sm[];
   u64* X = sm;      // [2][H] own half of the inverse, by link parity
   u64* D = sm + N;  // [2][H] own half of the transformed digits 0 and 1; N words at the end
   u64* a_ntt = D + N;
-  u64* tw = a_ntt + N;
-  u64* twp = tw + N;
-  u64* Wm = twp + N;  // room for three key rows, as in k_respond
-  u64* Y = Wm + 3 * N;
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(Y + 3 * N);
+  Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
+  ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
+  const KeyRows K{rows, rows + N, rows + 2 * N};
+  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
   uint16_t* s_tab = e_tab + N;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -1135,13 +1138,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
   const int ls = 4 * u + 2 * dg;  // local slots ls, ls + 1
   const int ug = rank * HU + u;   // global unit index of slots 4u..4u+3
 
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, twp, Wm, Y, e_tab, s_tab);
+  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
   expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  {
-    u64* const bufs[1] = {a_ntt};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
-  }
-  u64 cur[2], sb[2];
+  transform_a<LOGN, NT>(c, a_ntt, tw);
+  u64 cur[2];
+  Acc sb[2];
   u32 et[2];
 #pragma unroll
   for (int k = 0; k < 2; k++) et[k] = e_tab[own + ls + k];
@@ -1151,20 +1152,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = mont(a_ntt[tb], Srow[own + ls + k]);
-      sb[k] = 0;
+      cur[k] = mulq(a_ntt[tb], Srow[own + ls + k]);
+      sb[k] = Acc{0, 0, 0, 0};
     }
   }
   // Twiddles of the register passes: inverse stages 0-1 of unit ug, forward stages
   // logn-2, logn-1 of unit ug (fixed per thread).
-  u64 wl1, wl1p, wl2, wl2p;
-  inv_twiddle(tw, twp, H + 2 * ug + dg, wl1, wl1p);
-  inv_twiddle(tw, twp, H / 2 + ug, wl2, wl2p);
+  const Tw wl1 = tw[N - 1 - (2 * ug + dg)], wl2 = tw[H - 1 - ug];
   constexpr int MF = 1 << (LOGN - 2);
-  const u64 fa = tw[MF + ug], fap = twp[MF + ug];
-  const u64 fb = tw[2 * MF + 2 * ug], fbp = twp[2 * MF + 2 * ug];
-  const u64 fc = tw[2 * MF + 2 * ug + 1], fcp = twp[2 * MF + 2 * ug + 1];
-  const u64 wf = tw[1], wfp = twp[1];
+  const Tw fa = tw[MF + ug], fb = tw[2 * MF + 2 * ug], fc = tw[2 * MF + 2 * ug + 1];
+  const Tw wf = tw[1];
 #pragma unroll 1
   for (int i = (int)gamma - 2; i >= 0; i--) {
     const u64* Srow = sh.sums_R + (size_t)i * N;
@@ -1175,18 +1172,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
     {
       // Inverse stages 0-1 of unit ug: lane dg holds slots 4u + 2dg, +1.
       u64 p = cur[0], q = cur[1];
-      bf_inv4(p, q, wl1, wl1p);
+      bf_inv<3>(p, q, wl1);
       const u64 recv = __shfl_xor_sync(0xffffffffu, dg == 0 ? q : p, 1);
       u64 x0 = dg == 0 ? p : recv, x1 = dg == 0 ? recv : q;  // (slot 4u, 4u+2) or (4u+1, 4u+3)
-      bf_inv4(x0, x1, wl2, wl2p);
-      xh[sw(4 * u + dg)] = x0;
+      bf_inv<3>(x0, x1, wl2);
+      xh[sw(4 * u + dg)] = red60(x0);
       xh[sw(4 * u + dg + 2)] = x1;
     }
     __syncthreads();
-    int s = 2;
-#pragma unroll 1
-    for (; s + 1 <= LOGN - 2; s += 2) inv_part_r4<LOGN, 2>(xh, s, rank, tw, twp);
-    if (s == LOGN - 2) inv_part_r2<LOGN, 2>(xh, s, rank, tw, twp);
+    inv_part<LOGN, 2, 2>(xh, rank, tw);
     cluster.sync();
     {
       // Elements [0, H) of the inverse live in rank 0's X, elements [H, N) in rank 1's.
@@ -1196,36 +1190,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
       for (int j = 0; j < 2; j++) {
         const int b = tid + j * NT;
         const u64 x0 = lo[sw(b)], x1 = hi[sw(b)];
-        // The inverse's last stage and n^-1 as one product per output: n^-1 on the sum,
-        // n^-1 times the stage's twiddle on the difference.
-        const u64 r0 = shoup(x0 + x1, c.ninv, c.ninvp), r1 = shoup(x0 - x1 + 4 * Q, c.nlast, c.nlastp);
-        u64 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + H
-        if (exact) {
-          p0 = r0 & DMASK;
-          p1 = (r0 >> 20) & DMASK;
-          q0 = r1 & DMASK;
-          q1 = (r1 >> 20) & DMASK;
-        } else {
-          const u64 rr0 = (r0 + (1ULL << 19)) >> 20, rr1 = (r1 + (1ULL << 19)) >> 20;
-          p0 = rr0 & DMASK;
-          p1 = rr0 >> 20;
-          q0 = rr1 & DMASK;
-          q1 = rr1 >> 20;
-        }
+        u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + H
+        split_digits(canon(x0 + x1), exact, p0, p1);
+        split_digits(canon(mulw(x1 - x0 + 5 * Q, wf)), exact, q0, q1);
         // Forward cross stage: slot b gets p + w q, slot b + H gets p - w q.
-        const u64 t0 = shoup_digit((u32)q0, wf, wfp), t1 = shoup_digit((u32)q1, wf, wfp);
-        D[sw(b)] = rank == 0 ? p0 + t0 : p0 + 4 * Q - t0;
-        D[H + sw(b)] = rank == 0 ? p1 + t1 : p1 + 4 * Q - t1;
+        const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
+        D[sw(b)] = rank == 0 ? p0 + t0 : p0 + 3 * Q - t0;
+        D[H + sw(b)] = rank == 0 ? p1 + t1 : p1 + 3 * Q - t1;
       }
     }
     __syncthreads();
-    s = 1;
-    if (!(LOGN & 1)) {
-      fwd_part_r2<LOGN, 2>(D, 1, rank, tw, twp);
-      s = 2;
-    }
-#pragma unroll 1
-    for (; s < LOGN - 2; s += 2) fwd_part_r4<LOGN, 2>(D, s, rank, tw, twp);
+    fwd_part<LOGN, 2, 1, LOGN - 2, 3>(D, rank, tw);
     // Forward stages logn-2, logn-1 of unit ug for digit dg, then each lane takes the other
     // digit at its own two slots from its partner.
     u64 d0[2], d1[2];
@@ -1234,10 +1209,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
       const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(x + sw(4 * u));
       const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(x + sw(4 * u + 2));
       u64 a0 = v01.x, a1 = v01.y, a2 = v23.x, a3 = v23.y;
-      bf_fwd8(a0, a2, fa, fap);
-      bf_fwd8(a1, a3, fa, fap);
-      bf_fwd8(a0, a1, fb, fbp);
-      bf_fwd8(a2, a3, fc, fcp);
+      fwd_unit<(fwd_bound(LOGN, 1, 3) > FWD_FREE)>(a0, a1, a2, a3, fa, fb, fc);
       const u64 g0 = __shfl_xor_sync(0xffffffffu, dg == 0 ? a2 : a0, 1);
       const u64 g1 = __shfl_xor_sync(0xffffffffu, dg == 0 ? a3 : a1, 1);
       const u64 m0 = dg == 0 ? a0 : a2, m1 = dg == 0 ? a1 : a3;
@@ -1249,14 +1221,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      u128 nb = wide(d0[k], Y[tb]) + wide(d1[k], Y[N + tb]);
-      u128 nc = wide(a_ntt[tb], k == 0 ? sv.x : sv.y) + wide(d0[k], Wm[tb]) + wide(d1[k], Wm[N + tb]);
-      if (exact) {  // the rows are folded: R_{i+1} stands in for digit 2
-        nb += wide(cur[k], Y[2 * N + tb]);
-        nc += wide(cur[k], Wm[2 * N + tb]);
-      }
-      sb[k] = addq(sb[k], redc_wide(nb));
-      cur[k] = redc_wide(nc);
+      cur[k] = link_slot(sb[k], d0[k], d1[k], cur[k], k == 0 ? sv.x : sv.y, a_ntt, K, tb, exact);
+    }
+    if (i % SB_FOLD_LINKS == 0) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) sb[k] = acc_from(acc_fold(sb[k]));
     }
   }
   // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each
@@ -1267,8 +1236,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
   const u64* pf = peerX + H;
 #pragma unroll
   for (int k = 0; k < 2; k++) {
-    xf[ls + k] = rank == 0 ? sb[k] : cur[k];
-    D[own + ls + k] = rank == 0 ? cur[k] : sb[k];
+    const u64 sum = acc_fold(sb[k]);
+    xf[ls + k] = rank == 0 ? sum : cur[k];
+    D[own + ls + k] = rank == 0 ? cur[k] : sum;
   }
   cluster.sync();
 #pragma unroll
@@ -1276,13 +1246,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
   cluster.sync();  // each CTA's X stays alive until its peer has read it
   {
     u64* const bufs[1] = {D};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int t = tid + k * NT;
     if (rank == 0)
-      a_out[(size_t)qi * N + t] = finish_a(c, D[t], qd.ms);
+      a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
     else
       b_out[(size_t)qi * N + t] = finish_b(c, D[t], t, gamma, b_fold + qd.fold_off, qd.ms);
   }
@@ -1313,16 +1283,14 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
   namespace cg = cooperative_groups;
   constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4, SPT = P / NT;  // two slots a thread
   constexpr u32 M2N = 2 * N - 1;
-  constexpr u64 DMASK = (1ULL << 20) - 1;
   extern __shared__ __align__(16) u64 sm[];
   u64* X = sm;          // [2][P] own quarter of the inverse, by link parity
   u64* D = sm + 2 * P;  // [2][P] own quarter of digits 0 and 1; N words for the last transform
   u64* a_ntt = D + N;
-  u64* tw = a_ntt + N;
-  u64* twp = tw + N;
-  u64* Wm = twp + N;  // room for three key rows, as in k_respond
-  u64* Y = Wm + 3 * N;
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(Y + 3 * N);
+  Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
+  ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
+  const KeyRows K{rows, rows + N, rows + 2 * N};
+  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
   uint16_t* s_tab = e_tab + N;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -1339,30 +1307,25 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
   const bool exact = ps.approx == 0;
   // This thread's slots: rank P + tid + j NT, j < SPT.
 
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, twp, Wm, Y, e_tab, s_tab);
+  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
   expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  {
-    u64* const bufs[1] = {a_ntt};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
-  }
+  transform_a<LOGN, NT>(c, a_ntt, tw);
   u32 et[SPT];
-  u64 cur[SPT], sb[SPT];
+  u64 cur[SPT];
+  Acc sb[SPT];
 #pragma unroll
   for (int j = 0; j < SPT; j++) {
     const int slot = rank * P + tid + j * NT;
     et[j] = e_tab[slot];
     const u32 gp = ps.gpow[gamma - 1];
     const u32 tb = s_tab[((gp * et[j]) & M2N) >> 1];
-    cur[j] = mont(a_ntt[tb], sh.sums_R[(size_t)(gamma - 1) * N + slot]);
-    sb[j] = 0;
+    cur[j] = mulq(a_ntt[tb], sh.sums_R[(size_t)(gamma - 1) * N + slot]);
+    sb[j] = Acc{0, 0, 0, 0};
   }
-  // Twiddles of the cross pass: the inverse's stage logn-2 (indices 2 and 3), the forward's
-  // stage 0 (index 1) and stage 1 (index 2 for the first half, 3 for the second).
-  u64 wi2, wi2p, wi3, wi3p;
-  inv_twiddle(tw, twp, 2, wi2, wi2p);
-  inv_twiddle(tw, twp, 3, wi3, wi3p);
-  const u64 wf1 = tw[1], wf1p = twp[1];
-  const u64 wfs = tw[2 + (rank >> 1)], wfsp = twp[2 + (rank >> 1)];
+  // Twiddles of the cross pass: stage logn-2 of the inverse takes the mirrored entries 3 and 2, its
+  // last stage and stage 0 of the forward entry 1, stage 1 entry 2 for the first half, 3 for the second.
+  const Tw w1 = tw[1], w2 = tw[2], w3 = tw[3];
+  const Tw wfs = tw[2 + (rank >> 1)];
 #pragma unroll 1
   for (int i = (int)gamma - 2; i >= 0; i--) {
     u64 sv[SPT];
@@ -1374,73 +1337,54 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
 #pragma unroll
     for (int j = 0; j < SPT; j++) xq[sw(tid + j * NT)] = cur[j];
     __syncthreads();
-    int s = 0;
-#pragma unroll 1
-    for (; s + 1 <= LOGN - 3; s += 2) inv_part_r4<LOGN, 4>(xq, s, rank, tw, twp);
-    if (s == LOGN - 3) inv_part_r2<LOGN, 4>(xq, s, rank, tw, twp);
+    inv_part<LOGN, 4, 0>(xq, rank, tw);
     cluster.sync();
 #pragma unroll
     for (int j = 0; j < SPT; j++) {
       const int b = tid + j * NT;
       u64 x0 = peer[0][par + sw(b)], x1 = peer[1][par + sw(b)];
       u64 x2 = peer[2][par + sw(b)], x3 = peer[3][par + sw(b)];
-      bf_inv4(x0, x1, wi2, wi2p);  // (b, b + N/4), block 0 of stage logn-2
-      bf_inv4(x2, x3, wi3, wi3p);  // (b + N/2, b + 3N/4), block 1
-      u64 cf[4];                   // coefficients b, b + N/4, b + N/2, b + 3N/4
-      cf[0] = shoup(x0 + x2, c.ninv, c.ninvp);
-      cf[2] = shoup(x0 - x2 + 4 * Q, c.nlast, c.nlastp);
-      cf[1] = shoup(x1 + x3, c.ninv, c.ninvp);
-      cf[3] = shoup(x1 - x3 + 4 * Q, c.nlast, c.nlastp);
-      u64 g0[4], g1[4];  // digits 0 and 1
+      bf_inv<5>(x0, x1, w3);  // (b, b + N/4), block 0 of stage logn-2: sums up to 8+
+      bf_inv<5>(x2, x3, w2);  // (b + N/2, b + 3N/4), block 1
+      x0 = red60(x0);
+      x2 = red60(x2);
+      u64 cf[4];  // coefficients b, b + N/4, b + N/2, b + 3N/4
+      cf[0] = canon(x0 + x2);
+      cf[2] = canon(mulw(x2 - x0 + 3 * Q, w1));
+      cf[1] = canon(x1 + x3);
+      cf[3] = canon(mulw(x3 - x1 + 3 * Q, w1));
+      u32 g0[4], g1[4];  // digits 0 and 1
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        if (exact) {
-          g0[k] = cf[k] & DMASK;
-          g1[k] = (cf[k] >> 20) & DMASK;
-        } else {
-          const u64 rr = (cf[k] + (1ULL << 19)) >> 20;
-          g0[k] = rr & DMASK;
-          g1[k] = rr >> 20;
-        }
-      }
+      for (int k = 0; k < 4; k++) split_digits(cf[k], exact, g0[k], g1[k]);
       // Forward stage 0 (b with b + N/2, b + N/4 with b + 3N/4), then stage 1 on this
-      // quarter's half: a bf_fwd8 whose output r & 1 is the quarter's word.
-      auto fwd = [&](const u64(&g)[4]) -> u64 {
-        const u64 t2 = shoup_digit((u32)g[2], wf1, wf1p), t3 = shoup_digit((u32)g[3], wf1, wf1p);
+      // quarter's half, of which output rank & 1 is the quarter's word, at most 6.
+      auto fwd = [&](const u32(&g)[4]) -> u64 {
+        const u64 t2 = mulw_digit(g[2], w1), t3 = mulw_digit(g[3], w1);
         u64 lo, hi;
         if (rank < 2) {
           lo = g[0] + t2;
           hi = g[1] + t3;
         } else {
-          lo = g[0] + 4 * Q - t2;
-          hi = g[1] + 4 * Q - t3;
+          lo = g[0] + 3 * Q - t2;
+          hi = g[1] + 3 * Q - t3;
         }
-        bf_fwd8(lo, hi, wfs, wfsp);
-        return (rank & 1) ? hi : lo;
+        const u64 t = mulw(hi, wfs);
+        return (rank & 1) ? lo - t + 3 * Q : lo + t;
       };
       D[sw(b)] = fwd(g0);
       D[P + sw(b)] = fwd(g1);
     }
     __syncthreads();
-    s = 2;
-    if ((LOGN - 2) & 1) {
-      fwd_part_r2<LOGN, 4>(D, 2, rank, tw, twp);
-      s = 3;
-    }
-#pragma unroll 1
-    for (; s < LOGN; s += 2) fwd_part_r4<LOGN, 4>(D, s, rank, tw, twp);
+    fwd_part<LOGN, 4, 2, LOGN, 6>(D, rank, tw);
 #pragma unroll
     for (int j = 0; j < SPT; j++) {
       const u64 d0 = D[sw(tid + j * NT)], d1 = D[P + sw(tid + j * NT)];
       const u32 tb = s_tab[((gp * et[j]) & M2N) >> 1];
-      u128 nb = wide(d0, Y[tb]) + wide(d1, Y[N + tb]);
-      u128 nc = wide(a_ntt[tb], sv[j]) + wide(d0, Wm[tb]) + wide(d1, Wm[N + tb]);
-      if (exact) {  // the rows are folded: R_{i+1} stands in for digit 2
-        nb += wide(cur[j], Y[2 * N + tb]);
-        nc += wide(cur[j], Wm[2 * N + tb]);
-      }
-      sb[j] = addq(sb[j], redc_wide(nb));
-      cur[j] = redc_wide(nc);
+      cur[j] = link_slot(sb[j], d0, d1, cur[j], sv[j], a_ntt, K, tb, exact);
+    }
+    if (i % SB_FOLD_LINKS == 0) {
+#pragma unroll
+      for (int j = 0; j < SPT; j++) sb[j] = acc_from(acc_fold(sb[j]));
     }
   }
   // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each from
@@ -1449,7 +1393,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
 #pragma unroll
   for (int j = 0; j < SPT; j++) {
     X[tid + j * NT] = cur[j];
-    X[P + tid + j * NT] = sb[j];
+    X[P + tid + j * NT] = acc_fold(sb[j]);
   }
   cluster.sync();
   if (rank < 2) {
@@ -1463,13 +1407,13 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
   __syncthreads();
   {
     u64* const bufs[1] = {D};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
   }
 #pragma unroll
   for (int k = 0; k < N / NT; k++) {
     const int t = tid + k * NT;
     if (rank == 0)
-      a_out[(size_t)qi * N + t] = finish_a(c, D[t], qd.ms);
+      a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
     else
       b_out[(size_t)qi * N + t] = finish_b(c, D[t], t, gamma, b_fold + qd.fold_off, qd.ms);
   }
@@ -1484,30 +1428,28 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
 //                as ciphertext 1 + j of the query;
 //   nopack_sum:  ciphertext 0 = the sum of the column ciphertexts mod q.
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 4) k_nopack_prep(CrsDev c, const QueryDev* queries, u64 r_mod_q,
-                                                                 u64 r_mod_qp, u64* AB_R, u32* status) {
+__global__ void __launch_bounds__((1 << LOGN) / 4) k_nopack_prep(CrsDev c, const QueryDev* queries, Tw r_mod_q,
+                                                                 u64* AB_R, u32* status) {
   constexpr int N = 1 << LOGN, NT = N / 4;
   extern __shared__ __align__(16) u64 sm[];
   u64* xa = sm;
   u64* xb = sm + N;
-  u64* tw = sm + 2 * N;
-  u64* twp = sm + 3 * N;
+  Tw* tw = reinterpret_cast<Tw*>(sm + 2 * N);
   const u32 qi = blockIdx.x;
   const QueryDev qd = queries[qi];
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
     xb[k] = reduce128(qd.b[k]);
   }
   expand_a<N, NT>(qd, xa, status, qi, 0);  // ends with a barrier
   {
     u64* const bufs[2] = {xa, xb};
-    ntt_fwd_r4<LOGN, NT, 2>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 2>(bufs, tw);
   }
   u64* o = AB_R + (size_t)qi * 2 * N;
   for (int k = threadIdx.x; k < N; k += NT) {
-    o[k] = shoup(xa[k], r_mod_q, r_mod_qp);
-    o[N + k] = shoup(xb[k], r_mod_q, r_mod_qp);
+    o[k] = canon(mulw(xa[k], r_mod_q));
+    o[N + k] = canon(mulw(xb[k], r_mod_q));
   }
 }
 
@@ -1519,36 +1461,34 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_nopack_cols(CrsDev c, const
   u64* x = sm;
   u64* ya = sm + N;
   u64* yb = sm + 2 * N;
-  u64* tw = sm + 3 * N;
-  u64* twp = sm + 4 * N;
+  Tw* tw = reinterpret_cast<Tw*>(sm + 3 * N);
   const u32 j = blockIdx.x, qi = blockIdx.y;
   const QueryDev qd = queries[qi];
   const u64* col = shards[qd.shard].columns + (size_t)j * N;
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
     x[k] = reduce128(col[k]);
   }
   __syncthreads();
   {
     u64* const bufs[1] = {x};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
   const u64* A = AB_R + (size_t)qi * 2 * N;
   for (int k = threadIdx.x; k < N; k += NT) {
-    const u64 h = csub(csub2(x[k]));
+    const u64 h = canon(x[k]);
     ya[k] = mont(A[k], h);
     yb[k] = mont(A[N + k], h);
   }
   __syncthreads();
   {
     u64* const bufs[2] = {ya, yb};
-    ntt_inv_r4<LOGN, NT, 2>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 2>(bufs, tw);
   }
   u64* o = out + ((size_t)qi * (c.gamma + 1) + 1 + j) * 2 * N;
   for (int k = threadIdx.x; k < N; k += NT) {
-    o[k] = shoup(ya[k], c.ninv, c.ninvp);
-    o[N + k] = shoup(yb[k], c.ninv, c.ninvp);
+    o[k] = canon(mulw(ya[k], c.ninv));
+    o[N + k] = canon(mulw(yb[k], c.ninv));
   }
 }
 
@@ -1583,15 +1523,13 @@ __global__ void k_nopack_sum(u32 n, u32 gamma, u64* out) {
 // waiting nodes sit in a per-query stack of log n node slots in global memory.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
-    k_tree(CrsDev c, const QueryDev* queries, const ShardDev* shards, u64 r_mod_q, u64 r_mod_qp, u64 ms_target,
-           u64* stack, u64* a_out, u64* b_out, u32* status) {
+    k_tree(CrsDev c, const QueryDev* queries, const ShardDev* shards, u64 ms_target, u64* stack, u64* a_out, u64* b_out,
+           u32* status) {
   constexpr int N = 1 << LOGN, NT = N / 4;
   constexpr u32 M2N = 2 * N - 1;
-  constexpr u64 DMASK = (1ULL << 20) - 1;
   extern __shared__ __align__(16) u64 sm[];
-  u64* tw = sm;
-  u64* twp = tw + N;
-  u64* aR = twp + N;     // NTT(a) in R-form
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* aR = sm + 2 * N;  // n^-1 NTT(a)
   u64* S1a = aR + N;     // E - y O, permuted by the automorphism
   u64* S1b = S1a + N;
   u64* X = S1b + N;      // the inverse in progress, then a leaf column
@@ -1609,23 +1547,20 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
 
   for (int k = tid; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
     e_tab[k] = c.slot_exp[k];
     s_tab[k] = c.exp_slot[k];
   }
   expand_a<N, NT>(qd, aR, status, qi, 0);  // ends with a barrier
   {
     u64* const bufs[1] = {aR};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
-  for (int k = tid; k < N; k += NT) aR[k] = shoup(aR[k], r_mod_q, r_mod_qp);
+  for (int k = tid; k < N; k += NT) aR[k] = canon(mulw(aR[k], c.ninv));
   __syncthreads();
 
   const int l0 = 4 * tid;
   u64 ca[4], cb[4];  // the current node at slots l0..l0+3 (thread tid's transform unit)
   bool cur_zero = true;
-  const u64 wf = tw[1], wfp = twp[1];
-  constexpr int H = N / 2, MF = 1 << (LOGN - 2);
   // Leaf `start`: the column through the transform times NTT(a); its b-value on the side.
   auto leaf = [&](u32 start) {
     u128 acc = 0;
@@ -1649,24 +1584,22 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
     }
     {
       u64* const bufs[1] = {X};
-      ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);  // ends with a barrier
+      ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);  // ends with a barrier
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      ca[j] = mont(csub(csub2(X[l0 + j])), aR[l0 + j]);
+      ca[j] = csub(mulq(X[l0 + j], aR[l0 + j]));
       cb[j] = 0;
     }
     __syncthreads();  // X is rewritten next
   };
   // The current node becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell, E from the
-  // stack slot ell - 1; the current node is O (zero when odd_zero). The transforms follow
-  // k_respond's link: the inverse's first two stages in registers, its last stage fused with
-  // n^-1, the digit split and the forward's first stage, the forward's last two stages in
-  // registers, X and D under the sw() layout.
+  // stack slot ell - 1; the current node is O (zero when odd_zero). Nodes are held scaled by n^-1,
+  // as k_respond's links hold R, and the key switch runs the same transforms.
   auto combine = [&](int ell, bool odd_zero) {
     const u64* E = stk + (size_t)(ell - 1) * 2 * N + l0;
     const u32 sy = (u32)(N >> ell), t = (1u << ell) + 1;
-    const u64* key = c.galois_R + (size_t)(LOGN - ell) * 6 * N + l0;
+    const u64* key = c.galois + (size_t)(LOGN - ell) * 6 * N + l0;
     u64 s0a[4], s0b[4], aa[4], ab[4];
     {
       const ulonglong2 e01 = *reinterpret_cast<const ulonglong2*>(E);
@@ -1700,156 +1633,20 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
       aa[j] = S1a[src];
       ab[j] = S1b[src];
     }
-    {
-      // Inverse stages 0-1 of unit tid (block B = tid, m = N/2).
-      u64 w0, w0p, w1, w1p, w2, w2p;
-      inv_twiddle(tw, twp, H + 2 * tid, w0, w0p);
-      inv_twiddle(tw, twp, H + 2 * tid + 1, w1, w1p);
-      inv_twiddle(tw, twp, H / 2 + tid, w2, w2p);
-      u64 a0 = aa[0], a1 = aa[1], a2 = aa[2], a3 = aa[3];
-      bf_inv4(a0, a1, w0, w0p);
-      bf_inv4(a2, a3, w1, w1p);
-      bf_inv4(a0, a2, w2, w2p);
-      bf_inv4(a1, a3, w2, w2p);
-      *reinterpret_cast<ulonglong2*>(X + sw(l0)) = make_ulonglong2(a0, a1);
-      *reinterpret_cast<ulonglong2*>(X + sw(l0 + 2)) = make_ulonglong2(a2, a3);
-    }
-    __syncthreads();
-    // Inverse stages 2 .. logn-2 (radix-4 pairs, a radix-2 stage last when logn is even).
-    int s = 2;
-#pragma unroll 1
-    for (; s + 1 <= LOGN - 2; s += 2) {
-      const int tt = 1 << s, m = N >> (s + 1);
-      const int B = tid >> s, o = tid & (tt - 1);
-      const int e0 = B * 4 * tt + o;
-      u64 w0, w0p, w1, w1p, w2, w2p;
-      inv_twiddle(tw, twp, m + 2 * B, w0, w0p);
-      inv_twiddle(tw, twp, m + 2 * B + 1, w1, w1p);
-      inv_twiddle(tw, twp, (m >> 1) + B, w2, w2p);
-      u64 a0 = X[sw(e0)], a1 = X[sw(e0 + tt)], a2 = X[sw(e0 + 2 * tt)], a3 = X[sw(e0 + 3 * tt)];
-      bf_inv4(a0, a1, w0, w0p);
-      bf_inv4(a2, a3, w1, w1p);
-      bf_inv4(a0, a2, w2, w2p);
-      bf_inv4(a1, a3, w2, w2p);
-      X[sw(e0)] = a0;
-      X[sw(e0 + tt)] = a1;
-      X[sw(e0 + 2 * tt)] = a2;
-      X[sw(e0 + 3 * tt)] = a3;
-      __syncthreads();
-    }
-    if (s == LOGN - 2) {
-      const int tt = 1 << s, m = N >> (s + 1);
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int v = tid + r * NT;
-        const int B = v >> s, o = v & (tt - 1);
-        const int e = B * 2 * tt + o;
-        u64 w, wp;
-        inv_twiddle(tw, twp, m + B, w, wp);
-        u64 a = X[sw(e)], b = X[sw(e + tt)];
-        bf_inv4(a, b, w, wp);
-        X[sw(e)] = a;
-        X[sw(e + tt)] = b;
-      }
-      __syncthreads();
-    }
-    // Inverse stage logn-1, n^-1, digit split and forward stage 0, per pair (b, b + N/2).
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int b = tid + j * NT;
-      const u64 x0 = X[sw(b)], x1 = X[sw(b + H)];
-      // The inverse's last stage and n^-1 as one product per output: n^-1 on the sum,
-      // n^-1 times the stage's twiddle on the difference.
-      const u64 r0 = shoup(x0 + x1, c.ninv, c.ninvp), r1 = shoup(x0 - x1 + 4 * Q, c.nlast, c.nlastp);
-      const u64 p0 = r0 & DMASK, p1 = (r0 >> 20) & DMASK, q0 = r1 & DMASK, q1 = (r1 >> 20) & DMASK;
-      const u64 t0 = shoup_digit((u32)q0, wf, wfp), t1 = shoup_digit((u32)q1, wf, wfp);
-      D[sw(b)] = p0 + t0;
-      D[sw(b + H)] = p0 + 4 * Q - t0;
-      D[N + sw(b)] = p1 + t1;
-      D[N + sw(b + H)] = p1 + 4 * Q - t1;
-    }
-    __syncthreads();
-    // Forward stages 1 .. logn-3 (a radix-2 stage first when logn is even), both digits.
-    s = 1;
-    if (!(LOGN & 1)) {
-      const int lt = LOGN - 2, tt = 1 << lt;
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int v = tid + r * NT;
-        const int ib = v >> lt, o = v & (tt - 1);
-        const int e = ib * 2 * tt + o;
-        const u64 w = tw[2 + ib], wp = twp[2 + ib];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-          u64* x = D + k * N;
-          u64 a = x[sw(e)], b = x[sw(e + tt)];
-          bf_fwd8(a, b, w, wp);
-          x[sw(e)] = a;
-          x[sw(e + tt)] = b;
-        }
-      }
-      __syncthreads();
-      s = 2;
-    }
-#pragma unroll 1
-    for (; s < LOGN - 2; s += 2) {
-      const int tt = N >> (s + 1), m = 1 << s, h = tt >> 1;
-      const int ib = tid / h, o = tid - ib * h;
-      const int e0 = ib * 2 * tt + o;
-      const u64 wa = tw[m + ib], wap = twp[m + ib];
-      const u64 wb = tw[2 * m + 2 * ib], wbp = twp[2 * m + 2 * ib];
-      const u64 wc = tw[2 * m + 2 * ib + 1], wcp = twp[2 * m + 2 * ib + 1];
-      const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + tt), i3 = sw(e0 + tt + h);
-      u64* x0 = D;
-      u64* x1 = D + N;
-      u64 a0 = x0[i0], a1 = x0[i1], a2 = x0[i2], a3 = x0[i3];
-      u64 c0 = x1[i0], c1 = x1[i1], c2 = x1[i2], c3 = x1[i3];
-      bf_fwd8(a0, a2, wa, wap);
-      bf_fwd8(c0, c2, wa, wap);
-      bf_fwd8(a1, a3, wa, wap);
-      bf_fwd8(c1, c3, wa, wap);
-      bf_fwd8(a0, a1, wb, wbp);
-      bf_fwd8(c0, c1, wb, wbp);
-      bf_fwd8(a2, a3, wc, wcp);
-      bf_fwd8(c2, c3, wc, wcp);
-      x0[i0] = a0;
-      x0[i1] = a1;
-      x0[i2] = a2;
-      x0[i3] = a3;
-      x1[i0] = c0;
-      x1[i1] = c1;
-      x1[i2] = c2;
-      x1[i3] = c3;
-      __syncthreads();
-    }
-    // Forward stages logn-2, logn-1 of unit tid, both digits, in registers.
     u64 d0[4], d1[4];
-    {
-      const u64 fa = tw[MF + tid], fap = twp[MF + tid];
-      const u64 fb = tw[2 * MF + 2 * tid], fbp = twp[2 * MF + 2 * tid];
-      const u64 fc = tw[2 * MF + 2 * tid + 1], fcp = twp[2 * MF + 2 * tid + 1];
-      const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(D + sw(l0));
-      const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(D + sw(l0 + 2));
-      const ulonglong2 g01 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0));
-      const ulonglong2 g23 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0 + 2));
-      d0[0] = v01.x, d0[1] = v01.y, d0[2] = v23.x, d0[3] = v23.y;
-      d1[0] = g01.x, d1[1] = g01.y, d1[2] = g23.x, d1[3] = g23.y;
-      bf_fwd8(d0[0], d0[2], fa, fap);
-      bf_fwd8(d1[0], d1[2], fa, fap);
-      bf_fwd8(d0[1], d0[3], fa, fap);
-      bf_fwd8(d1[1], d1[3], fa, fap);
-      bf_fwd8(d0[0], d0[1], fb, fbp);
-      bf_fwd8(d1[0], d1[1], fb, fbp);
-      bf_fwd8(d0[2], d0[3], fc, fcp);
-      bf_fwd8(d1[2], d1[3], fc, fcp);
-    }
+    link_transforms<LOGN>(aa, d0, d1, X, D, tw, true);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      // The keys' digit rows are folded (fold_gadget3): aa stands in for digit 2.
-      const u64 na = redc_wide(wide(d0[j], key[j]) + wide(d1[j], key[2 * N + j]) + wide(aa[j], key[4 * N + j]));
-      const u64 nb = redc_wide(wide(d0[j], key[N + j]) + wide(d1[j], key[3 * N + j]) + wide(aa[j], key[5 * N + j]));
-      ca[j] = addq(s0a[j], na);
-      cb[j] = addq(s0b[j], addq(ab[j], nb));
+      // The keys' digit rows are folded (fold_gadget_keys): aa stands in for digit 2.
+      Acc na{0, 0, 0, 0}, nb{0, 0, 0, 0};
+      mac(na, d0[j], key[j]);
+      mac(nb, d0[j], key[N + j]);
+      mac(na, d1[j], key[2 * N + j]);
+      mac(nb, d1[j], key[3 * N + j]);
+      mac(na, aa[j], key[4 * N + j]);
+      mac(nb, aa[j], key[5 * N + j]);
+      ca[j] = addq(s0a[j], csub(acc_fold(na)));
+      cb[j] = addq(s0b[j], addq(ab[j], csub(acc_fold(nb))));
     }
     __syncthreads();  // S1, X and D are rewritten next
   };
@@ -1899,14 +1696,14 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
   __syncthreads();
   {
     u64* const bufs[2] = {X, D};
-    ntt_inv_r4<LOGN, NT, 2>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 2>(bufs, tw);
   }
   const u64 scale = gamma == 1 ? 1 : (u64)N;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int k = tid + j * NT;
-    u64 av = shoup(X[k], c.ninv, c.ninvp);
-    u64 bv = gamma == 1 ? (k == 0 ? bval[0] : 0) : shoup(D[k], c.ninv, c.ninvp);
+    u64 av = canon(X[k]);
+    u64 bv = gamma == 1 ? (k == 0 ? bval[0] : 0) : canon(D[k]);
     if (gamma > 1 && (u32)k < gamma) bv = addq(bv, reduce128(wide(bval[k], scale)));
     if (ms_target) {
       av = mod_switch_word(av, ms_target);
@@ -2072,31 +1869,29 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_client_query(CrsDev c, cons
                                                                   u32* status) {
   constexpr int N = 1 << LOGN, NT = N / 4;
   extern __shared__ __align__(16) u64 sm[];
-  u64* x = sm;
-  u64* tw = sm + N;
-  u64* twp = tw + N;
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* x = sm + 2 * N;
   const u32 qi = blockIdx.x;
   const QueryDev qd = queries[qi];
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
   }
   expand_a<N, NT>(qd, x, status, qi, 0);  // ends with a barrier
   {
     u64* const bufs[1] = {x};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
-  for (int k = threadIdx.x; k < N; k += NT) x[k] = mont(csub(csub2(x[k])), s_R[k]);
+  for (int k = threadIdx.x; k < N; k += NT) x[k] = mont(canon(x[k]), s_R[k]);
   __syncthreads();
   {
     u64* const bufs[1] = {x};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
   }
   const u32 local = locals[qi];
   const int pos = local == 0 ? 0 : N - (int)local;
   const u64 mono = local == 0 ? delta : Q - delta;  // Delta X^-local (encode_db.rs:43-70)
   for (int k = threadIdx.x; k < N; k += NT) {
-    const u64 as = shoup(x[k], c.ninv, c.ninvp);
+    const u64 as = canon(mulw(x[k], c.ninv));
     const i64 ev = samples[(size_t)qi * N + k];
     u64 b = addq(negq(as), ev < 0 ? Q - (u64)(-ev) : (u64)ev);
     if (k == pos) b = addq(b, mono);
@@ -2115,29 +1910,27 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_client_extract(CrsDev c, co
                                                                     u64 dinv, u32 entry_size, uint8_t* out) {
   constexpr int N = 1 << LOGN, NT = N / 4;
   extern __shared__ __align__(16) u64 sm[];
-  u64* x = sm;
-  u64* tw = sm + N;
-  u64* twp = tw + N;
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* x = sm + 2 * N;
   const u32 qi = blockIdx.x;
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-    twp[k] = c.twp[k];
     x[k] = a[(size_t)qi * N + k];
   }
   __syncthreads();
   {
     u64* const bufs[1] = {x};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
-  for (int k = threadIdx.x; k < N; k += NT) x[k] = mont(csub(csub2(x[k])), s_R[k]);
+  for (int k = threadIdx.x; k < N; k += NT) x[k] = mont(canon(x[k]), s_R[k]);
   __syncthreads();
   {
     u64* const bufs[1] = {x};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw, twp);
+    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
   }
   const u32 cols = (entry_size + 1) / 2;
   for (u32 k = threadIdx.x; k < cols && k < (u32)N; k += NT) {
-    u64 as = shoup(x[k], c.ninv, c.ninvp);
+    u64 as = canon(mulw(x[k], c.ninv));
     if (modulus != Q) {
       const bool neg = as > (Q >> 1);
       const u64 mag = (neg ? Q - as : as) % modulus;
@@ -2155,20 +1948,20 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_client_extract(CrsDev c, co
 }
 
 // ------------------------------------------------------------------------------------
-// Integer roofline probe: the recursion kernels' lazy forward butterflies (bf_fwd8: one
-// Shoup product, two 64-bit adds and a conditional subtraction each, the transforms' unit
-// of work) on values held in registers, eight independent chains per thread, no memory
-// traffic. Its rate is the ceiling the respond kernels' butterflies are measured against.
-__global__ void __launch_bounds__(256) k_butterfly_peak(u64* out, int iters, u64 w, u64 wp) {
+// Integer roofline probe: the recursion kernels' lazy forward butterflies (bf_fwd: one product by
+// a twiddle and two 64-bit sums, the transforms' unit of work) on values held in registers, eight
+// per thread, no memory traffic. Its rate is the ceiling the respond kernels' butterflies are
+// measured against.
+__global__ void __launch_bounds__(256) k_butterfly_peak(u64* out, int iters, Tw w) {
   u64 x[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) x[k] = (u64)(blockIdx.x * 8191u + threadIdx.x * 131u + k) * 0x9E3779B97F4A7C15ULL % Q;
 #pragma unroll 1
   for (int it = 0; it < iters; it++) {
 #pragma unroll
-    for (int k = 0; k < 8; k += 2) bf_fwd8(x[k], x[k + 1], w, wp);
+    for (int k = 0; k < 8; k += 2) bf_fwd(x[k], x[k + 1], w);
 #pragma unroll
-    for (int k = 0; k < 4; k++) bf_fwd8(x[k], x[k + 4], w, wp);
+    for (int k = 0; k < 4; k++) bf_fwd(x[k], x[k + 4], w);
   }
   u64 acc = 0;
 #pragma unroll
@@ -2195,14 +1988,14 @@ cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t
   return cudaGetLastError();
 }
 
-cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, u64 scalep, cudaStream_t s) {
+cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, cudaStream_t s) {
   if (rows == 0) return cudaSuccess;
   const size_t smem = 3 * (size_t)c.n * 8;
   IG_DISPATCH_LOGN(c.logn, {
     auto k = k_ntt_rows<L>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<rows, (1 << L) / 4, smem, s>>>(c, in, out, scale, scalep);
+    k<<<rows, (1 << L) / 4, smem, s>>>(c, in, out, make_tw(scale));
   });
   return cudaGetLastError();
 }
@@ -2287,7 +2080,7 @@ cudaError_t nopack(const CrsDev& c, const QueryDev* queries, const ShardDev* sha
       const size_t smem = 4 * (size_t)N * 8;
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      k<<<nq, N / 4, smem, s>>>(c, queries, r_mod_q, shoup_companion(r_mod_q), AB_R, status);
+      k<<<nq, N / 4, smem, s>>>(c, queries, make_tw(r_mod_q), AB_R, status);
     }
     {
       auto k = k_nopack_cols<L>;
@@ -2347,24 +2140,23 @@ cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64
 
 size_t tree_smem_bytes(const CrsDev& c) { return ((size_t)8 * c.n + c.n / 2 + 32) * 8 + 2 * (size_t)c.n * 2; }
 
-cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 r_mod_q, u64 ms_target,
-                 u64* stack, u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
+cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 ms_target, u64* stack,
+                 u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
-  if (!c.galois_R || c.gamma > c.n / 2) return cudaErrorInvalidValue;
+  if (!c.galois || c.gamma > c.n / 2) return cudaErrorInvalidValue;
   const size_t smem = tree_smem_bytes(c);
   IG_DISPATCH_LOGN(c.logn, {
     auto k = k_tree<L>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<nq, (1 << L) / 4, smem, s>>>(c, queries, shards, r_mod_q, shoup_companion(r_mod_q), ms_target, stack, a_out,
-                                      b_out, status);
+    k<<<nq, (1 << L) / 4, smem, s>>>(c, queries, shards, ms_target, stack, a_out, b_out, status);
   });
   return cudaGetLastError();
 }
 
 cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s) {
   const u64 w = 0x0123456789ABCDEULL % Q;
-  k_butterfly_peak<<<blocks, 256, 0, s>>>(out, iters, w, shoup_companion(w));
+  k_butterfly_peak<<<blocks, 256, 0, s>>>(out, iters, make_tw(w));
   return cudaGetLastError();
 }
 

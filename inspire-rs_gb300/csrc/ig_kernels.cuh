@@ -17,9 +17,10 @@ enum DeviceStatus : u32 {
 // Per parameter-set constants, resident in device memory.
 struct CrsDev {
   u32 n, logn, gamma, rows, approx;
-  const u64 *tw, *twp;    // forward ladder psi^brv(m), Shoup companions (index m in [1, n))
-  u64 ninv, ninvp;        // n^-1 mod q, Shoup
-  u64 nlast, nlastp;      // n^-1 times the inverse's last twiddle (q - tw[1]), Shoup
+  const Tw* tw;           // forward ladder psi^brv(m), index m in [1, n)
+  // Scalars: n^-1; n^-1 2^-64, 2^-64 and n 2^-64, which take the recursion's R-form operands to
+  // the scaled standard form its links use (stage_constants).
+  Tw ninv, s_ninv_rinv, s_rinv, s_n_rinv;
   const uint16_t* slot_exp;  // odd exponent e_t of slot t's root relative to slot 0's
   const uint16_t* exp_slot;  // slot holding exponent e, indexed e/2
   const u32* gpow;           // g^i mod 2n, i < gamma
@@ -32,9 +33,9 @@ struct CrsDev {
   // base^-2, -base^-2 and -base^-1, by which the key rows are folded (fold_gadget3).
   u64 ld_inv_R, ld_c0_R, ld_c1_R;
   // Galois keys of the automorphism tree (OnePacking), null when the CRS carries none:
-  // key i (t = n / 2^i + 1) as 3 rows of (a, b), each n words, R-form NTT, folded at
-  // upload (fold_gadget_keys) so the node stands in for the third digit.
-  const u64* galois_R;
+  // key i (t = n / 2^i + 1) as 3 rows of (a, b), each n words, standard-form NTT, folded and
+  // scaled at upload (fold_gadget_keys) so the node stands in for the third digit.
+  const u64* galois;
 };
 
 // One query of a launch.
@@ -97,12 +98,12 @@ namespace igk {
 using namespace ig;
 
 // The Galois keys ([key][3 digits][2 parts][n], R-form NTT) folded in place for consumers
-// that take R in place of the derived third digit.
+// that take the node in place of the derived third digit, and brought to the standard form
+// and the scale of the tree's nodes (n^-1 times their values).
 cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t s);
-// Forward NTT of `rows` polynomials: out[r] = scale * NTT(in[r] mod q), scale given with
-// its Shoup companion (scale = 1 for standard form, 2^64 mod q for R-form).
-cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, u64 scalep,
-                     cudaStream_t s);
+// Forward NTT of `rows` polynomials: out[r] = scale * NTT(in[r] mod q), canonical (scale = 1 for
+// standard form, 2^64 mod q for R-form).
+cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, cudaStream_t s);
 
 // Shard scan over `nq` queries: for query q and column j < gamma_q,
 // b_fold[fold_off_q + j] = coeff0(b_q * column_j); a query on a stale shard gets
@@ -169,8 +170,8 @@ cudaError_t client_query(const CrsDev& c, const QueryDev* queries, u32 nq, const
                          const i64* samples, u64 delta, u64* b_out, u32* status, cudaStream_t s);
 cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64* a, const u64* b, u64 modulus,
                            u64 delta, u64 p, u64 dinv, u32 entry_size, uint8_t* out, cudaStream_t s);
-cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 r_mod_q, u64 ms_target,
-                 u64* stack, u64* a_out, u64* b_out, u32* status, cudaStream_t s);
+cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 ms_target, u64* stack,
+                 u64* a_out, u64* b_out, u32* status, cudaStream_t s);
 
 // Integer roofline probe: blocks x 256 threads x iters x 8 lazy butterflies in registers.
 cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s);

@@ -405,7 +405,7 @@ int fold_store(ig_ctx* c, CrsObj& o, const u64* cols, u64* sums) {
   if (rc) return rc;
   long k = prof_begin(c, REGION_FOLD);
   c->launches++;
-  IG_CUDA(c, igk::ntt_rows(o.dev, cols, (u64*)H, o.gamma, 1, shoup_companion(1), c->stream));
+  IG_CUDA(c, igk::ntt_rows(o.dev, cols, (u64*)H, o.gamma, 1, c->stream));
   IG_CUDA(c, igk::store_fold(o.dev, (const u64*)H, sums, c->stream));
   prof_end(c, k);
   return IG_OK;
@@ -722,8 +722,8 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   const u64 two_n = 2ULL * n;
   const u64 psi = find_root(two_n);
   std::vector<u64> tw = ladder(n, psi);
-  std::vector<u64> twp(n);
-  for (u32 m = 0; m < n; m++) twp[m] = shoup_companion(tw[m]);
+  std::vector<Tw> twd(n);
+  for (u32 m = 0; m < n; m++) twd[m] = make_tw(tw[m]);
   // Slot roots: slot t of the forward transform of X holds root w_t = w0^e_t.
   std::vector<u64> X(n, 0);
   X[1] = 1;
@@ -782,7 +782,7 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   d.rows = o.rows;
   d.approx = o.approx;
   int rc;
-  if ((rc = upload(c, o, tw, &d.tw)) || (rc = upload(c, o, twp, &d.twp)) || (rc = upload(c, o, slot_exp, &d.slot_exp)) ||
+  if ((rc = upload(c, o, twd, &d.tw)) || (rc = upload(c, o, slot_exp, &d.slot_exp)) ||
       (rc = upload(c, o, exp_slot, &d.exp_slot)) || (rc = upload(c, o, gpow, &d.gpow)) ||
       (rc = upload(c, o, cpow, &d.cpow)) || (rc = upload(c, o, m_of_i, &d.m_of_i)) ||
       (rc = upload(c, o, pow_root_R, &d.pow_root_R))) {
@@ -790,10 +790,11 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
     c->obj_bytes -= o.bytes;
     return rc;
   }
-  d.ninv = invmod(n);
-  d.ninvp = shoup_companion(d.ninv);
-  d.nlast = mulmod(d.ninv, negq(tw[1]));
-  d.nlastp = shoup_companion(d.nlast);
+  const u64 ninv = invmod(n), rinv = invmod(R_MOD_Q);
+  d.ninv = make_tw(ninv);
+  d.s_ninv_rinv = make_tw(mulmod(ninv, rinv));
+  d.s_rinv = make_tw(rinv);
+  d.s_n_rinv = make_tw(mulmod(n, rinv));
   d.inv_gamma_R = mulmod(invmod(gamma), R_MOD_Q);
   d.inv_gamma_Rp = shoup_companion(d.inv_gamma_R);
   // Last exact digit: base^-2 (R - D0 - base D1) (inspiring2.rs:1094-1161). The kernels
@@ -814,7 +815,7 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   }
   o.allocs.push_back(wm);
   IG_CUDA(c, cudaMemcpyAsync(mraw, mask.data(), mask.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  IG_CUDA(c, igk::ntt_rows(d, (const u64*)mraw, (u64*)wm, o.rows, R_MOD_Q, shoup_companion(R_MOD_Q), c->stream));
+  IG_CUDA(c, igk::ntt_rows(d, (const u64*)mraw, (u64*)wm, o.rows, R_MOD_Q, c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
   d.wmask_R = (const u64*)wm;
   if ((rc = sync_crs_self(c, o))) {
@@ -1102,7 +1103,7 @@ static int make_seat(ig_ctx* c, CrsObj& o, const uint64_t* y_body, uint32_t rows
     IG_CUDA(c, cudaMemcpyAsync(raw, y_body, (size_t)rows * o.n * 8, cudaMemcpyHostToDevice, c->stream));
     src = (const u64*)raw;
   }
-  IG_CUDA(c, igk::ntt_rows(o.dev, src, dst, rows, R_MOD_Q, shoup_companion(R_MOD_Q), c->stream));
+  IG_CUDA(c, igk::ntt_rows(o.dev, src, dst, rows, R_MOD_Q, c->stream));
   return IG_OK;
 }
 
@@ -1547,7 +1548,7 @@ int ig_client_create(ig_ctx* c, uint64_t crs, const uint64_t* secret, double sig
   cl.allocs.push_back(acc);
   IG_CUDA(c, cudaMemcpyAsync(raw, secret, n * 8, cudaMemcpyHostToDevice, c->stream));
   IG_CUDA(c, cudaMemcpyAsync(acc, table.data(), table.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  IG_CUDA(c, igk::ntt_rows(o->dev, (const u64*)raw, (u64*)sR, 1, R_MOD_Q, shoup_companion(R_MOD_Q), c->stream));
+  IG_CUDA(c, igk::ntt_rows(o->dev, (const u64*)raw, (u64*)sR, 1, R_MOD_Q, c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
   cl.s_R = (u64*)sR;
   cl.accept = (u64*)acc;
@@ -1737,13 +1738,12 @@ int ig_crs_set_galois_keys(ig_ctx* c, uint64_t crs, uint32_t count, uint32_t row
   if (!rc) rc = dalloc(c, &dk, words * 8, &o->bytes);
   if (rc) return rc;
   IG_CUDA(c, cudaMemcpyAsync(raw, keys, words * 8, cudaMemcpyHostToDevice, c->stream));
-  IG_CUDA(c, igk::ntt_rows(o->dev, (const u64*)raw, (u64*)dk, (u32)(words / o->n), R_MOD_Q, shoup_companion(R_MOD_Q),
-                           c->stream));
+  IG_CUDA(c, igk::ntt_rows(o->dev, (const u64*)raw, (u64*)dk, (u32)(words / o->n), R_MOD_Q, c->stream));
   IG_CUDA(c, igk::fold_gadget_keys(o->dev, (u64*)dk, count, c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (o->dev.galois_R) {
+  if (o->dev.galois) {
     for (auto it = o->allocs.begin(); it != o->allocs.end(); ++it)
-      if (*it == (void*)o->dev.galois_R) {
+      if (*it == (void*)o->dev.galois) {
         cudaFree(*it);
         o->allocs.erase(it);
         o->bytes -= words * 8;
@@ -1752,7 +1752,7 @@ int ig_crs_set_galois_keys(ig_ctx* c, uint64_t crs, uint32_t count, uint32_t row
       }
   }
   o->allocs.push_back(dk);
-  o->dev.galois_R = (const u64*)dk;
+  o->dev.galois = (const u64*)dk;
   return sync_crs_self(c, *o);
 }
 
@@ -1774,7 +1774,7 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
   if (!db) return fail(c, IG_ERR_HANDLE, "unknown database handle %llu", (unsigned long long)dbh);
   CrsObj& o = *get_crs(c, db->crs);
   const size_t n = o.n;
-  if (!o.dev.galois_R)
+  if (!o.dev.galois)
     return fail(c, IG_ERR_SHAPE,
                 "respond_one_packing: 0 galois keys, but ring_dim %u packs through %u tree levels; this CRS cannot "
                 "drive automorphism packing",
@@ -1831,8 +1831,8 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     return rc;
   cudaStream_t s = igint::host_call_stream(c, hc);
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
-  IG_CUDA(c, igk::tree(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, R_MOD_Q, ms_target,
-                       (u64*)d_stack, (u64*)d_a, (u64*)d_b, (u32*)d_status, s));
+  IG_CUDA(c, igk::tree(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, ms_target, (u64*)d_stack,
+                       (u64*)d_a, (u64*)d_b, (u32*)d_status, s));
   c->launches++;
   IG_CUDA(c, cudaMemcpyAsync((void*)h_status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
   if ((rc = igint::host_call_launched(c, hc))) return rc;
