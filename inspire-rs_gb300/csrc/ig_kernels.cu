@@ -18,6 +18,8 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "ig_kernels.cuh"
 
 namespace igk {
@@ -628,6 +630,17 @@ struct KeyRows {
 //   c_i = (n^-1 a)[tau] S + sum_k (n^-1 W_k)[tau] D_k,   sum_b += sum_k Y_k[tau] D_k,
 // and with the exact gadget (rows folded by fold_gadget3), where R_{i+1} = n c_{i+1} takes the third
 // digit's place, W_2 stays and Y_2 is scaled by n.
+__device__ __forceinline__ void stage_key_rows(const CrsDev& c, const SetView& v, const u64* yR, const KeyRows& K, int n,
+                                               int k, int to) {
+  u64 w[3] = {v.wmask_R[k], v.wmask_R[n + k], 0}, y[3] = {yR[k], yR[n + k], 0};
+  if (v.approx == 0) {
+    fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, v.wmask_R + k, w, n, 1);
+    fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, yR + k, y, n, 1);
+  }
+  K.W01[to] = make_ulonglong2(canon(mulw(w[0], c.s_ninv_rinv)), canon(mulw(w[1], c.s_ninv_rinv)));
+  K.Y01[to] = make_ulonglong2(canon(mulw(y[0], c.s_rinv)), canon(mulw(y[1], c.s_rinv)));
+  K.WY2[to] = make_ulonglong2(canon(mulw(w[2], c.s_rinv)), canon(mulw(y[2], c.s_n_rinv)));
+}
 template <int N, int NT>
 __device__ __forceinline__ void stage_constants(const CrsDev& c, const SetView& v, const u64* yR, Tw* tw,
                                                 const KeyRows& K, uint16_t* e_tab, uint16_t* s_tab) {
@@ -635,14 +648,7 @@ __device__ __forceinline__ void stage_constants(const CrsDev& c, const SetView& 
     tw[k] = c.tw[k];
     e_tab[k] = c.slot_exp[k];
     s_tab[k] = c.exp_slot[k];
-    u64 w[3] = {v.wmask_R[k], v.wmask_R[N + k], 0}, y[3] = {yR[k], yR[N + k], 0};
-    if (v.approx == 0) {
-      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, v.wmask_R + k, w, N, 1);
-      fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, yR + k, y, N, 1);
-    }
-    K.W01[k] = make_ulonglong2(canon(mulw(w[0], c.s_ninv_rinv)), canon(mulw(w[1], c.s_ninv_rinv)));
-    K.Y01[k] = make_ulonglong2(canon(mulw(y[0], c.s_rinv)), canon(mulw(y[1], c.s_rinv)));
-    K.WY2[k] = make_ulonglong2(canon(mulw(w[2], c.s_rinv)), canon(mulw(y[2], c.s_n_rinv)));
+    stage_key_rows(c, v, yR, K, N, k, k);
   }
 }
 
@@ -659,8 +665,9 @@ __device__ __forceinline__ void transform_a(const CrsDev& c, u64* a, const Tw* t
 
 // The pointwise step of one slot at the gathered position tb: adds sum_k Y_k D_k to sb and returns
 // c_i. d0, d1 at most 15q, cur at most 1+: sb takes at most 31 q^2 < 2^125 a call.
+template <bool EXACT>
 __device__ __forceinline__ u64 link_slot(Acc& sb, u64 d0, u64 d1, u64 cur, u64 s_R, const u64* a_ntt,
-                                         const KeyRows& K, u32 tb, bool exact) {
+                                         const KeyRows& K, u32 tb) {
   const ulonglong2 w = K.W01[tb], y = K.Y01[tb];
   Acc r{0, 0, 0, 0};
   mac(r, a_ntt[tb], s_R);
@@ -668,7 +675,7 @@ __device__ __forceinline__ u64 link_slot(Acc& sb, u64 d0, u64 d1, u64 cur, u64 s
   mac(sb, d0, y.x);
   mac(r, d1, w.y);
   mac(sb, d1, y.y);
-  if (exact) {  // the rows are folded: c_{i+1} stands in for digit 2
+  if constexpr (EXACT) {  // the rows are folded: c_{i+1} stands in for digit 2
     const ulonglong2 z = K.WY2[tb];
     mac(r, cur, z.x);
     mac(sb, cur, z.y);
@@ -750,9 +757,10 @@ __device__ __forceinline__ int sw(int e) { return e ^ (((e >> 4) & 3) << 2); }
 // ------------------------------------------------------------------------------------
 // The digits 0 and 1 of a canonical coefficient: base 2^20, of the coefficient itself (exact) or of
 // its rounding to a multiple of 2^20 with the lowest digit dropped (the top carry is kept).
-__device__ __forceinline__ void split_digits(u64 r, bool exact, u32& g0, u32& g1) {
+template <bool EXACT>
+__device__ __forceinline__ void split_digits(u64 r, u32& g0, u32& g1) {
   constexpr u32 DMASK = (1u << 20) - 1;
-  if (exact) {
+  if constexpr (EXACT) {
     g0 = (u32)r & DMASK;
     g1 = (u32)(r >> 20) & DMASK;
   } else {
@@ -857,7 +865,7 @@ __device__ __forceinline__ void fwd_middle(u64* D, const Tw* tw) {
 // split and the forward's first stage are one pass over the pairs (b, b + N/2). X: N words, D: 2N.
 template <int LOGN>
 __device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4], u64 (&d1)[4], u64* X, u64* D,
-                                                const Tw* tw, bool exact) {
+                                                const Tw* tw) {
   constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2, MF = 1 << (LOGN - 2);
   const int tid = threadIdx.x, l0 = 4 * tid;
   {
@@ -874,8 +882,8 @@ __device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4
     const int b = sw(tid + j * NT), b2 = sw(tid + j * NT + H);
     const u64 x0 = X[b], x1 = X[b2];
     u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + N/2
-    split_digits(canon(x0 + x1), exact, p0, p1);
-    split_digits(canon(mulw(x1 - x0 + 5 * Q, wf)), exact, q0, q1);
+    split_digits<true>(canon(x0 + x1), p0, p1);
+    split_digits<true>(canon(mulw(x1 - x0 + 5 * Q, wf)), q0, q1);
     const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
     D[b] = p0 + t0;
     D[b2] = p0 + 3 * Q - t0;
@@ -898,7 +906,314 @@ __device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4
   }
 }
 
-// One CTA per query (batches that fill the GPU). Thread u owns slots 4u..4u+3 of every
+// ------------------------------------------------------------------------------------
+// Radix-8 transforms of one CTA of N/8 threads (the one-CTA respond kernel): three stages a
+// shared-memory round trip on units of eight words a thread. Against radix-4 passes on N/4 threads
+// a link takes 6 barriers instead of 10 and half the shared-memory wavefronts (2.26 M -> 1.14 M a query at
+// gamma 256), and each phase between barriers is long enough to hide its loads: 7.14 -> 6.79 ms for 509
+// queries. What bounds it now is the two warps a sub-partition that its shared memory leaves room for:
+// the heavy multiply pipe is busy 70% of cycles, the warps' fixed-latency waits take the rest.
+//
+// Layouts, free of bank conflicts in every pass of the 2048 ring:
+//   sw8    words of the transform buffers: bits 4-5 of the index XORed into bits 1-2 spread the
+//          16-byte accesses of contiguous units, bit 6 into bit 3 those of the stride-8 passes;
+//   tw8    ladder entries: the levels N/4 and N/2, used only by the passes on contiguous units, hold
+//          the entries that a unit takes N/8 apart, so a warp's loads are contiguous;
+//   slot8  gathered operands (a_ntt, the key rows): slot t at (t & 7) N/8 + (t >> 3). The slots
+//          8 l + k of a warp's lanes l go to slots whose t >> 3 differ modulo any power of two that
+//          theirs do (an odd affine map of the bit-reversed index), so a gather hits distinct banks.
+__device__ __forceinline__ int sw8(int e) { return e ^ (((e >> 4) & 3) << 1) ^ (((e >> 6) & 1) << 3); }
+template <int LOGN>
+__device__ __forceinline__ int tw8(int m) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  if (m >= N / 2) return N / 2 + (m & 3) * E + ((m - N / 2) >> 2);
+  if (m >= N / 4) return N / 4 + (m & 1) * E + ((m - N / 4) >> 1);
+  return m;
+}
+template <int LOGN>
+__device__ __forceinline__ int slot8(int t) {
+  return ((t & 7) << (LOGN - 3)) | (t >> 3);
+}
+
+// Three forward stages; out <= in + 9. RED brings the words that are not multiplied first down to 1.
+template <bool RED>
+__device__ __forceinline__ void fwd_unit8(u64 (&x)[8], const Tw& w0, const Tw (&w1)[2], const Tw (&w2)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (RED) x[k] = red60(x[k]);
+    bf_fwd(x[k], x[k + 4], w0);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    bf_fwd(x[k], x[k + 2], w1[0]);
+    bf_fwd(x[k + 4], x[k + 6], w1[1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) bf_fwd(x[2 * k], x[2 * k + 1], w2[k]);
+}
+constexpr int FWD_FREE8 = 6;  // 6 + 9 < 16
+
+// Three inverse stages on words up to 2+; out at most 2+. The first word's sum after two stages (8+)
+// is reduced before it meets its equal, and the four sums at the end.
+__device__ __forceinline__ void inv_unit8(u64 (&x)[8], const Tw (&f0)[4], const Tw (&f1)[2], const Tw& f2) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) bf_inv<3>(x[2 * k], x[2 * k + 1], f0[k]);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    bf_inv<5>(x[4 * k], x[4 * k + 2], f1[k]);
+    bf_inv<3>(x[4 * k + 1], x[4 * k + 3], f1[k]);
+  }
+  x[0] = red60(x[0]);
+  bf_inv<2>(x[0], x[4], f2);
+  bf_inv<5>(x[1], x[5], f2);
+  bf_inv<3>(x[2], x[6], f2);
+  bf_inv<3>(x[3], x[7], f2);
+#pragma unroll
+  for (int k = 0; k < 4; k++) x[k] = red60(x[k]);
+}
+
+// Stages a middle pass takes with `rem` left: three, but two and two of four, and two of two.
+__host__ __device__ constexpr int pass_stages(int rem) { return rem == 4 || rem == 2 ? 2 : 3; }
+
+// Inverse stages S .. logn-3 of NB buffers N words apart, words up to 2+ in and out. Each pass ends with
+// a barrier.
+template <int LOGN, int NB, int S = 3>
+__device__ __forceinline__ void inv_middle8(u64* X, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 8;
+  if constexpr (S < LOGN - 2) {
+    constexpr int K = pass_stages(LOGN - 2 - S), t = 1 << S, M = N >> (S + 1);
+    if constexpr (K == 3) {
+      const int u = threadIdx.x, B = u >> S, o = u & (t - 1), e0 = B * 8 * t + o;
+      Tw f0[4], f1[2];
+#pragma unroll
+      for (int j = 0; j < 4; j++) f0[j] = tw[2 * M - 1 - 4 * B - j];
+#pragma unroll
+      for (int j = 0; j < 2; j++) f1[j] = tw[M - 1 - 2 * B - j];
+      const Tw f2 = tw[M / 2 - 1 - B];
+#pragma unroll
+      for (int n = 0; n < NB; n++) {
+        u64 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = X[n * N + sw8(e0 + k * t)];
+        inv_unit8(x, f0, f1, f2);
+#pragma unroll
+        for (int k = 0; k < 8; k++) X[n * N + sw8(e0 + k * t)] = x[k];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int u = threadIdx.x + r * NT, B = u >> S, o = u & (t - 1), e0 = B * 4 * t + o;
+#pragma unroll
+        for (int n = 0; n < NB; n++) {
+          u64 x[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) x[k] = X[n * N + sw8(e0 + k * t)];
+          inv_unit(x[0], x[1], x[2], x[3], tw[2 * M - 1 - 2 * B], tw[2 * M - 2 - 2 * B], tw[M - 1 - B]);
+#pragma unroll
+          for (int k = 0; k < 4; k++) X[n * N + sw8(e0 + k * t)] = x[k];
+        }
+      }
+    }
+    __syncthreads();
+    inv_middle8<LOGN, NB, S + K>(X, tw);
+  }
+}
+
+// Forward stages S .. logn-4 of NB buffers N words apart, words up to BIN in and fwd_bound8 out. Each pass
+// ends with a barrier.
+__host__ __device__ constexpr int fwd_bound8(int logn, int s, int b) {
+  for (; s < logn - 3; s += pass_stages(logn - 3 - s)) {
+    const int k = pass_stages(logn - 3 - s);
+    b = (b > 15 - 3 * k ? 1 : b) + 3 * k;
+  }
+  return b;
+}
+template <int LOGN, int NB, int BIN, int S = 2>
+__device__ __forceinline__ void fwd_middle8(u64* D, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 8;
+  if constexpr (S < LOGN - 3) {
+    constexpr int K = pass_stages(LOGN - 3 - S), m = 1 << S, h = N >> (S + K);
+    constexpr bool RED = BIN > 15 - 3 * K;
+    if constexpr (K == 3) {
+      const int u = threadIdx.x, i = u / h, o = u % h, e0 = i * 8 * h + o;
+      const Tw w0 = tw[m + i];
+      Tw w1[2], w2[4];
+#pragma unroll
+      for (int j = 0; j < 2; j++) w1[j] = tw[2 * m + 2 * i + j];
+#pragma unroll
+      for (int j = 0; j < 4; j++) w2[j] = tw[4 * m + 4 * i + j];
+#pragma unroll
+      for (int n = 0; n < NB; n++) {
+        u64 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = D[n * N + sw8(e0 + k * h)];
+        fwd_unit8<RED>(x, w0, w1, w2);
+#pragma unroll
+        for (int k = 0; k < 8; k++) D[n * N + sw8(e0 + k * h)] = x[k];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int u = threadIdx.x + r * NT, i = u / h, o = u % h, e0 = i * 4 * h + o;
+#pragma unroll
+        for (int n = 0; n < NB; n++) {
+          u64 x[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) x[k] = D[n * N + sw8(e0 + k * h)];
+          fwd_unit<RED>(x[0], x[1], x[2], x[3], tw[m + i], tw[2 * m + 2 * i], tw[2 * m + 2 * i + 1]);
+#pragma unroll
+          for (int k = 0; k < 4; k++) D[n * N + sw8(e0 + k * h)] = x[k];
+        }
+      }
+    }
+    __syncthreads();
+    fwd_middle8<LOGN, NB, (RED ? 1 : BIN) + 3 * K, S + K>(D, tw);
+  }
+}
+
+// The first three inverse stages of thread tid's unit (slots 8 tid .. 8 tid + 7, words up to 2+), from
+// registers to X.
+template <int LOGN>
+__device__ __forceinline__ void inv_first8(u64 (&x)[8], u64* X, const Tw* tw) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  const int tid = threadIdx.x, r = E - 1 - tid;  // the mirrored unit
+  Tw f0[4], f1[2];
+#pragma unroll
+  for (int j = 0; j < 4; j++) f0[j] = tw[N / 2 + (3 - j) * E + r];
+#pragma unroll
+  for (int j = 0; j < 2; j++) f1[j] = tw[N / 4 + (1 - j) * E + r];
+  inv_unit8(x, f0, f1, tw[E + r]);
+#pragma unroll
+  for (int k = 0; k < 8; k += 2)
+    *reinterpret_cast<ulonglong2*>(X + sw8(8 * tid + k)) = make_ulonglong2(x[k], x[k + 1]);
+}
+
+// The last three forward stages of thread tid's unit of NB buffers, to registers: at most 15.
+template <int LOGN, int NB, int BIN>
+__device__ __forceinline__ void fwd_last8(u64 (&x)[NB][8], const u64* D, const Tw* tw) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  constexpr bool RED = BIN > FWD_FREE8;
+  const int tid = threadIdx.x;
+  const Tw w0 = tw[E + tid];
+  Tw w1[2], w2[4];
+#pragma unroll
+  for (int j = 0; j < 2; j++) w1[j] = tw[N / 4 + j * E + tid];
+#pragma unroll
+  for (int j = 0; j < 4; j++) w2[j] = tw[N / 2 + j * E + tid];
+#pragma unroll
+  for (int n = 0; n < NB; n++) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(D + n * N + sw8(8 * tid + k));
+      x[n][k] = v.x;
+      x[n][k + 1] = v.y;
+    }
+    fwd_unit8<RED>(x[n], w0, w1, w2);
+  }
+}
+
+// One link's transforms: thread tid holds the NTT-domain words cur of its unit (at most 1+, scaled by
+// n^-1) and gets the transforms of digits 0 and 1 of their inverse transform at the same slots, at most
+// 15. The inverse's last two stages, the digit split and the forward's first two are one radix-4 pass
+// over the words b + k N/4. D: 2N words; the inverse runs in the first N, which the pass rewrites in
+// place as digit 0. No thread touches another's unit after the last barrier, so the next link may
+// follow without one.
+template <int LOGN, bool EXACT>
+__device__ __forceinline__ void link_transforms8(const u64 (&cur)[8], u64 (&d)[2][8], u64* D, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
+  {
+    u64 x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = cur[k];
+    inv_first8<LOGN>(x, D, tw);
+  }
+  __syncthreads();
+  inv_middle8<LOGN, 1>(D, tw);
+  const Tw w1 = tw[1], w2 = tw[2], w3 = tw[3];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int b = threadIdx.x + j * NT;
+    u64 x[4];
+    int at[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = D[at[k] = sw8(b + k * P)];
+    bf_inv<3>(x[0], x[1], w3);
+    bf_inv<3>(x[2], x[3], w2);
+    u32 g[2][4];
+    split_digits<EXACT>(canon(x[0] + x[2]), g[0][0], g[1][0]);
+    split_digits<EXACT>(canon(x[1] + x[3]), g[0][1], g[1][1]);
+    split_digits<EXACT>(canon(mulw(x[2] - x[0] + 5 * Q, w1)), g[0][2], g[1][2]);
+    split_digits<EXACT>(canon(mulw(x[3] - x[1] + 3 * Q, w1)), g[0][3], g[1][3]);
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+      const u64 t2 = mulw_digit(g[n][2], w1), t3 = mulw_digit(g[n][3], w1);
+      u64 y0 = g[n][0] + t2, y2 = g[n][0] + 3 * Q - t2, y1 = g[n][1] + t3, y3 = g[n][1] + 3 * Q - t3;
+      bf_fwd(y0, y1, w2);
+      bf_fwd(y2, y3, w3);
+      D[n * N + at[0]] = y0;
+      D[n * N + at[1]] = y1;
+      D[n * N + at[2]] = y2;
+      D[n * N + at[3]] = y3;
+    }
+  }
+  __syncthreads();
+  fwd_middle8<LOGN, 2, 6>(D, tw);
+  fwd_last8<LOGN, 2, fwd_bound8(LOGN, 2, 6)>(d, D, tw);
+}
+
+// The query's `a` (coefficient form in src, plain order) to n^-1 2^-64 NTT(a) at its slots' positions in
+// a_ntt. D: N words of scratch other than src.
+template <int LOGN>
+__device__ __forceinline__ void transform_a8(const CrsDev& c, const u64* src, u64* D, u64* a_ntt, const Tw* tw) {
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int b = threadIdx.x + j * NT;
+    u64 x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = src[b + k * P];
+    fwd_unit<false>(x[0], x[1], x[2], x[3], tw[1], tw[2], tw[3]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) D[sw8(b + k * P)] = x[k];
+  }
+  __syncthreads();
+  fwd_middle8<LOGN, 1, 7>(D, tw);
+  u64 x[1][8];
+  fwd_last8<LOGN, 1, fwd_bound8(LOGN, 2, 7)>(x, D, tw);
+#pragma unroll
+  for (int k = 0; k < 8; k++) a_ntt[k * NT + threadIdx.x] = canon(mulw(x[0][k], c.s_ninv_rinv));
+  __syncthreads();
+}
+
+// The recursion's links gamma - 2 .. 0 on thread tid's slots (sums: the store's row 0 at its first slot).
+template <int LOGN, bool EXACT>
+__device__ __forceinline__ void respond_links8(u64 (&cur)[8], Acc (&sb)[8], const u32 (&et)[8], u32 gamma,
+                                               const u32* gpow, const u64* sums, u64* D, const u64* a_ntt,
+                                               const Tw* tw, const KeyRows& K, const uint16_t* s_tab) {
+  constexpr int N = 1 << LOGN;
+  constexpr u32 M2N = 2 * N - 1;
+#pragma unroll 1
+  for (int i = (int)gamma - 2; i >= 0; i--) {
+    const ulonglong2* Srow = reinterpret_cast<const ulonglong2*>(sums + (size_t)i * N);
+    ulonglong2 sv[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) sv[k] = Srow[k];
+    const u32 gp = gpow[i];
+    u64 d[2][8];
+    link_transforms8<LOGN, EXACT>(cur, d, D, tw);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
+      cur[k] = link_slot<EXACT>(sb[k], d[0][k], d[1][k], cur[k], k & 1 ? sv[k / 2].y : sv[k / 2].x, a_ntt, K, tb);
+    }
+    if (i % SB_FOLD_LINKS == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) sb[k] = acc_from(acc_fold(sb[k]));
+    }
+  }
+}
+
+// One CTA per query (batches that fill the GPU). Thread u owns slots 8u..8u+7 of every
 // NTT-domain vector (one transform unit). Each link of the recursion (i from gamma-2 down
 // to 0) holds n^-1 R_{i+1} in NTT form (`cur`, in registers):
 //   r = INTT(R_{i+1});  d_k = base-2^20 digits of r (rounded, top carry kept, when the
@@ -911,22 +1226,20 @@ __device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4
 // a fixed linear combination, so the key rows are folded at staging (fold_gadget3) and
 // R_{i+1} takes digit 2's place in the sums.
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 4, 1)
+__global__ void __launch_bounds__((1 << LOGN) / 8, 1)
     k_respond(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out, u64* b_out,
               u32* status, int force_serial) {
-  constexpr int N = 1 << LOGN, NT = N / 4;
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
   constexpr u32 M2N = 2 * N - 1;
   extern __shared__ __align__(16) u64 sm[];
-  u64* X = sm;       // N: the inverse in progress
-  u64* D = sm + N;   // 2N: digits 0 and 1 (forward in progress)
+  u64* D = sm;  // 2N: the inverse in progress in the first N, then digits 0 and 1
   u64* a_ntt = D + 2 * N;
   Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
   // Room for three key rows whatever the query's gadget, so queries of different sets
   // share a launch.
   ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);
   const KeyRows K{rows, rows + N, rows + 2 * N};
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
-  uint16_t* s_tab = e_tab + N;
+  uint16_t* s_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);  // position of the slot of exponent 2e + 1
 
   const int tid = threadIdx.x;
   const QueryDev qd = queries[blockIdx.x];
@@ -935,62 +1248,62 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
   const SetView ps = set_view(c, qd.crs);
   const u32 gamma = ps.gamma;
   const bool exact = ps.approx == 0;
-  const int l0 = 4 * tid;
+  const int l0 = 8 * tid;
 
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
-  expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  transform_a<LOGN, NT>(c, a_ntt, tw);
+  for (int k = tid; k < N; k += NT) {
+    tw[tw8<LOGN>(k)] = c.tw[k];
+    s_tab[k] = (uint16_t)slot8<LOGN>(c.exp_slot[k]);
+    stage_key_rows(c, ps, qd.seat_R, K, N, k, slot8<LOGN>(k));
+  }
+  expand_a<N, NT>(qd, D + N, status, qi, force_serial);  // ends with a barrier
+  transform_a8<LOGN>(c, D + N, D, a_ntt, tw);
 
-  u64 cur[4];
-  Acc sb[4];
-  u32 et[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) et[k] = e_tab[l0 + k];
+  u64 cur[8];
+  Acc sb[8];
+  u32 et[8];
   {
     const u32 gp = ps.gpow[gamma - 1];
-    const u64* Srow = sh.sums_R + (size_t)(gamma - 1) * N;
+    const u64* Srow = sh.sums_R + (size_t)(gamma - 1) * N + l0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = mulq(a_ntt[tb], Srow[l0 + k]);
+    for (int k = 0; k < 8; k++) {
+      et[k] = c.slot_exp[l0 + k];
+      cur[k] = mulq(a_ntt[s_tab[((gp * et[k]) & M2N) >> 1]], Srow[k]);
       sb[k] = Acc{0, 0, 0, 0};
     }
   }
-#pragma unroll 1
-  for (int i = (int)gamma - 2; i >= 0; i--) {
-    const u64* Srow = sh.sums_R + (size_t)i * N + l0;
-    const ulonglong2 sv01 = *reinterpret_cast<const ulonglong2*>(Srow);
-    const ulonglong2 sv23 = *reinterpret_cast<const ulonglong2*>(Srow + 2);
-    const u32 gp = ps.gpow[i];
-    u64 d0[4], d1[4];
-    link_transforms<LOGN>(cur, d0, d1, X, D, tw, exact);
-    const u64 sv[4] = {sv01.x, sv01.y, sv23.x, sv23.y};
+  if (exact)
+    respond_links8<LOGN, true>(cur, sb, et, gamma, ps.gpow, sh.sums_R + l0, D, a_ntt, tw, K, s_tab);
+  else
+    respond_links8<LOGN, false>(cur, sb, et, gamma, ps.gpow, sh.sums_R + l0, D, a_ntt, tw, K, s_tab);
+  // Final inverse transforms of c_0 (to a) and of the online sum (to b), in the two halves of D.
+  {
+    u64 x[8];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = link_slot(sb[k], d0[k], d1[k], cur[k], sv[k], a_ntt, K, tb, exact);
-    }
-    if (i % SB_FOLD_LINKS == 0) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) sb[k] = acc_from(acc_fold(sb[k]));
-    }
-  }
-  __syncthreads();  // every thread is past its last read of D
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    D[l0 + k] = cur[k];
-    D[N + l0 + k] = acc_fold(sb[k]);
+    for (int k = 0; k < 8; k++) x[k] = acc_fold(sb[k]);
+    inv_first8<LOGN>(cur, D, tw);
+    inv_first8<LOGN>(x, D + N, tw);
   }
   __syncthreads();
-  {
-    u64* const bufs[2] = {D, D + N};
-    ntt_inv_r4<LOGN, NT, 2>(bufs, tw);
-  }
+  inv_middle8<LOGN, 2>(D, tw);
+  const Tw w1 = tw[1], w2 = tw[2], w3 = tw[3];
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int t = tid + k * NT;
-    a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
-    b_out[(size_t)qi * N + t] = finish_b(c, D[N + t], t, gamma, b_fold + qd.fold_off, qd.ms);
+  for (int j = 0; j < 2; j++) {
+    const int b = tid + j * NT;
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+      u64 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = D[n * N + sw8(b + k * P)];
+      inv_unit(x[0], x[1], x[2], x[3], w3, w2, w1);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int t = b + k * P;
+        if (n == 0)
+          a_out[(size_t)qi * N + t] = finish_a(x[k], qd.ms);
+        else
+          b_out[(size_t)qi * N + t] = finish_b(c, x[k], t, gamma, b_fold + qd.fold_off, qd.ms);
+      }
+    }
   }
 }
 
@@ -1162,6 +1475,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
   constexpr int MF = 1 << (LOGN - 2);
   const Tw fa = tw[MF + ug], fb = tw[2 * MF + 2 * ug], fc = tw[2 * MF + 2 * ug + 1];
   const Tw wf = tw[1];
+  // One instance of the links a gadget: the choice stays out of the slots' straight-line code.
+  auto links = [&](auto gadget) {
+    constexpr bool EXACT = decltype(gadget)::value;
 #pragma unroll 1
   for (int i = (int)gamma - 2; i >= 0; i--) {
     const u64* Srow = sh.sums_R + (size_t)i * N;
@@ -1191,8 +1507,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
         const int b = tid + j * NT;
         const u64 x0 = lo[sw(b)], x1 = hi[sw(b)];
         u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + H
-        split_digits(canon(x0 + x1), exact, p0, p1);
-        split_digits(canon(mulw(x1 - x0 + 5 * Q, wf)), exact, q0, q1);
+        split_digits<EXACT>(canon(x0 + x1), p0, p1);
+        split_digits<EXACT>(canon(mulw(x1 - x0 + 5 * Q, wf)), q0, q1);
         // Forward cross stage: slot b gets p + w q, slot b + H gets p - w q.
         const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
         D[sw(b)] = rank == 0 ? p0 + t0 : p0 + 3 * Q - t0;
@@ -1221,13 +1537,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = link_slot(sb[k], d0[k], d1[k], cur[k], k == 0 ? sv.x : sv.y, a_ntt, K, tb, exact);
+      cur[k] = link_slot<EXACT>(sb[k], d0[k], d1[k], cur[k], k == 0 ? sv.x : sv.y, a_ntt, K, tb);
     }
     if (i % SB_FOLD_LINKS == 0) {
 #pragma unroll
       for (int k = 0; k < 2; k++) sb[k] = acc_from(acc_fold(sb[k]));
     }
   }
+  };
+  if (exact)
+    links(std::true_type{});
+  else
+    links(std::false_type{});
   // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each
   // from its own half and the peer's half (exchanged through the half of X that link 0
   // did not use; the peer read it last at link 1, before the barrier of link 0).
@@ -1326,6 +1647,9 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
   // last stage and stage 0 of the forward entry 1, stage 1 entry 2 for the first half, 3 for the second.
   const Tw w1 = tw[1], w2 = tw[2], w3 = tw[3];
   const Tw wfs = tw[2 + (rank >> 1)];
+  // One instance of the links a gadget: the choice stays out of the slots' straight-line code.
+  auto links = [&](auto gadget) {
+    constexpr bool EXACT = decltype(gadget)::value;
 #pragma unroll 1
   for (int i = (int)gamma - 2; i >= 0; i--) {
     u64 sv[SPT];
@@ -1355,7 +1679,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
       cf[3] = canon(mulw(x3 - x1 + 3 * Q, w1));
       u32 g0[4], g1[4];  // digits 0 and 1
 #pragma unroll
-      for (int k = 0; k < 4; k++) split_digits(cf[k], exact, g0[k], g1[k]);
+      for (int k = 0; k < 4; k++) split_digits<EXACT>(cf[k], g0[k], g1[k]);
       // Forward stage 0 (b with b + N/2, b + N/4 with b + 3N/4), then stage 1 on this
       // quarter's half, of which output rank & 1 is the quarter's word, at most 6.
       auto fwd = [&](const u32(&g)[4]) -> u64 {
@@ -1380,13 +1704,18 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
     for (int j = 0; j < SPT; j++) {
       const u64 d0 = D[sw(tid + j * NT)], d1 = D[P + sw(tid + j * NT)];
       const u32 tb = s_tab[((gp * et[j]) & M2N) >> 1];
-      cur[j] = link_slot(sb[j], d0, d1, cur[j], sv[j], a_ntt, K, tb, exact);
+      cur[j] = link_slot<EXACT>(sb[j], d0, d1, cur[j], sv[j], a_ntt, K, tb);
     }
     if (i % SB_FOLD_LINKS == 0) {
 #pragma unroll
       for (int j = 0; j < SPT; j++) sb[j] = acc_from(acc_fold(sb[j]));
     }
   }
+  };
+  if (exact)
+    links(std::true_type{});
+  else
+    links(std::false_type{});
   // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each from
   // the four quarters exchanged through X once every peer is past its last cross-pass read.
   cluster.sync();
@@ -1634,7 +1963,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
       ab[j] = S1b[src];
     }
     u64 d0[4], d1[4];
-    link_transforms<LOGN>(aa, d0, d1, X, D, tw, true);
+    link_transforms<LOGN>(aa, d0, d1, X, D, tw);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       // The keys' digit rows are folded (fold_gadget_keys): aa stands in for digit 2.
@@ -2163,7 +2492,7 @@ cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s) {
 size_t respond_smem_bytes(const CrsDev& c, int ctas) {
   // X, D and a_ntt, the two ladders, three key rows of W and Y, two u16 slot tables.
   const size_t n = c.n;
-  const size_t words = ctas == 4 ? n / 2 + 4 * n : ctas == 2 ? 5 * n : 6 * n;
+  const size_t words = ctas == 4 ? n / 2 + 4 * n : 5 * n;
   return (words + 2 * (size_t)3 * n) * 8 + 2 * n * 2;
 }
 
@@ -2188,7 +2517,7 @@ cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* sh
       auto k = k_respond<L>;
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      k<<<nq, (1 << L) / 4, smem, s>>>(c, queries, shards, b_fold, a_out, b_out, status, force_serial_expand);
+      k<<<nq, (1 << L) / 8, smem, s>>>(c, queries, shards, b_fold, a_out, b_out, status, force_serial_expand);
     }
   });
   return cudaGetLastError();
