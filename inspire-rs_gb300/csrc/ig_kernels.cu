@@ -205,54 +205,75 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_ntt_rows(CrsDev c, const u6
 //   acc_i[t] = DFT_zeta(u)[(e_t * m_i) mod gamma].
 // The sum lands at S_i[t'] with table_i[t'] = t, i.e. t' = slot of exponent c_i * e_t,
 // scaled by gamma^-1 and stored in R-form.
+//
+// One launch folds several shards (blockIdx.y): a shard alone leaves most of the GPU idle. The powers of
+// w0 come from global memory (one gather a word, 64 KB, kept in L1 and L2) and only the DFT's gamma / 2
+// twiddles are staged, where staging every power took 32 KB of loads for a tile of 16 KB.
 constexpr int FOLD_TILE = 2048;
 constexpr int FOLD_THREADS = 256;
 
+// The shard a store kernel works on: entry blockIdx.y of a device table, or the one given.
+struct ShardArg {
+  const ShardDev* table;
+  ShardDev one;
+};
+__device__ __forceinline__ ShardDev shard_of(const ShardArg& a) { return a.table ? a.table[blockIdx.y] : a.one; }
+
 template <int LOGN>
-__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, u64* sums_R, u32 SL) {
+__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, ShardArg shards, u32 SL) {
   constexpr int N = 1 << LOGN;
   constexpr u32 M2N = 2 * N - 1;
   extern __shared__ __align__(16) u64 sm[];
-  const u32 gamma = c.gamma;
-  const u32 tile = SL * gamma;   // SL slots per CTA, tile <= FOLD_TILE words
-  u64* x = sm;                   // [slot][j]
-  u64* pw = sm + FOLD_TILE;      // w0^e R-form, 2N words
+  const u32 gamma = c.gamma, half = gamma >> 1;
+  const u32 tile = SL * gamma, row = gamma + 1;  // SL slots per CTA, tile <= FOLD_TILE words
+  Tw* zeta = reinterpret_cast<Tw*>(sm);
+  u64* x = sm + 2 * half;  // [slot][j], a word of padding per slot
   const u32 t0 = blockIdx.x * SL;
-  u32 lg = 0;
-  while ((1u << lg) < gamma) lg++;
-  for (int k = threadIdx.x; k < 2 * N; k += FOLD_THREADS) pw[k] = c.pow_root_R[k];
-  __syncthreads();
+  const u32 lg = 31 - __clz(gamma);
+  H += (size_t)blockIdx.y * gamma * N;
+  u64* sums = const_cast<u64*>(shard_of(shards).sums_R);
+  for (u32 k = threadIdx.x; k < half; k += FOLD_THREADS) zeta[k] = c.zeta[k];
   for (u32 idx = threadIdx.x; idx < tile; idx += FOLD_THREADS) {
     const u32 j = idx / SL, s = idx % SL;
     const u32 t = t0 + s;
-    const u32 e = c.slot_exp[t];
-    const u64 h = H[(size_t)j * N + t];
-    x[s * gamma + j] = mont(h, pw[(e * j) & M2N]);
+    x[s * row + j] = mulw(H[(size_t)j * N + t], c.pow_root[(c.slot_exp[t] * j) & M2N]);
   }
   __syncthreads();
-  // Gentleman-Sande DFT of length gamma per slot, bit-reversed output.
-  for (u32 len = gamma >> 1; len >= 1; len >>= 1) {
-    const u32 half_total = SL * (gamma >> 1);
-    for (u32 b = threadIdx.x; b < half_total; b += FOLD_THREADS) {
-      const u32 s = b / (gamma >> 1);
-      const u32 bb = b % (gamma >> 1);
-      const u32 blk = bb / len, j = bb % len;
-      const u32 i0 = s * gamma + blk * 2 * len + j;
-      const u64 u = x[i0], v = x[i0 + len];
-      x[i0] = addq(u, v);
-      x[i0 + len] = mont(subq(u, v), pw[(j * (N / len)) & M2N]);
+  // Gentleman-Sande DFT of length gamma per slot, bit-reversed output, two stages a pass on words up to
+  // 2+ (sums up to 8+ and 4+ reduced, products 2+), a last stage alone when log gamma is odd.
+  u32 len = half;
+  for (; len >= 2; len >>= 2) {
+    const u32 q = len >> 1, step = half / len;
+    for (u32 b = threadIdx.x; b < tile / 4; b += FOLD_THREADS) {
+      const u32 s = b / (gamma >> 2), bb = b % (gamma >> 2);
+      const u32 j = bb & (q - 1), i0 = s * row + (bb - j) * 4 + j;
+      u64 a0 = x[i0], a1 = x[i0 + q], a2 = x[i0 + len], a3 = x[i0 + len + q];
+      const u64 s0 = a0 + a2, s1 = a1 + a3;
+      const u64 d0 = mulw(a0 - a2 + 3 * Q, zeta[j * step]), d1 = mulw(a1 - a3 + 3 * Q, zeta[(j + q) * step]);
+      const Tw w = zeta[2 * j * step];
+      x[i0] = red60(s0 + s1);
+      x[i0 + q] = mulw(s0 - s1 + 5 * Q, w);
+      x[i0 + len] = red60(d0 + d1);
+      x[i0 + len + q] = mulw(d0 - d1 + 3 * Q, w);
+    }
+    __syncthreads();
+  }
+  if (len == 1) {
+    for (u32 b = threadIdx.x; b < tile / 2; b += FOLD_THREADS) {
+      const u32 s = b / half, i0 = s * row + 2 * (b % half);
+      const u64 u = x[i0], v = x[i0 + 1];
+      x[i0] = u + v;
+      x[i0 + 1] = u - v + 3 * Q;
     }
     __syncthreads();
   }
   for (u32 idx = threadIdx.x; idx < tile; idx += FOLD_THREADS) {
     const u32 i = idx / SL, s = idx % SL;
-    const u32 t = t0 + s;
-    const u32 e = c.slot_exp[t];
+    const u32 e = c.slot_exp[t0 + s];
     const u32 k = (e * c.m_of_i[i]) & (gamma - 1);
     const u32 kr = lg ? (__brev(k) >> (32 - lg)) : 0;
-    const u64 val = x[s * gamma + kr];
     const u32 tp = c.exp_slot[((c.cpow[i] * e) & M2N) >> 1];
-    sums_R[(size_t)i * N + tp] = shoup(val, c.inv_gamma_R, c.inv_gamma_Rp);
+    sums[(size_t)i * N + tp] = canon(mulw(x[s * row + kr], c.inv_gamma_R));
   }
 }
 
@@ -296,36 +317,64 @@ __device__ __forceinline__ u128 shfl_xor_u128(u128 v, int m) {
   return ((u128)hi << 64) | lo;
 }
 
-// Tags of `gamma` columns: one warp per column. With `expect` set, a tag that differs sets
-// *mismatch instead of being written.
+__device__ __forceinline__ u64 tag_residue(u128 tag) {
+  u128 t = (tag & TAG_PRIME) + (tag >> 61);
+  t = (t & TAG_PRIME) + (t >> 61);
+  u64 tv = (u64)t;
+  while (tv >= TAG_PRIME) tv -= TAG_PRIME;
+  return tv;
+}
+// Writes column j's tag, or with a mismatch word given compares it with the stored one.
+__device__ __forceinline__ void put_tag(const ShardDev& sh, u32 j, u64 tag, u32* mismatch) {
+  if (!mismatch)
+    const_cast<u64*>(sh.tags)[j] = tag;
+  else if (tag != sh.tags[j])
+    atomicOr(mismatch + blockIdx.y, 1u);
+}
+
+// A shard's tag key: 2n words below 2^61 - 1 from the ChaCha20 keystream of a seed drawn from OS entropy
+// (shard_store.rs:127-135), stream `stream` + the shard's place in the launch. A candidate at the bound
+// (probability 2^-61) gives way to the same word of the streams 2^32 further on.
+struct TagSeed {
+  u32 w[8];
+};
+__global__ void k_tag_keys(u32 n, const ShardDev* table, TagSeed seed, u64 stream) {
+  const u32 b = blockIdx.x * blockDim.x + threadIdx.x;  // one block of eight words
+  if (b >= n / 4) return;
+  u64* key = const_cast<u64*>(table[blockIdx.y].tag_key) + 8 * (size_t)b;
+  u32 blk[16];
+  chacha20_block(seed.w, b, stream + blockIdx.y, blk);
+#pragma unroll 1
+  for (int k = 0; k < 8; k++) {
+    u64 v = (((u64)blk[2 * k + 1] << 32) | blk[2 * k]) >> 3;
+    for (u64 more = 1; v >= TAG_PRIME && more < 64; more++) {
+      u32 alt[16];
+      chacha20_block(seed.w, b, stream + blockIdx.y + (more << 32), alt);
+      v = (((u64)alt[2 * k + 1] << 32) | alt[2 * k]) >> 3;
+    }
+    key[k] = v;
+  }
+}
+
+// Tags of the columns of wide shards (words of 2^16 and above): one warp per column.
 template <int LOGN>
-__global__ void __launch_bounds__(256) k_column_tags(u32 gamma, const u64* cols, const u64* key, u64* tags_out,
-                                                     const u64* expect, u32* mismatch) {
+__global__ void __launch_bounds__(256) k_column_tags(u32 gamma, const ShardDev* table, u32* mismatch) {
   constexpr int N = 1 << LOGN;
+  const ShardDev sh = table[blockIdx.y];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const u32 j = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (j >= gamma) return;
-  const u64* col = cols + (size_t)j * N;
+  if (j >= gamma || sh.cols16) return;
+  const u64* col = sh.columns + (size_t)j * N;
   u128 tag = 0;
 #pragma unroll 4
   for (int k = lane; k < N; k += 32) {
     const u64 w = col[k];
-    const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(key + 2 * k);
+    const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(sh.tag_key + 2 * k);
     tag += (u128)(w & 0xffffffffULL) * kk.x + (u128)(w >> 32) * kk.y;
   }
 #pragma unroll
   for (int m = 16; m >= 1; m >>= 1) tag += shfl_xor_u128(tag, m);
-  if (lane == 0) {
-    u128 t = (tag & TAG_PRIME) + (tag >> 61);
-    t = (t & TAG_PRIME) + (t >> 61);
-    u64 tv = (u64)t;
-    while (tv >= TAG_PRIME) tv -= TAG_PRIME;
-    if (expect) {
-      if (tv != expect[j]) atomicOr(mismatch, 1u);
-    } else {
-      tags_out[j] = tv;
-    }
-  }
+  if (lane == 0) put_tag(sh, j, tag_residue(tag), mismatch);
 }
 
 // Shared memory of the compact path: the vector V, then per warp a ring of SCAN_STAGES
@@ -378,12 +427,92 @@ __device__ __forceinline__ void warp_reduce8(u64 (&v)[8], int lane) {
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// Sums word_k v_k over `rows` (at most SCAN_ROWS) columns at col for a vector of 64-bit words v: fill(V)
+// writes v's 32-bit limbs (shared by the CTA's warps, V[k & 7][k >> 3]) while the warp's first copies are
+// in flight, out(r, sum) gets row r's 128-bit sum on one lane. All the CTA's threads call it.
+template <int LOGN, class Fill, class Out>
+__device__ __forceinline__ void scan_columns16(uint4* scan_sm, const uint16_t* col, int rows, Fill fill, Out out) {
+  constexpr int N = 1 << LOGN, M = N / 8, ITER = M / 32;
+  uint2* V = reinterpret_cast<uint2*>(scan_sm);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint4* ring = scan_sm + N / 2 + (size_t)warp * SCAN_STAGES * SCAN_ROWS * 32;
+  // Lane l copies, for step it, the 16-byte chunk at positions 8m..8m+7 (m = l + 32 it)
+  // of each of the warp's rows into its own ring slots.
+  auto issue = [&](int it) {
+    if (it < ITER) {
+      uint4* dst = ring + (it % SCAN_STAGES) * SCAN_ROWS * 32 + lane;
+      const int m = lane + 32 * it;
+      for (int r = 0; r < rows; r++) cp_async16(dst + r * 32, col + (size_t)r * N + 8 * m);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int it = 0; it < SCAN_STAGES - 1; it++) issue(it);
+  fill(V);
+  __syncthreads();
+  if (rows == 0) {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    return;
+  }
+  u64 acc[8];  // acc[2r] = low-limb sum of row r, acc[2r + 1] = high-limb sum
+#pragma unroll
+  for (int k = 0; k < 8; k++) acc[k] = 0;
+#pragma unroll 1
+  for (int it = 0; it < ITER; it++) {
+    issue(it + SCAN_STAGES - 1);
+    cp_async_wait<SCAN_STAGES - 1>();  // step it's copies have landed
+    const int m = lane + 32 * it;
+    const uint4* src = ring + (it % SCAN_STAGES) * SCAN_ROWS * 32 + lane;
+    uint4 w[SCAN_ROWS];
+#pragma unroll
+    for (int r = 0; r < SCAN_ROWS; r++) w[r] = r < rows ? src[r * 32] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+      const uint2 v = V[p * M + m];
+#pragma unroll
+      for (int r = 0; r < SCAN_ROWS; r++) {
+        const u32 word = p & 1 ? (((&w[r].x)[p >> 1]) >> 16) : (((&w[r].x)[p >> 1]) & 0xffffu);
+        acc[2 * r] += (u64)word * v.x;
+        acc[2 * r + 1] += (u64)word * v.y;
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  warp_reduce8(acc, lane);
+  // Lane l holds value x = ((l >> 4) & 1) 4 + ((l >> 3) & 1) 2 + ((l >> 2) & 1): row x / 2,
+  // limb x & 1; a row's high limb sits four lanes above its low limb.
+  const u64 hi = __shfl_down_sync(0xffffffffu, acc[0], 4);
+  const int r = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+  if ((lane & 7) == 0 && r < rows) out(r, (u128)acc[0] + ((u128)hi << 32));
+}
+
+// Tags of the columns of compact shards: the same sums over the words of the tag key that meet a column
+// word's low half (its high half is zero). 64 columns a CTA share one staging of the key, where a warp a
+// column read all of it each: 18.8 us a shard alone, part of one launch over all shards here.
+template <int LOGN>
+__global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_column_tags16(u32 gamma, const ShardDev* table, u32* mismatch) {
+  constexpr int N = 1 << LOGN, M = N / 8;
+  extern __shared__ __align__(16) uint4 scan_sm[];
+  const ShardDev sh = table[blockIdx.y];
+  if (!sh.cols16) return;
+  const u32 j0 = blockIdx.x * SCAN_COLS + (threadIdx.x >> 5) * SCAN_ROWS;
+  const int rows = j0 < gamma ? min(SCAN_ROWS, (int)(gamma - j0)) : 0;
+  scan_columns16<LOGN>(
+      scan_sm, sh.cols16 + (size_t)j0 * N, rows,
+      [&](uint2* V) {
+        for (int k = threadIdx.x; k < N; k += SCAN_WARPS * 32) {
+          const u64 v = sh.tag_key[2 * k];
+          V[(k & 7) * M + (k >> 3)] = make_uint2((u32)v, (u32)(v >> 32));
+        }
+      },
+      [&](int r, u128 sum) { put_tag(sh, j0 + r, tag_residue(sum), mismatch); });
+}
+
 template <int LOGN>
 __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_scan(CrsDev c, const QueryDev* queries, const ShardDev* shards,
                                                           const u32* work, u32 chunks, u64* b_fold, u32* status) {
-  constexpr int N = 1 << LOGN, M = N / 8, ITER = M / 32;
+  constexpr int N = 1 << LOGN, M = N / 8;
   extern __shared__ __align__(16) uint4 scan_sm[];
-  uint2* V = reinterpret_cast<uint2*>(scan_sm);  // [8][M]: b_rev[k] lo, hi
   u32 qi, chunk;
   if (work) {
     const u32 w = work[blockIdx.x];
@@ -412,62 +541,18 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_scan(CrsDev c, const Que
   const int rows = j0 < gamma ? min(SCAN_ROWS, (int)(gamma - j0)) : 0;
 
   if (sh.cols16) {
-    const uint16_t* col = sh.cols16 + (size_t)j0 * N;
-    uint4* ring = scan_sm + N / 2 + (size_t)warp * SCAN_STAGES * SCAN_ROWS * 32;
-    // Lane l copies, for step it, the 16-byte chunk at positions 8m..8m+7 (m = l + 32 it)
-    // of each of the warp's rows into its own ring slots.
-    auto issue = [&](int it) {
-      if (it < ITER) {
-        uint4* dst = ring + (it % SCAN_STAGES) * SCAN_ROWS * 32 + lane;
-        const int m = lane + 32 * it;
-        for (int r = 0; r < rows; r++) cp_async16(dst + r * 32, col + (size_t)r * N + 8 * m);
-      }
-      cp_async_commit();
-    };
+    scan_columns16<LOGN>(
+        scan_sm, sh.cols16 + (size_t)j0 * N, rows,
+        [&](uint2* V) {
 #pragma unroll
-    for (int it = 0; it < SCAN_STAGES - 1; it++) issue(it);
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-      const int k = threadIdx.x + j * SCAN_WARPS * 32;
-      if (k >= N) break;
-      const u64 bv = k == 0 ? reduce128(braw[j]) : negq(reduce128(braw[j]));
-      V[(k & 7) * M + (k >> 3)] = make_uint2((u32)bv, (u32)(bv >> 32));
-    }
-    __syncthreads();
-    if (rows == 0) {
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-      return;
-    }
-    u64 acc[8];  // acc[2r] = low-limb sum of row r, acc[2r + 1] = high-limb sum
-#pragma unroll
-    for (int k = 0; k < 8; k++) acc[k] = 0;
-#pragma unroll 1
-    for (int it = 0; it < ITER; it++) {
-      issue(it + SCAN_STAGES - 1);
-      cp_async_wait<SCAN_STAGES - 1>();  // step it's copies have landed
-      const int m = lane + 32 * it;
-      const uint4* src = ring + (it % SCAN_STAGES) * SCAN_ROWS * 32 + lane;
-      uint4 w[SCAN_ROWS];
-#pragma unroll
-      for (int r = 0; r < SCAN_ROWS; r++) w[r] = r < rows ? src[r * 32] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int p = 0; p < 8; p++) {
-        const uint2 v = V[p * M + m];
-#pragma unroll
-        for (int r = 0; r < SCAN_ROWS; r++) {
-          const u32 word = p & 1 ? (((&w[r].x)[p >> 1]) >> 16) : (((&w[r].x)[p >> 1]) & 0xffffu);
-          acc[2 * r] += (u64)word * v.x;
-          acc[2 * r + 1] += (u64)word * v.y;
-        }
-      }
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    warp_reduce8(acc, lane);
-    // Lane l holds value x = ((l >> 4) & 1) 4 + ((l >> 3) & 1) 2 + ((l >> 2) & 1): row x / 2,
-    // limb x & 1; a row's high limb sits four lanes above its low limb.
-    const u64 hi = __shfl_down_sync(0xffffffffu, acc[0], 4);
-    const int r = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
-    if ((lane & 7) == 0 && r < rows) fold_out[j0 + r] = reduce128((u128)acc[0] + ((u128)hi << 32));
+          for (int j = 0; j < PER; j++) {
+            const int k = threadIdx.x + j * SCAN_WARPS * 32;
+            if (k >= N) break;
+            const u64 bv = k == 0 ? reduce128(braw[j]) : negq(reduce128(braw[j]));
+            V[(k & 7) * M + (k >> 3)] = make_uint2((u32)bv, (u32)(bv >> 32));
+          }
+        },
+        [&](int r, u128 sum) { fold_out[j0 + r] = reduce128(sum); });
     return;
   }
 
@@ -530,23 +615,46 @@ __global__ void k_wire(const u64* a, const u64* b, u32 n, u32 retained, u32 bits
 
 // encode_database's column split (pir/encode_db.rs:74-168) for one shard: column j, row k
 // holds bytes 2j and 2j+1 of entry k little-endian (one byte when the entry ends there,
-// zero past it), rows past `entries` are zero. Writes the u64 words and their u16 copy.
-__global__ void k_encode_records(const uint8_t* rec, u32 entries, u32 entry_size, u32 n, u32 gamma, u64* cols,
-                                 uint16_t* cols16) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)gamma * n) return;
-  const u32 j = (u32)(idx / n), k = (u32)(idx % n);
-  u32 v = 0;
-  if (k < entries) {
-    const uint8_t* e = rec + (size_t)k * entry_size;
-    const u32 off = 2 * j;
-    if (off + 1 < entry_size)
-      v = (u32)e[off] | ((u32)e[off + 1] << 8);
-    else if (off < entry_size)
-      v = e[off];
+// zero past it), rows past the last entry are zero. Writes the u64 words and their u16 copy.
+//
+// The entries are the rows of a transpose: a CTA takes ENC_ROWS entries by ENC_COLS columns through shared
+// memory, reading along the entries and writing along the columns (a thread a word read its two bytes
+// entry_size apart from its neighbours': 7.1 us a shard alone). Shard blockIdx.z of the launch holds entries
+// n blockIdx.z onward of `rec`.
+constexpr int ENC_ROWS = 64, ENC_COLS = 32;
+__global__ void __launch_bounds__(256) k_encode_records(const uint8_t* rec, u64 total, u32 entry_size, u32 n, u32 gamma,
+                                                        const ShardDev* table) {
+  __shared__ uint16_t tile[ENC_COLS][ENC_ROWS + 2];
+  const ShardDev sh = table[blockIdx.z];
+  u64* cols = const_cast<u64*>(sh.columns);
+  uint16_t* cols16 = const_cast<uint16_t*>(sh.cols16);
+  const u64 first = (u64)blockIdx.z * n;
+  const u32 entries = (u32)min((u64)n, total - first);
+  rec += first * entry_size;
+  const u32 k0 = blockIdx.y * ENC_ROWS, j0 = blockIdx.x * ENC_COLS;
+  // Two-byte loads where every entry starts on a two-byte boundary, single bytes otherwise.
+  const bool pairs = !(entry_size & 1) && !((size_t)rec & 1);
+  for (u32 i = threadIdx.x; i < ENC_ROWS * ENC_COLS; i += 256) {
+    const u32 j = j0 + i % ENC_COLS, k = k0 + i / ENC_COLS, off = 2 * j;
+    u32 v = 0;
+    if (k < entries && off < entry_size) {
+      const uint8_t* e = rec + (size_t)k * entry_size + off;
+      if (pairs)
+        v = *reinterpret_cast<const uint16_t*>(e);
+      else
+        v = off + 1 < entry_size ? (u32)e[0] | ((u32)e[1] << 8) : e[0];
+    }
+    tile[i % ENC_COLS][i / ENC_COLS] = (uint16_t)v;
   }
-  cols[idx] = v;
-  cols16[idx] = (uint16_t)v;
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < ENC_ROWS * ENC_COLS / 2; i += 256) {
+    const u32 j = j0 + i / (ENC_ROWS / 2), k = 2 * (i % (ENC_ROWS / 2));
+    if (j >= gamma) continue;
+    const u32 v = *reinterpret_cast<const u32*>(&tile[i / (ENC_ROWS / 2)][k]);
+    const size_t at = (size_t)j * n + k0 + k;
+    *reinterpret_cast<ulonglong2*>(cols + at) = make_ulonglong2(v & 0xffffu, v >> 16);
+    *reinterpret_cast<u32*>(cols16 + at) = v;
+  }
 }
 
 // Compact copy of a shard's columns: out[k] = w[k] when every word is below 2^16; any
@@ -1183,6 +1291,57 @@ __device__ __forceinline__ void transform_a8(const CrsDev& c, const u64* src, u6
 #pragma unroll
   for (int k = 0; k < 8; k++) a_ntt[k * NT + threadIdx.x] = canon(mulw(x[0][k], c.s_ninv_rinv));
   __syncthreads();
+}
+
+// The column transforms of a store build, several shards a launch (blockIdx.y): H row j is the transform of
+// column j, left lazy (at most 15, the fold takes any word). A CTA stages the ladder once for
+// STORE_ROWS columns; compact columns are read from their u16 copy, and their first stage takes the
+// 32-bit product.
+constexpr int STORE_ROWS = 4;
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8) k_store_ntt(CrsDev c, ShardArg shards, u64* H) {
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
+  extern __shared__ __align__(16) u64 sm[];
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* D = sm + 2 * N;
+  const ShardDev sh = shard_of(shards);
+  for (int k = threadIdx.x; k < N; k += NT) tw[tw8<LOGN>(k)] = c.tw[k];
+  __syncthreads();
+  H += (size_t)blockIdx.y * c.gamma * N;
+#pragma unroll 1
+  for (u32 j = blockIdx.x * STORE_ROWS; j < min(c.gamma, (blockIdx.x + 1) * STORE_ROWS); j++) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int b = threadIdx.x + r * NT;
+      u64 x[4];
+      if (sh.cols16) {
+        u32 w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = sh.cols16[(size_t)j * N + b + k * P];
+        const u64 t2 = mulw_digit(w[2], tw[1]), t3 = mulw_digit(w[3], tw[1]);
+        x[0] = w[0] + t2;
+        x[1] = w[1] + t3;
+        x[2] = w[0] + 3 * Q - t2;
+        x[3] = w[1] + 3 * Q - t3;
+        bf_fwd(x[0], x[1], tw[2]);
+        bf_fwd(x[2], x[3], tw[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = red60(sh.columns[(size_t)j * N + b + k * P]);
+        fwd_unit<false>(x[0], x[1], x[2], x[3], tw[1], tw[2], tw[3]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) D[sw8(b + k * P)] = x[k];
+    }
+    __syncthreads();
+    fwd_middle8<LOGN, 1, 7>(D, tw);
+    u64 x[1][8];
+    fwd_last8<LOGN, 1, fwd_bound8(LOGN, 2, 7)>(x, D, tw);
+    ulonglong2* o = reinterpret_cast<ulonglong2*>(H + (size_t)j * N + 8 * threadIdx.x);
+#pragma unroll
+    for (int k = 0; k < 4; k++) o[k] = make_ulonglong2(x[0][2 * k], x[0][2 * k + 1]);
+    __syncthreads();  // D is rewritten by the next column
+  }
 }
 
 // The recursion's links gamma - 2 .. 0 on thread tid's slots (sums: the store's row 0 at its first slot).
@@ -1941,9 +2100,9 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, 1)
       for (int j = 0; j < 4; j++) {
         u64 ya = 0, yb = 0;
         if (!odd_zero) {
-          const u64 y = c.pow_root_R[(e_tab[l0 + j] * sy) & M2N];
-          ya = mont(ca[j], y);
-          yb = mont(cb[j], y);
+          const Tw y = c.pow_root[(e_tab[l0 + j] * sy) & M2N];
+          ya = canon(mulw(ca[j], y));
+          yb = canon(mulw(cb[j], y));
         }
         s0a[j] = addq(ea[j], ya);
         s0b[j] = addq(eb[j], yb);
@@ -2329,20 +2488,30 @@ cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 sca
   return cudaGetLastError();
 }
 
-cudaError_t store_fold(const CrsDev& c, const u64* H, u64* sums_R, cudaStream_t s) {
+static cudaError_t store_sums(const CrsDev& c, const ShardArg& shards, u32 count, u64* H, cudaStream_t s) {
+  if (count == 0) return cudaSuccess;
   if (c.gamma > (u32)FOLD_TILE || c.gamma == 0 || c.gamma > c.n) return cudaErrorInvalidValue;
   u32 SL = FOLD_TILE / c.gamma;
   if (SL > c.n) SL = c.n;
   if (c.n % SL) return cudaErrorInvalidValue;
-  const u32 blocks = c.n / SL;
-  const size_t smem = (FOLD_TILE + 2 * (size_t)c.n) * 8;
+  const size_t smem_ntt = 3 * (size_t)c.n * 8;
+  const size_t smem_fold = (c.gamma / 2) * sizeof(Tw) + (size_t)SL * (c.gamma + 1) * 8;
   IG_DISPATCH_LOGN(c.logn, {
-    auto k = k_store_fold<L>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kn = k_store_ntt<L>;
+    auto kf = k_store_fold<L>;
+    cudaError_t e = cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ntt);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fold);
     if (e != cudaSuccess) return e;
-    k<<<blocks, FOLD_THREADS, smem, s>>>(c, H, sums_R, SL);
+    kn<<<dim3((c.gamma + STORE_ROWS - 1) / STORE_ROWS, count), (1 << L) / 8, smem_ntt, s>>>(c, shards, H);
+    kf<<<dim3(c.n / SL, count), FOLD_THREADS, smem_fold, s>>>(c, H, shards, SL);
   });
   return cudaGetLastError();
+}
+cudaError_t store_sums(const CrsDev& c, const ShardDev* table, u32 count, u64* H, cudaStream_t s) {
+  return store_sums(c, ShardArg{table, {}}, count, H, s);
+}
+cudaError_t store_sums_one(const CrsDev& c, const ShardDev& shard, u64* H, cudaStream_t s) {
+  return store_sums(c, ShardArg{nullptr, shard}, 1, H, s);
 }
 
 u32 scan_chunks(u32 gamma) { return (gamma + SCAN_COLS - 1) / SCAN_COLS; }
@@ -2363,21 +2532,34 @@ cudaError_t shard_scan(const CrsDev& c, const QueryDev* queries, const ShardDev*
   return cudaGetLastError();
 }
 
-cudaError_t column_tags(const CrsDev& c, const u64* cols, const u64* key, u64* tags_out, const u64* expect,
-                        u32* mismatch, cudaStream_t s) {
-  if (c.gamma == 0) return cudaSuccess;
+cudaError_t tag_keys(const CrsDev& c, const ShardDev* table, u32 count, const u32 (&seed)[8], u64 stream, cudaStream_t s) {
+  if (count == 0) return cudaSuccess;
+  TagSeed t;
+  for (int k = 0; k < 8; k++) t.w[k] = seed[k];
+  k_tag_keys<<<dim3((c.n / 4 + 127) / 128, count), 128, 0, s>>>(c.n, table, t, stream);
+  return cudaGetLastError();
+}
+
+cudaError_t column_tags(const CrsDev& c, const ShardDev* table, u32 count, bool any_wide, u32* mismatch, cudaStream_t s) {
+  if (c.gamma == 0 || count == 0) return cudaSuccess;
   constexpr u32 per_cta = 8;  // warps of 256 threads, one column each
+  const size_t smem = scan_smem_bytes((int)c.n);
   IG_DISPATCH_LOGN(c.logn, {
-    k_column_tags<L><<<(c.gamma + per_cta - 1) / per_cta, per_cta * 32, 0, s>>>(c.gamma, cols, key, tags_out,
-                                                                              expect, mismatch);
+    auto k = k_column_tags16<L>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(scan_chunks(c.gamma), count), SCAN_WARPS * 32, smem, s>>>(c.gamma, table, mismatch);
+    if (any_wide)
+      k_column_tags<L><<<dim3((c.gamma + per_cta - 1) / per_cta, count), per_cta * 32, 0, s>>>(c.gamma, table, mismatch);
   });
   return cudaGetLastError();
 }
 
-cudaError_t encode_records(const uint8_t* rec, u32 entries, u32 entry_size, u32 n, u32 gamma, u64* cols,
-                           uint16_t* cols16, cudaStream_t s) {
-  const size_t words = (size_t)gamma * n;
-  k_encode_records<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(rec, entries, entry_size, n, gamma, cols, cols16);
+cudaError_t encode_records(const uint8_t* rec, u64 entries, u32 entry_size, u32 n, u32 gamma, const ShardDev* table,
+                           u32 count, cudaStream_t s) {
+  if (count == 0) return cudaSuccess;
+  k_encode_records<<<dim3((gamma + ENC_COLS - 1) / ENC_COLS, n / ENC_ROWS, count), 256, 0, s>>>(rec, entries, entry_size, n,
+                                                                                            gamma, table);
   return cudaGetLastError();
 }
 

@@ -26,8 +26,9 @@ struct CrsDev {
   const u32* gpow;           // g^i mod 2n, i < gamma
   const u32* cpow;           // g^-i mod 2n, i < gamma
   const u32* m_of_i;         // (g^-i - 1) / (2n/gamma)
-  const u64* pow_root_R;     // w0^e * 2^64 mod q for e < 2n (w0 = slot 0's root)
-  u64 inv_gamma_R, inv_gamma_Rp;  // gamma^-1 * 2^64 mod q, Shoup
+  const Tw* pow_root;        // w0^e for e < 2n (w0 = slot 0's root)
+  const Tw* zeta;            // zeta^j for j < gamma / 2, zeta = w0^(2n/gamma)
+  Tw inv_gamma_R;            // gamma^-1 * 2^64 mod q
   const u64* wmask_R;        // rows x n: NTT of the kept mask rows, R-form
   // The last exact-gadget digit's factors (D2 = base^-2 (R - D0 - base D1)) in R-form:
   // base^-2, -base^-2 and -base^-1, by which the key rows are folded (fold_gadget3).
@@ -114,15 +115,16 @@ u32 scan_chunks(u32 gamma);
 cudaError_t shard_scan(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u32* work,
                        u32 nwork, u64* b_fold, u32* status, cudaStream_t s);
 
-// Keyed tags of a shard's gamma columns (u64 words, key: 2n words below 2^61 - 1) into
-// tags_out; with `expect` set, *mismatch gets 1 when a tag differs from expect instead.
-cudaError_t column_tags(const CrsDev& c, const u64* cols, const u64* key, u64* tags_out, const u64* expect,
-                        u32* mismatch, cudaStream_t s);
+// Tag keys of `count` shards of a device table (2n words below 2^61 - 1 each) from a 32-byte seed.
+cudaError_t tag_keys(const CrsDev& c, const ShardDev* table, u32 count, const u32 (&seed)[8], u64 stream, cudaStream_t s);
+// Keyed tags of the shards' gamma columns; with `mismatch` set, mismatch[i] gets 1 when a tag of shard i
+// differs from the stored one instead. any_wide: some shard has no u16 copy.
+cudaError_t column_tags(const CrsDev& c, const ShardDev* table, u32 count, bool any_wide, u32* mismatch, cudaStream_t s);
 
-// One shard's columns from its records (entries of entry_size bytes, at most n of them):
-// the gamma x n u64 words and their u16 copy.
-cudaError_t encode_records(const uint8_t* rec, u32 entries, u32 entry_size, u32 n, u32 gamma, u64* cols,
-                           uint16_t* cols16, cudaStream_t s);
+// The columns of `count` shards from their records (`entries` entries of entry_size bytes, n a shard, the last
+// shard's rest zero): the gamma x n u64 words and their u16 copy.
+cudaError_t encode_records(const uint8_t* rec, u64 entries, u32 entry_size, u32 n, u32 gamma, const ShardDev* table,
+                           u32 count, cudaStream_t s);
 
 // ServerResponse bytes of `count` responses into out[len * r ..] from the zero-coefficient
 // template (a: n coefficients at a_off, b: `retained` at b_off, `bits` each).
@@ -134,8 +136,10 @@ cudaError_t wire(const u64* a, const u64* b, u32 count, u32 n, u32 retained, u32
 // 2^16 or above (the copy is then unusable).
 cudaError_t compact16(const u64* cols, size_t words, uint16_t* out, u32* wide, cudaStream_t s);
 
-// Step-1 sums of one shard from the NTTs of its columns (H: gamma x n standard form).
-cudaError_t store_fold(const CrsDev& c, const u64* H, u64* sums_R, cudaStream_t s);
+// Step-1 sums (the packing store) of `count` shards of a device table, or of one shard, from their columns.
+// H: count x gamma x n words of scratch.
+cudaError_t store_sums(const CrsDev& c, const ShardDev* table, u32 count, u64* H, cudaStream_t s);
+cudaError_t store_sums_one(const CrsDev& c, const ShardDev& shard, u64* H, cudaStream_t s);
 
 // Fused per-query respond: expansion of `a`, store gather, backward recursion with the
 // online gather, final transforms, the mod switch to each query's target (QueryDev::ms).

@@ -390,95 +390,130 @@ int sync_crs_self(ig_ctx* c, CrsObj& o) {
   return IG_OK;
 }
 
-int sync_table_entry(ig_ctx* c, DbObj& db, u32 s) {
-  const ShardDev d = db.shards[s].dev();
-  IG_CUDA(c, cudaMemcpyAsync(db.d_table + s, &d, sizeof d, cudaMemcpyHostToDevice, c->stream));
+// Shards of a store build that share a launch: enough column transforms to fill the GPU, their H words
+// (a group's, 32 MB) kept in L2 between the two kernels.
+u32 store_group(const CrsObj& o) { return std::max<u32>(1, (u32)((32u << 20) / ((size_t)o.gamma * o.n * 8))); }
+
+// Shards a launch takes at most (a grid's y and z run to 65,535).
+enum : u32 { LAUNCH_SHARDS = 16384 };
+
+// Writes the table entries of shards [first, first + count) on the context stream.
+int sync_table(ig_ctx* c, DbObj& db, u32 first, u32 count) {
+  std::vector<ShardDev> d(count);
+  for (u32 k = 0; k < count; k++) d[k] = db.shards[first + k].dev();
+  IG_CUDA(c, cudaMemcpyAsync(db.d_table + first, d.data(), count * sizeof(ShardDev), cudaMemcpyHostToDevice, c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
   return IG_OK;
 }
 
-// Folds step 1 over `cols` into `sums` (gamma x n, R-form): gamma forward transforms,
-// then the per-slot DFT fold.
-int fold_store(ig_ctx* c, CrsObj& o, const u64* cols, u64* sums) {
+// Folds step 1 over a shard's columns into its sums (gamma x n, R-form).
+int fold_store(ig_ctx* c, CrsObj& o, const ShardDev& sh) {
   void* H;
   int rc = scratch(c, "fold_H", (size_t)o.gamma * o.n * 8, &H);
   if (rc) return rc;
   long k = prof_begin(c, REGION_FOLD);
   c->launches++;
-  IG_CUDA(c, igk::ntt_rows(o.dev, cols, (u64*)H, o.gamma, 1, c->stream));
-  IG_CUDA(c, igk::store_fold(o.dev, (const u64*)H, sums, c->stream));
+  IG_CUDA(c, igk::store_sums_one(o.dev, sh, (u64*)H, c->stream));
   prof_end(c, k);
   return IG_OK;
 }
 
-int build_store(ig_ctx* c, DbObj& db, CrsObj& o, u32 s) {
-  ShardSlot& sl = db.shards[s];
-  if (!sl.cols)
-    return fail(c, IG_ERR_ARG, "shard %u: no columns uploaded; precompute_packing needs the shard's columns", s);
+// Stores of shards [first, first + count): keyed tags and step-1 sums, one launch sequence a group of shards
+// and one wait at the end. A shard that cannot be built ends the range: those before it are built, the
+// call then fails.
+int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
   const size_t n = o.n, g = o.gamma;
-  if (!sl.sums) {
-    // All three buffers or none: a shard counts as stored when `sums` is set.
-    u64 *sums = nullptr, *key = nullptr, *tags = nullptr;
-    size_t got = 0;
-    int rc = dalloc(c, (void**)&sums, g * n * 8, &got);
-    if (!rc) rc = dalloc(c, (void**)&key, 2 * n * 8, &got);
-    if (!rc) rc = dalloc(c, (void**)&tags, g * 8, &got);
-    if (rc) {
-      if (sums) dfree(c, sums, g * n * 8);
-      if (key) dfree(c, key, 2 * n * 8);
-      return rc;
+  int failed = IG_OK;
+  u32 ready = 0;
+  bool wide = false;
+  for (; ready < count; ready++) {
+    ShardSlot& sl = db.shards[first + ready];
+    if (!sl.cols) {
+      failed = fail(c, IG_ERR_ARG, "shard %u: no columns uploaded; precompute_packing needs the shard's columns",
+                    first + ready);
+      break;
     }
-    db.bytes += got;
-    sl.sums = sums;
-    sl.tag_key = key;
-    sl.tags = tags;
+    if (!sl.sums) {
+      // All three buffers or none: a shard counts as stored when `sums` is set.
+      u64 *sums = nullptr, *key = nullptr, *tags = nullptr;
+      size_t got = 0;
+      failed = dalloc(c, (void**)&sums, g * n * 8, &got);
+      if (!failed) failed = dalloc(c, (void**)&key, 2 * n * 8, &got);
+      if (!failed) failed = dalloc(c, (void**)&tags, g * 8, &got);
+      if (failed) {
+        if (sums) dfree(c, sums, g * n * 8);
+        if (key) dfree(c, key, 2 * n * 8);
+        break;
+      }
+      db.bytes += got;
+      sl.sums = sums;
+      sl.tag_key = key;
+      sl.tags = tags;
+    }
+    wide |= !sl.compact;
   }
-  // Tag key: two words per column word below 2^61 - 1, drawn from OS entropy and never
-  // leaving the device (shard_store.rs:127-135).
-  std::random_device rd;
-  uint8_t seed[32];
-  for (int i = 0; i < 8; i++) {
-    u32 v = rd();
-    memcpy(seed + 4 * i, &v, 4);
+  if (ready) {
+    const u32 group = std::min(ready, store_group(o));
+    void* H;
+    int rc = scratch(c, "fold_H", (size_t)group * g * n * 8, &H);
+    if (rc) return rc;
+    // Tag keys: two words per column word below 2^61 - 1, expanded on the device from OS entropy; they
+    // never leave it (shard_store.rs:127-135).
+    std::random_device rd;
+    u32 seed[8];
+    for (auto& w : seed) w = rd();
+    for (u32 k = 0; k < ready; k++) db.shards[first + k].stale = false;
+    rc = sync_table(c, db, first, ready);
+    if (rc) return rc;
+    const ShardDev* table = db.d_table + first;
+    for (u32 k = 0; k < ready; k += LAUNCH_SHARDS) {
+      const u32 m = std::min<u32>(LAUNCH_SHARDS, ready - k);
+      IG_CUDA(c, igk::tag_keys(o.dev, table + k, m, seed, k, c->stream));
+      IG_CUDA(c, igk::column_tags(o.dev, table + k, m, wide, nullptr, c->stream));
+      c->launches += wide ? 3 : 2;
+    }
+    for (u32 k = 0; k < ready; k += group) {
+      long p = prof_begin(c, REGION_FOLD);
+      c->launches++;
+      IG_CUDA(c, igk::store_sums(o.dev, table + k, std::min(group, ready - k), (u64*)H, c->stream));
+      prof_end(c, p);
+    }
+    IG_CUDA(c, cudaStreamSynchronize(c->stream));
   }
-  HostChaCha rng(seed, 0);
-  std::vector<u64> key(2 * n);
-  for (auto& k : key) {
-    u64 cand;
-    do cand = rng.next_u64() >> 3;
-    while (cand >= (1ULL << 61) - 1);
-    k = cand;
-  }
-  IG_CUDA(c, cudaMemcpyAsync(sl.tag_key, key.data(), key.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  IG_CUDA(c, igk::column_tags(o.dev, sl.cols, sl.tag_key, sl.tags, nullptr, nullptr, c->stream));
-  int rc = fold_store(c, o, sl.cols, sl.sums);
-  if (rc) return rc;
-  c->launches++;
-  IG_CUDA(c, cudaStreamSynchronize(c->stream));
-  sl.stale = false;
-  return sync_table_entry(c, db, s);
+  return failed;
 }
 
-// After new columns land in a shard that holds a store: the columns' tags against the
-// store's (the check shard_store.rs:197-264 makes at every respond, made here once per
-// change, since the library writes every column word itself). A mismatch marks the shard
-// stale; columns equal to the stored ones keep it served.
-int check_store_tags(ig_ctx* c, CrsObj& o, ShardSlot& sl) {
-  if (!sl.sums) {
-    sl.stale = false;
-    return IG_OK;
+// After new columns land in shards [first, first + count), with their table entries written: the columns'
+// tags against the stores' (the check shard_store.rs:197-264 makes at every respond, made here once per
+// change, since the library writes every column word itself). A mismatch marks the shard stale; columns
+// equal to the stored ones keep it served.
+int check_store_tags(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
+  bool stored = false, wide = false, changed = false;
+  for (u32 k = 0; k < count; k++) {
+    stored |= db.shards[first + k].sums != nullptr;
+    wide |= !db.shards[first + k].compact;
   }
-  void* flag;
-  int rc = scratch(c, "tag_mismatch", 4, &flag);
-  if (rc) return rc;
-  IG_CUDA(c, cudaMemsetAsync(flag, 0, 4, c->stream));
-  IG_CUDA(c, igk::column_tags(o.dev, sl.cols, sl.tag_key, nullptr, sl.tags, (u32*)flag, c->stream));
-  c->launches++;
-  u32 mismatch = 1;
-  IG_CUDA(c, cudaMemcpyAsync(&mismatch, flag, 4, cudaMemcpyDeviceToHost, c->stream));
+  std::vector<u32> mismatch(count, 0);
+  if (stored) {
+    void* flags;
+    int rc = scratch(c, "tag_mismatch", count * 4, &flags);
+    if (rc) return rc;
+    IG_CUDA(c, cudaMemsetAsync(flags, 0, count * 4, c->stream));
+    for (u32 k = 0; k < count; k += LAUNCH_SHARDS) {
+      const u32 m = std::min<u32>(LAUNCH_SHARDS, count - k);
+      IG_CUDA(c, igk::column_tags(o.dev, db.d_table + first + k, m, wide, (u32*)flags + k, c->stream));
+      c->launches += wide ? 2 : 1;
+    }
+    IG_CUDA(c, cudaMemcpyAsync(mismatch.data(), flags, count * 4, cudaMemcpyDeviceToHost, c->stream));
+  }
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
-  sl.stale = mismatch != 0;
-  return IG_OK;
+  for (u32 k = 0; k < count; k++) {
+    ShardSlot& sl = db.shards[first + k];
+    const bool stale = sl.sums && mismatch[k];
+    changed |= stale != sl.stale;
+    sl.stale = stale;
+  }
+  return changed ? sync_table(c, db, first, count) : IG_OK;
 }
 
 }  // namespace
@@ -760,12 +795,13 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
     a = a * g % two_n;
     b = b * ginv % two_n;
   }
-  std::vector<u64> pow_root_R(two_n);
+  std::vector<Tw> pow_root(two_n), zeta(std::max<u32>(gamma / 2, 1));
   u64 acc = 1;
   for (u64 e = 0; e < two_n; e++) {
-    pow_root_R[e] = mulmod(acc, R_MOD_Q);
+    pow_root[e] = make_tw(acc);
     acc = mulmod(acc, w0);
   }
+  for (size_t j = 0; j < zeta.size(); j++) zeta[j] = pow_root[j * L];
   // Offline mask rows: ChaCha20(w_seed) on stream 0 (exact) or gamma (approximate),
   // next_u64 mod q, the dropped digits' rows skipped (inspiring2.rs:839-887).
   HostChaCha rng(w_seed, o.approx ? gamma : 0);
@@ -785,7 +821,7 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   if ((rc = upload(c, o, twd, &d.tw)) || (rc = upload(c, o, slot_exp, &d.slot_exp)) ||
       (rc = upload(c, o, exp_slot, &d.exp_slot)) || (rc = upload(c, o, gpow, &d.gpow)) ||
       (rc = upload(c, o, cpow, &d.cpow)) || (rc = upload(c, o, m_of_i, &d.m_of_i)) ||
-      (rc = upload(c, o, pow_root_R, &d.pow_root_R))) {
+      (rc = upload(c, o, pow_root, &d.pow_root)) || (rc = upload(c, o, zeta, &d.zeta))) {
     for (void* p2 : o.allocs) cudaFree(p2);
     c->obj_bytes -= o.bytes;
     return rc;
@@ -795,8 +831,7 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   d.s_ninv_rinv = make_tw(mulmod(ninv, rinv));
   d.s_rinv = make_tw(rinv);
   d.s_n_rinv = make_tw(mulmod(n, rinv));
-  d.inv_gamma_R = mulmod(invmod(gamma), R_MOD_Q);
-  d.inv_gamma_Rp = shoup_companion(d.inv_gamma_R);
+  d.inv_gamma_R = make_tw(mulmod(invmod(gamma), R_MOD_Q));
   // Last exact digit: base^-2 (R - D0 - base D1) (inspiring2.rs:1094-1161). The kernels
   // fold these three factors into the key rows (fold_gadget3) rather than form the digit.
   const u64 inv = invmod(1ULL << 40);
@@ -934,9 +969,9 @@ static int set_shard(ig_ctx* c, uint64_t dbh, uint32_t s, const uint64_t* cols, 
   IG_CUDA(c, cudaMemcpyAsync(&wide_h, wide, 4, cudaMemcpyDeviceToHost, c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
   sl.compact = wide_h == 0;
-  rc = check_store_tags(c, *o, sl);
+  rc = sync_table(c, *db, s, 1);
   if (rc) return rc;
-  return sync_table_entry(c, *db, s);
+  return check_store_tags(c, *db, *o, s, 1);
 }
 
 int ig_db_encode_records(ig_ctx* c, uint64_t dbh, uint32_t first_shard, const uint8_t* records, size_t nbytes,
@@ -961,35 +996,40 @@ int ig_db_encode_records(ig_ctx* c, uint64_t dbh, uint32_t first_shard, const ui
     return fail(c, IG_ERR_ARG,
                 "encode_database: %zu entries fill %zu shards of %u from shard %u; the database holds %u", entries,
                 shards, n, first_shard, db->num_shards);
-  const size_t shard_bytes = (size_t)n * entry_size;
+  // Shards [first, first + count) from `src` (device memory): one launch, one tag check. A shard that
+  // cannot be allocated ends the range: those before it are encoded, the call then fails.
+  auto encode = [&](u32 first, u32 count, const uint8_t* src, size_t n_entries) -> int {
+    int failed = IG_OK;
+    u32 ready = 0;
+    for (; ready < count; ready++) {
+      ShardSlot& sl = db->shards[first + ready];
+      failed = alloc_columns(c, *db, sl, (size_t)g * n * 8);
+      if (failed) break;
+      sl.compact = true;
+    }
+    if (ready) {
+      int rc = sync_table(c, *db, first, ready);
+      if (rc) return rc;
+      for (u32 k = 0; k < ready; k += LAUNCH_SHARDS) {
+        const u32 m = std::min<u32>(LAUNCH_SHARDS, ready - k);
+        const size_t from = (size_t)k * n;
+        IG_CUDA(c, igk::encode_records(src + from * entry_size, std::min<size_t>(n_entries - from, (size_t)m * n),
+                                       entry_size, n, g, db->d_table + first + k, m, c->stream));
+        c->launches++;
+      }
+      rc = check_store_tags(c, *db, o, first, ready);
+      if (rc) return rc;
+    }
+    return failed;
+  };
+  if (on_device) return encode(first_shard, (u32)shards, records, entries);
   void* staging = nullptr;
-  if (!on_device) {
-    int rc = scratch(c, "encode_records", shard_bytes, &staging);
-    if (rc) return rc;
-  }
+  int rc = scratch(c, "encode_records", (size_t)n * entry_size, &staging);
+  if (rc) return rc;
   for (size_t s = 0; s < shards; s++) {
-    ShardSlot& sl = db->shards[first_shard + s];
-    const size_t words = (size_t)g * n;
-    {
-      int rc = alloc_columns(c, *db, sl, words * 8);
-      if (rc) return rc;
-    }
-    const size_t first = s * n;
-    const u32 count = (u32)std::min<size_t>(n, entries - first);
-    const uint8_t* src = records + first * entry_size;
-    if (!on_device) {
-      int rc = stage_h2d(c, staging, src, (size_t)count * entry_size);
-      if (rc) return rc;
-      src = (const uint8_t*)staging;
-    }
-    IG_CUDA(c, igk::encode_records(src, count, entry_size, n, g, sl.cols, sl.cols16, c->stream));
-    c->launches++;
-    sl.compact = true;
-    // The staging buffer is reused by the next shard only after this encode has read it.
-    if (!on_device) IG_CUDA(c, cudaStreamSynchronize(c->stream));
-    int rc = check_store_tags(c, o, sl);
-    if (rc) return rc;
-    rc = sync_table_entry(c, *db, first_shard + (u32)s);
+    const size_t count = std::min<size_t>(n, entries - s * n);
+    rc = stage_h2d(c, staging, records + s * n * entry_size, count * entry_size);
+    if (!rc) rc = encode(first_shard + (u32)s, 1, (const uint8_t*)staging, count);  // waits for the encode
     if (rc) return rc;
   }
   return IG_OK;
@@ -1009,7 +1049,7 @@ int ig_db_precompute_packing(ig_ctx* c, uint64_t dbh, uint32_t s) {
   DbObj* db = get_db(c, dbh);
   if (!db) return fail(c, IG_ERR_HANDLE, "unknown database handle %llu", (unsigned long long)dbh);
   if (s >= db->num_shards) return fail(c, IG_ERR_ARG, "shard %u out of range (%u shards)", s, db->num_shards);
-  return build_store(c, *db, *get_crs(c, db->crs), s);
+  return build_stores(c, *db, *get_crs(c, db->crs), s, 1);
 }
 
 int ig_db_precompute_packing_all(ig_ctx* c, uint64_t dbh) {
@@ -1018,12 +1058,7 @@ int ig_db_precompute_packing_all(ig_ctx* c, uint64_t dbh) {
   cudaSetDevice(c->device);
   DbObj* db = get_db(c, dbh);
   if (!db) return fail(c, IG_ERR_HANDLE, "unknown database handle %llu", (unsigned long long)dbh);
-  CrsObj* o = get_crs(c, db->crs);
-  for (u32 s = 0; s < db->num_shards; s++) {
-    int rc = build_store(c, *db, *o, s);
-    if (rc) return rc;
-  }
-  return IG_OK;
+  return build_stores(c, *db, *get_crs(c, db->crs), 0, db->num_shards);
 }
 
 int ig_db_drop_packing_store(ig_ctx* c, uint64_t dbh, uint32_t s) {
@@ -1046,7 +1081,7 @@ int ig_db_drop_packing_store(ig_ctx* c, uint64_t dbh, uint32_t s) {
     sl.sums = sl.tag_key = sl.tags = nullptr;
   }
   sl.stale = false;
-  return sync_table_entry(c, *db, s);
+  return sync_table(c, *db, s, 1);
 }
 
 int ig_db_has_store(ig_ctx* c, uint64_t dbh, uint32_t s, int* out) {
@@ -1315,9 +1350,9 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
       table[k] = sl.dev();
     } else {
       u64* sums = (u64*)tsums + (size_t)tk++ * g * n;
-      rc = fold_store(c, o, sl.cols, sums);
-      if (rc) return rc;
       table[k] = ShardDev{sl.cols, sums, zkey, nullptr, sl.compact ? sl.cols16 : nullptr};
+      rc = fold_store(c, o, table[k]);
+      if (rc) return rc;
     }
   }
   void *d_table, *d_q, *d_seeds, *d_bs, *d_a, *d_b, *d_fold, *d_status;
