@@ -749,28 +749,6 @@ __device__ __forceinline__ void stage_key_rows(const CrsDev& c, const SetView& v
   K.Y01[to] = make_ulonglong2(canon(mulw(y[0], c.s_rinv)), canon(mulw(y[1], c.s_rinv)));
   K.WY2[to] = make_ulonglong2(canon(mulw(w[2], c.s_rinv)), canon(mulw(y[2], c.s_n_rinv)));
 }
-template <int N, int NT>
-__device__ __forceinline__ void stage_constants(const CrsDev& c, const SetView& v, const u64* yR, Tw* tw,
-                                                const KeyRows& K, uint16_t* e_tab, uint16_t* s_tab) {
-  for (int k = threadIdx.x; k < N; k += NT) {
-    tw[k] = c.tw[k];
-    e_tab[k] = c.slot_exp[k];
-    s_tab[k] = c.exp_slot[k];
-    stage_key_rows(c, v, yR, K, N, k, k);
-  }
-}
-
-// The query's `a` (coefficient form, in place) to n^-1 2^-64 NTT(a): the factor that takes an R-form
-// store word to c_i's scale. Ends with a barrier.
-template <int LOGN, int NT>
-__device__ __forceinline__ void transform_a(const CrsDev& c, u64* a, const Tw* tw) {
-  u64* const bufs[1] = {a};
-  ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
-#pragma unroll
-  for (int k = threadIdx.x; k < (1 << LOGN); k += NT) a[k] = canon(mulw(a[k], c.s_ninv_rinv));
-  __syncthreads();
-}
-
 // The pointwise step of one slot at the gathered position tb: adds sum_k Y_k D_k to sb and returns
 // c_i. d0, d1 at most 15q, cur at most 1+: sb takes at most 31 q^2 < 2^125 a call.
 template <bool EXACT>
@@ -1467,443 +1445,381 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 }
 
 // ------------------------------------------------------------------------------------
-// Split transforms for the two-CTA kernel. The inverse (Gentleman-Sande, from t = 1
-// upward) combines indices within blocks of growing size: its stages 0 .. logn-2 stay
-// inside each half of N/2 words, and only the last stage (t = N/2) mixes the halves. The
-// forward (Cooley-Tukey, from t = N/2 downward) mixes the halves in its first stage only.
-// So each CTA of a pair runs the local stages on the half of the slots it owns, and the
-// two cross stages run once per link, fused with the digit split. Unit and butterfly
-// numbering is the full transform's, so the twiddles are the full transform's.
-
-// The same split holds for R parts of N/R words: the inverse's stages 0 .. logn-1-log R and
-// the forward's stages log R .. logn-1 stay inside a part. The helpers below run a local
-// pass on the part of rank `rank` of a cluster of R CTAs (R = 2 or 4).
-
-// Inverse stages S .. logn-1-log R over this CTA's part xp (N/R words, local index), words up to 2+:
-// radix-4 passes, one unit per thread below N/(4R), then a radix-2 stage when the count is odd
-// (its sums up to 4+). Each pass ends with a barrier.
-template <int LOGN, int R, int S>
-__device__ __forceinline__ void inv_part(u64* xp, int rank, const Tw* tw) {
-  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4, LR = R == 4 ? 2 : 1;
-  const int tid = threadIdx.x;
-  if constexpr (S + 1 <= LOGN - 1 - LR) {
-    constexpr int t = 1 << S, m = N >> (S + 1);
-    if (tid < PU) {
-      const int u = rank * PU + tid;
-      const int B = u >> S, o = u & (t - 1);
-      const int e0 = B * 4 * t + o - rank * P;
-      const int i0 = sw(e0), i1 = sw(e0 + t), i2 = sw(e0 + 2 * t), i3 = sw(e0 + 3 * t);
-      u64 a0 = xp[i0], a1 = xp[i1], a2 = xp[i2], a3 = xp[i3];
-      inv_unit(a0, a1, a2, a3, tw[2 * m - 1 - 2 * B], tw[2 * m - 2 - 2 * B], tw[m - 1 - B]);
-      xp[i0] = a0;
-      xp[i1] = a1;
-      xp[i2] = a2;
-      xp[i3] = a3;
+// A cluster of R = 2 or 4 CTAs per query, for batches that leave SMs idle with one CTA each: a query's
+// recursion spread over R SMs, where the time of a link is its chain of dependent steps.
+//
+// CTA r owns part r, words [r P, (r+1) P), P = N/R, of every NTT-domain vector, two words a thread. The
+// inverse (Gentleman-Sande, from t = 1 upward) stays inside a part for its first log P stages and the forward
+// (Cooley-Tukey, downward) for its last log P; the log R stages between them mix word e of every part.
+// Per link:
+//   1. local inverse: one butterfly a thread and stage. The pair's index bit moves from 0 upward by a
+//      lane exchange (shuffles) for bits 0-5, through shared memory at bit 6, by lane exchanges again. No
+//      thread idles and one barrier is left, where radix-4 passes through shared memory kept half the threads
+//      and a barrier for every two stages (1,650 cycles for nine stages).
+//   2. each word goes to the CTA that crosses its e (CTA e / (P/R)), by a store to its shared memory; cluster
+//      barrier.
+//   3. the cross: the inverse's last log R stages, the digit split, the forward's first log R stages, for
+//      P/R words a CTA and not all P (each CTA computing every cross and keeping its own part took 2,160
+//      cycles); the digits' words go back to their owners by remote stores; cluster barrier.
+//   4. local forward of both digits, the inverse's path backwards, ending with the thread's two slots.
+//   5. the pointwise step. The online sum is off the chain, so its products run in the first cluster
+//      barrier's shadow.
+// Two cluster barriers a link order every buffer's reuse: a CTA rewrites a peer's cross words only after the
+// second barrier of the link before, which the peer reached after reading them, and its digit words only after
+// the first barrier of the next link, which the peer reached after its forward had read them.
+template <int LOGN, int R>
+struct Part {
+  static constexpr int N = 1 << LOGN, LR = R == 4 ? 2 : 1, LP = LOGN - LR, P = 1 << LP, NT = P / 2;
+  static constexpr int K = LP > 6 ? LP - 6 : 0;  // index bits above a warp's 64 words
+  // Word (with bit B zero) that this thread's pair holds while the pair's bit is B.
+  template <int B>
+  static __device__ __forceinline__ int word() {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if constexpr (B < 6) {
+      return (w << 6) | ((l >> B) << (B + 1)) | (l & ((1 << B) - 1));
+    } else {
+      // Lanes' low 6 - K bits and the warp: index bits 0-5; the lanes' high bits: the bits above 6.
+      const int hi = l >> (6 - K), q = B - 6;
+      return (l & ((1 << (6 - K)) - 1)) | (w << (6 - K)) | ((((hi >> q) << (q + 1)) | (hi & ((1 << q) - 1))) << 6);
     }
-    __syncthreads();
-    inv_part<LOGN, R, S + 2>(xp, rank, tw);
-  } else if constexpr (S == LOGN - 1 - LR) {
-    constexpr int t = 1 << S, m = N >> (S + 1);
-    for (int v0 = tid; v0 < P / 2; v0 += blockDim.x) {
-      const int v = rank * (P / 2) + v0;
-      const int B = v >> S, o = v & (t - 1);
-      const int e = sw(B * 2 * t + o - rank * P), f = sw(B * 2 * t + o - rank * P + t);
-      u64 a = xp[e], b = xp[f];
-      bf_inv<3>(a, b, tw[2 * m - 1 - B]);
-      xp[e] = a;
-      xp[f] = b;
-    }
-    __syncthreads();
   }
+  // Lane mask of the exchange between pair bits B and B + 1.
+  static __device__ __forceinline__ constexpr int mask(int B) { return B < 6 ? 1 << B : 1 << (6 - K + B - 6); }
+  // Shared-memory positions without bank conflicts: the bits above 6 (7 for the exchange at bit 6) that a
+  // half-warp's lanes carry go into the low bits they leave free.
+  static __device__ __forceinline__ int swt(int e) { return K >= 3 ? e ^ (((e >> 7) & 3) << (6 - K)) : e; }
+  static __device__ __forceinline__ int swd(int e) { return K >= 3 ? e ^ (((e >> 6) & 3) << (6 - K)) : e; }
+};
+
+// Twiddles of a thread's local butterflies by pair bit. They are the same in every link: four CTAs keep them
+// in registers, two (512 threads, 128 registers each) read them from the ladder in shared memory.
+template <int LOGN, int R>
+struct PartTw {
+  using G = Part<LOGN, R>;
+  static constexpr bool REG = R == 4;
+  const Tw* tw;
+  int base;
+  Tw fi[REG ? G::LP : 1], ff[REG ? G::LP : 1];
+  template <int B>
+  __device__ __forceinline__ Tw load(bool inverse) const {
+    constexpr int M = G::N >> (B + 1);
+    const int i = (base + G::template word<B>()) >> (B + 1);
+    return tw[inverse ? 2 * M - 1 - i : M + i];
+  }
+  template <int B>
+  __device__ __forceinline__ void fill() {
+    if constexpr (REG && B < G::LP) {
+      fi[B] = load<B>(true);
+      ff[B] = load<B>(false);
+      fill<B + 1>();
+    }
+  }
+  template <int B>
+  __device__ __forceinline__ Tw inv() const {
+    if constexpr (REG)
+      return fi[B];
+    else
+      return load<B>(true);
+  }
+  template <int B>
+  __device__ __forceinline__ Tw fwd() const {
+    if constexpr (REG)
+      return ff[B];
+    else
+      return load<B>(false);
+  }
+};
+
+// The pair's bit and lane bit `mask` change places.
+__device__ __forceinline__ void lane_exchange(u64& x0, u64& x1, int mask) {
+  const bool up = threadIdx.x & mask;
+  const u64 got = __shfl_xor_sync(0xffffffffu, up ? x0 : x1, mask);
+  x0 = up ? got : x0;
+  x1 = up ? x1 : got;
 }
 
-// Forward stages S .. END-1 (S >= log R) over this CTA's part of two buffers D[0..P) and D[P..2P),
-// P = N/R, words up to BIN in and fwd_bound out: a radix-2 stage first when the count is odd, then
-// radix-4 passes, one unit per thread below N/(2R). Each pass ends with a barrier.
-template <int LOGN, int R, int S, int END, int BIN>
-__device__ __forceinline__ void fwd_part(u64* D, int rank, const Tw* tw) {
-  constexpr int N = 1 << LOGN, P = N / R, PU = P / 4;
-  const int tid = threadIdx.x;
-  if constexpr (S < END && ((END - S) & 1)) {
-    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S;
-    for (int v0 = tid; v0 < P / 2; v0 += blockDim.x) {
-      const int v = rank * (P / 2) + v0;
-      const int i = v >> lt, o = v & (t - 1);
-      const int e = sw(i * 2 * t + o - rank * P), f = sw(i * 2 * t + o - rank * P + t);
-      const Tw w = tw[m + i];
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        u64* x = D + k * P;
-        u64 a = x[e], b = x[f];
-        bf_fwd(a, b, w);
-        x[e] = a;
-        x[f] = b;
+// Local inverse stages B .. log P - 1 on words up to W (2 out). T: P words of scratch.
+template <int LOGN, int R, int B, int W>
+__device__ __forceinline__ void part_inverse(u64& x0, u64& x1, u64* T, const PartTw<LOGN, R>& tw) {
+  using G = Part<LOGN, R>;
+  if constexpr (B < G::LP) {
+    bf_inv<W + 1>(x0, x1, tw.template inv<B>());
+    // Sums double, products are 2+; the last stage leaves at most 2+.
+    constexpr bool RED = 2 * W >= 8 || (B == G::LP - 1 && W > 1);
+    if (RED) x0 = red60(x0);
+    if constexpr (B + 1 < G::LP) {
+      if constexpr (B == 5) {
+        const int e = G::template word<5>(), f = G::template word<6>();
+        T[G::swt(e)] = x0;
+        T[G::swt(e | 32)] = x1;
+        __syncthreads();
+        x0 = T[G::swt(f)];
+        x1 = T[G::swt(f | 64)];
+      } else {
+        lane_exchange(x0, x1, G::mask(B));
       }
+      part_inverse<LOGN, R, B + 1, (RED || W < 1 ? 2 : 2 * W)>(x0, x1, T, tw);
     }
-    __syncthreads();
-    fwd_part<LOGN, R, S + 1, END, BIN + 3>(D, rank, tw);
-  } else if constexpr (S < END) {
-    constexpr bool RED = BIN > FWD_FREE;
-    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S, h = t >> 1;
-    if (tid < 2 * PU) {
-      u64* x = D + (tid >= PU ? P : 0);
-      const int u = rank * PU + (tid & (PU - 1));
-      const int i = u >> (lt - 1), o = u & (h - 1);
-      const int e0 = i * 2 * t + o - rank * P;
-      const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + t), i3 = sw(e0 + t + h);
-      u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
-      fwd_unit<RED>(a0, a1, a2, a3, tw[m + i], tw[2 * m + 2 * i], tw[2 * m + 2 * i + 1]);
-      x[i0] = a0;
-      x[i1] = a1;
-      x[i2] = a2;
-      x[i3] = a3;
-    }
-    __syncthreads();
-    fwd_part<LOGN, R, S + 2, END, (RED ? 1 : BIN) + 6>(D, rank, tw);
   }
 }
 
-// ------------------------------------------------------------------------------------
-// Two CTAs per query (a thread-block cluster), for batches that leave SMs idle with one
-// CTA each. CTA r owns slots [r N/2, (r+1) N/2) of every NTT-domain vector. Per link:
-//   own half of R_{i+1} -> local inverse stages -> cluster barrier -> cross stage over
-//   (own half, peer's half read through distributed shared memory), n^-1, digit split and
-//   the forward cross stage, keeping this CTA's half of digits 0 and 1 -> local forward
-//   stages -> pointwise at own slots.
-// Thread pair (2u, 2u+1) owns local slots 4u..4u+3, two each: the first inverse pass
-// (stages 0 and 1, one 4-slot unit) and the last forward pass (same units, one digit per
-// lane) run in registers with one lane exchange, next to the pointwise link.
-// One cluster barrier per link: the exchange buffer X alternates between two halves by
-// link parity, so a CTA rewrites the half its peer read at link i only at link i-2, after
-// both passed the barrier of link i-1. With the exact gadget the third digit's transform
-// comes from the other two: D_2 = base^-2 (R_{i+1} - D_0 - base D_1)
-// (inspiring2.rs:1094-1161).
+// Local forward stages of both digits from pair bit B down to 0, words up to W; at most 15 out. T: 2P words.
+template <int LOGN, int R, int B, int W>
+__device__ __forceinline__ void part_forward(u64 (&x)[2][2], u64* T, const PartTw<LOGN, R>& tw) {
+  using G = Part<LOGN, R>;
+  constexpr bool RED = W > 12;
+  const Tw w = tw.template fwd<B>();
+#pragma unroll
+  for (int n = 0; n < 2; n++) {
+    if (RED) x[n][0] = red60(x[n][0]);
+    bf_fwd(x[n][0], x[n][1], w);
+  }
+  if constexpr (B > 0) {
+    if constexpr (B == 6) {
+      const int e = G::template word<6>(), f = G::template word<5>();
+#pragma unroll
+      for (int n = 0; n < 2; n++) {
+        T[n * G::P + G::swt(e)] = x[n][0];
+        T[n * G::P + G::swt(e | 64)] = x[n][1];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int n = 0; n < 2; n++) {
+        x[n][0] = T[n * G::P + G::swt(f)];
+        x[n][1] = T[n * G::P + G::swt(f | 32)];
+      }
+    } else {
+#pragma unroll
+      for (int n = 0; n < 2; n++) lane_exchange(x[n][0], x[n][1], G::mask(B - 1));
+    }
+    part_forward<LOGN, R, B - 1, (RED ? 1 : W) + 3>(x, T, tw);
+  }
+}
+
+// The inverse's last log R stages on word e of the R parts (words up to 2+): canonical coefficients.
+template <int R>
+__device__ __forceinline__ void cross_inverse(const u64 (&x)[R], u64 (&cf)[R], const Tw& w1, const Tw& w2, const Tw& w3) {
+  if constexpr (R == 2) {
+    cf[0] = canon(x[0] + x[1]);
+    cf[1] = canon(mulw(x[1] - x[0] + 3 * Q, w1));
+  } else {
+    u64 a0 = x[0], a1 = x[1], a2 = x[2], a3 = x[3];
+    bf_inv<3>(a0, a1, w3);
+    bf_inv<3>(a2, a3, w2);
+    cf[0] = canon(a0 + a2);
+    cf[1] = canon(a1 + a3);
+    cf[2] = canon(mulw(a2 - a0 + 5 * Q, w1));
+    cf[3] = canon(mulw(a3 - a1 + 3 * Q, w1));
+  }
+}
+
+// The forward's first log R stages on one digit of the R coefficients: at most 3 log R.
+template <int R>
+__device__ __forceinline__ void cross_forward(const u32 (&g)[R], u64 (&y)[R], const Tw& w1, const Tw& w2, const Tw& w3) {
+#pragma unroll
+  for (int k = 0; k < R / 2; k++) {
+    const u64 t = mulw_digit(g[k + R / 2], w1);
+    y[k] = g[k] + t;
+    y[k + R / 2] = g[k] + 3 * Q - t;
+  }
+  if constexpr (R == 4) {
+    bf_fwd(y[0], y[1], w2);
+    bf_fwd(y[2], y[3], w3);
+  }
+}
+
+// Position of slot t's gathered operands: a warp's lanes (slots 2 l + k) gather from distinct banks, as slot8
+// arranges for units of eight.
 template <int LOGN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((1 << LOGN) / 4, 1)
-    k_respond_pair(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out,
-                   u64* b_out, u32* status, int force_serial) {
+__device__ __forceinline__ int slot2(int t) {
+  return ((t & 1) << (LOGN - 1)) | (t >> 1);
+}
+
+template <int LOGN, int R>
+__global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
+    k_respond_cluster(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out,
+                      u64* b_out, u32* status, int force_serial) {
   namespace cg = cooperative_groups;
-  constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2, HU = N / 8;
+  using G = Part<LOGN, R>;
+  constexpr int N = G::N, P = G::P, NT = G::NT, LP = G::LP, C = P / R;  // C cross words a CTA
   constexpr u32 M2N = 2 * N - 1;
   extern __shared__ __align__(16) u64 sm[];
-  u64* X = sm;      // [2][H] own half of the inverse, by link parity
-  u64* D = sm + N;  // [2][H] own half of the transformed digits 0 and 1; N words at the end
-  u64* a_ntt = D + N;
+  u64* XB = sm;           // [R][C] the parts' words that this CTA crosses
+  u64* D = XB + P;        // [2][P] this part of digits 0 and 1
+  u64* T = D + 2 * P;     // [P] the local inverse's exchange, then [2][P] the forward's
+  u64* a_ntt = T + 3 * P;
   Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
   ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
-  const KeyRows K{rows, rows + N, rows + 2 * N};
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
-  uint16_t* s_tab = e_tab + N;
+  const KeyRows KR{rows, rows + N, rows + 2 * N};
+  uint16_t* s_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);  // position of the slot of exponent 2e + 1
 
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const u64* peerX = cluster.map_shared_rank(X, rank ^ 1);
-  const int tid = threadIdx.x;
-  const QueryDev qd = queries[blockIdx.x >> 1];
+  const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
+  u64* peer[R];
+#pragma unroll
+  for (int k = 0; k < R; k++) peer[k] = cluster.map_shared_rank(sm, k);
+  const QueryDev qd = queries[blockIdx.x / R];
   const u32 qi = qd.row;  // output and status row
   const ShardDev sh = shards[qd.shard];
   const SetView ps = set_view(c, qd.crs);
   const u32 gamma = ps.gamma;
-  const bool exact = ps.approx == 0;
-  const int own = rank * H, other = (rank ^ 1) * H;
-  const int u = tid >> 1, dg = tid & 1;
-  const int ls = 4 * u + 2 * dg;  // local slots ls, ls + 1
-  const int ug = rank * HU + u;   // global unit index of slots 4u..4u+3
 
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
-  expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  transform_a<LOGN, NT>(c, a_ntt, tw);
+  for (int k = tid; k < N; k += NT) {
+    tw[k] = c.tw[k];
+    s_tab[k] = (uint16_t)slot2<LOGN>(c.exp_slot[k]);
+    stage_key_rows(c, ps, qd.seat_R, KR, N, k, slot2<LOGN>(k));
+  }
+  // The query's a: expanded and transformed in the exchange buffers' place, kept at its slots' positions.
+  static_assert(6 * P >= N, "a fits the buffers");
+  expand_a<N, NT>(qd, sm, status, qi, force_serial);  // ends with a barrier
+  {
+    u64* const bufs[1] = {sm};
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
+  }
+  for (int k = tid; k < N; k += NT) a_ntt[slot2<LOGN>(k)] = canon(mulw(sm[k], c.s_ninv_rinv));
+  PartTw<LOGN, R> ptw;
+  ptw.tw = tw;
+  ptw.base = rank * P;
+  ptw.template fill<0>();
+  const int l0 = rank * P + 2 * tid;  // this thread's slots: l0, l0 + 1
+  const u32 et[2] = {c.slot_exp[l0], c.slot_exp[l0 + 1]};
+  __syncthreads();
   u64 cur[2];
   Acc sb[2];
-  u32 et[2];
-#pragma unroll
-  for (int k = 0; k < 2; k++) et[k] = e_tab[own + ls + k];
   {
     const u32 gp = ps.gpow[gamma - 1];
-    const u64* Srow = sh.sums_R + (size_t)(gamma - 1) * N;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = mulq(a_ntt[tb], Srow[own + ls + k]);
+      cur[k] = mulq(a_ntt[s_tab[((gp * et[k]) & M2N) >> 1]], sh.sums_R[(size_t)(gamma - 1) * N + l0 + k]);
       sb[k] = Acc{0, 0, 0, 0};
     }
   }
-  // Twiddles of the register passes: inverse stages 0-1 of unit ug, forward stages
-  // logn-2, logn-1 of unit ug (fixed per thread).
-  const Tw wl1 = tw[N - 1 - (2 * ug + dg)], wl2 = tw[H - 1 - ug];
-  constexpr int MF = 1 << (LOGN - 2);
-  const Tw fa = tw[MF + ug], fb = tw[2 * MF + 2 * ug], fc = tw[2 * MF + 2 * ug + 1];
-  const Tw wf = tw[1];
-  // One instance of the links a gadget: the choice stays out of the slots' straight-line code.
+  const Tw w1 = tw[1], w2 = R == 4 ? tw[2] : w1, w3 = R == 4 ? tw[3] : w1;
+  // This thread's cross word and, with four CTAs, its digit.
+  const int q = tid & (C - 1), dg = tid / C;
+  cluster.sync();  // every CTA is past its use of the exchange buffers
+
+  // The thread's pair of words to the CTAs that cross them (the pair's bit is log P - 1).
+  auto push = [&](u64 x0, u64 x1) {
+    const int e = G::template word<LP - 1>();
+    const int at = rank * C + (e & (C - 1));
+    if constexpr (R == 2) {
+      peer[0][at] = x0;
+      peer[1][at] = x1;
+    } else {
+      const bool up = e >= C;
+      (up ? peer[1] : peer[0])[at] = x0;
+      (up ? peer[3] : peer[2])[at] = x1;
+    }
+  };
   auto links = [&](auto gadget) {
     constexpr bool EXACT = decltype(gadget)::value;
-#pragma unroll 1
-  for (int i = (int)gamma - 2; i >= 0; i--) {
-    const u64* Srow = sh.sums_R + (size_t)i * N;
-    const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(Srow + own + ls);
-    const u32 gp = ps.gpow[i];
-    const int par = (i & 1) * H;
-    u64* xh = X + par;
-    {
-      // Inverse stages 0-1 of unit ug: lane dg holds slots 4u + 2dg, +1.
-      u64 p = cur[0], q = cur[1];
-      bf_inv<3>(p, q, wl1);
-      const u64 recv = __shfl_xor_sync(0xffffffffu, dg == 0 ? q : p, 1);
-      u64 x0 = dg == 0 ? p : recv, x1 = dg == 0 ? recv : q;  // (slot 4u, 4u+2) or (4u+1, 4u+3)
-      bf_inv<3>(x0, x1, wl2);
-      xh[sw(4 * u + dg)] = red60(x0);
-      xh[sw(4 * u + dg + 2)] = x1;
-    }
-    __syncthreads();
-    inv_part<LOGN, 2, 2>(xh, rank, tw);
-    cluster.sync();
-    {
-      // Elements [0, H) of the inverse live in rank 0's X, elements [H, N) in rank 1's.
-      const u64* lo = (rank == 0 ? (const u64*)X : peerX) + par;
-      const u64* hi = (rank == 0 ? peerX : (const u64*)X) + par;
+    // The online sum's operands of the link before.
+    u64 pd0[2] = {0, 0}, pd1[2] = {0, 0}, pc[2] = {0, 0};
+    u32 pt[2] = {0, 0};
+    auto online = [&](int i) {
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int b = tid + j * NT;
-        const u64 x0 = lo[sw(b)], x1 = hi[sw(b)];
-        u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + H
-        split_digits<EXACT>(canon(x0 + x1), p0, p1);
-        split_digits<EXACT>(canon(mulw(x1 - x0 + 5 * Q, wf)), q0, q1);
-        // Forward cross stage: slot b gets p + w q, slot b + H gets p - w q.
-        const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
-        D[sw(b)] = rank == 0 ? p0 + t0 : p0 + 3 * Q - t0;
-        D[H + sw(b)] = rank == 0 ? p1 + t1 : p1 + 3 * Q - t1;
+      for (int k = 0; k < 2; k++) {
+        const ulonglong2 y = KR.Y01[pt[k]];
+        mac(sb[k], pd0[k], y.x);
+        mac(sb[k], pd1[k], y.y);
+        if constexpr (EXACT) mac(sb[k], pc[k], KR.WY2[pt[k]].y);
+        if (i % SB_FOLD_LINKS == 0) sb[k] = acc_from(acc_fold(sb[k]));
+      }
+    };
+#pragma unroll 1
+    for (int i = (int)gamma - 2; i >= 0; i--) {
+      const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(sh.sums_R + (size_t)i * N + l0);
+      const u32 gp = ps.gpow[i];
+      {
+        u64 x0 = cur[0], x1 = cur[1];
+        part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
+        push(x0, x1);
+      }
+      cluster.barrier_arrive();
+      online(i);
+      cluster.barrier_wait();
+      {
+        u64 x[R], cf[R], y[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) x[k] = XB[k * C + q];
+        cross_inverse<R>(x, cf, w1, w2, w3);
+        u32 g[2][R];
+#pragma unroll
+        for (int k = 0; k < R; k++) split_digits<EXACT>(cf[k], g[0][k], g[1][k]);
+        const int at = G::swd(rank * C + q);
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+          u32 h[R];
+          if constexpr (R == 4) {
+            if (n) break;  // one digit a thread
+#pragma unroll
+            for (int k = 0; k < R; k++) h[k] = dg ? g[1][k] : g[0][k];
+          } else {
+#pragma unroll
+            for (int k = 0; k < R; k++) h[k] = g[n][k];
+          }
+          cross_forward<R>(h, y, w1, w2, w3);
+          const int to = P + (R == 4 ? dg : n) * P + at;
+#pragma unroll
+          for (int k = 0; k < R; k++) peer[k][to] = y[k];
+        }
+      }
+      cluster.sync();
+      u64 d[2][2];
+      {
+        const int e = G::template word<LP - 1>();
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+          d[n][0] = D[n * P + G::swd(e)];
+          d[n][1] = D[n * P + G::swd(e | (P / 2))];
+        }
+        part_forward<LOGN, R, LP - 1, 3 * G::LR>(d, T + P, ptw);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
+        const ulonglong2 w = KR.W01[tb];
+        Acc r{0, 0, 0, 0};
+        mac(r, a_ntt[tb], k ? sv.y : sv.x);
+        if constexpr (EXACT) mac(r, cur[k], KR.WY2[tb].x);
+        mac(r, d[0][k], w.x);
+        mac(r, d[1][k], w.y);
+        pd0[k] = d[0][k];
+        pd1[k] = d[1][k];
+        pc[k] = cur[k];
+        pt[k] = tb;
+        cur[k] = acc_fold(r);
       }
     }
-    __syncthreads();
-    fwd_part<LOGN, 2, 1, LOGN - 2, 3>(D, rank, tw);
-    // Forward stages logn-2, logn-1 of unit ug for digit dg, then each lane takes the other
-    // digit at its own two slots from its partner.
-    u64 d0[2], d1[2];
-    {
-      const u64* x = D + dg * H;
-      const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(x + sw(4 * u));
-      const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(x + sw(4 * u + 2));
-      u64 a0 = v01.x, a1 = v01.y, a2 = v23.x, a3 = v23.y;
-      fwd_unit<(fwd_bound(LOGN, 1, 3) > FWD_FREE)>(a0, a1, a2, a3, fa, fb, fc);
-      const u64 g0 = __shfl_xor_sync(0xffffffffu, dg == 0 ? a2 : a0, 1);
-      const u64 g1 = __shfl_xor_sync(0xffffffffu, dg == 0 ? a3 : a1, 1);
-      const u64 m0 = dg == 0 ? a0 : a2, m1 = dg == 0 ? a1 : a3;
-      d0[0] = dg == 0 ? m0 : g0;
-      d0[1] = dg == 0 ? m1 : g1;
-      d1[0] = dg == 0 ? g0 : m0;
-      d1[1] = dg == 0 ? g1 : m1;
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-      cur[k] = link_slot<EXACT>(sb[k], d0[k], d1[k], cur[k], k == 0 ? sv.x : sv.y, a_ntt, K, tb);
-    }
-    if (i % SB_FOLD_LINKS == 0) {
-#pragma unroll
-      for (int k = 0; k < 2; k++) sb[k] = acc_from(acc_fold(sb[k]));
-    }
-  }
+    online(0);
   };
-  if (exact)
+  if (ps.approx == 0)
     links(std::true_type{});
   else
     links(std::false_type{});
-  // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each
-  // from its own half and the peer's half (exchanged through the half of X that link 0
-  // did not use; the peer read it last at link 1, before the barrier of link 0).
-  __syncthreads();  // every lane is past its last read of D
-  u64* xf = X + H;
-  const u64* pf = peerX + H;
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const u64 sum = acc_fold(sb[k]);
-    xf[ls + k] = rank == 0 ? sum : cur[k];
-    D[own + ls + k] = rank == 0 ? cur[k] : sum;
-  }
-  cluster.sync();
-#pragma unroll
-  for (int k = 0; k < 2; k++) D[other + tid + k * NT] = pf[tid + k * NT];
-  cluster.sync();  // each CTA's X stays alive until its peer has read it
-  {
-    u64* const bufs[1] = {D};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int t = tid + k * NT;
-    if (rank == 0)
-      a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
-    else
-      b_out[(size_t)qi * N + t] = finish_b(c, D[t], t, gamma, b_fold + qd.fold_off, qd.ms);
-  }
-}
-
-// ------------------------------------------------------------------------------------
-// Four CTAs per query (a cluster of 4), for small batches whose latency sets the tail: a
-// query's recursion spread over four SMs. CTA r owns quarter r, slots [r N/4, (r+1) N/4), of
-// every NTT-domain vector, two slots per thread (N/8 threads: the quarter-local passes keep
-// half of them busy or all, where N/4 threads left three quarters or half idle at every
-// barrier). The inverse's stages 0 .. logn-3 and the
-// forward's stages 2 .. logn-1 stay inside a quarter (the part helpers above); the two
-// stages on each side that mix quarters combine the four elements b, b + N/4, b + N/2,
-// b + 3N/4 of each b < N/4, so they run as one radix-4 cross pass per link: thread b reads
-// its four elements (three through distributed shared memory), takes the inverse's last two
-// stages with n^-1 folded into the last (n^-1 on the sum, n^-1 times the stage's twiddle on
-// the difference), splits the four coefficients into digits and runs the forward's first
-// two stages, of which it keeps its own quarter's output (three products a digit). One
-// cluster barrier per link: the inverse's exchange buffer alternates between two quarters
-// by link parity, so a CTA rewrites what its peers read at link i only at link i-2, after
-// all passed the barrier of link i-1. With the exact gadget the third digit's transform
-// comes from the other two (inspiring2.rs:1094-1161), folded into the key rows as in
-// k_respond.
-template <int LOGN>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 1)
-    k_respond_quad(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out,
-                   u64* b_out, u32* status, int force_serial) {
-  namespace cg = cooperative_groups;
-  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4, SPT = P / NT;  // two slots a thread
-  constexpr u32 M2N = 2 * N - 1;
-  extern __shared__ __align__(16) u64 sm[];
-  u64* X = sm;          // [2][P] own quarter of the inverse, by link parity
-  u64* D = sm + 2 * P;  // [2][P] own quarter of digits 0 and 1; N words for the last transform
-  u64* a_ntt = D + N;
-  Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
-  ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
-  const KeyRows K{rows, rows + N, rows + 2 * N};
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);
-  uint16_t* s_tab = e_tab + N;
-
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const u64* peer[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) peer[k] = cluster.map_shared_rank(X, k);
-  const int tid = threadIdx.x;
-  const QueryDev qd = queries[blockIdx.x >> 2];
-  const u32 qi = qd.row;  // output and status row
-  const ShardDev sh = shards[qd.shard];
-  const SetView ps = set_view(c, qd.crs);
-  const u32 gamma = ps.gamma;
-  const bool exact = ps.approx == 0;
-  // This thread's slots: rank P + tid + j NT, j < SPT.
-
-  stage_constants<N, NT>(c, ps, qd.seat_R, tw, K, e_tab, s_tab);
-  expand_a<N, NT>(qd, a_ntt, status, qi, force_serial);
-  transform_a<LOGN, NT>(c, a_ntt, tw);
-  u32 et[SPT];
-  u64 cur[SPT];
-  Acc sb[SPT];
-#pragma unroll
-  for (int j = 0; j < SPT; j++) {
-    const int slot = rank * P + tid + j * NT;
-    et[j] = e_tab[slot];
-    const u32 gp = ps.gpow[gamma - 1];
-    const u32 tb = s_tab[((gp * et[j]) & M2N) >> 1];
-    cur[j] = mulq(a_ntt[tb], sh.sums_R[(size_t)(gamma - 1) * N + slot]);
-    sb[j] = Acc{0, 0, 0, 0};
-  }
-  // Twiddles of the cross pass: stage logn-2 of the inverse takes the mirrored entries 3 and 2, its
-  // last stage and stage 0 of the forward entry 1, stage 1 entry 2 for the first half, 3 for the second.
-  const Tw w1 = tw[1], w2 = tw[2], w3 = tw[3];
-  const Tw wfs = tw[2 + (rank >> 1)];
-  // One instance of the links a gadget: the choice stays out of the slots' straight-line code.
-  auto links = [&](auto gadget) {
-    constexpr bool EXACT = decltype(gadget)::value;
+  // Final inverse transforms of c_0 (to a) and of the online sum (to b): local stages, then the cross.
 #pragma unroll 1
-  for (int i = (int)gamma - 2; i >= 0; i--) {
-    u64 sv[SPT];
-#pragma unroll
-    for (int j = 0; j < SPT; j++) sv[j] = sh.sums_R[(size_t)i * N + rank * P + tid + j * NT];
-    const u32 gp = ps.gpow[i];
-    const int par = (i & 1) * P;
-    u64* xq = X + par;
-#pragma unroll
-    for (int j = 0; j < SPT; j++) xq[sw(tid + j * NT)] = cur[j];
-    __syncthreads();
-    inv_part<LOGN, 4, 0>(xq, rank, tw);
+  for (int n = 0; n < 2; n++) {
+    u64 x0 = n ? acc_fold(sb[0]) : cur[0], x1 = n ? acc_fold(sb[1]) : cur[1];
+    part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
+    push(x0, x1);
     cluster.sync();
+    u64 x[R], cf[R];
 #pragma unroll
-    for (int j = 0; j < SPT; j++) {
-      const int b = tid + j * NT;
-      u64 x0 = peer[0][par + sw(b)], x1 = peer[1][par + sw(b)];
-      u64 x2 = peer[2][par + sw(b)], x3 = peer[3][par + sw(b)];
-      bf_inv<5>(x0, x1, w3);  // (b, b + N/4), block 0 of stage logn-2: sums up to 8+
-      bf_inv<5>(x2, x3, w2);  // (b + N/2, b + 3N/4), block 1
-      x0 = red60(x0);
-      x2 = red60(x2);
-      u64 cf[4];  // coefficients b, b + N/4, b + N/2, b + 3N/4
-      cf[0] = canon(x0 + x2);
-      cf[2] = canon(mulw(x2 - x0 + 3 * Q, w1));
-      cf[1] = canon(x1 + x3);
-      cf[3] = canon(mulw(x3 - x1 + 3 * Q, w1));
-      u32 g0[4], g1[4];  // digits 0 and 1
+    for (int k = 0; k < R; k++) x[k] = XB[k * C + q];
+    if (n == 0) cluster.sync();  // the words are read before the next are pushed
+    // Unscaled residues: finish_a takes the coefficient as it is, finish_b times n^-1.
+    cross_inverse<R>(x, cf, w1, w2, w3);
+    if (dg) continue;
 #pragma unroll
-      for (int k = 0; k < 4; k++) split_digits<EXACT>(cf[k], g0[k], g1[k]);
-      // Forward stage 0 (b with b + N/2, b + N/4 with b + 3N/4), then stage 1 on this
-      // quarter's half, of which output rank & 1 is the quarter's word, at most 6.
-      auto fwd = [&](const u32(&g)[4]) -> u64 {
-        const u64 t2 = mulw_digit(g[2], w1), t3 = mulw_digit(g[3], w1);
-        u64 lo, hi;
-        if (rank < 2) {
-          lo = g[0] + t2;
-          hi = g[1] + t3;
-        } else {
-          lo = g[0] + 3 * Q - t2;
-          hi = g[1] + 3 * Q - t3;
-        }
-        const u64 t = mulw(hi, wfs);
-        return (rank & 1) ? lo - t + 3 * Q : lo + t;
-      };
-      D[sw(b)] = fwd(g0);
-      D[P + sw(b)] = fwd(g1);
+    for (int k = 0; k < R; k++) {
+      const int t = k * P + rank * C + q;
+      if (n == 0)
+        a_out[(size_t)qi * N + t] = finish_a(cf[k], qd.ms);
+      else
+        b_out[(size_t)qi * N + t] = finish_b(c, cf[k], t, gamma, b_fold + qd.fold_off, qd.ms);
     }
-    __syncthreads();
-    fwd_part<LOGN, 4, 2, LOGN, 6>(D, rank, tw);
-#pragma unroll
-    for (int j = 0; j < SPT; j++) {
-      const u64 d0 = D[sw(tid + j * NT)], d1 = D[P + sw(tid + j * NT)];
-      const u32 tb = s_tab[((gp * et[j]) & M2N) >> 1];
-      cur[j] = link_slot<EXACT>(sb[j], d0, d1, cur[j], sv[j], a_ntt, K, tb);
-    }
-    if (i % SB_FOLD_LINKS == 0) {
-#pragma unroll
-      for (int j = 0; j < SPT; j++) sb[j] = acc_from(acc_fold(sb[j]));
-    }
-  }
-  };
-  if (exact)
-    links(std::true_type{});
-  else
-    links(std::false_type{});
-  // Final transforms: rank 0 assembles R_0 (-> a), rank 1 the online sum (-> b), each from
-  // the four quarters exchanged through X once every peer is past its last cross-pass read.
-  cluster.sync();
-#pragma unroll
-  for (int j = 0; j < SPT; j++) {
-    X[tid + j * NT] = cur[j];
-    X[P + tid + j * NT] = acc_fold(sb[j]);
-  }
-  cluster.sync();
-  if (rank < 2) {
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int j = 0; j < SPT; j++) D[k * P + tid + j * NT] = peer[k][rank * P + tid + j * NT];
-  }
-  cluster.sync();  // each CTA's X stays alive until ranks 0 and 1 have read it
-  if (rank >= 2) return;
-  __syncthreads();
-  {
-    u64* const bufs[1] = {D};
-    ntt_inv_r4<LOGN, NT, 1>(bufs, tw);
-  }
-#pragma unroll
-  for (int k = 0; k < N / NT; k++) {
-    const int t = tid + k * NT;
-    if (rank == 0)
-      a_out[(size_t)qi * N + t] = finish_a(D[t], qd.ms);
-    else
-      b_out[(size_t)qi * N + t] = finish_b(c, D[t], t, gamma, b_fold + qd.fold_off, qd.ms);
   }
 }
 
@@ -2672,10 +2588,11 @@ cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s) {
 }
 
 size_t respond_smem_bytes(const CrsDev& c, int ctas) {
-  // X, D and a_ntt, the two ladders, three key rows of W and Y, two u16 slot tables.
+  // Transform buffers (2n words, or six parts of n / ctas), a_ntt and the ladder, three key rows of W and Y, the
+  // u16 slot table.
   const size_t n = c.n;
-  const size_t words = ctas == 4 ? n / 2 + 4 * n : 5 * n;
-  return (words + 2 * (size_t)3 * n) * 8 + 2 * n * 2;
+  const size_t words = (ctas == 1 ? 2 * n : 6 * n / ctas) + 3 * n + 6 * n;
+  return words * 8 + n * 2;
 }
 
 cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq,
@@ -2685,16 +2602,23 @@ cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* sh
   if (ctas != 1 && ctas != 2 && ctas != 4) return cudaErrorInvalidValue;
   const size_t smem = respond_smem_bytes(c, ctas);
   IG_DISPATCH_LOGN(c.logn, {
-    if (ctas == 4) {
-      auto k = k_respond_quad<L>;
+    if (ctas > 1) {
+      auto k = ctas == 4 ? k_respond_cluster<L, 4> : k_respond_cluster<L, 2>;
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      k<<<4 * nq, (1 << L) / 8, smem, s>>>(c, queries, shards, b_fold, a_out, b_out, status, force_serial_expand);
-    } else if (ctas == 2) {
-      auto k = k_respond_pair<L>;
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaLaunchAttribute cluster{};
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      cluster.val.clusterDim.x = (unsigned)ctas;
+      cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(ctas * nq);
+      cfg.blockDim = dim3((1u << L) / ctas / 2);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = s;
+      cfg.attrs = &cluster;
+      cfg.numAttrs = 1;
+      e = cudaLaunchKernelEx(&cfg, k, c, queries, shards, b_fold, a_out, b_out, status, force_serial_expand);
       if (e != cudaSuccess) return e;
-      k<<<2 * nq, (1 << L) / 4, smem, s>>>(c, queries, shards, b_fold, a_out, b_out, status, force_serial_expand);
     } else {
       auto k = k_respond<L>;
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
