@@ -1456,17 +1456,17 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 //      lane exchange (shuffles) for bits 0-5, through shared memory at bit 6, by lane exchanges again. No
 //      thread idles and one barrier is left, where radix-4 passes through shared memory kept half the threads
 //      and a barrier for every two stages (1,650 cycles for nine stages).
-//   2. each word goes to the CTA that crosses its e (CTA e / (P/R)), by a store to its shared memory; cluster
-//      barrier.
+//   2. each word goes to the CTA that crosses its e (CTA e / (P/R)), by an asynchronous store to its shared
+//      memory that counts on an mbarrier there.
 //   3. the cross: the inverse's last log R stages, the digit split, the forward's first log R stages, for
 //      P/R words a CTA and not all P (each CTA computing every cross and keeping its own part took 2,160
-//      cycles); the digits' words go back to their owners by remote stores; cluster barrier.
+//      cycles); the digits' words go back to their owners the same way.
 //   4. local forward of both digits, the inverse's path backwards, ending with the thread's two slots.
-//   5. the pointwise step. The online sum is off the chain, so its products run in the first cluster
-//      barrier's shadow.
-// Two cluster barriers a link order every buffer's reuse: a CTA rewrites a peer's cross words only after the
-// second barrier of the link before, which the peer reached after reading them, and its digit words only after
-// the first barrier of the next link, which the peer reached after its forward had read them.
+//   5. the pointwise step. The online sum is off the chain, so its products run while the cross words travel.
+// The data's own arrivals order every buffer's reuse. A CTA sends a link's cross words after its forward of the
+// link before, which took digits from every peer, and a peer sends those after reading its cross words; it sends
+// digits after taking cross words from every peer, and a peer's threads send those after reading their
+// digits of the link before.
 template <int LOGN, int R>
 struct Part {
   static constexpr int N = 1 << LOGN, LR = R == 4 ? 2 : 1, LP = LOGN - LR, P = 1 << LP, NT = P / 2;
@@ -1635,6 +1635,42 @@ __device__ __forceinline__ int slot2(int t) {
   return ((t & 1) << (LOGN - 1)) | (t >> 1);
 }
 
+// Words between the CTAs of a cluster: st.async stores a word in a CTA's shared memory and counts its bytes
+// on an mbarrier there, so a receiver waits for its data alone. A cluster barrier's release made every
+// thread wait until its remote stores had landed and its loads were back (1,400 cycles of a 6,480-cycle
+// link, twice).
+__device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ u32 cluster_addr(u32 addr, int rank) {
+  u32 a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void send_word(u32 to, u64 v, u32 bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to), "l"(v), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void inbox_init(u32 bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// One thread opens a phase of `bytes`; every thread waits for its end.
+__device__ __forceinline__ void inbox_expect(u32 bar, u32 bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase of the given parity, a bounded number of tries (each suspends the thread up to a
+// hardware time limit); false when they ran out.
+constexpr int INBOX_TRIES = 1 << 20;
+__device__ __forceinline__ bool inbox_wait(u32 bar, u32 parity) {
+  for (int k = 0; k < INBOX_TRIES; k++) {
+    u32 done;
+    asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 template <int LOGN, int R>
 __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
     k_respond_cluster(CrsDev c, const QueryDev* queries, const ShardDev* shards, const u64* b_fold, u64* a_out,
@@ -1653,11 +1689,24 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   const KeyRows KR{rows, rows + N, rows + 2 * N};
   uint16_t* s_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);  // position of the slot of exponent 2e + 1
 
+  __shared__ __align__(8) u64 inbox[2];  // arrivals of cross words and of digit words
+
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
-  u64* peer[R];
+  // Shared memory of the R CTAs (their buffers, then their inboxes).
+  const u32 in_words = smem_addr(&inbox[0]), in_digits = smem_addr(&inbox[1]);
+  u32 peer[R], peer_words[R], peer_digits[R];
 #pragma unroll
-  for (int k = 0; k < R; k++) peer[k] = cluster.map_shared_rank(sm, k);
+  for (int k = 0; k < R; k++) {
+    peer[k] = cluster_addr(smem_addr(sm), k);
+    peer_words[k] = cluster_addr(in_words, k);
+    peer_digits[k] = cluster_addr(in_digits, k);
+  }
+  if (tid == 0) {
+    inbox_init(in_words);
+    inbox_init(in_digits);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   const QueryDev qd = queries[blockIdx.x / R];
   const u32 qi = qd.row;  // output and status row
   const ShardDev sh = shards[qd.shard];
@@ -1702,14 +1751,23 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   // The thread's pair of words to the CTAs that cross them (the pair's bit is log P - 1).
   auto push = [&](u64 x0, u64 x1) {
     const int e = G::template word<LP - 1>();
-    const int at = rank * C + (e & (C - 1));
+    const u32 at = 8 * (rank * C + (e & (C - 1)));
     if constexpr (R == 2) {
-      peer[0][at] = x0;
-      peer[1][at] = x1;
+      send_word(peer[0] + at, x0, peer_words[0]);
+      send_word(peer[1] + at, x1, peer_words[1]);
     } else {
       const bool up = e >= C;
-      (up ? peer[1] : peer[0])[at] = x0;
-      (up ? peer[3] : peer[2])[at] = x1;
+      send_word((up ? peer[1] : peer[0]) + at, x0, up ? peer_words[1] : peer_words[0]);
+      send_word((up ? peer[3] : peer[2]) + at, x1, up ? peer_words[3] : peer_words[2]);
+    }
+  };
+  // A wait that runs out marks the query failed; the links then run on without waiting, to their end.
+  bool alive = true;
+  u32 parity = 0;  // of the next phase of either inbox
+  auto await = [&](u32 bar) {
+    if (alive && !inbox_wait(bar, parity)) {
+      alive = false;
+      atomicOr(status + qi, (u32)DEV_PEER_TIMEOUT);
     }
   };
   auto links = [&](auto gadget) {
@@ -1731,14 +1789,17 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
     for (int i = (int)gamma - 2; i >= 0; i--) {
       const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(sh.sums_R + (size_t)i * N + l0);
       const u32 gp = ps.gpow[i];
+      if (tid == 0 && alive) {
+        inbox_expect(in_words, P * 8);
+        inbox_expect(in_digits, 2 * P * 8);
+      }
       {
         u64 x0 = cur[0], x1 = cur[1];
         part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
         push(x0, x1);
       }
-      cluster.barrier_arrive();
       online(i);
-      cluster.barrier_wait();
+      await(in_words);
       {
         u64 x[R], cf[R], y[R];
 #pragma unroll
@@ -1760,12 +1821,13 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
             for (int k = 0; k < R; k++) h[k] = g[n][k];
           }
           cross_forward<R>(h, y, w1, w2, w3);
-          const int to = P + (R == 4 ? dg : n) * P + at;
+          const u32 to = 8 * (P + (R == 4 ? dg : n) * P + at);
 #pragma unroll
-          for (int k = 0; k < R; k++) peer[k][to] = y[k];
+          for (int k = 0; k < R; k++) send_word(peer[k] + to, y[k], peer_digits[k]);
         }
       }
-      cluster.sync();
+      await(in_digits);
+      parity ^= 1;
       u64 d[2][2];
       {
         const int e = G::template word<LP - 1>();
@@ -1802,13 +1864,15 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
 #pragma unroll 1
   for (int n = 0; n < 2; n++) {
     u64 x0 = n ? acc_fold(sb[0]) : cur[0], x1 = n ? acc_fold(sb[1]) : cur[1];
+    if (tid == 0 && alive) inbox_expect(in_words, P * 8);
     part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
     push(x0, x1);
-    cluster.sync();
+    await(in_words);
+    parity ^= 1;
     u64 x[R], cf[R];
 #pragma unroll
     for (int k = 0; k < R; k++) x[k] = XB[k * C + q];
-    if (n == 0) cluster.sync();  // the words are read before the next are pushed
+    cluster.sync();  // the words are read before the next are pushed, and before a CTA ends
     // Unscaled residues: finish_a takes the coefficient as it is, finish_b times n^-1.
     cross_inverse<R>(x, cf, w1, w2, w3);
     if (dg) continue;

@@ -11,7 +11,8 @@ namespace ig {
 enum DeviceStatus : u32 {
   DEV_OK = 0,
   DEV_TAG_MISMATCH = 1,     // a column is not the column the store was built from
-  DEV_EXPAND_EXHAUSTED = 2  // query `a` expansion ran past its candidate budget
+  DEV_EXPAND_EXHAUSTED = 2,  // query `a` expansion ran past its candidate budget
+  DEV_PEER_TIMEOUT = 4       // a CTA of the query's cluster waited too long for its peers' words
 };
 
 // Per parameter-set constants, resident in device memory.
