@@ -1452,16 +1452,18 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 // inverse (Gentleman-Sande, from t = 1 upward) stays inside a part for its first log P stages and the forward
 // (Cooley-Tukey, downward) for its last log P; the log R stages between them mix word e of every part.
 // Per link:
-//   1. local inverse: one butterfly a thread and stage. The pair's index bit moves from 0 upward by a
-//      lane exchange (shuffles) for bits 0-5, through shared memory at bit 6, by lane exchanges again. No
-//      thread idles and one barrier is left, where radix-4 passes through shared memory kept half the threads
-//      and a barrier for every two stages (1,650 cycles for nine stages).
+//   1. local inverse: stage 0 on the thread's own pair, then radix-4 units through shared memory on half the
+//      threads (one unit a thread, its two stages in registers). Units on bits 1-6 stay within the 128
+//      words of a warp, so a warp barrier between them is enough; bits 7 and up take a CTA barrier. (One
+//      butterfly a thread with lane exchanges keeps every thread busy, but its selects cost the ALU
+//      port half as much again as the products: 1,300 cycles for nine stages.)
 //   2. each word goes to the CTA that crosses its e (CTA e / (P/R)), by an asynchronous store to its shared
 //      memory that counts on an mbarrier there.
 //   3. the cross: the inverse's last log R stages, the digit split, the forward's first log R stages, for
 //      P/R words a CTA and not all P (each CTA computing every cross and keeping its own part took 2,160
 //      cycles); the digits' words go back to their owners the same way.
-//   4. local forward of both digits, the inverse's path backwards, ending with the thread's two slots.
+//   4. local forward of both digits, the inverse's passes backwards with a unit of one digit a thread, ending with
+//      both digits of the thread's own pair.
 //   5. the pointwise step. The online sum is off the chain, so its products run while the cross words travel.
 // The data's own arrivals order every buffer's reuse. A CTA sends a link's cross words after its forward of the
 // link before, which took digits from every peer, and a peer sends those after reading its cross words; it sends
@@ -1470,129 +1472,92 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 template <int LOGN, int R>
 struct Part {
   static constexpr int N = 1 << LOGN, LR = R == 4 ? 2 : 1, LP = LOGN - LR, P = 1 << LP, NT = P / 2;
-  static constexpr int K = LP > 6 ? LP - 6 : 0;  // index bits above a warp's 64 words
-  // Word (with bit B zero) that this thread's pair holds while the pair's bit is B.
-  template <int B>
-  static __device__ __forceinline__ int word() {
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if constexpr (B < 6) {
-      return (w << 6) | ((l >> B) << (B + 1)) | (l & ((1 << B) - 1));
-    } else {
-      // Lanes' low 6 - K bits and the warp: index bits 0-5; the lanes' high bits: the bits above 6.
-      const int hi = l >> (6 - K), q = B - 6;
-      return (l & ((1 << (6 - K)) - 1)) | (w << (6 - K)) | ((((hi >> q) << (q + 1)) | (hi & ((1 << q) - 1))) << 6);
-    }
-  }
-  // Lane mask of the exchange between pair bits B and B + 1.
-  static __device__ __forceinline__ constexpr int mask(int B) { return B < 6 ? 1 << B : 1 << (6 - K + B - 6); }
-  // Shared-memory positions without bank conflicts: the bits above 6 (7 for the exchange at bit 6) that a
-  // half-warp's lanes carry go into the low bits they leave free.
-  static __device__ __forceinline__ int swt(int e) { return K >= 3 ? e ^ (((e >> 7) & 3) << (6 - K)) : e; }
-  static __device__ __forceinline__ int swd(int e) { return K >= 3 ? e ^ (((e >> 6) & 3) << (6 - K)) : e; }
+  static constexpr int C = P / R;  // words whose cross a CTA computes
+  // The part's words in shared memory: every pass's accesses are free of bank conflicts.
+  static __device__ __forceinline__ int sw(int e) { return e ^ (((e >> 4) & 3) << 1) ^ (((e >> 5) & 1) << 3); }
+  // First word of unit u of a pass on `n` index bits from bit b (word k of the unit: + k 2^b).
+  static __device__ __forceinline__ int unit(int u, int b, int n) { return ((u >> b) << (b + n)) | (u & ((1 << b) - 1)); }
+  static __host__ __device__ constexpr int bits(int b) { return b + 1 < LP ? 2 : 1; }  // of the pass from bit b (odd)
 };
 
-// Twiddles of a thread's local butterflies by pair bit. They are the same in every link: four CTAs keep them
-// in registers, two (512 threads, 128 registers each) read them from the ladder in shared memory.
-template <int LOGN, int R>
-struct PartTw {
-  using G = Part<LOGN, R>;
-  static constexpr bool REG = R == 4;
-  const Tw* tw;
-  int base;
-  Tw fi[REG ? G::LP : 1], ff[REG ? G::LP : 1];
-  template <int B>
-  __device__ __forceinline__ Tw load(bool inverse) const {
-    constexpr int M = G::N >> (B + 1);
-    const int i = (base + G::template word<B>()) >> (B + 1);
-    return tw[inverse ? 2 * M - 1 - i : M + i];
-  }
-  template <int B>
-  __device__ __forceinline__ void fill() {
-    if constexpr (REG && B < G::LP) {
-      fi[B] = load<B>(true);
-      ff[B] = load<B>(false);
-      fill<B + 1>();
-    }
-  }
-  template <int B>
-  __device__ __forceinline__ Tw inv() const {
-    if constexpr (REG)
-      return fi[B];
-    else
-      return load<B>(true);
-  }
-  template <int B>
-  __device__ __forceinline__ Tw fwd() const {
-    if constexpr (REG)
-      return ff[B];
-    else
-      return load<B>(false);
-  }
-};
-
-// The pair's bit and lane bit `mask` change places.
-__device__ __forceinline__ void lane_exchange(u64& x0, u64& x1, int mask) {
-  const bool up = threadIdx.x & mask;
-  const u64 got = __shfl_xor_sync(0xffffffffu, up ? x0 : x1, mask);
-  x0 = up ? got : x0;
-  x1 = up ? x1 : got;
-}
-
-// Local inverse stages B .. log P - 1 on words up to W (2 out). T: P words of scratch.
-template <int LOGN, int R, int B, int W>
-__device__ __forceinline__ void part_inverse(u64& x0, u64& x1, u64* T, const PartTw<LOGN, R>& tw) {
+// Local inverse stages from bit B up, on the part's words X (2+ in and out); put(e, word) takes the last
+// pass's words instead of X. `base`: the part's first index.
+template <int LOGN, int R, int B, class Put>
+__device__ __forceinline__ void part_inverse(u64* X, int base, const Tw* tw, Put put) {
   using G = Part<LOGN, R>;
   if constexpr (B < G::LP) {
-    bf_inv<W + 1>(x0, x1, tw.template inv<B>());
-    // Sums double, products are 2+; the last stage leaves at most 2+.
-    constexpr bool RED = 2 * W >= 8 || (B == G::LP - 1 && W > 1);
-    if (RED) x0 = red60(x0);
-    if constexpr (B + 1 < G::LP) {
-      if constexpr (B == 5) {
-        const int e = G::template word<5>(), f = G::template word<6>();
-        T[G::swt(e)] = x0;
-        T[G::swt(e | 32)] = x1;
-        __syncthreads();
-        x0 = T[G::swt(f)];
-        x1 = T[G::swt(f | 64)];
+    constexpr int n = G::bits(B), t = 1 << B, M = G::N >> (B + 1);
+    constexpr bool last = B + n == G::LP;
+    if ((int)threadIdx.x < (G::P >> n)) {
+      const int e = G::unit(threadIdx.x, B, n), i = (base + e) >> (B + 1);
+      u64 x[1 << n];
+#pragma unroll
+      for (int k = 0; k < 1 << n; k++) x[k] = X[G::sw(e + k * t)];
+      if constexpr (n == 2) {
+        inv_unit(x[0], x[1], x[2], x[3], tw[2 * M - 1 - i], tw[2 * M - 2 - i], tw[M - 1 - (i >> 1)]);
       } else {
-        lane_exchange(x0, x1, G::mask(B));
+        bf_inv<3>(x[0], x[1], tw[2 * M - 1 - i]);
+        x[0] = red60(x[0]);
       }
-      part_inverse<LOGN, R, B + 1, (RED || W < 1 ? 2 : 2 * W)>(x0, x1, T, tw);
+#pragma unroll
+      for (int k = 0; k < 1 << n; k++) {
+        if constexpr (last)
+          put(e + k * t, k, x[k]);
+        else
+          X[G::sw(e + k * t)] = x[k];
+      }
     }
+    if constexpr (!last) {
+      if constexpr (B + n >= 7)
+        __syncthreads();
+      else
+        __syncwarp();
+    }
+    part_inverse<LOGN, R, B + n>(X, base, tw, put);
   }
 }
 
-// Local forward stages of both digits from pair bit B down to 0, words up to W; at most 15 out. T: 2P words.
+// Local forward stages from the pass at bit B down to bit 1, both digits in place (D[0..P), D[P..2P)), words
+// up to W in and part_bound out. Ends with a CTA barrier.
+__host__ __device__ constexpr int part_bound(int lp, int b, int w) {
+  for (; b >= 1; b -= 2) w = b + 1 < lp ? (w > FWD_FREE ? 1 : w) + 6 : (w > 12 ? 1 : w) + 3;
+  return w;
+}
 template <int LOGN, int R, int B, int W>
-__device__ __forceinline__ void part_forward(u64 (&x)[2][2], u64* T, const PartTw<LOGN, R>& tw) {
+__device__ __forceinline__ void part_forward(u64* D, int base, const Tw* tw) {
   using G = Part<LOGN, R>;
-  constexpr bool RED = W > 12;
-  const Tw w = tw.template fwd<B>();
+  if constexpr (B >= 1) {
+    constexpr int n = G::bits(B), t = 1 << B, m = G::N >> (B + n);
+    constexpr bool RED = n == 2 ? W > FWD_FREE : W > 12;
+    if constexpr (n == 2) {  // a unit of one digit a thread
+      const int u = threadIdx.x & (G::P / 4 - 1);
+      u64* x = D + ((int)threadIdx.x < G::P / 4 ? 0 : G::P);
+      const int e = G::unit(u, B, 2), i = (base + e) >> (B + 2);
+      const int i0 = G::sw(e), i1 = G::sw(e + t), i2 = G::sw(e + 2 * t), i3 = G::sw(e + 3 * t);
+      u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
+      fwd_unit<RED>(a0, a1, a2, a3, tw[m + i], tw[2 * m + 2 * i], tw[2 * m + 2 * i + 1]);
+      x[i0] = a0;
+      x[i1] = a1;
+      x[i2] = a2;
+      x[i3] = a3;
+    } else {  // a pair of each digit a thread
+      const int e = G::unit(threadIdx.x, B, 1), i0 = G::sw(e), i1 = G::sw(e + t);
+      const Tw w = tw[m + ((base + e) >> (B + 1))];
 #pragma unroll
-  for (int n = 0; n < 2; n++) {
-    if (RED) x[n][0] = red60(x[n][0]);
-    bf_fwd(x[n][0], x[n][1], w);
-  }
-  if constexpr (B > 0) {
-    if constexpr (B == 6) {
-      const int e = G::template word<6>(), f = G::template word<5>();
-#pragma unroll
-      for (int n = 0; n < 2; n++) {
-        T[n * G::P + G::swt(e)] = x[n][0];
-        T[n * G::P + G::swt(e | 64)] = x[n][1];
+      for (int d = 0; d < 2; d++) {
+        u64* x = D + d * G::P;
+        u64 a = x[i0], c = x[i1];
+        if (RED) a = red60(a);
+        bf_fwd(a, c, w);
+        x[i0] = a;
+        x[i1] = c;
       }
-      __syncthreads();
-#pragma unroll
-      for (int n = 0; n < 2; n++) {
-        x[n][0] = T[n * G::P + G::swt(f)];
-        x[n][1] = T[n * G::P + G::swt(f | 32)];
-      }
-    } else {
-#pragma unroll
-      for (int n = 0; n < 2; n++) lane_exchange(x[n][0], x[n][1], G::mask(B - 1));
     }
-    part_forward<LOGN, R, B - 1, (RED ? 1 : W) + 3>(x, T, tw);
+    if constexpr (B >= 7 || B == 1)
+      __syncthreads();
+    else
+      __syncwarp();
+    part_forward<LOGN, R, B - 2, (RED ? 1 : W) + 3 * n>(D, base, tw);
   }
 }
 
@@ -1677,13 +1642,14 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
                       u64* b_out, u32* status, int force_serial) {
   namespace cg = cooperative_groups;
   using G = Part<LOGN, R>;
-  constexpr int N = G::N, P = G::P, NT = G::NT, LP = G::LP, C = P / R;  // C cross words a CTA
+  constexpr int N = G::N, P = G::P, NT = G::NT, LP = G::LP, C = G::C;
+  constexpr int TOP = LP & 1 ? LP - 2 : LP - 1;  // bit of the forward's first local pass
   constexpr u32 M2N = 2 * N - 1;
   extern __shared__ __align__(16) u64 sm[];
   u64* XB = sm;           // [R][C] the parts' words that this CTA crosses
   u64* D = XB + P;        // [2][P] this part of digits 0 and 1
-  u64* T = D + 2 * P;     // [P] the local inverse's exchange, then [2][P] the forward's
-  u64* a_ntt = T + 3 * P;
+  u64* X = D + 2 * P;     // [P] the local inverse
+  u64* a_ntt = X + P;
   Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
   ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
   const KeyRows KR{rows, rows + N, rows + 2 * N};
@@ -1719,18 +1685,14 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
     stage_key_rows(c, ps, qd.seat_R, KR, N, k, slot2<LOGN>(k));
   }
   // The query's a: expanded and transformed in the exchange buffers' place, kept at its slots' positions.
-  static_assert(6 * P >= N, "a fits the buffers");
+  static_assert(4 * P >= N, "a fits the buffers");
   expand_a<N, NT>(qd, sm, status, qi, force_serial);  // ends with a barrier
   {
     u64* const bufs[1] = {sm};
     ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
   for (int k = tid; k < N; k += NT) a_ntt[slot2<LOGN>(k)] = canon(mulw(sm[k], c.s_ninv_rinv));
-  PartTw<LOGN, R> ptw;
-  ptw.tw = tw;
-  ptw.base = rank * P;
-  ptw.template fill<0>();
-  const int l0 = rank * P + 2 * tid;  // this thread's slots: l0, l0 + 1
+  const int base = rank * P, l0 = base + 2 * tid;  // this thread's slots: l0, l0 + 1
   const u32 et[2] = {c.slot_exp[l0], c.slot_exp[l0 + 1]};
   __syncthreads();
   u64 cur[2];
@@ -1748,18 +1710,21 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   const int q = tid & (C - 1), dg = tid / C;
   cluster.sync();  // every CTA is past its use of the exchange buffers
 
-  // The thread's pair of words to the CTAs that cross them (the pair's bit is log P - 1).
-  auto push = [&](u64 x0, u64 x1) {
-    const int e = G::template word<LP - 1>();
-    const u32 at = 8 * (rank * C + (e & (C - 1)));
-    if constexpr (R == 2) {
-      send_word(peer[0] + at, x0, peer_words[0]);
-      send_word(peer[1] + at, x1, peer_words[1]);
-    } else {
-      const bool up = e >= C;
-      send_word((up ? peer[1] : peer[0]) + at, x0, up ? peer_words[1] : peer_words[0]);
-      send_word((up ? peer[3] : peer[2]) + at, x1, up ? peer_words[3] : peer_words[2]);
-    }
+  // Twiddles of the thread's own pair: stage 0 of the inverse, the last of the forward.
+  const Tw wi0 = tw[N - 1 - (l0 >> 1)], wf0 = tw[N / 2 + (l0 >> 1)];
+  // The thread's pair through the local inverse, its words to the CTAs that cross them.
+  auto inverse_to_cross = [&](u64 x0, u64 x1) {
+    bf_inv<2>(x0, x1, wi0);
+    *reinterpret_cast<ulonglong2*>(X + G::sw(2 * tid)) = make_ulonglong2(x0, x1);
+    __syncthreads();
+    part_inverse<LOGN, R, 1>(X, base, tw, [&](int e, int k, u64 x) {
+      const u32 at = 8 * (rank * C + (e & (C - 1)));
+      if constexpr (G::bits(LP & 1 ? LP - 2 : LP - 1) == G::LR) {  // the pass holds the bits of the crossing CTA
+        send_word(peer[k] + at, x, peer_words[k]);
+      } else {
+        send_word(cluster_addr(smem_addr(sm) + at, e / C), x, cluster_addr(in_words, e / C));
+      }
+    });
   };
   // A wait that runs out marks the query failed; the links then run on without waiting, to their end.
   bool alive = true;
@@ -1793,11 +1758,7 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
         inbox_expect(in_words, P * 8);
         inbox_expect(in_digits, 2 * P * 8);
       }
-      {
-        u64 x0 = cur[0], x1 = cur[1];
-        part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
-        push(x0, x1);
-      }
+      inverse_to_cross(cur[0], cur[1]);
       online(i);
       await(in_words);
       {
@@ -1808,7 +1769,7 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
         u32 g[2][R];
 #pragma unroll
         for (int k = 0; k < R; k++) split_digits<EXACT>(cf[k], g[0][k], g[1][k]);
-        const int at = G::swd(rank * C + q);
+        const int at = G::sw(rank * C + q);
 #pragma unroll
         for (int n = 0; n < 2; n++) {
           u32 h[R];
@@ -1828,15 +1789,14 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
       }
       await(in_digits);
       parity ^= 1;
+      part_forward<LOGN, R, TOP, 3 * G::LR>(D, base, tw);
       u64 d[2][2];
-      {
-        const int e = G::template word<LP - 1>();
 #pragma unroll
-        for (int n = 0; n < 2; n++) {
-          d[n][0] = D[n * P + G::swd(e)];
-          d[n][1] = D[n * P + G::swd(e | (P / 2))];
-        }
-        part_forward<LOGN, R, LP - 1, 3 * G::LR>(d, T + P, ptw);
+      for (int n = 0; n < 2; n++) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(D + n * P + G::sw(2 * tid));
+        d[n][0] = part_bound(LP, TOP, 3 * G::LR) > 12 ? red60(v.x) : v.x;
+        d[n][1] = v.y;
+        bf_fwd(d[n][0], d[n][1], wf0);
       }
 #pragma unroll
       for (int k = 0; k < 2; k++) {
@@ -1863,10 +1823,8 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   // Final inverse transforms of c_0 (to a) and of the online sum (to b): local stages, then the cross.
 #pragma unroll 1
   for (int n = 0; n < 2; n++) {
-    u64 x0 = n ? acc_fold(sb[0]) : cur[0], x1 = n ? acc_fold(sb[1]) : cur[1];
     if (tid == 0 && alive) inbox_expect(in_words, P * 8);
-    part_inverse<LOGN, R, 0, 1>(x0, x1, T, ptw);
-    push(x0, x1);
+    inverse_to_cross(n ? acc_fold(sb[0]) : cur[0], n ? acc_fold(sb[1]) : cur[1]);
     await(in_words);
     parity ^= 1;
     u64 x[R], cf[R];
@@ -2652,10 +2610,10 @@ cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s) {
 }
 
 size_t respond_smem_bytes(const CrsDev& c, int ctas) {
-  // Transform buffers (2n words, or six parts of n / ctas), a_ntt and the ladder, three key rows of W and Y, the
+  // Transform buffers (2n words, or four parts of n / ctas), a_ntt and the ladder, three key rows of W and Y, the
   // u16 slot table.
   const size_t n = c.n;
-  const size_t words = (ctas == 1 ? 2 * n : 6 * n / ctas) + 3 * n + 6 * n;
+  const size_t words = (ctas == 1 ? 2 * n : 4 * n / ctas) + 3 * n + 6 * n;
   return words * 8 + n * 2;
 }
 
