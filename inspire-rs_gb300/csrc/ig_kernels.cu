@@ -832,15 +832,6 @@ __device__ __forceinline__ u64 finish_b(const CrsDev& c, u64 x, u32 t, u32 gamma
   return ms ? mod_switch_word(v, ms) : v;
 }
 
-// ------------------------------------------------------------------------------------
-// Shared-memory position of word e of the one-CTA kernel's per-link transform buffers
-// (8-byte words, 16 to a 128-byte bank row): bits 4 and 5 of e are XORed into bits 2 and 3,
-// which puts every half-warp of the small-stride radix-4 passes (t = 4, 16 in the inverse;
-// h = 4, 16 in the forward) on 16 distinct bank pairs. 2-word pairs stay contiguous and
-// 16-byte aligned, and each 16-word row maps onto itself.
-__device__ __forceinline__ int sw(int e) { return e ^ (((e >> 4) & 3) << 2); }
-
-// ------------------------------------------------------------------------------------
 // The digits 0 and 1 of a canonical coefficient: base 2^20, of the coefficient itself (exact) or of
 // its rounding to a multiple of 2^20 with the lowest digit dropped (the top carry is kept).
 template <bool EXACT>
@@ -856,141 +847,7 @@ __device__ __forceinline__ void split_digits(u64 r, u32& g0, u32& g1) {
   }
 }
 
-// Inverse stages S .. logn-2 in shared memory, words up to 2+ (radix-4 pairs; a radix-2 stage last
-// when logn is even, its sums up to 4+). Each pass ends with a barrier.
-template <int LOGN, int S>
-__device__ __forceinline__ void inv_middle(u64* X, const Tw* tw) {
-  constexpr int N = 1 << LOGN, NT = N / 4;
-  const int tid = threadIdx.x;
-  if constexpr (S + 1 <= LOGN - 2) {
-    constexpr int t = 1 << S, m = N >> (S + 1);
-    const int B = tid >> S, o = tid & (t - 1);
-    const int e0 = B * 4 * t + o;
-    const int i0 = sw(e0), i1 = sw(e0 + t), i2 = sw(e0 + 2 * t), i3 = sw(e0 + 3 * t);
-    u64 a0 = X[i0], a1 = X[i1], a2 = X[i2], a3 = X[i3];
-    inv_unit(a0, a1, a2, a3, tw[2 * m - 1 - 2 * B], tw[2 * m - 2 - 2 * B], tw[m - 1 - B]);
-    X[i0] = a0;
-    X[i1] = a1;
-    X[i2] = a2;
-    X[i3] = a3;
-    __syncthreads();
-    inv_middle<LOGN, S + 2>(X, tw);
-  } else if constexpr (S == LOGN - 2) {
-    constexpr int t = 1 << S, m = N >> (S + 1);
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int v = tid + r * NT;
-      const int B = v >> S, o = v & (t - 1);
-      const int e = sw(B * 2 * t + o), f = sw(B * 2 * t + o + t);
-      u64 a = X[e], b = X[f];
-      bf_inv<3>(a, b, tw[2 * m - 1 - B]);
-      X[e] = a;
-      X[f] = b;
-    }
-    __syncthreads();
-  }
-}
-
-// Forward stages S .. logn-3 of digits 0 and 1 (x and x + N) in shared memory, words up to BIN in
-// (a radix-2 stage first when their count is odd), up to fwd_bound out. Each pass ends with a barrier.
-constexpr int FWD_FREE = 9;  // a unit whose words are at most this needs no reduction: 9 + 6 < 16
-__host__ __device__ constexpr int fwd_bound(int logn, int s, int b) {
-  if ((logn - 2 - s) & 1) b += 3, s++;
-  for (; s < logn - 2; s += 2) b = (b > FWD_FREE ? 1 : b) + 6;
-  return b;
-}
-template <int LOGN, int S, int BIN>
-__device__ __forceinline__ void fwd_middle(u64* D, const Tw* tw) {
-  constexpr int N = 1 << LOGN, NT = N / 4;
-  const int tid = threadIdx.x;
-  if constexpr (S < LOGN - 2 && ((LOGN - 2 - S) & 1)) {
-    constexpr int lt = LOGN - S - 1, t = 1 << lt;
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int v = tid + r * NT;
-      const int ib = v >> lt, o = v & (t - 1);
-      const int e = sw(ib * 2 * t + o), f = sw(ib * 2 * t + o + t);
-      const Tw w = tw[(1 << S) + ib];
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        u64* x = D + k * N;
-        u64 a = x[e], b = x[f];
-        bf_fwd(a, b, w);
-        x[e] = a;
-        x[f] = b;
-      }
-    }
-    __syncthreads();
-    fwd_middle<LOGN, S + 1, BIN + 3>(D, tw);
-  } else if constexpr (S < LOGN - 2) {
-    constexpr int lt = LOGN - S - 1, t = 1 << lt, m = 1 << S, h = t >> 1;
-    constexpr bool RED = BIN > FWD_FREE;
-    const int ib = tid >> (lt - 1), o = tid & (h - 1);
-    const int e0 = ib * 2 * t + o;
-    const Tw wa = tw[m + ib], wb = tw[2 * m + 2 * ib], wc = tw[2 * m + 2 * ib + 1];
-    const int i0 = sw(e0), i1 = sw(e0 + h), i2 = sw(e0 + t), i3 = sw(e0 + t + h);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      u64* x = D + k * N;
-      u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
-      fwd_unit<RED>(a0, a1, a2, a3, wa, wb, wc);
-      x[i0] = a0;
-      x[i1] = a1;
-      x[i2] = a2;
-      x[i3] = a3;
-    }
-    __syncthreads();
-    fwd_middle<LOGN, S + 2, (RED ? 1 : BIN) + 6>(D, tw);
-  }
-}
-
-// One link's transforms on one CTA of N/4 threads: thread tid holds the NTT-domain words cur of its
-// unit (slots 4 tid .. 4 tid + 3, at most 1+, scaled by n^-1) and gets the transforms d0, d1 of digits
-// 0 and 1 of their inverse transform at the same slots, at most 15. The inverse's first two stages and
-// the forward's last two act within a unit and run in registers; the inverse's last stage, the digit
-// split and the forward's first stage are one pass over the pairs (b, b + N/2). X: N words, D: 2N.
-template <int LOGN>
-__device__ __forceinline__ void link_transforms(const u64 (&cur)[4], u64 (&d0)[4], u64 (&d1)[4], u64* X, u64* D,
-                                                const Tw* tw) {
-  constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2, MF = 1 << (LOGN - 2);
-  const int tid = threadIdx.x, l0 = 4 * tid;
-  {
-    u64 a0 = cur[0], a1 = cur[1], a2 = cur[2], a3 = cur[3];
-    inv_unit(a0, a1, a2, a3, tw[N - 1 - 2 * tid], tw[N - 2 - 2 * tid], tw[H - 1 - tid]);
-    *reinterpret_cast<ulonglong2*>(X + sw(l0)) = make_ulonglong2(a0, a1);
-    *reinterpret_cast<ulonglong2*>(X + sw(l0 + 2)) = make_ulonglong2(a2, a3);
-  }
-  __syncthreads();
-  inv_middle<LOGN, 2>(X, tw);
-  const Tw wf = tw[1];
-#pragma unroll
-  for (int j = 0; j < 2; j++) {
-    const int b = sw(tid + j * NT), b2 = sw(tid + j * NT + H);
-    const u64 x0 = X[b], x1 = X[b2];
-    u32 p0, p1, q0, q1;  // digits 0 and 1 of coefficients b and b + N/2
-    split_digits<true>(canon(x0 + x1), p0, p1);
-    split_digits<true>(canon(mulw(x1 - x0 + 5 * Q, wf)), q0, q1);
-    const u64 t0 = mulw_digit(q0, wf), t1 = mulw_digit(q1, wf);
-    D[b] = p0 + t0;
-    D[b2] = p0 + 3 * Q - t0;
-    D[N + b] = p1 + t1;
-    D[N + b2] = p1 + 3 * Q - t1;
-  }
-  __syncthreads();
-  fwd_middle<LOGN, 1, 3>(D, tw);
-  {
-    constexpr bool RED = fwd_bound(LOGN, 1, 3) > FWD_FREE;
-    const Tw fa = tw[MF + tid], fb = tw[2 * MF + 2 * tid], fc = tw[2 * MF + 2 * tid + 1];
-    const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(D + sw(l0));
-    const ulonglong2 v23 = *reinterpret_cast<const ulonglong2*>(D + sw(l0 + 2));
-    const ulonglong2 g01 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0));
-    const ulonglong2 g23 = *reinterpret_cast<const ulonglong2*>(D + N + sw(l0 + 2));
-    d0[0] = v01.x, d0[1] = v01.y, d0[2] = v23.x, d0[3] = v23.y;
-    d1[0] = g01.x, d1[1] = g01.y, d1[2] = g23.x, d1[3] = g23.y;
-    fwd_unit<RED>(d0[0], d0[1], d0[2], d0[3], fa, fb, fc);
-    fwd_unit<RED>(d1[0], d1[1], d1[2], d1[3], fa, fb, fc);
-  }
-}
+constexpr int FWD_FREE = 9;  // a radix-4 unit whose words are at most this needs no reduction: 9 + 6 < 16
 
 // ------------------------------------------------------------------------------------
 // Radix-8 transforms of one CTA of N/8 threads (the one-CTA respond kernel): three stages a
@@ -1247,10 +1104,10 @@ __device__ __forceinline__ void link_transforms8(const u64 (&cur)[8], u64 (&d)[2
   fwd_last8<LOGN, 2, fwd_bound8(LOGN, 2, 6)>(d, D, tw);
 }
 
-// The query's `a` (coefficient form in src, plain order) to n^-1 2^-64 NTT(a) at its slots' positions in
-// a_ntt. D: N words of scratch other than src.
+// scale NTT(src), canonical, at the thread's slots (src: N coefficients in plain order). D: N words of scratch
+// other than src.
 template <int LOGN>
-__device__ __forceinline__ void transform_a8(const CrsDev& c, const u64* src, u64* D, u64* a_ntt, const Tw* tw) {
+__device__ __forceinline__ void transform_slots8(const u64* src, u64* D, const Tw* tw, const Tw& scale, u64 (&out)[8]) {
   constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
 #pragma unroll
   for (int j = 0; j < 2; j++) {
@@ -1267,8 +1124,7 @@ __device__ __forceinline__ void transform_a8(const CrsDev& c, const u64* src, u6
   u64 x[1][8];
   fwd_last8<LOGN, 1, fwd_bound8(LOGN, 2, 7)>(x, D, tw);
 #pragma unroll
-  for (int k = 0; k < 8; k++) a_ntt[k * NT + threadIdx.x] = canon(mulw(x[0][k], c.s_ninv_rinv));
-  __syncthreads();
+  for (int k = 0; k < 8; k++) out[k] = canon(mulw(x[0][k], scale));
 }
 
 // The column transforms of a store build, several shards a launch (blockIdx.y): H row j is the transform of
@@ -1393,7 +1249,14 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
     stage_key_rows(c, ps, qd.seat_R, K, N, k, slot8<LOGN>(k));
   }
   expand_a<N, NT>(qd, D + N, status, qi, force_serial);  // ends with a barrier
-  transform_a8<LOGN>(c, D + N, D, a_ntt, tw);
+  {
+    // n^-1 2^-64 NTT(a): the factor that takes an R-form store word to c_i's scale.
+    u64 x[8];
+    transform_slots8<LOGN>(D + N, D, tw, c.s_ninv_rinv, x);
+#pragma unroll
+    for (int k = 0; k < 8; k++) a_ntt[k * NT + tid] = x[k];
+    __syncthreads();
+  }
 
   u64 cur[8];
   Acc sb[8];
@@ -1930,213 +1793,235 @@ __global__ void k_nopack_sum(u32 n, u32 gamma, u64* out) {
 
 // ------------------------------------------------------------------------------------
 // OnePacking: respond_one_packing (pir/respond.rs:696-729), the Galois-automorphism tree of
-// inspiring/automorph_pack.rs, one CTA per query. Leaf j (j < gamma) is the column product's
-// a part a h_j (b part zero) and b-value_j = coeff0(b h_j); leaves past gamma are the
-// padding's zero ciphertexts. Node (ell, start) = (E + y O) + keyswitch(tau_t(E - y O)) with
+// inspiring/automorph_pack.rs. Leaf j (j < gamma) is the column product's
+// a part a h_j (b part zero) and b-value_j = coeff0(b h_j), which the shard scan gives; leaves past gamma are
+// the padding's zero ciphertexts. Node (ell, start) = (E + y O) + keyswitch(tau_t(E - y O)) with
 // E, O its children (start, start + n/2^ell), y = X^(n >> ell), t = 2^ell + 1 and Galois key
 // log n - ell (pack_lwes_inner, automorph_pack.rs:96-163). Every node whose start is at or
 // past gamma is exactly zero, so only those below gamma are computed.
 //
-// Nodes live in the NTT domain: y O is a product by NTT(X^s), tau_t a slot permutation,
-// and only the key switch's digit split needs coefficients: a = INTT(tau_t(...).a), digits
-// 0 and 1 (base 2^20) transformed, digit 2's transform base^-2 (a - D0 - base D1) (the
+// Nodes live in the NTT domain, scaled by n^-1 as k_respond's links hold R: y O is a product by NTT(X^s),
+// tau_t a slot permutation, and only the key switch's digit split needs coefficients: a = INTT(tau_t(...).a),
+// digits 0 and 1 (base 2^20) transformed, digit 2's transform base^-2 (a - D0 - base D1) (the
 // unsigned split of rgsw/external_product.rs:58-99 leaves a = D0 + base D1 + base^2 D2
-// exactly), which the keys' folded rows (fold_gadget_keys) take from a itself. Key rows
-// are R-form NTT, so each sum of three products takes one reduction.
+// exactly), which the keys' folded rows (fold_gadget_keys) take from a itself.
 //
 // The walk is the recursion's depth-first order: leaf k of the walk is start = bitrev(k),
 // and a binary-counter carry combines each finished node with its waiting sibling; the
-// waiting nodes sit in a per-query stack of log n node slots in global memory.
+// waiting nodes sit in a stack of node slots in global memory. The leaves [j n/S, (j+1) n/S) of the walk make up
+// the subtree of start bitrev(j) at level log n - log S, so k_tree_part walks S subtrees of a query on as many
+// CTAs and k_tree_top the S - 1 nodes above them: a query alone on one CTA took 11 ms whatever the batch, and
+// 64 left most SMs idle. 103 KB of shared memory a CTA: two on an SM.
+struct TreeSmem {
+  Tw* tw;
+  u64 *S1a, *S1b, *D;  // E - y O of a node, by gather position; the transforms' buffers (2N)
+  uint16_t* s_tab;     // gather position of the slot of exponent 2e + 1
+};
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 4, 1)
-    k_tree(CrsDev c, const QueryDev* queries, const ShardDev* shards, u64 ms_target, u64* stack, u64* a_out, u64* b_out,
-           u32* status) {
-  constexpr int N = 1 << LOGN, NT = N / 4;
+__device__ __forceinline__ TreeSmem tree_stage(const CrsDev& c, u64* sm) {
+  constexpr int N = 1 << LOGN, NT = N / 8;
+  TreeSmem S{reinterpret_cast<Tw*>(sm), sm + 2 * N, sm + 3 * N, sm + 4 * N, reinterpret_cast<uint16_t*>(sm + 6 * N)};
+  for (int k = threadIdx.x; k < N; k += NT) {
+    S.tw[tw8<LOGN>(k)] = c.tw[k];
+    S.s_tab[k] = (uint16_t)slot8<LOGN>(c.exp_slot[k]);
+  }
+  return S;
+}
+// A node in global memory: (a, b) of 2N words, each thread's pairs of slots apart by the thread count.
+template <int LOGN>
+__device__ __forceinline__ void node_load(const u64* node, u64 (&a)[8], u64 (&b)[8]) {
+  constexpr int NT = (1 << LOGN) / 8;
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(node) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const ulonglong2 x = p[k * NT], y = p[(k + 4) * NT];
+    a[2 * k] = x.x, a[2 * k + 1] = x.y, b[2 * k] = y.x, b[2 * k + 1] = y.y;
+  }
+}
+template <int LOGN>
+__device__ __forceinline__ void node_store(u64* node, const u64 (&a)[8], const u64 (&b)[8]) {
+  constexpr int NT = (1 << LOGN) / 8;
+  ulonglong2* p = reinterpret_cast<ulonglong2*>(node) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    p[k * NT] = make_ulonglong2(a[2 * k], a[2 * k + 1]);
+    p[(k + 4) * NT] = make_ulonglong2(b[2 * k], b[2 * k + 1]);
+  }
+}
+// The current node (a, b at the thread's slots) becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell; it is
+// O, zero when odd_zero. Ends with a barrier.
+template <int LOGN>
+__device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S, const u64* E, int ell, bool odd_zero,
+                                             const u32 (&et)[8], u64 (&ca)[8], u64 (&cb)[8]) {
+  constexpr int N = 1 << LOGN, NT = N / 8;
   constexpr u32 M2N = 2 * N - 1;
+  const u32 sy = (u32)(N >> ell), t = (1u << ell) + 1;
+  u64 ea[8], eb[8];
+  node_load<LOGN>(E, ea, eb);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    u64 ya = 0, yb = 0;
+    if (!odd_zero) {
+      const Tw y = c.pow_root[(et[k] * sy) & M2N];
+      ya = canon(mulw(ca[k], y));
+      yb = canon(mulw(cb[k], y));
+    }
+    ca[k] = addq(ea[k], ya);
+    cb[k] = addq(eb[k], yb);
+    S.S1a[k * NT + threadIdx.x] = subq(ea[k], ya);
+    S.S1b[k * NT + threadIdx.x] = subq(eb[k], yb);
+  }
+  __syncthreads();
+  u64 d[2][8];
+  {
+    u64 aa[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) aa[k] = S.S1a[S.s_tab[((t * et[k]) & M2N) >> 1]];
+    link_transforms8<LOGN, true>(aa, d, S.D, S.tw);
+  }
+  const u64* key = c.galois + (size_t)(LOGN - ell) * 6 * N + 8 * threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const u32 at = S.s_tab[((t * et[k]) & M2N) >> 1];
+    const u64 aa = S.S1a[at];
+    Acc na{0, 0, 0, 0}, nb{0, 0, 0, 0};
+    mac(na, d[0][k], key[k]);
+    mac(nb, d[0][k], key[N + k]);
+    mac(na, d[1][k], key[2 * N + k]);
+    mac(nb, d[1][k], key[3 * N + k]);
+    mac(na, aa, key[4 * N + k]);
+    mac(nb, aa, key[5 * N + k]);
+    ca[k] = addq(ca[k], csub(acc_fold(na)));
+    cb[k] = addq(cb[k], addq(S.S1b[at], csub(acc_fold(nb))));
+  }
+  __syncthreads();  // S1 and D are rewritten next
+}
+
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8, 2)
+    k_tree_part(CrsDev c, const QueryDev* queries, const ShardDev* shards, u32 log_parts, u64* stack, u64* roots,
+                u32* status) {
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
   extern __shared__ __align__(16) u64 sm[];
-  Tw* tw = reinterpret_cast<Tw*>(sm);
-  u64* aR = sm + 2 * N;  // n^-1 NTT(a)
-  u64* S1a = aR + N;     // E - y O, permuted by the automorphism
-  u64* S1b = S1a + N;
-  u64* X = S1b + N;      // the inverse in progress, then a leaf column
-  u64* D = X + N;        // digits 0 and 1
-  u64* bval = D + 2 * N; // b-values of the leaves (gamma <= n/2)
-  u64* red = bval + N / 2;  // per-warp partial sums
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(red + 32);
-  uint16_t* s_tab = e_tab + N;
+  const TreeSmem S = tree_stage<LOGN>(c, sm);
   const int tid = threadIdx.x;
-  const u32 qi = blockIdx.x;
+  const u32 qi = blockIdx.x >> log_parts, part = blockIdx.x & ((1u << log_parts) - 1);
   const QueryDev qd = queries[qi];
   const ShardDev sh = shards[qd.shard];
   const u32 gamma = c.gamma;
-  u64* stk = stack + (size_t)qi * LOGN * 2 * N;
-
-  for (int k = tid; k < N; k += NT) {
-    tw[k] = c.tw[k];
-    e_tab[k] = c.slot_exp[k];
-    s_tab[k] = c.exp_slot[k];
-  }
-  expand_a<N, NT>(qd, aR, status, qi, 0);  // ends with a barrier
-  {
-    u64* const bufs[1] = {aR};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
-  }
-  for (int k = tid; k < N; k += NT) aR[k] = canon(mulw(aR[k], c.ninv));
-  __syncthreads();
-
-  const int l0 = 4 * tid;
-  u64 ca[4], cb[4];  // the current node at slots l0..l0+3 (thread tid's transform unit)
-  bool cur_zero = true;
-  // Leaf `start`: the column through the transform times NTT(a); its b-value on the side.
-  auto leaf = [&](u32 start) {
-    u128 acc = 0;
+  const int levels = LOGN - (int)log_parts;
+  u64* stk = stack + (size_t)blockIdx.x * levels * 2 * N;
+  u32 et[8];
+  u64 aR[8];  // n^-1 NTT(a) at the thread's slots
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = tid + j * NT;
-      const u64 h = sh.cols16 ? (u64)sh.cols16[(size_t)start * N + k] : reduce128(sh.columns[(size_t)start * N + k]);
-      const u64 br = k == 0 ? reduce128(qd.b[0]) : negq(reduce128(qd.b[N - k]));
-      acc += wide(h, br);
-      X[k] = h;
-    }
-    u64 v = reduce128(acc);
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) v = addq(v, __shfl_xor_sync(0xffffffffu, v, m));
-    if ((tid & 31) == 0) red[tid >> 5] = v;
-    __syncthreads();
-    if (tid == 0) {
-      u64 t = 0;
-      for (int w = 0; w < NT / 32; w++) t = addq(t, red[w]);
-      bval[start] = t;
-    }
-    {
-      u64* const bufs[1] = {X};
-      ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);  // ends with a barrier
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      ca[j] = csub(mulq(X[l0 + j], aR[l0 + j]));
-      cb[j] = 0;
-    }
-    __syncthreads();  // X is rewritten next
-  };
-  // The current node becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell, E from the
-  // stack slot ell - 1; the current node is O (zero when odd_zero). Nodes are held scaled by n^-1,
-  // as k_respond's links hold R, and the key switch runs the same transforms.
-  auto combine = [&](int ell, bool odd_zero) {
-    const u64* E = stk + (size_t)(ell - 1) * 2 * N + l0;
-    const u32 sy = (u32)(N >> ell), t = (1u << ell) + 1;
-    const u64* key = c.galois + (size_t)(LOGN - ell) * 6 * N + l0;
-    u64 s0a[4], s0b[4], aa[4], ab[4];
-    {
-      const ulonglong2 e01 = *reinterpret_cast<const ulonglong2*>(E);
-      const ulonglong2 e23 = *reinterpret_cast<const ulonglong2*>(E + 2);
-      const ulonglong2 f01 = *reinterpret_cast<const ulonglong2*>(E + N);
-      const ulonglong2 f23 = *reinterpret_cast<const ulonglong2*>(E + N + 2);
-      const u64 ea[4] = {e01.x, e01.y, e23.x, e23.y}, eb[4] = {f01.x, f01.y, f23.x, f23.y};
-      u64 da[4], db[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        u64 ya = 0, yb = 0;
-        if (!odd_zero) {
-          const Tw y = c.pow_root[(e_tab[l0 + j] * sy) & M2N];
-          ya = canon(mulw(ca[j], y));
-          yb = canon(mulw(cb[j], y));
-        }
-        s0a[j] = addq(ea[j], ya);
-        s0b[j] = addq(eb[j], yb);
-        da[j] = subq(ea[j], ya);
-        db[j] = subq(eb[j], yb);
-      }
-      *reinterpret_cast<ulonglong2*>(S1a + l0) = make_ulonglong2(da[0], da[1]);
-      *reinterpret_cast<ulonglong2*>(S1a + l0 + 2) = make_ulonglong2(da[2], da[3]);
-      *reinterpret_cast<ulonglong2*>(S1b + l0) = make_ulonglong2(db[0], db[1]);
-      *reinterpret_cast<ulonglong2*>(S1b + l0 + 2) = make_ulonglong2(db[2], db[3]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const u32 src = s_tab[((t * e_tab[l0 + j]) & M2N) >> 1];
-      aa[j] = S1a[src];
-      ab[j] = S1b[src];
-    }
-    u64 d0[4], d1[4];
-    link_transforms<LOGN>(aa, d0, d1, X, D, tw);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      // The keys' digit rows are folded (fold_gadget_keys): aa stands in for digit 2.
-      Acc na{0, 0, 0, 0}, nb{0, 0, 0, 0};
-      mac(na, d0[j], key[j]);
-      mac(nb, d0[j], key[N + j]);
-      mac(na, d1[j], key[2 * N + j]);
-      mac(nb, d1[j], key[3 * N + j]);
-      mac(na, aa[j], key[4 * N + j]);
-      mac(nb, aa[j], key[5 * N + j]);
-      ca[j] = addq(s0a[j], csub(acc_fold(na)));
-      cb[j] = addq(s0b[j], addq(ab[j], csub(acc_fold(nb))));
-    }
-    __syncthreads();  // S1, X and D are rewritten next
-  };
-
-  if (gamma == 1) {
-    // pack_lwes with one input returns it untouched: no tree and no d scaling.
-    leaf(0);
-    cur_zero = false;
-  } else {
-    u32 zero_slots = 0;  // bit L: the waiting node at level L is zero
+  for (int k = 0; k < 8; k++) et[k] = c.slot_exp[8 * tid + k];
+  expand_a<N, NT>(qd, S.D + N, status, qi, 0);  // ends with a barrier
+  transform_slots8<LOGN>(S.D + N, S.D, S.tw, c.ninv, aR);
+  u64 ca[8], cb[8];
+  u32 zero_slots = 0;  // bit L: the waiting node at level L is zero
 #pragma unroll 1
-    for (u32 k = 0; k < (u32)N; k++) {
-      const u32 start = __brev(k) >> (32 - LOGN);
-      cur_zero = start >= gamma;
-      if (!cur_zero) leaf(start);
-      int L = 0;
-      while ((k >> L) & 1) {
-        if ((zero_slots >> L) & 1) {
-          cur_zero = true;  // an even child at or past gamma makes its sibling zero too
-        } else {
-          combine(L + 1, cur_zero);
-          cur_zero = false;
+  for (u32 k = 0; k < (u32)N >> log_parts; k++) {
+    const u32 start = __brev((part << levels) | k) >> (32 - LOGN);
+    bool cur_zero = start >= gamma;
+    if (!cur_zero) {
+      // Leaf `start`: the column through the transform times NTT(a).
+      __syncthreads();  // every thread is past its last read of D
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int b = tid + r * NT;
+        u64 x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const size_t at = (size_t)start * N + b + j * P;
+          x[j] = sh.cols16 ? (u64)sh.cols16[at] : red60(sh.columns[at]);
         }
-        L++;
+        fwd_unit<false>(x[0], x[1], x[2], x[3], S.tw[1], S.tw[2], S.tw[3]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) S.D[sw8(b + j * P)] = x[j];
       }
-      if (L < LOGN) {
-        if (cur_zero) {
-          zero_slots |= 1u << L;
-        } else {
-          zero_slots &= ~(1u << L);
-          u64* slot = stk + (size_t)L * 2 * N + l0;
-          *reinterpret_cast<ulonglong2*>(slot) = make_ulonglong2(ca[0], ca[1]);
-          *reinterpret_cast<ulonglong2*>(slot + 2) = make_ulonglong2(ca[2], ca[3]);
-          *reinterpret_cast<ulonglong2*>(slot + N) = make_ulonglong2(cb[0], cb[1]);
-          *reinterpret_cast<ulonglong2*>(slot + N + 2) = make_ulonglong2(cb[2], cb[3]);
-        }
+      __syncthreads();
+      fwd_middle8<LOGN, 1, 7>(S.D, S.tw);
+      u64 x[1][8];
+      fwd_last8<LOGN, 1, fwd_bound8(LOGN, 2, 7)>(x, S.D, S.tw);
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        ca[j] = csub(mulq(x[0][j], aR[j]));
+        cb[j] = 0;
       }
     }
+    if (gamma == 1) break;  // a single leaf is the root
+    int L = 0;
+    while ((k >> L) & 1) {
+      if ((zero_slots >> L) & 1) {
+        cur_zero = true;  // an even child at or past gamma makes its sibling zero too
+      } else {
+        tree_combine<LOGN>(c, S, stk + (size_t)L * 2 * N, L + 1, cur_zero, et, ca, cb);
+        cur_zero = false;
+      }
+      L++;
+    }
+    if (L == levels) break;  // the subtree's root (start below gamma: never zero)
+    zero_slots = (zero_slots & ~(1u << L)) | (cur_zero ? 1u << L : 0);
+    if (!cur_zero) node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
   }
-  // The root to coefficients; b_z += n b-value_z for z < gamma (pack_lwes, automorph_pack.rs
-  // 327-338), except for a single input.
+  node_store<LOGN>(roots + (size_t)blockIdx.x * 2 * N, ca, cb);
+}
+
+// The nodes above the subtrees, then the root to coefficients; b_z += n b-value_z for z < gamma (pack_lwes,
+// automorph_pack.rs 327-338), except for a single input, which pack_lwes returns untouched: no tree and no d
+// scaling.
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8, 2)
+    k_tree_top(CrsDev c, const QueryDev* queries, u32 log_parts, u64 ms_target, u64* stack, const u64* roots,
+               const u64* b_fold, u64* a_out, u64* b_out) {
+  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
+  extern __shared__ __align__(16) u64 sm[];
+  const TreeSmem S = tree_stage<LOGN>(c, sm);
+  const int tid = threadIdx.x, levels = LOGN - (int)log_parts;
+  const u32 qi = blockIdx.x, gamma = c.gamma;
+  // The waiting nodes go where the query's first subtree kept its own; log_parts slots are free there or in
+  // the ones after.
+  u64* stk = stack + (size_t)(qi << log_parts) * levels * 2 * N;
+  u32 et[8];
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    X[l0 + j] = ca[j];
-    D[l0 + j] = cb[j];
-  }
+  for (int k = 0; k < 8; k++) et[k] = c.slot_exp[8 * tid + k];
   __syncthreads();
-  {
-    u64* const bufs[2] = {X, D};
-    ntt_inv_r4<LOGN, NT, 2>(bufs, tw);
+  u64 ca[8], cb[8];
+#pragma unroll 1
+  for (u32 j = 0; j < 1u << log_parts; j++) {
+    node_load<LOGN>(roots + ((size_t)(qi << log_parts) + j) * 2 * N, ca, cb);
+    int L = 0;
+    for (; (j >> L) & 1; L++) tree_combine<LOGN>(c, S, stk + (size_t)L * 2 * N, levels + L + 1, false, et, ca, cb);
+    if (L < (int)log_parts) node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
   }
-  const u64 scale = gamma == 1 ? 1 : (u64)N;
+  inv_first8<LOGN>(ca, S.D, S.tw);
+  inv_first8<LOGN>(cb, S.D + N, S.tw);
+  __syncthreads();
+  inv_middle8<LOGN, 2>(S.D, S.tw);
+  const u64* bval = b_fold + queries[qi].fold_off;
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const int k = tid + j * NT;
-    u64 av = canon(X[k]);
-    u64 bv = gamma == 1 ? (k == 0 ? bval[0] : 0) : canon(D[k]);
-    if (gamma > 1 && (u32)k < gamma) bv = addq(bv, reduce128(wide(bval[k], scale)));
-    if (ms_target) {
-      av = mod_switch_word(av, ms_target);
-      bv = mod_switch_word(bv, ms_target);
+  for (int r = 0; r < 2; r++) {
+    const int b = tid + r * NT;
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+      u64 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = S.D[n * N + sw8(b + k * P)];
+      inv_unit(x[0], x[1], x[2], x[3], S.tw[3], S.tw[2], S.tw[1]);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const u32 z = b + k * P;
+        u64 v = canon(x[k]);
+        if (n == 1) {
+          if (gamma == 1)
+            v = z == 0 ? bval[0] : 0;
+          else if (z < gamma)
+            v = addq(v, reduce128(wide(bval[z], (u64)N)));
+        }
+        if (ms_target) v = mod_switch_word(v, ms_target);
+        (n ? b_out : a_out)[(size_t)qi * N + z] = v;
+      }
     }
-    a_out[(size_t)qi * N + k] = av;
-    b_out[(size_t)qi * N + k] = bv;
   }
 }
 
@@ -2587,18 +2472,39 @@ cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64
   return cudaGetLastError();
 }
 
-size_t tree_smem_bytes(const CrsDev& c) { return ((size_t)8 * c.n + c.n / 2 + 32) * 8 + 2 * (size_t)c.n * 2; }
+// Subtrees of a query (a power of two): the split whose waves of two CTAs an SM and nodes above it take least, in
+// key switches (a leaf counts as one), with the stacks and roots within 256 MB.
+u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms) {
+  u64 work = c.gamma, best = ~0ULL;  // leaves and nodes of a whole tree
+  for (u32 k = 1; k <= c.logn; k++) work += c.gamma < (c.n >> k) ? c.gamma : c.n >> k;
+  u32 log_best = 0;
+  for (u32 lp = 0; lp <= 5 && (2u << lp) <= c.gamma; lp++) {
+    if (lp && tree_scratch_words(c, nq, lp) * 8 > (256ULL << 20)) break;
+    const u64 ctas = (u64)nq << lp, waves = (ctas + 2 * sms - 1) / (2 * sms);
+    const u64 cost = (waves * work >> lp) + ((1u << lp) - 1);
+    if (cost < best) best = cost, log_best = lp;
+  }
+  return log_best;
+}
+// Node stacks of the subtrees (and of the nodes above them, in their place), then their roots.
+u64 tree_scratch_words(const CrsDev& c, u32 nq, u32 log_parts) {
+  return ((u64)nq << log_parts) * (c.logn - log_parts + 1) * 2 * c.n;
+}
 
-cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 ms_target, u64* stack,
-                 u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
+cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u32 log_parts, u64 ms_target,
+                 u64* nodes, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   if (!c.galois || c.gamma > c.n / 2) return cudaErrorInvalidValue;
-  const size_t smem = tree_smem_bytes(c);
+  const size_t smem = (size_t)6 * c.n * 8 + 2 * (size_t)c.n;
+  u64* roots = nodes + ((u64)nq << log_parts) * (c.logn - log_parts) * 2 * c.n;
   IG_DISPATCH_LOGN(c.logn, {
-    auto k = k_tree<L>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto part = k_tree_part<L>;
+    auto top = k_tree_top<L>;
+    cudaError_t e = cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<nq, (1 << L) / 4, smem, s>>>(c, queries, shards, ms_target, stack, a_out, b_out, status);
+    part<<<nq << log_parts, (1 << L) / 8, smem, s>>>(c, queries, shards, log_parts, nodes, roots, status);
+    top<<<nq, (1 << L) / 8, smem, s>>>(c, queries, log_parts, ms_target, nodes, roots, b_fold, a_out, b_out);
   });
   return cudaGetLastError();
 }

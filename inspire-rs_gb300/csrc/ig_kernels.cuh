@@ -159,10 +159,13 @@ size_t respond_smem_bytes(const CrsDev& c, int ctas);
 cudaError_t nopack(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 r_mod_q,
                    u64* AB_R, u64* out, u32* status, cudaStream_t s);
 
-// OnePacking (respond_one_packing): one CTA per query walks the automorphism tree; stack
-// holds nq x logn x 2n words of waiting nodes. Outputs coefficient-form (a, b), switched to
-// ms_target when nonzero.
-size_t tree_smem_bytes(const CrsDev& c);
+// OnePacking (respond_one_packing): 2^log_parts CTAs per query walk the automorphism tree's subtrees, one the nodes
+// above them; nodes holds tree_scratch_words, b_fold the scan's b-values. Outputs coefficient-form
+// (a, b), switched to ms_target when nonzero.
+u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms);
+u64 tree_scratch_words(const CrsDev& c, u32 nq, u32 log_parts);
+cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u32 log_parts, u64 ms_target,
+                 u64* nodes, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s);
 
 // Client side: the sampler's keystream (ChaCha20 blocks of stream 0), the parallel parse of
 // W stream words from u32 offset `base` of ks into the first S samples (out) and the word
@@ -175,9 +178,6 @@ cudaError_t client_query(const CrsDev& c, const QueryDev* queries, u32 nq, const
                          const i64* samples, u64 delta, u64* b_out, u32* status, cudaStream_t s);
 cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64* a, const u64* b, u64 modulus,
                            u64 delta, u64 p, u64 dinv, u32 entry_size, uint8_t* out, cudaStream_t s);
-cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 ms_target, u64* stack,
-                 u64* a_out, u64* b_out, u32* status, cudaStream_t s);
-
 // Integer roofline probe: blocks x 256 threads x iters x 8 lazy butterflies in registers.
 cudaError_t butterfly_peak(u64* out, int blocks, int iters, cudaStream_t s);
 }  // namespace igk

@@ -1829,21 +1829,24 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     if (!local.count(s)) {
       local[s] = (u32)table.size();
       table.push_back(db->shards[s].dev());
+      table.back().stale = 0;  // the tree reads columns alone: no store to be out of date
     }
   }
   const size_t seed_bytes = as ? (size_t)count * n * 8 : (size_t)count * 32;
-  void *d_table, *d_q, *d_seeds, *d_bs, *d_stack, *d_a, *d_b, *d_status;
+  void *d_table, *d_q, *d_seeds, *d_bs, *d_nodes, *d_fold, *d_a, *d_b, *d_status;
   auto lane_scratch = [&](const char* name, size_t bytes, void** p) {
     char full[48];
     snprintf(full, sizeof full, "%s%u", name, k);
     return scratch(c, full, bytes, p);
   };
+  const u32 parts = igk::tree_log_parts(o.dev, count, c->sms);
   int rc;
   if ((rc = lane_scratch("tr_table", table.size() * sizeof(ShardDev), &d_table)) ||
       (rc = lane_scratch("tr_queries", count * sizeof(QueryDev), &d_q)) ||
       (rc = lane_scratch("tr_seeds", seed_bytes, &d_seeds)) ||
       (rc = lane_scratch("tr_bs", (size_t)count * n * 8, &d_bs)) ||
-      (rc = lane_scratch("tr_stack", (size_t)count * o.logn * 2 * n * 8, &d_stack)) ||
+      (rc = lane_scratch("tr_nodes", igk::tree_scratch_words(o.dev, count, parts) * 8, &d_nodes)) ||
+      (rc = lane_scratch("tr_fold", (size_t)count * o.gamma * 8, &d_fold)) ||
       (rc = lane_scratch("tr_a", (size_t)count * n * 8, &d_a)) ||
       (rc = lane_scratch("tr_b", (size_t)count * n * 8, &d_b)) || (rc = lane_scratch("tr_status", count * 4, &d_status)))
     return rc;
@@ -1858,6 +1861,8 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     qs[i].a = as ? (const u64*)d_seeds + (size_t)i * n : nullptr;
     qs[i].b = (const u64*)d_bs + (size_t)i * n;
     qs[i].seat_R = nullptr;
+    qs[i].fold_off = i * o.gamma;
+    qs[i].row = i;
   }
   if ((rc = stage_h2d(c, d_table, table.data(), table.size() * sizeof(ShardDev))) ||
       (rc = stage_h2d(c, d_q, qs.data(), count * sizeof(QueryDev))) ||
@@ -1866,9 +1871,11 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     return rc;
   cudaStream_t s = igint::host_call_stream(c, hc);
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
-  IG_CUDA(c, igk::tree(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, ms_target, (u64*)d_stack,
-                       (u64*)d_a, (u64*)d_b, (u32*)d_status, s));
-  c->launches++;
+  IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, nullptr, 0, (u64*)d_fold,
+                             (u32*)d_status, s));
+  IG_CUDA(c, igk::tree(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, parts, ms_target, (u64*)d_nodes,
+                       (const u64*)d_fold, (u64*)d_a, (u64*)d_b, (u32*)d_status, s));
+  c->launches += 3;
   IG_CUDA(c, cudaMemcpyAsync((void*)h_status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
   if ((rc = igint::host_call_launched(c, hc))) return rc;
   lk.unlock();  // other callers launch while this batch runs and copies out
