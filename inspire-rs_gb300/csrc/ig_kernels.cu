@@ -2472,16 +2472,19 @@ cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64
   return cudaGetLastError();
 }
 
-// Subtrees of a query (a power of two): the split whose waves of two CTAs an SM and nodes above it take least, in
-// key switches (a leaf counts as one), with the stacks and roots within 256 MB.
+// Subtrees of a query (a power of two): the split that takes least by a model in key switches (a leaf counts as
+// one; 10.2 us on an SM alone), with the stacks and roots within 256 MB. A subtree takes its own length on an idle
+// GPU; a full one gets through the batch's work at 1.2 subtrees an SM (two CTAs share it), with half a
+// subtree of idle tail; the nodes above follow. Measured at gamma 256 (ms, 1 / 8 / 32 subtrees): a query alone
+// 13.0 / 1.80 / 0.91, 64 queries 13.1 / 5.42 / 4.99 (16 subtrees 4.89), 152 13.4 / 10.8 / 10.8.
 u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms) {
   u64 work = c.gamma, best = ~0ULL;  // leaves and nodes of a whole tree
   for (u32 k = 1; k <= c.logn; k++) work += c.gamma < (c.n >> k) ? c.gamma : c.n >> k;
   u32 log_best = 0;
   for (u32 lp = 0; lp <= 5 && (2u << lp) <= c.gamma; lp++) {
     if (lp && tree_scratch_words(c, nq, lp) * 8 > (256ULL << 20)) break;
-    const u64 ctas = (u64)nq << lp, waves = (ctas + 2 * sms - 1) / (2 * sms);
-    const u64 cost = (waves * work >> lp) + ((1u << lp) - 1);
+    const u64 part = work >> lp, full = nq * work * 10 / (12 * (u64)sms) + part / 2;
+    const u64 cost = (part > full ? part : full) + ((1u << lp) - 1);
     if (cost < best) best = cost, log_best = lp;
   }
   return log_best;
