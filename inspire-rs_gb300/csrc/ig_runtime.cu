@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <random>
@@ -216,6 +217,10 @@ struct ig_ctx {
   // that many queries under 1, 2 and 4 CTAs per query.
   u32 force_ctas = 0;
   std::map<std::pair<u32, u32>, std::map<u32, std::array<double, 3>>> tune;
+  // Second and third stream of a mixed launch whose queries take several shapes, by lane, with the events that
+  // fork them from and join them to the lane's stream.
+  cudaStream_t side_stream[IG_MAX_LANES][2] = {};
+  cudaEvent_t side_fork[IG_MAX_LANES] = {}, side_done[IG_MAX_LANES][2] = {};
   cudaStream_t lane_stream[IG_MAX_LANES] = {};
   cudaEvent_t lane_in[IG_MAX_LANES] = {}, lane_done[IG_MAX_LANES] = {};
   bool lane_used[IG_MAX_LANES] = {};
@@ -685,6 +690,14 @@ void ig_ctx_destroy(ig_ctx* c) {
     }
     if (c->hlane[k].pin) cudaFreeHost(c->hlane[k].pin);
     if (c->hlane[k].done) cudaEventDestroy(c->hlane[k].done);
+    if (c->side_fork[k]) cudaEventDestroy(c->side_fork[k]);
+    for (int j = 0; j < 2; j++) {
+      if (c->side_stream[k][j]) {
+        cudaStreamSynchronize(c->side_stream[k][j]);
+        cudaStreamDestroy(c->side_stream[k][j]);
+      }
+      if (c->side_done[k][j]) cudaEventDestroy(c->side_done[k][j]);
+    }
   }
   if (c->sm && c->sm_destroy) c->sm_destroy(c, c->sm);
   for (auto& kv : c->crs)
@@ -1963,6 +1976,7 @@ struct MixedPlan {
   std::vector<ShardDev> table;   // distinct (database, shard) pairs of the launch
   std::vector<QueryDev> qs;      // launch order: longest recursion (gamma) first
   std::vector<u32> work;         // scan work items, position << 12 | chunk
+  std::vector<u32> gammas;       // the queries' widths in launch order
   size_t fold_words = 0;
   u32 max_gamma = 0;             // the longest recursion of the launch
 };
@@ -2027,9 +2041,99 @@ static int plan_mixed(ig_ctx* c, u32 count, const uint64_t* dbs, const uint64_t*
     const u32 gamma = order[p].first;
     for (u32 ch = 0; ch < igk::scan_chunks(gamma); ch++) P.work.push_back((p << 12) | ch);
     P.fold_words += gamma;
+    P.gammas.push_back(gamma);
     P.max_gamma = std::max(P.max_gamma, gamma);
   }
   P.qs.swap(sorted);
+  return IG_OK;
+}
+
+// A run of a mixed launch's queries and their shape.
+struct ShapeRun {
+  u32 first, count;
+  int ctas;
+};
+
+// Shapes of a mixed launch of several widths, whose queries need not share one: under a bound T on a query's own
+// time each query takes the fewest CTAs that keep it (four where none does), and T is the one whose launch
+// ends first when the queries start longest first as SMs come free. Times are the tuned table's for one query,
+// else 6.65, 4.62 and 2.76 us a link (measured at gamma 256 under one, two and four CTAs). 128 queries over gamma
+// 16, 256 and 1024 in equal parts took one CTA each: 7.65 ms, the time of the 43 longest, with most SMs
+// idle after 2 ms. Lanes share the SMs. More queries than four an SM fill the GPU in any order: one CTA each.
+static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u32 count) {
+  const bool uniform = P.gammas.front() == P.gammas.back();
+  const u32 sms = std::max<u32>(1, c->sms / c->lanes);
+  if (c->force_ctas || uniform || count > 4 * sms)
+    return {{0, count, igint::launch_ctas(c, n, P.max_gamma, count, count * c->lanes)}};
+  std::map<u32, std::array<double, 3>> times;  // by gamma: a query under 1, 2, 4 CTAs
+  std::vector<double> bounds;
+  for (u32 g : P.gammas)
+    if (!times.count(g)) {
+      std::array<double, 3> t{6.65 * g, 4.62 * g, 2.76 * g};
+      if (c->tune.count({n, g}))  // milliseconds, of this width only
+        for (int k = 0; k < 3; k++) t[k] = 1e3 * (*igint::tuned_row(c, n, g, 1))[k];
+      times[g] = t;
+      bounds.insert(bounds.end(), t.begin(), t.end());
+    }
+  auto shape_of = [&](u32 g, double bound) {
+    const std::array<double, 3>& t = times[g];
+    return t[0] <= bound ? 0 : t[1] <= bound ? 1 : 2;
+  };
+  double best = 0, best_bound = 0;
+  std::vector<double> busy;
+  for (double bound : bounds) {
+    busy.assign(sms, 0.0);  // a heap of the SMs' ends, the earliest first
+    double end = 0;
+    for (u32 g : P.gammas) {
+      const int k = shape_of(g, bound), r = std::min<int>(1 << k, (int)sms);
+      double start = 0;
+      for (int j = 0; j < r; j++) {
+        std::pop_heap(busy.begin(), busy.end() - j, std::greater<double>());
+        start = busy[busy.size() - 1 - j];
+      }
+      for (int j = r - 1; j >= 0; j--) {
+        busy[busy.size() - 1 - j] = start + times[g][k];
+        std::push_heap(busy.begin(), busy.end() - j, std::greater<double>());
+      }
+      end = std::max(end, start + times[g][k]);
+    }
+    if (best == 0 || end < 0.98 * best || (end <= best && bound > best_bound)) best = end, best_bound = bound;
+  }
+  std::vector<ShapeRun> runs;
+  for (u32 p = 0; p < count; p++) {
+    const int ctas = 1 << shape_of(P.gammas[p], best_bound);
+    if (runs.empty() || runs.back().ctas != ctas) runs.push_back({p, 0, ctas});
+    runs.back().count++;
+  }
+  return runs;
+}
+
+// The respond launches of a mixed batch after its scan on `s`: one a shape, side by side on the lane's side
+// streams (a run of longer recursions goes first and is placed first), joined to `s`.
+static int respond_runs(ig_ctx* c, const MixedPlan& P, const std::vector<ShapeRun>& runs, u32 lane, const QueryDev* dq,
+                        const ShardDev* dt, const u64* df, u64* da, u64* db, u32* dst, cudaStream_t s) {
+  if (runs.size() > 1) {
+    if (!c->side_fork[lane]) IG_CUDA(c, cudaEventCreateWithFlags(&c->side_fork[lane], cudaEventDisableTiming));
+    IG_CUDA(c, cudaEventRecord(c->side_fork[lane], s));
+  }
+  for (size_t r = 0; r < runs.size(); r++) {
+    cudaStream_t st = s;
+    if (r) {
+      cudaStream_t& side = c->side_stream[lane][(r - 1) % 2];
+      if (!side) IG_CUDA(c, cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+      IG_CUDA(c, cudaStreamWaitEvent(side, c->side_fork[lane], 0));
+      st = side;
+    }
+    IG_CUDA(c, igk::respond(P.ring, dq + runs[r].first, dt, runs[r].count, df, da, db, dst, c->force_serial, runs[r].ctas,
+                            st));
+    if (r) {
+      cudaEvent_t& done = c->side_done[lane][(r - 1) % 2];
+      if (!done) IG_CUDA(c, cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+      IG_CUDA(c, cudaEventRecord(done, st));
+    }
+  }
+  for (size_t r = 1; r < runs.size(); r++) IG_CUDA(c, cudaStreamWaitEvent(s, c->side_done[lane][(r - 1) % 2], 0));
+  c->launches += runs.size();
   return IG_OK;
 }
 
@@ -2073,12 +2177,12 @@ int ig_respond_mixed_batch_device(ig_ctx* c, uint32_t count, const uint64_t* dbs
   IG_CUDA(c, igk::shard_scan(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u32*)dw,
                              (u32)P.work.size(), (u64*)df, d_status, s));
   prof_end(c, pk, s);
-  const int ctas = igint::launch_ctas(c, (u32)n, P.max_gamma, count, count * c->lanes);
   pk = prof_begin(c, REGION_RESPOND, s);
-  IG_CUDA(c, igk::respond(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u64*)df, d_a, d_b, d_status,
-                          c->force_serial, ctas, s));
+  if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), lane < 0 ? 0 : (u32)lane, (const QueryDev*)dq,
+                         (const ShardDev*)dt, (const u64*)df, d_a, d_b, d_status, s)))
+    return rc;
   prof_end(c, pk, s);
-  c->launches += 2;
+  c->launches++;
   return igint::lane_release(c, lane);
 }
 
@@ -2134,11 +2238,10 @@ int ig_respond_mixed_batch(ig_ctx* c, uint32_t count, const uint64_t* dbs, const
   IG_CUDA(c, cudaMemsetAsync(dst, 0, count * 4, s));
   IG_CUDA(c, igk::shard_scan(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u32*)dw,
                              (u32)P.work.size(), (u64*)df, (u32*)dst, s));
-  IG_CUDA(c, igk::respond(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u64*)df, (u64*)da, (u64*)db_,
-                          (u32*)dst, c->force_serial,
-                          igint::launch_ctas(c, (u32)n, P.max_gamma, count, count * c->lanes),
-                          s));
-  c->launches += 2;
+  if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), k, (const QueryDev*)dq, (const ShardDev*)dt,
+                         (const u64*)df, (u64*)da, (u64*)db_, (u32*)dst, s)))
+    return rc;
+  c->launches++;
   IG_CUDA(c, cudaMemcpyAsync(h_status, dst, count * 4, cudaMemcpyDeviceToHost, s));
   IG_CUDA(c, cudaMemcpyAsync(h_a, da, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
   IG_CUDA(c, cudaMemcpyAsync(h_b, db_, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
