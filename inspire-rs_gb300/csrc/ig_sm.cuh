@@ -45,15 +45,13 @@ struct Prime32 {
   __host__ __device__ __forceinline__ i64 centred(u32 x) const { return x > (m >> 1) ? (i64)x - (i64)m : (i64)x; }
 };
 
-// One transform's constants: bit-reversed Montgomery-form powers of psi and psi^-1, and the
-// two factors of the inverse's fused last stage (arith.rs:131-166).
+// One transform's constants (arith.rs:131-166): bit-reversed Montgomery-form powers of psi and psi^-1.
 struct Ntt32Dev {
   Prime32 p;
   const u32* fwd;
   const u32* inv;
   const uint2* fwd_sh;  // the forward ladder in standard form with Shoup companions (w, w')
-  u32 n_inv, last;      // Montgomery form: 1/n, and 1/n times the inverse's last twiddle
-  u32 n_inv_s, n_inv_sp, last_s, last_sp;  // the same two in standard form with companions
+  u32 n_inv;            // 1/n in Montgomery form
 };
 
 struct SmDev {
@@ -68,6 +66,8 @@ struct SmDev {
   u32 inv_gamma_RR;          // gamma^-1 * 2^64 mod q: mont(x, .) = x gamma^-1 2^32
   u32 p_over_q, neg_off, p_inv_R;  // lifts between the limbs and 1/p mod q (R-form)
   u32 q_mu;                        // floor(2^32 / q), the Barrett factor of the lazy lift
+  u32 n_R;                         // n in Montgomery form mod q
+  u32 np_inv_s, np_inv_sp;         // 1/(n p) mod q in standard form with its Shoup companion
 };
 
 struct SmQueryDev {
@@ -94,7 +94,9 @@ cudaError_t table_columns(const SmDev& c, const uint8_t* cells, u32 rows, u32 ce
                           cudaStream_t s);
 // Step-1 table from the columns' transforms (H: gamma x n standard form): per-slot DFT.
 cudaError_t table_fold(const SmDev& c, const u32* H, u32* step1_R, cudaStream_t s);
-// Body fold: fold[q][k] = sum_m c_m values[m][k] (c_0 = centred b_0, c_m = -centred b_{n-m}).
+// Body fold: fold[q][chunk][k] = sum c_m values[m][k] over the rows m of a chunk (c_0 = centred b_0, c_m = -centred
+// b_{n-m}), k < gamma.
+constexpr int SM_FOLD_CHUNKS = 4;
 cudaError_t body_fold(const SmDev& c, const SmQueryDev* queries, u32 nq, i64* fold, cudaStream_t s);
 // The 2n-step recursion and the final transforms; one CTA per query.
 cudaError_t respond(const SmDev& c, const SmQueryDev* queries, u32 nq, const i64* fold, u32* mask_out, u32* body_out,

@@ -9,6 +9,8 @@
 // Every word is a canonical residue; products are Montgomery with R = 2^32 as in Prime32.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "ig_arith.cuh"
 #include "ig_sm.cuh"
 
@@ -56,42 +58,6 @@ __device__ __forceinline__ void fwd32(u32* x, const Ntt32Dev& T, const u32* tw) 
     v = P.mont(a3, wc);
     x[e0 + t] = P.add(a2, v);
     x[e0 + t + h] = P.sub(a2, v);
-    __syncthreads();
-  }
-}
-
-template <int LOGN>
-__device__ __forceinline__ void inv32(u32* x, const Ntt32Dev& T, const u32* itw) {
-  constexpr int N = 1 << LOGN, NT = N / 4;
-  static_assert(LOGN & 1, "odd log n: radix-4 pairs then the fused radix-2 stage");
-  const Prime32 P = T.p;
-  const int tid = threadIdx.x;
-#pragma unroll 1
-  for (int s = 0; s + 1 < LOGN; s += 2) {
-    const int t = 1 << s, m = N >> (s + 1);
-    const int B = tid >> s, o = tid & (t - 1);
-    const int e0 = B * 4 * t + o;
-    const u32 w0 = itw[m + 2 * B], w1 = itw[m + 2 * B + 1], w2 = itw[(m >> 1) + B];
-    u32 a0 = x[e0], a1 = x[e0 + t], a2 = x[e0 + 2 * t], a3 = x[e0 + 3 * t];
-    const u32 d01 = P.mont(a0 + P.m - a1, w0);
-    a0 = P.add(a0, a1);
-    const u32 d23 = P.mont(a2 + P.m - a3, w1);
-    a2 = P.add(a2, a3);
-    x[e0] = P.add(a0, a2);
-    x[e0 + 2 * t] = P.mont(a0 + P.m - a2, w2);
-    x[e0 + t] = P.add(d01, d23);
-    x[e0 + 3 * t] = P.mont(d01 + P.m - d23, w2);
-    __syncthreads();
-  }
-  {
-    constexpr int t = N / 2;
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int b = tid + r * NT;
-      const u32 u = x[b], v = x[b + t];
-      x[b] = P.mont(u + v, T.n_inv);
-      x[b + t] = P.mont(u + P.m - v, T.last);
-    }
     __syncthreads();
   }
 }
@@ -179,30 +145,43 @@ __global__ void __launch_bounds__(SM_FOLD_THREADS) k_sm_fold(SmDev c, const u32*
 }
 
 // ------------------------------------------------------------------------------------
-// Body fold: thread k < nb sums c_m values[m][k] over the shard's rows (exact in i64).
+// Body fold: fold[chunk][k] = sum c_m values[m][k] over the rows of one of SM_FOLD_CHUNKS chunks of the shard (exact
+// in i64; the respond kernel adds the chunks). A thread takes four columns of every fourth row, one 32-bit
+// load a row: a CTA a query walking all rows byte by byte was one long chain of loads (377 us for 256
+// queries, 1 MB of nibbles each).
+constexpr int SM_FOLD_ROWS = 4;  // rows a CTA reads side by side
 __global__ void __launch_bounds__(512) k_sm_body_fold(SmDev c, const SmQueryDev* queries, i64* fold) {
+  __shared__ i64 part[SM_FOLD_ROWS - 1][512];
   const SmQueryDev qd = queries[blockIdx.x];
-  const u32 k = threadIdx.x;
-  if (k >= c.nb) return;
+  const u32 lanes = blockDim.x / SM_FOLD_ROWS, k4 = threadIdx.x % lanes, r0 = threadIdx.x / lanes;
+  const u32 span = (qd.rows + SM_FOLD_CHUNKS - 1) / SM_FOLD_CHUNKS;
+  const u32 from = blockIdx.y * span, to = min(qd.rows, from + span);
   const Prime32 P = c.lq.p;
-  i64 acc = 0;
+  i64 acc[4] = {0, 0, 0, 0};
 #pragma unroll 8
-  for (u32 m = 0; m < qd.rows; m++) {
+  for (u32 m = from + r0; m < to; m += SM_FOLD_ROWS) {
     const u32 bw = qd.body[m == 0 ? 0 : c.n - m];
-    const i64 cm = m == 0 ? P.centred(bw) : -P.centred(bw);
-    acc += cm * (i64)qd.values[(size_t)m * c.gamma + k];
+    const int cm = (int)(m == 0 ? P.centred(bw) : -P.centred(bw));
+    const int8_t* row = qd.values + (size_t)m * c.gamma + 4 * k4;
+    char4 v = make_char4(0, 0, 0, 0);
+    if (c.gamma >= 4)
+      v = *reinterpret_cast<const char4*>(row);
+    else  // two columns
+      v.x = row[0], v.y = row[1];
+    acc[0] += (i64)cm * v.x;
+    acc[1] += (i64)cm * v.y;
+    acc[2] += (i64)cm * v.z;
+    acc[3] += (i64)cm * v.w;
   }
-  fold[(size_t)blockIdx.x * c.nb + k] = acc;
-}
-
-// Inverse twiddle m of a ladder (Gentleman-Sande, psi^-brv(m)) from the forward ladder's
-// Shoup pairs: for 2^s <= m < 2^(s+1), brv(3 2^s - 1 - m) = n - brv(m), so
-// psi^-brv(m) = -psi^brv(3 2^s - 1 - m); and the companion of pm - w is the complement of
-// w's (w != 0, pm prime above w).
-__device__ __forceinline__ uint2 inv_tw(const uint2* fs, u32 pm, int m) {
-  const int s = 31 - __clz(m);
-  const uint2 f = fs[3 * (1 << s) - 1 - m];
-  return make_uint2(pm - f.x, ~f.y);
+  if (r0)
+    for (int j = 0; j < 4; j++) part[r0 - 1][4 * k4 + j] = acc[j];
+  __syncthreads();
+  if (r0) return;
+  i64* out = fold + ((size_t)blockIdx.x * SM_FOLD_CHUNKS + blockIdx.y) * c.gamma + 4 * k4;
+  for (int j = 0; j < 4; j++) {
+    for (int r = 0; r < SM_FOLD_ROWS - 1; r++) acc[j] += part[r][4 * k4 + j];
+    if (4 * k4 + j < c.gamma) out[j] = acc[j];
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -271,336 +250,380 @@ __device__ __forceinline__ u32 q_to_p(const SmDev& c, u32 x) {
   return x > (c.lq.p.m >> 1) ? x + (c.lp.p.m - c.lq.p.m) : x;
 }
 
-// One CTA per query. Each link i = gamma-2 .. 0 (server.rs:434-487):
+// ------------------------------------------------------------------------------------
+// Radix-8 transforms of the recursion: N/8 threads, three stages a shared-memory round trip, layouts free of bank
+// conflicts (32-bit words, 32 to a bank row): sw spreads the 16-byte accesses of contiguous units (bit 5 into
+// bit 2) and the stride-8 passes (bits 6-7 into 3-4); the ladders' top two levels hold the entries that a unit
+// takes N/8 apart; gathered operands sit at (t & 7) N/8 + (t >> 3).
+//
+// Twiddle products are Shoup products against the forward ladder's (w, w') pairs. The inverse takes the same
+// ladder at the mirrored index: psi^-brv(m) = -psi^brv(3 2^s - 1 - m) for m in [2^s, 2^(s+1)), so
+// (X - Y) w^-1 = (Y - X) f.
+__device__ __forceinline__ int sw(int e) { return e ^ (((e >> 5) & 1) << 2) ^ (((e >> 6) & 3) << 3); }
+template <int LOGN>
+__device__ __forceinline__ int ladder_at(int m) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  if (m >= N / 2) return N / 2 + (m & 3) * E + ((m - N / 2) >> 2);
+  if (m >= N / 4) return N / 4 + (m & 1) * E + ((m - N / 4) >> 1);
+  return m;
+}
+template <int LOGN>
+__device__ __forceinline__ int slot_at(int t) {
+  return ((t & 7) << (LOGN - 3)) | (t >> 3);
+}
+
+// Butterflies of a limb. Full, for a prime below 2^31: the inverse's words are residues, the forward's stay below
+// 2m (X is brought below m where it is used). Lazy, for 8m <= 2^32: products stay in [0, 2m), the inverse's words
+// below 4m and the forward's below 8m inside a unit and 6m between; RED marks the sums that would pass that.
+struct FullLimb {
+  Prime32 P;
+  template <bool RED>
+  __device__ __forceinline__ void fwd(u32& X, u32& Y, uint2 w) const {
+    const u32 x = P.csub(X), v = P.shoup(Y, w.x, w.y);
+    X = x + v;
+    Y = x + P.m - v;
+  }
+  template <bool RED>
+  __device__ __forceinline__ void inv(u32& X, u32& Y, uint2 f) const {
+    const u32 d = Y + P.m - X;
+    X = P.add(X, Y);
+    Y = P.shoup(d, f.x, f.y);
+  }
+  __device__ __forceinline__ u32 residue_inv(u32 x) const { return x; }
+  __device__ __forceinline__ u32 residue_fwd(u32 x) const { return P.csub(x); }
+};
+struct LazyLimb {
+  Prime32 P;
+  template <bool RED>
+  __device__ __forceinline__ void fwd(u32& X, u32& Y, uint2 w) const {
+    const u32 x = RED ? csub_by(X, 4 * P.m) : X, v = P.shoupl(Y, w.x, w.y);
+    X = x + v;
+    Y = x + 2 * P.m - v;
+  }
+  template <bool RED>
+  __device__ __forceinline__ void inv(u32& X, u32& Y, uint2 f) const {
+    const u32 d = Y + 4 * P.m - X, t = X + Y;
+    X = RED ? csub_by(t, 4 * P.m) : t;
+    Y = P.shoupl(d, f.x, f.y);
+  }
+  __device__ __forceinline__ u32 residue_inv(u32 x) const { return P.csub(csub_by(x, 2 * P.m)); }  // below 4m
+  __device__ __forceinline__ u32 residue_fwd(u32 x) const { return residue_inv(csub_by(x, 4 * P.m)); }
+};
+
+template <class L>
+__device__ __forceinline__ void fwd_unit8(const L& l, u32 (&x)[8], uint2 w0, const uint2 (&w1)[2], const uint2 (&w2)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) l.template fwd<false>(x[k], x[k + 4], w0);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    l.template fwd<true>(x[k], x[k + 2], w1[0]);
+    l.template fwd<true>(x[k + 4], x[k + 6], w1[1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) l.template fwd<true>(x[2 * k], x[2 * k + 1], w2[k]);
+}
+template <class L>
+__device__ __forceinline__ void inv_unit8(const L& l, u32 (&x)[8], const uint2 (&f0)[4], const uint2 (&f1)[2], uint2 f2) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) l.template inv<true>(x[2 * k], x[2 * k + 1], f0[k]);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    l.template inv<true>(x[4 * k], x[4 * k + 2], f1[k]);
+    l.template inv<false>(x[4 * k + 1], x[4 * k + 3], f1[k]);  // products below 2m
+  }
+  l.template inv<true>(x[0], x[4], f2);
+  l.template inv<true>(x[1], x[5], f2);
+  l.template inv<false>(x[2], x[6], f2);
+  l.template inv<false>(x[3], x[7], f2);
+}
+
+// Inverse stages 0-2 of thread tid's unit, from registers to buf.
+template <int LOGN, class L>
+__device__ __forceinline__ void inv_first8(const L& l, u32 (&x)[8], u32* buf, const uint2* tw) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  const int tid = threadIdx.x, r = E - 1 - tid;
+  uint2 f0[4], f1[2];
+#pragma unroll
+  for (int j = 0; j < 4; j++) f0[j] = tw[N / 2 + (3 - j) * E + r];
+#pragma unroll
+  for (int j = 0; j < 2; j++) f1[j] = tw[N / 4 + (1 - j) * E + r];
+  inv_unit8(l, x, f0, f1, tw[E + r]);
+#pragma unroll
+  for (int k = 0; k < 8; k += 4)
+    *reinterpret_cast<uint4*>(buf + sw(8 * tid + k)) = make_uint4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+}
+// Inverse stages S .. logn-3 (a multiple of three), a barrier after each pass.
+template <int LOGN, int S, class L>
+__device__ __forceinline__ void inv_middle8(const L& l, u32* buf, const uint2* tw) {
+  constexpr int N = 1 << LOGN;
+  if constexpr (S < LOGN - 2) {
+    constexpr int t = 1 << S, M = N >> (S + 1);
+    const int B = threadIdx.x >> S, e0 = B * 8 * t + (threadIdx.x & (t - 1));
+    uint2 f0[4], f1[2];
+#pragma unroll
+    for (int j = 0; j < 4; j++) f0[j] = tw[2 * M - 1 - 4 * B - j];
+#pragma unroll
+    for (int j = 0; j < 2; j++) f1[j] = tw[M - 1 - 2 * B - j];
+    u32 x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = buf[sw(e0 + k * t)];
+    inv_unit8(l, x, f0, f1, tw[M / 2 - 1 - B]);
+#pragma unroll
+    for (int k = 0; k < 8; k++) buf[sw(e0 + k * t)] = x[k];
+    __syncthreads();
+    inv_middle8<LOGN, S + 3>(l, buf, tw);
+  }
+}
+// Forward stages S .. logn-4, a barrier after each pass.
+template <int LOGN, int S, class L>
+__device__ __forceinline__ void fwd_middle8(const L& l, u32* buf, const uint2* tw) {
+  constexpr int N = 1 << LOGN;
+  if constexpr (S < LOGN - 3) {
+    constexpr int m = 1 << S, h = N >> (S + 3);
+    const int i = threadIdx.x / h, e0 = i * 8 * h + threadIdx.x % h;
+    uint2 w1[2], w2[4];
+#pragma unroll
+    for (int j = 0; j < 2; j++) w1[j] = tw[2 * m + 2 * i + j];
+#pragma unroll
+    for (int j = 0; j < 4; j++) w2[j] = tw[4 * m + 4 * i + j];
+    u32 x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = buf[sw(e0 + k * h)];
+    fwd_unit8(l, x, tw[m + i], w1, w2);
+#pragma unroll
+    for (int k = 0; k < 8; k++) buf[sw(e0 + k * h)] = x[k];
+    __syncthreads();
+    fwd_middle8<LOGN, S + 3>(l, buf, tw);
+  }
+}
+// The last three forward stages of thread tid's unit, to registers.
+template <int LOGN, class L>
+__device__ __forceinline__ void fwd_last8(const L& l, u32 (&x)[8], const u32* buf, const uint2* tw) {
+  constexpr int N = 1 << LOGN, E = N / 8;
+  const int tid = threadIdx.x;
+  uint2 w1[2], w2[4];
+#pragma unroll
+  for (int j = 0; j < 2; j++) w1[j] = tw[N / 4 + j * E + tid];
+#pragma unroll
+  for (int j = 0; j < 4; j++) w2[j] = tw[N / 2 + j * E + tid];
+#pragma unroll
+  for (int k = 0; k < 8; k += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(buf + sw(8 * tid + k));
+    x[k] = v.x, x[k + 1] = v.y, x[k + 2] = v.z, x[k + 3] = v.w;
+  }
+  fwd_unit8(l, x, tw[E + tid], w1, w2);
+}
+// The inverse's last two stages on words b + k N/4, the forward's first two.
+template <class L>
+__device__ __forceinline__ void inv_cross(const L& l, u32 (&x)[4], uint2 w1, uint2 w2, uint2 w3) {
+  l.template inv<true>(x[0], x[1], w3);
+  l.template inv<true>(x[2], x[3], w2);
+  l.template inv<true>(x[0], x[2], w1);
+  l.template inv<true>(x[1], x[3], w1);
+}
+template <class L>
+__device__ __forceinline__ void fwd_cross(const L& l, u32 (&x)[4], uint2 w1, uint2 w2, uint2 w3) {
+  l.template fwd<false>(x[0], x[2], w1);
+  l.template fwd<false>(x[1], x[3], w1);
+  l.template fwd<true>(x[0], x[1], w2);
+  l.template fwd<true>(x[2], x[3], w3);
+}
+
+// One CTA of N/8 threads per query, two on an SM. Each link i = gamma-2 .. 0 (server.rs:434-487):
 //   tp = NTT_p(lift(INTT_q(R_{i+1})));  cp = INTT_p(tp . w_p[tau_i]);  rq = NTT_q(lift(cp));
 //   R_i = a[tau_i] S_i + (R_{i+1} w_q[tau_i] - rq) / p;
 //   acc_q += R_{i+1} key_q[tau_i];  acc_p += tp key_p[tau_i].
-// Thread u owns slots 4u..4u+3 (one transform unit), so the passes that act within a unit
-// run in registers beside the pointwise steps: the first inverse pass of INTT_q, the last
-// forward pass of NTT_p with the products by key_p and w_p and the first inverse pass of
-// INTT_p, and the last forward pass of NTT_q with the link's update. Each inverse's last
-// stage (t = n/2, carrying 1/n), the limb lift and the next forward's first stage (the
-// same index pairs) run as one pass in place.
+// Thread u owns slots 8u..8u+7. Its unit's stages run in registers beside the pointwise steps; each inverse's last
+// two stages, the limb lift and the next forward's first two are one pass in place over the words b + k N/4.
+// The kernel holds c_i = n^-1 R_i, so the inverses need no 1/n: a and w_q are scaled by n^-1 and 1/p, w_p by n^-1
+// and key_q by n when they are staged, rq takes one product by 1/(n p).
 //
-// Twiddle products are Shoup products against the forward ladders' (w, w') pairs (the
-// inverse ladders derived from them by inv_tw); products by R-form operands are
-// Montgomery products.
-//
-// LAZY (q below 2^29, so 8q < 2^32): the q-limb passes skip most reductions. montl and
-// shoupl leave [0, 2q) for any 32-bit left operand, and the values between passes stay in [0, 4q)
-// through INTT_q and in [0, 6q) through NTT_q; every sum and every difference (offset by
-// 2q or 4q) stays below 8q. Values are brought to [0, q) where the arithmetic needs a
-// residue: before the lift to p and at the end of the chain. The p limb (near 2^31) has
-// no headroom and stays reduced.
+// Against radix-4 passes on N/4 threads: 12 barriers a link instead of 20, under half the shared-memory
+// wavefronts (7,240 a link, a third of them bank conflicts, filled 65% of the time), no product by 1/n.
 template <int LOGN, bool LAZY>
-__global__ void __launch_bounds__((1 << LOGN) / 4, 2)
+__global__ void __launch_bounds__((1 << LOGN) / 8, 2)
     k_sm_respond(SmDev c, const SmQueryDev* queries, const i64* fold, u32* mask_out, u32* body_out, u32* status) {
-  constexpr int N = 1 << LOGN, NT = N / 4, H = N / 2;
+  constexpr int N = 1 << LOGN, NT = N / 8, P4 = N / 4;
   constexpr u32 M2N = 2 * N - 1;
+  using QLimb = std::conditional_t<LAZY, LazyLimb, FullLimb>;
   extern __shared__ __align__(16) u32 smw[];
   u32* buf = smw;
-  u32* a = smw + N;
-  u32* kq = smw + 2 * N;
-  u32* kp = smw + 3 * N;
-  u32* wq = smw + 4 * N;
-  u32* wp = smw + 5 * N;
-  uint2* fqs = reinterpret_cast<uint2*>(smw + 6 * N);  // forward ladders with Shoup companions
-  uint2* fps = reinterpret_cast<uint2*>(smw + 8 * N);
-  uint16_t* e_tab = reinterpret_cast<uint16_t*>(smw + 10 * N);
-  uint16_t* s_tab = e_tab + N;
+  u32* a = smw + N;                                    // n^-1 a, by gather position
+  uint4* keys = reinterpret_cast<uint4*>(smw + 2 * N);  // n key_q, w_q / p, key_p, w_p / n (R-form), by position
+  uint2* fq = reinterpret_cast<uint2*>(smw + 6 * N);   // forward ladders with Shoup companions
+  uint2* fp = reinterpret_cast<uint2*>(smw + 8 * N);
+  uint16_t* s_tab = reinterpret_cast<uint16_t*>(smw + 10 * N);
   const int tid = threadIdx.x;
   const u32 qi = blockIdx.x;
   const SmQueryDev qd = queries[qi];
   const Prime32 PQ = c.lq.p, PP = c.lp.p;
+  const QLimb lq{PQ};
+  const FullLimb lp{PP};
   for (int k = tid; k < N; k += NT) {
-    kq[k] = qd.seat[k];
-    kp[k] = qd.seat[N + k];
-    wq[k] = qd.seat[2 * N + k];
-    wp[k] = qd.seat[3 * N + k];
-    fqs[k] = c.lq.fwd_sh[k];
-    fps[k] = c.lp.fwd_sh[k];
-    e_tab[k] = c.slot_exp[k];
-    s_tab[k] = c.exp_slot[k];
+    keys[slot_at<LOGN>(k)] =
+        make_uint4(PQ.mont(qd.seat[k], c.n_R), PQ.mont(qd.seat[2 * N + k], c.p_inv_R), qd.seat[N + k],
+                   PP.mont(qd.seat[3 * N + k], c.lp.n_inv));
+    fq[ladder_at<LOGN>(k)] = c.lq.fwd_sh[k];
+    fp[ladder_at<LOGN>(k)] = c.lp.fwd_sh[k];
+    s_tab[k] = (uint16_t)slot_at<LOGN>(c.exp_slot[k]);
   }
-  sm_expand<N, NT>(qd, PQ.m, a, status, qi);
-  fwd32<LOGN>(a, c.lq, c.lq.fwd);
-
-  const int l0 = 4 * tid;
-  u32 cur[4], accq[4], accp[4], et[4];
+  sm_expand<N, NT>(qd, PQ.m, buf, status, qi);  // ends with a barrier
+  const uint2 wq1 = fq[1], wq2 = fq[2], wq3 = fq[3], wp1 = fp[1], wp2 = fp[2], wp3 = fp[3];
+  {
+    u32 y[2][4];  // read before any is rewritten at its swizzled place
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    et[k] = e_tab[l0 + k];
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) y[r][k] = buf[tid + r * NT + k * P4];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      fwd_cross(lq, y[r], wq1, wq2, wq3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) buf[sw(tid + r * NT + k * P4)] = y[r][k];
+    }
+    __syncthreads();
+    fwd_middle8<LOGN, 2>(lq, buf, fq);
+    u32 x[8];
+    fwd_last8<LOGN>(lq, x, buf, fq);
+#pragma unroll
+    for (int k = 0; k < 8; k++) a[k * NT + tid] = PQ.mont(lq.residue_fwd(x[k]), c.lq.n_inv);
+    __syncthreads();
+  }
+  const int l0 = 8 * tid;
+  u32 cur[8], accq[8], accp[8], et[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    et[k] = c.slot_exp[l0 + k];
     const u32 tb = s_tab[((c.gpow[c.gamma - 1] * et[k]) & M2N) >> 1];
     cur[k] = PQ.mont(a[tb], qd.step1_R[(size_t)(c.gamma - 1) * N + l0 + k]);
     accq[k] = 0;
     accp[k] = 0;
   }
-  // Inverse stages 0-1 of unit tid (t = 1, block tid), in registers, to buf[l0..l0+3].
-  auto inv_first = [&](const Prime32& P, const uint2* fs, u32 a0, u32 a1, u32 a2, u32 a3) {
-    const uint2 w0 = inv_tw(fs, P.m, H + 2 * tid), w1 = inv_tw(fs, P.m, H + 2 * tid + 1),
-                w2 = inv_tw(fs, P.m, H / 2 + tid);
-    const u32 d01 = P.shoup(a0 + P.m - a1, w0.x, w0.y);
-    a0 = P.add(a0, a1);
-    const u32 d23 = P.shoup(a2 + P.m - a3, w1.x, w1.y);
-    a2 = P.add(a2, a3);
-    *reinterpret_cast<uint4*>(buf + l0) = make_uint4(P.add(a0, a2), P.add(d01, d23), P.shoup(a0 + P.m - a2, w2.x, w2.y),
-                                                     P.shoup(d01 + P.m - d23, w2.x, w2.y));
-  };
-  // Inverse stages 2 .. logn-2 over buf (radix-4 pairs; logn is odd).
-  auto inv_middle = [&](const Prime32& P, const uint2* fs) {
-#pragma unroll 1
-    for (int s = 2; s + 1 < LOGN; s += 2) {
-      const int t = 1 << s, m = N >> (s + 1);
-      const int B = tid >> s, o = tid & (t - 1);
-      const int e0 = B * 4 * t + o;
-      const uint2 w0 = inv_tw(fs, P.m, m + 2 * B), w1 = inv_tw(fs, P.m, m + 2 * B + 1),
-                  w2 = inv_tw(fs, P.m, (m >> 1) + B);
-      u32 a0 = buf[e0], a1 = buf[e0 + t], a2 = buf[e0 + 2 * t], a3 = buf[e0 + 3 * t];
-      const u32 d01 = P.shoup(a0 + P.m - a1, w0.x, w0.y);
-      a0 = P.add(a0, a1);
-      const u32 d23 = P.shoup(a2 + P.m - a3, w1.x, w1.y);
-      a2 = P.add(a2, a3);
-      buf[e0] = P.add(a0, a2);
-      buf[e0 + 2 * t] = P.shoup(a0 + P.m - a2, w2.x, w2.y);
-      buf[e0 + t] = P.add(d01, d23);
-      buf[e0 + 3 * t] = P.shoup(d01 + P.m - d23, w2.x, w2.y);
-      __syncthreads();
-    }
-  };
-  // Forward stages 1 .. logn-3 over buf.
-  auto fwd_middle = [&](const Prime32& P, const uint2* fs) {
-#pragma unroll 1
-    for (int s = 1; s < LOGN - 2; s += 2) {
-      const int t = N >> (s + 1), m = 1 << s, h = t >> 1;
-      const int i = tid / h, o = tid - i * h;
-      const int e0 = i * 2 * t + o;
-      const uint2 wa = fs[m + i], wb = fs[2 * m + 2 * i], wc = fs[2 * m + 2 * i + 1];
-      u32 a0 = buf[e0], a1 = buf[e0 + h], a2 = buf[e0 + t], a3 = buf[e0 + t + h];
-      u32 v = P.shoup(a2, wa.x, wa.y);
-      a2 = P.sub(a0, v);
-      a0 = P.add(a0, v);
-      v = P.shoup(a3, wa.x, wa.y);
-      a3 = P.sub(a1, v);
-      a1 = P.add(a1, v);
-      v = P.shoup(a1, wb.x, wb.y);
-      buf[e0] = P.add(a0, v);
-      buf[e0 + h] = P.sub(a0, v);
-      v = P.shoup(a3, wc.x, wc.y);
-      buf[e0 + t] = P.add(a2, v);
-      buf[e0 + t + h] = P.sub(a2, v);
-      __syncthreads();
-    }
-  };
-  // Forward stages logn-2, logn-1 of unit tid, in registers, from buf[l0..l0+3].
-  auto fwd_last = [&](const Prime32& P, const uint2* fs, u32 (&x)[4]) {
-    constexpr int MF = 1 << (LOGN - 2);
-    const uint2 wa = fs[MF + tid], wb = fs[2 * MF + 2 * tid], wc = fs[2 * MF + 2 * tid + 1];
-    const uint4 v4 = *reinterpret_cast<const uint4*>(buf + l0);
-    u32 a0 = v4.x, a1 = v4.y, a2 = v4.z, a3 = v4.w;
-    u32 v = P.shoup(a2, wa.x, wa.y);
-    a2 = P.sub(a0, v);
-    a0 = P.add(a0, v);
-    v = P.shoup(a3, wa.x, wa.y);
-    a3 = P.sub(a1, v);
-    a1 = P.add(a1, v);
-    v = P.shoup(a1, wb.x, wb.y);
-    x[0] = P.add(a0, v);
-    x[1] = P.sub(a0, v);
-    v = P.shoup(a3, wc.x, wc.y);
-    x[2] = P.add(a2, v);
-    x[3] = P.sub(a2, v);
-  };
-  const u32 Q2 = 2 * PQ.m, Q4 = 4 * PQ.m, Q6 = 6 * PQ.m;
-  // Lazy INTT_q passes: inputs below 4q, outputs below 4q (three reductions per unit).
-  auto inv_unit_lazy = [&](uint2 w0, uint2 w1, uint2 w2, u32& a0, u32& a1, u32& a2, u32& a3) {
-    const u32 d01 = PQ.shoupl(a0 + Q4 - a1, w0.x, w0.y);
-    const u32 s01 = csub_by(a0 + a1, Q4);
-    const u32 d23 = PQ.shoupl(a2 + Q4 - a3, w1.x, w1.y);
-    const u32 s23 = csub_by(a2 + a3, Q4);
-    a0 = csub_by(s01 + s23, Q4);
-    a2 = PQ.shoupl(s01 + Q4 - s23, w2.x, w2.y);
-    a1 = d01 + d23;
-    a3 = PQ.shoupl(d01 + Q2 - d23, w2.x, w2.y);
-  };
-  auto inv_first_lazy = [&](u32 a0, u32 a1, u32 a2, u32 a3) {
-    inv_unit_lazy(inv_tw(fqs, PQ.m, H + 2 * tid), inv_tw(fqs, PQ.m, H + 2 * tid + 1), inv_tw(fqs, PQ.m, H / 2 + tid), a0,
-                  a1, a2, a3);
-    *reinterpret_cast<uint4*>(buf + l0) = make_uint4(a0, a1, a2, a3);
-  };
-  auto inv_middle_lazy = [&]() {
-#pragma unroll 1
-    for (int s = 2; s + 1 < LOGN; s += 2) {
-      const int t = 1 << s, m = N >> (s + 1);
-      const int B = tid >> s, o = tid & (t - 1);
-      const int e0 = B * 4 * t + o;
-      u32 a0 = buf[e0], a1 = buf[e0 + t], a2 = buf[e0 + 2 * t], a3 = buf[e0 + 3 * t];
-      inv_unit_lazy(inv_tw(fqs, PQ.m, m + 2 * B), inv_tw(fqs, PQ.m, m + 2 * B + 1), inv_tw(fqs, PQ.m, (m >> 1) + B), a0,
-                    a1, a2, a3);
-      buf[e0] = a0;
-      buf[e0 + t] = a1;
-      buf[e0 + 2 * t] = a2;
-      buf[e0 + 3 * t] = a3;
-      __syncthreads();
-    }
-  };
-  // Lazy NTT_q passes: inputs below 6q, outputs below 6q (two reductions per unit).
-  auto fwd_unit_lazy = [&](uint2 wa, uint2 wb, uint2 wc, u32& a0, u32& a1, u32& a2, u32& a3) {
-    u32 v = PQ.shoupl(a2, wa.x, wa.y);
-    a2 = a0 + Q2 - v;  // below 8q
-    a0 = a0 + v;
-    v = PQ.shoupl(a3, wa.x, wa.y);
-    a3 = a1 + Q2 - v;
-    a1 = a1 + v;
-    a0 = csub_by(a0, Q4);  // below 4q
-    v = PQ.shoupl(a1, wb.x, wb.y);
-    a1 = a0 + Q2 - v;
-    a0 = a0 + v;
-    a2 = csub_by(a2, Q4);
-    v = PQ.shoupl(a3, wc.x, wc.y);
-    a3 = a2 + Q2 - v;
-    a2 = a2 + v;
-  };
-  auto fwd_middle_lazy = [&]() {
-#pragma unroll 1
-    for (int s = 1; s < LOGN - 2; s += 2) {
-      const int t = N >> (s + 1), m = 1 << s, h = t >> 1;
-      const int i = tid / h, o = tid - i * h;
-      const int e0 = i * 2 * t + o;
-      u32 a0 = buf[e0], a1 = buf[e0 + h], a2 = buf[e0 + t], a3 = buf[e0 + t + h];
-      fwd_unit_lazy(fqs[m + i], fqs[2 * m + 2 * i], fqs[2 * m + 2 * i + 1], a0, a1, a2, a3);
-      buf[e0] = a0;
-      buf[e0 + h] = a1;
-      buf[e0 + t] = a2;
-      buf[e0 + t + h] = a3;
-      __syncthreads();
-    }
-  };
 #pragma unroll 1
   for (int i = (int)c.gamma - 2; i >= 0; i--) {
-    const uint4 sv4 = *reinterpret_cast<const uint4*>(qd.step1_R + (size_t)i * N + l0);
-    const u32 sv[4] = {sv4.x, sv4.y, sv4.z, sv4.w};
-    u32 tb[4];
+    const uint4* Srow = reinterpret_cast<const uint4*>(qd.step1_R + (size_t)i * N + l0);
+    const uint4 s0 = Srow[0], s1 = Srow[1];
     const u32 gp = c.gpow[i];
-#pragma unroll
-    for (int k = 0; k < 4; k++) tb[k] = s_tab[((gp * et[k]) & M2N) >> 1];
-    if constexpr (LAZY) {
-      inv_first_lazy(cur[0], cur[1], cur[2], cur[3]);
-      __syncthreads();
-      inv_middle_lazy();
-    } else {
-      inv_first(PQ, fqs, cur[0], cur[1], cur[2], cur[3]);
-      __syncthreads();
-      inv_middle(PQ, fqs);
-    }
-    // INTT_q's last stage with 1/n, the lift to p, and NTT_p's first stage, pair (b, b + n/2).
-    // The lift takes residues, so both products are reduced fully here.
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int b = tid + r * NT;
-      const u32 u = buf[b], v = buf[b + H];
-      const u32 y0 = q_to_p(c, PQ.shoup(u + v, c.lq.n_inv_s, c.lq.n_inv_sp));
-      const u32 y1 = q_to_p(c, PQ.shoup(u + (LAZY ? Q4 : PQ.m) - v, c.lq.last_s, c.lq.last_sp));
-      const u32 z = PP.shoup(y1, fps[1].x, fps[1].y);
-      buf[b] = PP.add(y0, z);
-      buf[b + H] = PP.sub(y0, z);
-    }
-    __syncthreads();
-    fwd_middle(PP, fps);
     {
-      u32 tp[4], y[4];
-      fwd_last(PP, fps, tp);
+      u32 x[8];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        accp[k] = PP.add(accp[k], PP.mont(tp[k], kp[tb[k]]));
-        y[k] = PP.mont(tp[k], wp[tb[k]]);
-      }
-      inv_first(PP, fps, y[0], y[1], y[2], y[3]);
+      for (int k = 0; k < 8; k++) x[k] = cur[k];
+      inv_first8<LOGN>(lq, x, buf, fq);
     }
     __syncthreads();
-    inv_middle(PP, fps);
-    // INTT_p's last stage with 1/n, the lift to q, and NTT_q's first stage.
+    inv_middle8<LOGN, 3>(lq, buf, fq);
+    // INTT_q's end, the lift to p (of residues), NTT_p's start.
 #pragma unroll
     for (int r = 0; r < 2; r++) {
       const int b = tid + r * NT;
-      const u32 u = buf[b], v = buf[b + H];
-      const u32 xp0 = PP.shoup(u + v, c.lp.n_inv_s, c.lp.n_inv_sp);
-      const u32 xp1 = PP.shoup(u + PP.m - v, c.lp.last_s, c.lp.last_sp);
-      if constexpr (LAZY) {
-        const u32 y0 = p_to_q_lazy(c, xp0);  // below 3q
-        const u32 z = PQ.shoupl(p_to_q_lazy(c, xp1), fqs[1].x, fqs[1].y);
-        buf[b] = y0 + z;  // below 5q
-        buf[b + H] = y0 + Q2 - z;
-      } else {
-        const u32 y0 = p_to_q(c, xp0), y1 = p_to_q(c, xp1);
-        const u32 z = PQ.shoup(y1, fqs[1].x, fqs[1].y);
-        buf[b] = PQ.add(y0, z);
-        buf[b + H] = PQ.sub(y0, z);
-      }
+      u32 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = buf[sw(b + k * P4)];
+      inv_cross(lq, x, wq1, wq2, wq3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = q_to_p(c, lq.residue_inv(x[k]));
+      fwd_cross(lp, x, wp1, wp2, wp3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) buf[sw(b + k * P4)] = x[k];
     }
     __syncthreads();
-    u32 rq[4];
-    if constexpr (LAZY) {
-      fwd_middle_lazy();
-      constexpr int MF = 1 << (LOGN - 2);
-      const uint4 v4 = *reinterpret_cast<const uint4*>(buf + l0);
-      rq[0] = v4.x, rq[1] = v4.y, rq[2] = v4.z, rq[3] = v4.w;
-      fwd_unit_lazy(fqs[MF + tid], fqs[2 * MF + 2 * tid], fqs[2 * MF + 2 * tid + 1], rq[0], rq[1], rq[2], rq[3]);
-      // cur below 4q, rq below 6q: R_i = a S_i + (cur w_q - rq) / p lands below 4q, acc_q
-      // stays below 2q.
+    fwd_middle8<LOGN, 2>(lp, buf, fp);
+    {
+      u32 tp[8];
+      fwd_last8<LOGN>(lp, tp, buf, fp);
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const u32 cq = PQ.montl(cur[k], wq[tb[k]]);
-        accq[k] = csub_by(accq[k] + PQ.montl(cur[k], kq[tb[k]]), Q2);
-        cur[k] = PQ.montl(a[tb[k]], sv[k]) + PQ.montl(cq + Q6 - rq[k], c.p_inv_R);
+      for (int k = 0; k < 8; k++) {
+        const uint4 key = keys[s_tab[((gp * et[k]) & M2N) >> 1]];
+        accp[k] = PP.add(accp[k], PP.mont(tp[k], key.z));
+        tp[k] = PP.mont(tp[k], key.w);
       }
+      inv_first8<LOGN>(lp, tp, buf, fp);
+    }
+    __syncthreads();
+    inv_middle8<LOGN, 3>(lp, buf, fp);
+    // INTT_p's end, the lift to q, NTT_q's start.
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int b = tid + r * NT;
+      u32 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = buf[sw(b + k * P4)];
+      inv_cross(lp, x, wp1, wp2, wp3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = LAZY ? p_to_q_lazy(c, x[k]) : p_to_q(c, x[k]);
+      fwd_cross(lq, x, wq1, wq2, wq3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) buf[sw(b + k * P4)] = x[k];
+    }
+    __syncthreads();
+    fwd_middle8<LOGN, 2>(lq, buf, fq);
+    u32 rq[8];
+    fwd_last8<LOGN>(lq, rq, buf, fq);
+    const u32 sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
+      const uint2 key = *reinterpret_cast<const uint2*>(keys + tb);
+      if constexpr (LAZY) {
+        // Products below 2q each: c_i = n^-1 a S + c_{i+1} w_q / p - rq / (n p) below 6q, brought below 4q.
+        accq[k] = csub_by(accq[k] + PQ.montl(cur[k], key.x), 2 * PQ.m);
+        cur[k] = csub_by(PQ.montl(a[tb], sv[k]) + PQ.montl(cur[k], key.y) + 2 * PQ.m -
+                             PQ.shoupl(rq[k], c.np_inv_s, c.np_inv_sp),
+                         4 * PQ.m);
+      } else {
+        accq[k] = PQ.add(accq[k], PQ.mont(cur[k], key.x));
+        cur[k] = PQ.add(PQ.mont(a[tb], sv[k]),
+                        PQ.sub(PQ.mont(cur[k], key.y), PQ.shoup(rq[k], c.np_inv_s, c.np_inv_sp)));
+      }
+    }
+  }
+  // mask = INTT_q(R_0); body = mod_down(INTT_q(acc_q), INTT_p(acc_p)) + fold. No thread touches another's unit
+  // of buf before the first barrier of a transform.
+  u32 xq[2][4];
+#pragma unroll 1
+  for (int part = 0; part < 3; part++) {
+    u32 x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = part == 0 ? cur[k] : part == 1 ? accq[k] : accp[k];
+    if (part < 2) {
+      inv_first8<LOGN>(lq, x, buf, fq);
+      __syncthreads();
+      inv_middle8<LOGN, 3>(lq, buf, fq);
     } else {
-      fwd_middle(PQ, fqs);
-      fwd_last(PQ, fqs, rq);
+      inv_first8<LOGN>(lp, x, buf, fp);
+      __syncthreads();
+      inv_middle8<LOGN, 3>(lp, buf, fp);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int b = tid + r * NT;
+      u32 y[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) y[k] = buf[sw(b + k * P4)];
+      if (part < 2)
+        inv_cross(lq, y, wq1, wq2, wq3);
+      else
+        inv_cross(lp, y, wp1, wp2, wp3);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const u32 cq = PQ.mont(cur[k], wq[tb[k]]);
-        accq[k] = PQ.add(accq[k], PQ.mont(cur[k], kq[tb[k]]));
-        cur[k] = PQ.add(PQ.mont(a[tb[k]], sv[k]), PQ.mont(PQ.sub(cq, rq[k]), c.p_inv_R));
+        const int t = b + k * P4;
+        if (part == 0) {
+          mask_out[(size_t)qi * N + t] = lq.residue_inv(y[k]);
+        } else if (part == 1) {
+          xq[r][k] = PQ.mont(lq.residue_inv(y[k]), c.lq.n_inv);
+        } else if ((u32)t < c.nb) {
+          const u32 down = PQ.mont(PQ.sub(xq[r][k], p_to_q(c, PP.mont(y[k], c.lp.n_inv))), c.p_inv_R);
+          const i64* chunk = fold + (size_t)qi * SM_FOLD_CHUNKS * c.gamma + t;
+          i64 f = 0;
+          for (int j = 0; j < SM_FOLD_CHUNKS; j++) f += chunk[j * c.gamma];
+          f %= (i64)PQ.m;
+          if (f < 0) f += PQ.m;
+          body_out[(size_t)qi * c.nb + t] = PQ.add(down, (u32)f);
+        }
       }
     }
-  }
-  if constexpr (LAZY) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      cur[k] = PQ.csub(csub_by(cur[k], Q2));
-      accq[k] = PQ.csub(accq[k]);
-    }
-  }
-  // mask = INTT_q(R_0); body = mod_down(INTT_q(acc_q), INTT_p(acc_p)) + fold.
-  __syncthreads();  // every thread is past its last read of buf
-#pragma unroll
-  for (int k = 0; k < 4; k++) buf[l0 + k] = cur[k];
-  __syncthreads();
-  inv32<LOGN>(buf, c.lq, c.lq.inv);
-#pragma unroll
-  for (int k = 0; k < 4; k++) mask_out[(size_t)qi * N + tid + k * NT] = buf[tid + k * NT];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; k++) buf[l0 + k] = accq[k];
-  __syncthreads();
-  inv32<LOGN>(buf, c.lq, c.lq.inv);
-  u32 xq[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) xq[k] = buf[tid + k * NT];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; k++) buf[l0 + k] = accp[k];
-  __syncthreads();
-  inv32<LOGN>(buf, c.lp, c.lp.inv);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int t = tid + k * NT;
-    if ((u32)t < c.nb) {
-      const u32 down = PQ.mont(PQ.sub(xq[k], p_to_q(c, buf[t])), c.p_inv_R);
-      i64 f = fold[(size_t)qi * c.nb + t] % (i64)PQ.m;
-      if (f < 0) f += PQ.m;
-      body_out[(size_t)qi * c.nb + t] = PQ.add(down, (u32)f);
-    }
+    __syncthreads();  // buf is rewritten by the next part
   }
 }
 
@@ -630,7 +653,9 @@ cudaError_t table_fold(const SmDev& c, const u32* H, u32* step1_R, cudaStream_t 
 cudaError_t body_fold(const SmDev& c, const SmQueryDev* queries, u32 nq, i64* fold, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   if (c.nb > 512) return cudaErrorInvalidValue;
-  k_sm_body_fold<<<nq, 512, 0, s>>>(c, queries, fold);
+  // Only the first nb columns reach a response: 512 at most.
+  const u32 lanes = c.gamma < 4 ? 1 : (c.gamma < 512 ? c.gamma : 512) / 4;
+  k_sm_body_fold<<<dim3(nq, SM_FOLD_CHUNKS), SM_FOLD_ROWS * lanes, 0, s>>>(c, queries, fold);
   return cudaGetLastError();
 }
 
@@ -638,13 +663,13 @@ cudaError_t respond(const SmDev& c, const SmQueryDev* queries, u32 nq, const i64
                     u32* status, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   if (c.logn != 11) return cudaErrorInvalidValue;
-  const size_t smem = (10 * (size_t)c.n) * 4 + 2 * (size_t)c.n * 2;
+  const size_t smem = (10 * (size_t)c.n) * 4 + (size_t)c.n * 2;
   // The lazy q-limb passes need every value below 8q to fit 32 bits.
   const bool lazy = (u64)c.lq.p.m * 8 <= (1ULL << 32);
   auto kern = lazy ? k_sm_respond<11, true> : k_sm_respond<11, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<nq, 512, smem, s>>>(c, queries, fold, mask_out, body_out, status);
+  kern<<<nq, 256, smem, s>>>(c, queries, fold, mask_out, body_out, status);
   return cudaGetLastError();
 }
 

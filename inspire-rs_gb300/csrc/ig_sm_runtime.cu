@@ -299,21 +299,6 @@ int ig_sm_server_create(ig_ctx* c, uint32_t ring_dim, uint32_t gamma, uint64_t q
   dv.lp.p = Prime32{(u32)special_prime, hp.neg_minv};
   dv.lq.n_inv = hq.n_inv;
   dv.lp.n_inv = hp.n_inv;
-  // last = mont(inv[1], n_inv) = inv[1] n_inv 2^-32
-  dv.lq.last = dv.lq.p.mont(hq.inv[1], hq.n_inv);
-  dv.lp.last = dv.lp.p.mont(hp.inv[1], hp.n_inv);
-  // Standard-form Shoup pairs of the same: 1/n, and 1/n (m - fwd[1]) (the inverse's last
-  // twiddle is the negated second forward one).
-  for (Ntt32Dev* T : {&dv.lq, &dv.lp}) {
-    const HostNtt32& H = T == &dv.lq ? hq : hp;
-    const u64 m = H.m;
-    const u64 ninv = powm(H.n % m, m - 2, m);
-    const u64 last = ninv * ((m - H.fwd_std[1]) % m) % m;
-    T->n_inv_s = (u32)ninv;
-    T->n_inv_sp = (u32)((ninv << 32) / m);
-    T->last_s = (u32)last;
-    T->last_sp = (u32)((last << 32) / m);
-  }
   // The forward ladders as (w, floor(w 2^32 / m)) pairs for Shoup products.
   auto shoup_ladder = [](const HostNtt32& T) {
     std::vector<u32> v(2 * T.n);
@@ -342,6 +327,9 @@ int ig_sm_server_create(ig_ctx* c, uint32_t ring_dim, uint32_t gamma, uint64_t q
   dv.neg_off = (u32)((q - special_prime % q) % q);
   dv.q_mu = (u32)((1ULL << 32) / q);
   dv.p_inv_R = (u32)(((u128)powm(special_prime % q, q - 2, q) << 32) % q);
+  dv.n_R = (u32)(((u128)d << 32) % q);
+  dv.np_inv_s = (u32)powm((u64)d * (special_prime % q) % q, q - 2, q);
+  dv.np_inv_sp = (u32)(((u64)dv.np_inv_s << 32) / q);
   SmState& st = state(c);
   const u64 h = st.next++;
   st.servers[h] = o;
@@ -538,7 +526,7 @@ int ig_sm_respond_batch(ig_ctx* c, uint64_t server, uint32_t count, const uint64
   if ((rc = lane_scratch("sm_q", count * sizeof(SmQueryDev), &dq)) ||
       (rc = lane_scratch("sm_seeds", count * 32, &dseeds)) ||
       (rc = lane_scratch("sm_bodies", count * d * 4, &dbodies)) ||
-      (rc = lane_scratch("sm_fold", count * nb * 8, &dfold)) ||
+      (rc = lane_scratch("sm_fold", (size_t)count * igsmk::SM_FOLD_CHUNKS * o->dev.gamma * 8, &dfold)) ||
       (rc = lane_scratch("sm_mask", count * d * 4, &dmask)) ||
       (rc = lane_scratch("sm_body", count * nb * 4, &dbody)) ||
       (rc = lane_scratch("sm_status", count * 4, &dstatus)))
@@ -601,7 +589,7 @@ int ig_sm_respond_batch_device(ig_ctx* c, uint64_t server, uint32_t count, const
   snprintf(fname, sizeof fname, "smd_fold%d", lane);
   void *dq, *dfold;
   if ((rc = igint::scratch(c, qname, count * sizeof(SmQueryDev), &dq)) ||
-      (rc = igint::scratch(c, fname, count * nb * 8, &dfold)))
+      (rc = igint::scratch(c, fname, (size_t)count * igsmk::SM_FOLD_CHUNKS * o->dev.gamma * 8, &dfold)))
     return rc;
   for (u32 i = 0; i < count; i++) {
     qs[i].seed = (const u32*)(d_seeds + (size_t)i * 32);
