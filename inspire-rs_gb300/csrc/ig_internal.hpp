@@ -63,7 +63,39 @@ int lanes(ig_ctx* c);
 struct HostCall {
   unsigned k = 0;
   std::unique_lock<std::mutex> lane_lock;
+  cudaStream_t queued[2] = {};  // streams with copies of this call's host memory in flight
+  ~HostCall() {
+    for (cudaStream_t s : queued)
+      if (s) cudaStreamSynchronize(s);
+  }
 };
+// A host-buffer call's arrays: one device block (scratch of the lane) and its image in the lane's pinned buffer, in this
+// order, so the small arrays cross in one copy each way (a lone query of gamma 16 131 -> 120 us, where seven copies and a
+// memset went around its two launches). Arrays of COPY_DIRECT_BYTES and more are copied straight between the caller's memory and the device where the
+// GPU reads pageable memory through the host's page tables (an MB in 16 us, against 50 in and 71 out through the pinned
+// image; below 256 KB the image's copy is the shorter). A caller's result memory that no one has touched yet costs the
+// direct copy 180 us an MB in faults that the CPU takes in 10: wait() touches it while the device works. 64 queries
+// 1.455 -> 1.285 ms, 128 mixed ones 5.00 -> 4.46 ms, 256 special_modulus ones 4.43 -> 4.07 ms.
+constexpr size_t COPY_DIRECT_BYTES = 256 << 10;
+struct HostIO {
+  size_t table, queries, work, seeds, bs, status, a, b, end;  // offsets
+  size_t table_bytes, query_bytes, work_bytes, seed_bytes, bs_bytes, status_bytes, a_bytes, b_bytes;
+  uint8_t *dev, *pin;
+};
+// Lays the block out (byte counts in its order; status words are `count`) and allocates it.
+int host_io_open(ig_ctx* c, HostCall& hc, HostIO& io, size_t table, size_t queries, size_t work, size_t seeds, size_t bs,
+                 size_t count, size_t a, size_t b);
+// Queues the inputs and zeroed status words on the call's stream, after all context-stream work so far.
+int host_io_send(ig_ctx* c, HostCall& hc, HostIO& io, const void* table, const void* queries, const void* work,
+                 const void* seeds, const void* bs);
+// Queues the results' copies after the launches; under the context lock.
+int host_io_receive(ig_ctx* c, HostCall& hc, HostIO& io);
+// Waits for them (without the context lock). The status words are then at pin + status.
+int host_io_wait(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out);
+// Hands the results over: called once the status words are found clean, so a refused call writes no results.
+int host_io_finish(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out);
+// The lane's copy stream, ordered after nothing: copies that wait for the call's own events alone.
+cudaStream_t host_call_copy_stream(ig_ctx* c, HostCall& hc);
 void host_call_begin(ig_ctx* c, HostCall& hc);
 int host_call_pinned(ig_ctx* c, HostCall& hc, size_t bytes, void** pin);
 cudaStream_t host_call_stream(ig_ctx* c, HostCall& hc);

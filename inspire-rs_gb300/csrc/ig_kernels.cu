@@ -2412,27 +2412,30 @@ cudaError_t compact16(const u64* cols, size_t words, uint16_t* out, u32* wide, c
   return cudaGetLastError();
 }
 
-cudaError_t nopack(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 r_mod_q,
-                   u64* AB_R, u64* out, u32* status, cudaStream_t s) {
+cudaError_t nopack_prep(const CrsDev& c, const QueryDev* queries, u32 nq, u64 r_mod_q, u64* AB_R, u32* status,
+                        cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
+  const size_t smem = 4 * (size_t)c.n * 8;
   IG_DISPATCH_LOGN(c.logn, {
-    constexpr int N = 1 << L;
-    {
-      auto k = k_nopack_prep<L>;
-      const size_t smem = 4 * (size_t)N * 8;
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      k<<<nq, N / 4, smem, s>>>(c, queries, make_tw(r_mod_q), AB_R, status);
-    }
-    {
-      auto k = k_nopack_cols<L>;
-      const size_t smem = 5 * (size_t)N * 8;
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      k<<<dim3(c.gamma, nq), N / 4, smem, s>>>(c, queries, shards, AB_R, out);
-    }
-    k_nopack_sum<<<dim3((2 * N + 255) / 256, nq), 256, 0, s>>>(N, c.gamma, out);
+    auto k = k_nopack_prep<L>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<nq, (1 << L) / 4, smem, s>>>(c, queries, make_tw(r_mod_q), AB_R, status);
   });
+  return cudaGetLastError();
+}
+
+cudaError_t nopack_cols(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u64* AB_R,
+                        u64* out, cudaStream_t s) {
+  if (nq == 0) return cudaSuccess;
+  const size_t smem = 5 * (size_t)c.n * 8;
+  IG_DISPATCH_LOGN(c.logn, {
+    auto k = k_nopack_cols<L>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(c.gamma, nq), (1 << L) / 4, smem, s>>>(c, queries, shards, AB_R, out);
+  });
+  k_nopack_sum<<<dim3((2 * c.n + 255) / 256, nq), 256, 0, s>>>(c.n, c.gamma, out);
   return cudaGetLastError();
 }
 

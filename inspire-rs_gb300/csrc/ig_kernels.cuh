@@ -153,11 +153,12 @@ cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* sh
 
 size_t respond_smem_bytes(const CrsDev& c, int ctas);
 
-// NoPacking respond of `nq` queries: out[q] holds gamma + 1 ciphertexts of (a, b), n words
-// each in coefficient form, the column sum first (respond.rs:614-643). AB_R: nq x 2n words
-// of scratch. r_mod_q = 2^64 mod q.
-cudaError_t nopack(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u64 r_mod_q,
-                   u64* AB_R, u64* out, u32* status, cudaStream_t s);
+// NoPacking respond of `nq` queries: prep transforms them into AB_R (nq x 2n words, r_mod_q = 2^64 mod q); cols gives
+// out[q], gamma + 1 ciphertexts of (a, b), n words each in coefficient form, the column sum first (respond.rs:614-643).
+cudaError_t nopack_prep(const CrsDev& c, const QueryDev* queries, u32 nq, u64 r_mod_q, u64* AB_R, u32* status,
+                        cudaStream_t s);
+cudaError_t nopack_cols(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u64* AB_R,
+                        u64* out, cudaStream_t s);
 
 // OnePacking (respond_one_packing): 2^log_parts CTAs per query walk the automorphism tree's subtrees, one the nodes
 // above them; nodes holds tree_scratch_words, b_fold the scan's b-values. Outputs coefficient-form

@@ -2,6 +2,7 @@
 // per-parameter-set constants, shards, packing stores and seats, request validation with
 // the reference's refusal rules, and the launch sequence of a respond batch.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <array>
@@ -229,10 +230,14 @@ struct ig_ctx {
   // threads can have batches in flight while the context lock is held only to launch.
   struct HostLane {
     std::mutex mu;
-    void* pin = nullptr;  // pinned status, a and b of the call in flight
+    void* pin = nullptr;  // pinned image of the call in flight (HostIO)
     size_t pin_bytes = 0;
     cudaEvent_t done = nullptr;
+    cudaStream_t copy = nullptr;  // copies between the device and the caller's own memory
+    cudaEvent_t copied = nullptr;
+    std::vector<cudaEvent_t> parts;  // ends of a batch's parts, each copied out while the next runs
   };
+  bool direct_copies = false;  // the GPU reads pageable memory through the host's page tables
   HostLane hlane[IG_MAX_LANES];
   std::atomic<u32> hlane_next{0};
   // special_modulus objects (ig_sm_runtime.cu) and their destructor.
@@ -634,6 +639,117 @@ int host_call_wait(ig_ctx* c, HostCall& hc) {
   IG_CUDA(c, cudaEventSynchronize(c->hlane[hc.k].done));
   return IG_OK;
 }
+// A lane's copy stream and event, made with the lane: a call finds them there.
+static bool host_lane_streams(cudaStream_t& copy, cudaEvent_t& copied) {
+  return (copied || cudaEventCreateWithFlags(&copied, cudaEventDisableTiming) == cudaSuccess) &&
+         (copy || cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking) == cudaSuccess);
+}
+cudaStream_t host_call_copy_stream(ig_ctx* c, HostCall& hc) { return c->hlane[hc.k].copy; }
+static bool host_io_direct(const ig_ctx* c, size_t bytes) { return c->direct_copies && bytes >= COPY_DIRECT_BYTES; }
+int host_io_open(ig_ctx* c, HostCall& hc, HostIO& io, size_t table, size_t queries, size_t work, size_t seeds, size_t bs,
+                 size_t count, size_t a, size_t b) {
+  size_t at = 0;
+  auto put = [&](size_t bytes, size_t& off, size_t& len) {
+    off = at;
+    len = bytes;
+    at = (at + bytes + 255) & ~(size_t)255;
+  };
+  put(table, io.table, io.table_bytes);
+  put(queries, io.queries, io.query_bytes);
+  put(work, io.work, io.work_bytes);
+  put(seeds, io.seeds, io.seed_bytes);
+  put(bs, io.bs, io.bs_bytes);
+  put(count * 4, io.status, io.status_bytes);
+  put(a, io.a, io.a_bytes);
+  put(b, io.b, io.b_bytes);
+  io.end = at;
+  char name[32];
+  snprintf(name, sizeof name, "call%u", hc.k);
+  void *d, *h;
+  int rc = ::scratch(c, name, at, &d);
+  if (!rc) rc = host_call_pinned(c, hc, at, &h);
+  if (rc) return rc;
+  io.dev = (uint8_t*)d;
+  io.pin = (uint8_t*)h;
+  return IG_OK;
+}
+int host_io_send(ig_ctx* c, HostCall& hc, HostIO& io, const void* table, const void* queries, const void* work,
+                 const void* seeds, const void* bs) {
+  if (io.table_bytes) memcpy(io.pin + io.table, table, io.table_bytes);
+  memcpy(io.pin + io.queries, queries, io.query_bytes);
+  if (io.work_bytes) memcpy(io.pin + io.work, work, io.work_bytes);
+  memset(io.pin + io.status, 0, io.status_bytes);
+  // The large inputs go first, on the copy stream: nothing else uses their part of the block, so they need not wait for
+  // the context's work.
+  const bool ds = host_io_direct(c, io.seed_bytes), db = host_io_direct(c, io.bs_bytes);
+  cudaStream_t s = host_call_stream(c, hc), copy = nullptr;
+  int rc;
+  if (ds || db) {
+    hc.queued[1] = copy = host_call_copy_stream(c, hc);
+    if (ds) IG_CUDA(c, cudaMemcpyAsync(io.dev + io.seeds, seeds, io.seed_bytes, cudaMemcpyHostToDevice, copy));
+    if (db) IG_CUDA(c, cudaMemcpyAsync(io.dev + io.bs, bs, io.bs_bytes, cudaMemcpyHostToDevice, copy));
+    IG_CUDA(c, cudaEventRecord(c->hlane[hc.k].copied, copy));
+  }
+  if (!ds) memcpy(io.pin + io.seeds, seeds, io.seed_bytes);
+  if (!db) memcpy(io.pin + io.bs, bs, io.bs_bytes);
+  if ((rc = host_call_enter(c, hc))) return rc;
+  hc.queued[0] = s;
+  if (copy) IG_CUDA(c, cudaStreamWaitEvent(s, c->hlane[hc.k].copied, 0));
+  // One copy up to the first array that went by itself, another past the last one.
+  const size_t first = ds ? io.seeds : db ? io.bs : io.a, last = db ? io.status : ds ? io.bs : io.a;
+  if (first) IG_CUDA(c, cudaMemcpyAsync(io.dev, io.pin, first, cudaMemcpyHostToDevice, s));
+  if (last < io.a) IG_CUDA(c, cudaMemcpyAsync(io.dev + last, io.pin + last, io.a - last, cudaMemcpyHostToDevice, s));
+  return IG_OK;
+}
+int host_io_receive(ig_ctx* c, HostCall& hc, HostIO& io) {
+  const size_t last = !host_io_direct(c, io.b_bytes)   ? io.end
+                      : !host_io_direct(c, io.a_bytes) ? io.b
+                                                       : io.a;
+  cudaStream_t s = host_call_stream(c, hc);
+  const size_t first = host_io_direct(c, io.a_bytes) && last == io.end ? io.b : io.a;
+  if (first == io.b) {  // a goes by itself, b through the image
+    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.status, io.dev + io.status, io.a - io.status, cudaMemcpyDeviceToHost, s));
+    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.b, io.dev + io.b, io.end - io.b, cudaMemcpyDeviceToHost, s));
+  } else {
+    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.status, io.dev + io.status, last - io.status, cudaMemcpyDeviceToHost, s));
+  }
+  return host_call_launched(c, hc);
+}
+// Faults the pages of a result buffer in without changing a byte of it.
+static void touch_pages(void* p, size_t bytes) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  for (size_t at = 0; at < bytes; at += page) {
+    volatile uint8_t* b = (volatile uint8_t*)p + at;
+    *b = *b;
+  }
+  if (bytes) {
+    volatile uint8_t* b = (volatile uint8_t*)p + bytes - 1;
+    *b = *b;
+  }
+}
+int host_io_wait(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out) {
+  if (host_io_direct(c, io.a_bytes)) touch_pages(a_out, io.a_bytes);
+  if (host_io_direct(c, io.b_bytes)) touch_pages(b_out, io.b_bytes);
+  int rc = host_call_wait(c, hc);
+  if (!rc) hc.queued[0] = hc.queued[1] = nullptr;
+  return rc;
+}
+int host_io_finish(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out) {
+  const bool da = host_io_direct(c, io.a_bytes), db = host_io_direct(c, io.b_bytes);
+  if (!da) memcpy(a_out, io.pin + io.a, io.a_bytes);
+  if (!db) memcpy(b_out, io.pin + io.b, io.b_bytes);
+  if (!da && !db) return IG_OK;
+  // The copy stream waits for nothing but the batch, which has ended: other callers' launches on the context stream do
+  // not hold the results back.
+  cudaStream_t copy = host_call_copy_stream(c, hc);
+  cudaError_t e = cudaSuccess;
+  if (da) e = cudaMemcpyAsync(a_out, io.dev + io.a, io.a_bytes, cudaMemcpyDeviceToHost, copy);
+  if (e == cudaSuccess && db) e = cudaMemcpyAsync(b_out, io.dev + io.b, io.b_bytes, cudaMemcpyDeviceToHost, copy);
+  const cudaError_t w = cudaStreamSynchronize(copy);
+  if (e == cudaSuccess) e = w;
+  if (e != cudaSuccess) return fail(c, IG_ERR_CUDA, "copy of the responses failed: %s", cudaGetErrorString(e));
+  return IG_OK;
+}
 int lane_enter(ig_ctx* c, int lane) {
   if (lane < 0) return IG_OK;
   IG_CUDA(c, cudaEventRecord(c->lane_in[lane], c->stream));
@@ -669,7 +785,12 @@ int ig_ctx_create(int device, ig_ctx** out) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   c->pair_threshold = (u32)(sms / 2);
   c->sms = (u32)sms;
-  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  int tables = 0;
+  if (cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) != cudaSuccess)
+    cudaGetLastError();
+  c->direct_copies = tables != 0;
+  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      !igint::host_lane_streams(c->hlane[0].copy, c->hlane[0].copied)) {
     delete c;
     return IG_ERR_CUDA;
   }
@@ -690,6 +811,12 @@ void ig_ctx_destroy(ig_ctx* c) {
     }
     if (c->hlane[k].pin) cudaFreeHost(c->hlane[k].pin);
     if (c->hlane[k].done) cudaEventDestroy(c->hlane[k].done);
+    if (c->hlane[k].copy) {
+      cudaStreamSynchronize(c->hlane[k].copy);
+      cudaStreamDestroy(c->hlane[k].copy);
+    }
+    if (c->hlane[k].copied) cudaEventDestroy(c->hlane[k].copied);
+    for (cudaEvent_t e : c->hlane[k].parts) cudaEventDestroy(e);
     if (c->side_fork[k]) cudaEventDestroy(c->side_fork[k]);
     for (int j = 0; j < 2; j++) {
       if (c->side_stream[k][j]) {
@@ -1368,45 +1495,33 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
       if (rc) return rc;
     }
   }
-  void *d_table, *d_q, *d_seeds, *d_bs, *d_a, *d_b, *d_fold, *d_status;
-  const size_t seed_bytes = as ? (size_t)count * n * 8 : (size_t)count * 32;
-  auto lane_scratch = [&](const char* name, size_t bytes, void** out) {
-    char full[48];
-    snprintf(full, sizeof full, "%s%u", name, k);
-    return scratch(c, full, bytes, out);
-  };
-  if ((rc = lane_scratch("table", table.size() * sizeof(ShardDev), &d_table)) ||
-      (rc = lane_scratch("queries", count * sizeof(QueryDev), &d_q)) ||
-      (rc = lane_scratch("seeds", seed_bytes, &d_seeds)) || (rc = lane_scratch("bs", count * n * 8, &d_bs)) ||
-      (rc = lane_scratch("a_out", count * n * 8, &d_a)) || (rc = lane_scratch("b_out", count * n * 8, &d_b)) ||
-      (rc = lane_scratch("fold", count * g * 8, &d_fold)) || (rc = lane_scratch("status", count * 4, &d_status)))
+  const size_t words = (size_t)count * n * 8;
+  igint::HostIO io;
+  void* d_fold;
+  char fname[32];
+  snprintf(fname, sizeof fname, "fold%u", k);
+  if ((rc = igint::host_io_open(c, hc, io, table.size() * sizeof(ShardDev), count * sizeof(QueryDev), 0,
+                                as ? words : (size_t)count * 32, words, count, words, words)) ||
+      (rc = scratch(c, fname, count * g * 8, &d_fold)))
     return rc;
-  // Pinned landing buffer of the lane: status words, then a, then b.
-  const size_t st_bytes = ((size_t)count * 4 + 15) & ~(size_t)15;
-  void* pin;
-  if ((rc = igint::host_call_pinned(c, hc, st_bytes + 2 * (size_t)count * n * 8, &pin))) return rc;
-  u32* h_status = (u32*)pin;
-  u64* h_a = (u64*)((uint8_t*)pin + st_bytes);
-  u64* h_b = h_a + (size_t)count * n;
+  const QueryDev* d_q = (const QueryDev*)(io.dev + io.queries);
+  const ShardDev* d_table = (const ShardDev*)(io.dev + io.table);
+  u32* d_status = (u32*)(io.dev + io.status);
   std::vector<QueryDev> qs(count);
   for (u32 i = 0; i < count; i++) {
     qs[i] = QueryDev{};
     qs[i].shard = local[shard_ids[i]];
     qs[i].fold_off = i * (u32)g;
-    qs[i].seed = as ? nullptr : (const u32*)((const uint8_t*)d_seeds + (size_t)i * 32);
-    qs[i].a = as ? (const u64*)d_seeds + (size_t)i * n : nullptr;
-    qs[i].b = (const u64*)d_bs + (size_t)i * n;
+    qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
+    qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
+    qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
     qs[i].seat_R = seat;
     qs[i].ms = ms_target;
     qs[i].row = i;
   }
   cudaStream_t s = igint::host_call_stream(c, hc);
-  if ((rc = stage_h2d(c, d_table, table.data(), table.size() * sizeof(ShardDev))) ||
-      (rc = stage_h2d(c, d_q, qs.data(), count * sizeof(QueryDev))) ||
-      (rc = stage_h2d(c, d_seeds, as ? (const void*)as : (const void*)seeds, seed_bytes)) ||
-      (rc = stage_h2d(c, d_bs, bs, (size_t)count * n * 8)) || (rc = igint::host_call_enter(c, hc)))
+  if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
     return rc;
-  IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
   // RAVEN_PROFILE_RESPOND (respond.rs:1295-1345): CUDA events around the two regions of the
   // batch, printed to stderr in the reference's line format.
   cudaEvent_t env_ev[3] = {};
@@ -1415,15 +1530,12 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
     for (auto& e : env_ev) cudaEventCreate(&e);
   if (env_prof) cudaEventRecord(env_ev[0], s);
   long pk = prof_begin(c, REGION_SCAN, s);
-  IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, nullptr, 0, (u64*)d_fold,
-                             (u32*)d_status, s));
+  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
   prof_end(c, pk, s);
   if (env_prof) cudaEventRecord(env_ev[1], s);
   pk = prof_begin(c, REGION_RESPOND, s);
-  IG_CUDA(c, igk::respond(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, (const u64*)d_fold,
-                          (u64*)d_a, (u64*)d_b, (u32*)d_status, c->force_serial,
-                          igint::launch_ctas(c, (u32)n, (u32)g, count, count * lanes),
-                          s));
+  IG_CUDA(c, igk::respond(o.dev, d_q, d_table, count, (const u64*)d_fold, (u64*)(io.dev + io.a), (u64*)(io.dev + io.b),
+                          d_status, c->force_serial, igint::launch_ctas(c, (u32)n, (u32)g, count, count * lanes), s));
   prof_end(c, pk, s);
   if (env_prof) {
     cudaEventRecord(env_ev[2], s);
@@ -1435,12 +1547,10 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
             (unsigned)count, 1e3 * scan_ms, 1e3 * pack_ms);
     for (auto& e : env_ev) cudaEventDestroy(e);
   }
-  IG_CUDA(c, cudaMemcpyAsync(h_status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
-  IG_CUDA(c, cudaMemcpyAsync(h_a, d_a, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
-  IG_CUDA(c, cudaMemcpyAsync(h_b, d_b, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
-  if ((rc = igint::host_call_launched(c, hc))) return rc;
+  if ((rc = igint::host_io_receive(c, hc, io))) return rc;
   lk.unlock();  // other callers launch while this batch runs
-  if ((rc = igint::host_call_wait(c, hc))) return rc;
+  if ((rc = igint::host_io_wait(c, hc, io, a_out, b_out))) return rc;
+  const u32* h_status = (const u32*)(io.pin + io.status);
   for (u32 i = 0; i < count; i++) {
     if (h_status[i] & DEV_TAG_MISMATCH)
       return fail(c, IG_ERR_STORE_REFUSED,
@@ -1449,9 +1559,7 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
                   shard_ids[i]);
     if (h_status[i]) return fail(c, IG_ERR_DEVICE, "query %u: respond kernel status %u", i, h_status[i]);
   }
-  memcpy(a_out, h_a, (size_t)count * n * 8);
-  memcpy(b_out, h_b, (size_t)count * n * 8);
-  return IG_OK;
+  return igint::host_io_finish(c, hc, io, a_out, b_out);
 }
 
 int ig_respond_seeded_batch(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, const uint64_t* inline_y,
@@ -1503,51 +1611,68 @@ int ig_respond_nopacking_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const ui
       table.push_back(db->shards[s].dev());
     }
   }
-  const size_t seed_bytes = as ? (size_t)count * n * 8 : (size_t)count * 32;
-  const size_t out_words = (size_t)count * (g + 1) * 2 * n;
-  void *d_table, *d_q, *d_seeds, *d_bs, *d_ab, *d_out, *d_status;
+  const size_t words = (size_t)count * n * 8;
+  const size_t row_words = (g + 1) * 2 * n;
+  igint::HostIO io;
+  void *d_ab, *d_out;
   auto lane_scratch = [&](const char* name, size_t bytes, void** p) {
     char full[48];
     snprintf(full, sizeof full, "%s%u", name, k);
     return scratch(c, full, bytes, p);
   };
   int rc;
-  if ((rc = lane_scratch("np_table", table.size() * sizeof(ShardDev), &d_table)) ||
-      (rc = lane_scratch("np_queries", count * sizeof(QueryDev), &d_q)) ||
-      (rc = lane_scratch("np_seeds", seed_bytes, &d_seeds)) ||
-      (rc = lane_scratch("np_bs", (size_t)count * n * 8, &d_bs)) ||
+  if ((rc = igint::host_io_open(c, hc, io, table.size() * sizeof(ShardDev), count * sizeof(QueryDev), 0,
+                                as ? words : (size_t)count * 32, words, count, 0, 0)) ||
       (rc = lane_scratch("np_ab", (size_t)count * 2 * n * 8, &d_ab)) ||
-      (rc = lane_scratch("np_out", out_words * 8, &d_out)) || (rc = lane_scratch("np_status", count * 4, &d_status)))
+      (rc = lane_scratch("np_out", count * row_words * 8, &d_out)))
     return rc;
-  void* pin;
-  if ((rc = igint::host_call_pinned(c, hc, (size_t)count * 4, &pin))) return rc;
-  const u32* h_status = (const u32*)pin;
+  u32* d_status = (u32*)(io.dev + io.status);
   std::vector<QueryDev> qs(count);
   for (u32 i = 0; i < count; i++) {
     qs[i] = QueryDev{};
     qs[i].shard = local[shard_ids[i]];
-    qs[i].seed = as ? nullptr : (const u32*)((const uint8_t*)d_seeds + (size_t)i * 32);
-    qs[i].a = as ? (const u64*)d_seeds + (size_t)i * n : nullptr;
-    qs[i].b = (const u64*)d_bs + (size_t)i * n;
+    qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
+    qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
+    qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
     qs[i].seat_R = nullptr;
   }
-  if ((rc = stage_h2d(c, d_table, table.data(), table.size() * sizeof(ShardDev))) ||
-      (rc = stage_h2d(c, d_q, qs.data(), count * sizeof(QueryDev))) ||
-      (rc = stage_h2d(c, d_seeds, as ? (const void*)as : (const void*)seeds, seed_bytes)) ||
-      (rc = stage_h2d(c, d_bs, bs, (size_t)count * n * 8)) || (rc = igint::host_call_enter(c, hc)))
+  cudaStream_t s = igint::host_call_stream(c, hc), copy = igint::host_call_copy_stream(c, hc);
+  if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
     return rc;
-  cudaStream_t s = igint::host_call_stream(c, hc);
-  IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
-  IG_CUDA(c, igk::nopack(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, R_MOD_Q, (u64*)d_ab,
-                         (u64*)d_out, (u32*)d_status, s));
-  c->launches += 3;
-  IG_CUDA(c, cudaMemcpyAsync((void*)h_status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
-  if ((rc = igint::host_call_launched(c, hc))) return rc;
+  IG_CUDA(c, igk::nopack_prep(o.dev, (const QueryDev*)(io.dev + io.queries), count, R_MOD_Q, (u64*)d_ab, d_status, s));
+  c->launches++;
+  // The columns in parts, each copied out while the next runs: the copy (190 GB/s) takes twice the kernels' time, so a
+  // part need only be long enough to hide its launches: 16 MB, two queries of gamma 256 (16 of them 1.07 -> 0.86 ms, of
+  // which the copy is 0.70).
+  const u32 part = (u32)std::min<size_t>(count, std::max<size_t>(1, (16 << 20) / (row_words * 8)));
+  auto& ends = c->hlane[k].parts;
+  for (u32 i = 0, p = 0; i < count; i += part, p++) {
+    const u32 nq = std::min(part, count - i);
+    IG_CUDA(c, igk::nopack_cols(o.dev, (const QueryDev*)(io.dev + io.queries) + i, (const ShardDev*)(io.dev + io.table),
+                                nq, (const u64*)d_ab + (size_t)i * 2 * n, (u64*)d_out + i * row_words, s));
+    c->launches += 2;
+    if (p == ends.size()) {
+      cudaEvent_t e;
+      IG_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ends.push_back(e);
+    }
+    IG_CUDA(c, cudaEventRecord(ends[p], s));
+  }
+  if ((rc = igint::host_io_receive(c, hc, io))) return rc;
   lk.unlock();  // other callers launch while this batch runs and copies out
-  // The lane's stream and scratch stay this call's until it returns (the lane lock).
-  cudaError_t e = cudaMemcpyAsync(out, d_out, out_words * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  // The lane's scratch stays this call's until it returns (the lane lock).
+  hc.queued[1] = copy;
+  cudaError_t e = cudaSuccess;
+  for (u32 i = 0, p = 0; i < count && e == cudaSuccess; i += part, p++) {
+    e = cudaStreamWaitEvent(copy, ends[p], 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out + i * row_words, (const u64*)d_out + i * row_words,
+                          std::min(part, count - i) * row_words * 8, cudaMemcpyDeviceToHost, copy);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(copy);
   if (e != cudaSuccess) return fail(c, IG_ERR_CUDA, "respond: copy of the ciphertexts failed: %s", cudaGetErrorString(e));
+  if ((rc = igint::host_io_wait(c, hc, io, nullptr, nullptr))) return rc;
+  const u32* h_status = (const u32*)(io.pin + io.status);
   for (u32 i = 0; i < count; i++)
     if (h_status[i]) return fail(c, IG_ERR_DEVICE, "query %u: respond kernel status %u", i, h_status[i]);
   return IG_OK;
@@ -1845,62 +1970,49 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
       table.back().stale = 0;  // the tree reads columns alone: no store to be out of date
     }
   }
-  const size_t seed_bytes = as ? (size_t)count * n * 8 : (size_t)count * 32;
-  void *d_table, *d_q, *d_seeds, *d_bs, *d_nodes, *d_fold, *d_a, *d_b, *d_status;
+  const size_t words = (size_t)count * n * 8;
+  const u32 parts = igk::tree_log_parts(o.dev, count, c->sms);
+  igint::HostIO io;
+  void *d_nodes, *d_fold;
   auto lane_scratch = [&](const char* name, size_t bytes, void** p) {
     char full[48];
     snprintf(full, sizeof full, "%s%u", name, k);
     return scratch(c, full, bytes, p);
   };
-  const u32 parts = igk::tree_log_parts(o.dev, count, c->sms);
   int rc;
-  if ((rc = lane_scratch("tr_table", table.size() * sizeof(ShardDev), &d_table)) ||
-      (rc = lane_scratch("tr_queries", count * sizeof(QueryDev), &d_q)) ||
-      (rc = lane_scratch("tr_seeds", seed_bytes, &d_seeds)) ||
-      (rc = lane_scratch("tr_bs", (size_t)count * n * 8, &d_bs)) ||
+  if ((rc = igint::host_io_open(c, hc, io, table.size() * sizeof(ShardDev), count * sizeof(QueryDev), 0,
+                                as ? words : (size_t)count * 32, words, count, words, words)) ||
       (rc = lane_scratch("tr_nodes", igk::tree_scratch_words(o.dev, count, parts) * 8, &d_nodes)) ||
-      (rc = lane_scratch("tr_fold", (size_t)count * o.gamma * 8, &d_fold)) ||
-      (rc = lane_scratch("tr_a", (size_t)count * n * 8, &d_a)) ||
-      (rc = lane_scratch("tr_b", (size_t)count * n * 8, &d_b)) || (rc = lane_scratch("tr_status", count * 4, &d_status)))
+      (rc = lane_scratch("tr_fold", (size_t)count * o.gamma * 8, &d_fold)))
     return rc;
-  void* pin;
-  if ((rc = igint::host_call_pinned(c, hc, (size_t)count * 4, &pin))) return rc;
-  const u32* h_status = (const u32*)pin;
+  const QueryDev* d_q = (const QueryDev*)(io.dev + io.queries);
+  const ShardDev* d_table = (const ShardDev*)(io.dev + io.table);
+  u32* d_status = (u32*)(io.dev + io.status);
   std::vector<QueryDev> qs(count);
   for (u32 i = 0; i < count; i++) {
     qs[i] = QueryDev{};
     qs[i].shard = local[shard_ids[i]];
-    qs[i].seed = as ? nullptr : (const u32*)((const uint8_t*)d_seeds + (size_t)i * 32);
-    qs[i].a = as ? (const u64*)d_seeds + (size_t)i * n : nullptr;
-    qs[i].b = (const u64*)d_bs + (size_t)i * n;
+    qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
+    qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
+    qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
     qs[i].seat_R = nullptr;
     qs[i].fold_off = i * o.gamma;
     qs[i].row = i;
   }
-  if ((rc = stage_h2d(c, d_table, table.data(), table.size() * sizeof(ShardDev))) ||
-      (rc = stage_h2d(c, d_q, qs.data(), count * sizeof(QueryDev))) ||
-      (rc = stage_h2d(c, d_seeds, as ? (const void*)as : (const void*)seeds, seed_bytes)) ||
-      (rc = stage_h2d(c, d_bs, bs, (size_t)count * n * 8)) || (rc = igint::host_call_enter(c, hc)))
-    return rc;
   cudaStream_t s = igint::host_call_stream(c, hc);
-  IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
-  IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, nullptr, 0, (u64*)d_fold,
-                             (u32*)d_status, s));
-  IG_CUDA(c, igk::tree(o.dev, (const QueryDev*)d_q, (const ShardDev*)d_table, count, parts, ms_target, (u64*)d_nodes,
-                       (const u64*)d_fold, (u64*)d_a, (u64*)d_b, (u32*)d_status, s));
+  if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
+    return rc;
+  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
+  IG_CUDA(c, igk::tree(o.dev, d_q, d_table, count, parts, ms_target, (u64*)d_nodes, (const u64*)d_fold,
+                       (u64*)(io.dev + io.a), (u64*)(io.dev + io.b), d_status, s));
   c->launches += 3;
-  IG_CUDA(c, cudaMemcpyAsync((void*)h_status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
-  if ((rc = igint::host_call_launched(c, hc))) return rc;
-  lk.unlock();  // other callers launch while this batch runs and copies out
-  // The lane's stream and scratch stay this call's until it returns (the lane lock).
-  cudaError_t e = cudaMemcpyAsync(a_out, d_a, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(b_out, d_b, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess)
-    return fail(c, IG_ERR_CUDA, "respond_one_packing: copy of the responses failed: %s", cudaGetErrorString(e));
+  if ((rc = igint::host_io_receive(c, hc, io))) return rc;
+  lk.unlock();  // other callers launch while this batch runs
+  if ((rc = igint::host_io_wait(c, hc, io, a_out, b_out))) return rc;
+  const u32* h_status = (const u32*)(io.pin + io.status);
   for (u32 i = 0; i < count; i++)
     if (h_status[i]) return fail(c, IG_ERR_DEVICE, "query %u: tree kernel status %u", i, h_status[i]);
-  return IG_OK;
+  return igint::host_io_finish(c, hc, io, a_out, b_out);
 }
 
 int ig_respond_seeded_batch_device(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, uint32_t count,
@@ -2202,52 +2314,33 @@ int ig_respond_mixed_batch(ig_ctx* c, uint32_t count, const uint64_t* dbs, const
   int rc = plan_mixed(c, count, dbs, stores, handles, shard_ids, ms_targets, P);
   if (rc) return rc;
   const size_t n = P.ring.n;
-  void *dq, *dt, *dw, *df, *dseeds, *dbs_, *da, *db_, *dst;
-  auto lane_scratch = [&](const char* name, size_t bytes, void** out) {
-    char full[48];
-    snprintf(full, sizeof full, "%s%u", name, k);
-    return scratch(c, full, bytes, out);
-  };
-  if ((rc = lane_scratch("hmix_queries", count * sizeof(QueryDev), &dq)) ||
-      (rc = lane_scratch("hmix_table", P.table.size() * sizeof(ShardDev), &dt)) ||
-      (rc = lane_scratch("hmix_work", P.work.size() * 4, &dw)) ||
-      (rc = lane_scratch("hmix_fold", P.fold_words * 8, &df)) ||
-      (rc = lane_scratch("hmix_seeds", (size_t)count * 32, &dseeds)) ||
-      (rc = lane_scratch("hmix_bs", (size_t)count * n * 8, &dbs_)) ||
-      (rc = lane_scratch("hmix_a", (size_t)count * n * 8, &da)) ||
-      (rc = lane_scratch("hmix_b", (size_t)count * n * 8, &db_)) ||
-      (rc = lane_scratch("hmix_status", (size_t)count * 4, &dst)))
+  const size_t words = (size_t)count * n * 8;
+  igint::HostIO io;
+  void* df;
+  char fname[32];
+  snprintf(fname, sizeof fname, "hmix_fold%u", k);
+  if ((rc = igint::host_io_open(c, hc, io, P.table.size() * sizeof(ShardDev), count * sizeof(QueryDev), P.work.size() * 4,
+                                (size_t)count * 32, words, count, words, words)) ||
+      (rc = scratch(c, fname, P.fold_words * 8, &df)))
     return rc;
   for (QueryDev& q : P.qs) {
-    q.seed = (const u32*)((const uint8_t*)dseeds + (size_t)q.row * 32);
-    q.b = (const u64*)dbs_ + (size_t)q.row * n;
+    q.seed = (const u32*)(io.dev + io.seeds + (size_t)q.row * 32);
+    q.b = (const u64*)(io.dev + io.bs) + (size_t)q.row * n;
   }
-  const size_t st_bytes = ((size_t)count * 4 + 15) & ~(size_t)15;
-  void* pin;
-  if ((rc = igint::host_call_pinned(c, hc, st_bytes + 2 * (size_t)count * n * 8, &pin))) return rc;
-  u32* h_status = (u32*)pin;
-  u64* h_a = (u64*)((uint8_t*)pin + st_bytes);
-  u64* h_b = h_a + (size_t)count * n;
+  const QueryDev* dq = (const QueryDev*)(io.dev + io.queries);
+  const ShardDev* dt = (const ShardDev*)(io.dev + io.table);
+  u32* dst = (u32*)(io.dev + io.status);
   cudaStream_t s = igint::host_call_stream(c, hc);
-  if ((rc = stage_h2d(c, dq, P.qs.data(), count * sizeof(QueryDev))) ||
-      (rc = stage_h2d(c, dt, P.table.data(), P.table.size() * sizeof(ShardDev))) ||
-      (rc = stage_h2d(c, dw, P.work.data(), P.work.size() * 4)) ||
-      (rc = stage_h2d(c, dseeds, seeds, (size_t)count * 32)) ||
-      (rc = stage_h2d(c, dbs_, bs, (size_t)count * n * 8)) || (rc = igint::host_call_enter(c, hc)))
-    return rc;
-  IG_CUDA(c, cudaMemsetAsync(dst, 0, count * 4, s));
-  IG_CUDA(c, igk::shard_scan(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u32*)dw,
-                             (u32)P.work.size(), (u64*)df, (u32*)dst, s));
-  if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), k, (const QueryDev*)dq, (const ShardDev*)dt,
-                         (const u64*)df, (u64*)da, (u64*)db_, (u32*)dst, s)))
+  if ((rc = igint::host_io_send(c, hc, io, P.table.data(), P.qs.data(), P.work.data(), seeds, bs))) return rc;
+  IG_CUDA(c, igk::shard_scan(P.ring, dq, dt, count, (const u32*)(io.dev + io.work), (u32)P.work.size(), (u64*)df, dst, s));
+  if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), k, dq, dt, (const u64*)df, (u64*)(io.dev + io.a),
+                         (u64*)(io.dev + io.b), dst, s)))
     return rc;
   c->launches++;
-  IG_CUDA(c, cudaMemcpyAsync(h_status, dst, count * 4, cudaMemcpyDeviceToHost, s));
-  IG_CUDA(c, cudaMemcpyAsync(h_a, da, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
-  IG_CUDA(c, cudaMemcpyAsync(h_b, db_, (size_t)count * n * 8, cudaMemcpyDeviceToHost, s));
-  if ((rc = igint::host_call_launched(c, hc))) return rc;
+  if ((rc = igint::host_io_receive(c, hc, io))) return rc;
   lk.unlock();  // other callers launch while this batch runs
-  if ((rc = igint::host_call_wait(c, hc))) return rc;
+  if ((rc = igint::host_io_wait(c, hc, io, a_out, b_out))) return rc;
+  const u32* h_status = (const u32*)(io.pin + io.status);
   for (u32 i = 0; i < count; i++) {
     if (h_status[i] & DEV_TAG_MISMATCH)
       return fail(c, IG_ERR_STORE_REFUSED,
@@ -2256,9 +2349,7 @@ int ig_respond_mixed_batch(ig_ctx* c, uint32_t count, const uint64_t* dbs, const
                   shard_ids[i]);
     if (h_status[i]) return fail(c, IG_ERR_DEVICE, "query %u: respond kernel status %u", i, h_status[i]);
   }
-  memcpy(a_out, h_a, (size_t)count * n * 8);
-  memcpy(b_out, h_b, (size_t)count * n * 8);
-  return IG_OK;
+  return igint::host_io_finish(c, hc, io, a_out, b_out);
 }
 
 int ig_ctx_set_lanes(ig_ctx* c, uint32_t lanes) {
@@ -2268,6 +2359,8 @@ int ig_ctx_set_lanes(ig_ctx* c, uint32_t lanes) {
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   for (u32 k = 0; k < lanes; k++) {
+    if (!igint::host_lane_streams(c->hlane[k].copy, c->hlane[k].copied))
+      return fail(c, IG_ERR_CUDA, "ig_ctx_set_lanes: no stream for lane %u's copies", k);
     if (c->lane_stream[k]) continue;
     IG_CUDA(c, cudaStreamCreateWithFlags(&c->lane_stream[k], cudaStreamNonBlocking));
     IG_CUDA(c, cudaEventCreateWithFlags(&c->lane_in[k], cudaEventDisableTiming));

@@ -3,6 +3,7 @@
 // the batched respond, with the refusal rules of src/special_modulus/server.rs.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 
 #include <cstring>
@@ -515,54 +516,40 @@ int ig_sm_respond_batch(ig_ctx* c, uint64_t server, uint32_t count, const uint64
   int rc = sm_prepare(c, st, server, count, tables, seats, &o, qs);
   if (rc) return rc;
   const size_t d = o->n, nb = o->dev.nb;
-  for (size_t k = 0; k < (size_t)count * d; k++)
-    if (bodies[k] >= o->q) return fail(c, IG_ERR_SHAPE, "query %zu does not fit the set", k / d);
-  void *dq, *dseeds, *dbodies, *dfold, *dmask, *dbody, *dstatus;
-  auto lane_scratch = [&](const char* name, size_t bytes, void** out) {
-    char full[48];
-    snprintf(full, sizeof full, "%s%u", name, hc.k);
-    return igint::scratch(c, full, bytes, out);
-  };
-  if ((rc = lane_scratch("sm_q", count * sizeof(SmQueryDev), &dq)) ||
-      (rc = lane_scratch("sm_seeds", count * 32, &dseeds)) ||
-      (rc = lane_scratch("sm_bodies", count * d * 4, &dbodies)) ||
-      (rc = lane_scratch("sm_fold", (size_t)count * igsmk::SM_FOLD_CHUNKS * o->dev.gamma * 8, &dfold)) ||
-      (rc = lane_scratch("sm_mask", count * d * 4, &dmask)) ||
-      (rc = lane_scratch("sm_body", count * nb * 4, &dbody)) ||
-      (rc = lane_scratch("sm_status", count * 4, &dstatus)))
-    return rc;
-  // Pinned landing buffer: status words, mask, body.
-  const size_t st_bytes = ((size_t)count * 4 + 15) & ~(size_t)15;
-  void* pin;
-  if ((rc = igint::host_call_pinned(c, hc, st_bytes + (size_t)count * (d + nb) * 4, &pin))) return rc;
-  u32* h_status = (u32*)pin;
-  u32* h_mask = (u32*)((uint8_t*)pin + st_bytes);
-  u32* h_body = h_mask + (size_t)count * d;
   for (u32 i = 0; i < count; i++) {
-    qs[i].seed = (const u32*)((const uint8_t*)dseeds + (size_t)i * 32);
-    qs[i].body = (const u32*)dbodies + (size_t)i * d;
+    // The largest word, eight at a time and without a branch a word (d is a power of two): half a million words a call.
+    u32 top[8] = {};
+    for (size_t k = 0; k < d; k += 8)
+      for (int j = 0; j < 8; j++) top[j] = std::max(top[j], bodies[i * d + k + j]);
+    for (u32 t : top)
+      if (t >= o->q) return fail(c, IG_ERR_SHAPE, "query %zu does not fit the set", (size_t)i);
   }
-  cudaStream_t s = igint::host_call_stream(c, hc);
-  if ((rc = igint::stage_h2d(c, dq, qs.data(), count * sizeof(SmQueryDev))) ||
-      (rc = igint::stage_h2d(c, dseeds, seeds, (size_t)count * 32)) ||
-      (rc = igint::stage_h2d(c, dbodies, bodies, (size_t)count * d * 4)) || (rc = igint::host_call_enter(c, hc)))
+  igint::HostIO io;
+  void* dfold;
+  char fname[32];
+  snprintf(fname, sizeof fname, "sm_fold%u", hc.k);
+  if ((rc = igint::host_io_open(c, hc, io, 0, count * sizeof(SmQueryDev), 0, (size_t)count * 32, (size_t)count * d * 4,
+                                count, (size_t)count * d * 4, (size_t)count * nb * 4)) ||
+      (rc = igint::scratch(c, fname, (size_t)count * igsmk::SM_FOLD_CHUNKS * o->dev.gamma * 8, &dfold)))
     return rc;
-  SM_CUDA(c, cudaMemsetAsync(dstatus, 0, count * 4, s));
-  SM_CUDA(c, igsmk::body_fold(o->dev, (const SmQueryDev*)dq, count, (i64*)dfold, s));
-  SM_CUDA(c, igsmk::respond(o->dev, (const SmQueryDev*)dq, count, (const i64*)dfold, (u32*)dmask, (u32*)dbody,
-                            (u32*)dstatus, s));
+  for (u32 i = 0; i < count; i++) {
+    qs[i].seed = (const u32*)(io.dev + io.seeds + (size_t)i * 32);
+    qs[i].body = (const u32*)(io.dev + io.bs) + (size_t)i * d;
+  }
+  const SmQueryDev* dq = (const SmQueryDev*)(io.dev + io.queries);
+  cudaStream_t s = igint::host_call_stream(c, hc);
+  if ((rc = igint::host_io_send(c, hc, io, nullptr, qs.data(), nullptr, seeds, bodies))) return rc;
+  SM_CUDA(c, igsmk::body_fold(o->dev, dq, count, (i64*)dfold, s));
+  SM_CUDA(c, igsmk::respond(o->dev, dq, count, (const i64*)dfold, (u32*)(io.dev + io.a), (u32*)(io.dev + io.b),
+                            (u32*)(io.dev + io.status), s));
   igint::add_launches(c, 2);
-  SM_CUDA(c, cudaMemcpyAsync(h_status, dstatus, count * 4, cudaMemcpyDeviceToHost, s));
-  SM_CUDA(c, cudaMemcpyAsync(h_mask, dmask, (size_t)count * d * 4, cudaMemcpyDeviceToHost, s));
-  SM_CUDA(c, cudaMemcpyAsync(h_body, dbody, (size_t)count * nb * 4, cudaMemcpyDeviceToHost, s));
-  if ((rc = igint::host_call_launched(c, hc))) return rc;
+  if ((rc = igint::host_io_receive(c, hc, io))) return rc;
   lk.unlock();
-  if ((rc = igint::host_call_wait(c, hc))) return rc;
+  if ((rc = igint::host_io_wait(c, hc, io, mask_out, body_out))) return rc;
+  const u32* h_status = (const u32*)(io.pin + io.status);
   for (u32 i = 0; i < count; i++)
     if (h_status[i]) return fail(c, IG_ERR_DEVICE, "query %u: respond kernel status %u", i, h_status[i]);
-  memcpy(mask_out, h_mask, (size_t)count * d * 4);
-  memcpy(body_out, h_body, (size_t)count * nb * 4);
-  return IG_OK;
+  return igint::host_io_finish(c, hc, io, mask_out, body_out);
 }
 
 int ig_sm_respond_batch_device(ig_ctx* c, uint64_t server, uint32_t count, const uint64_t* tables,
