@@ -727,29 +727,58 @@ __global__ void k_fold_gadget_keys(CrsDev c, u64* keys, u32 count) {
   x[4 * n] = canon(mulw(x[4 * n], c.s_rinv));
 }
 
-// Key rows of one query in shared memory, standard form: the rows of digits 0 and 1 side by side
-// for the mask (W01) and the seat (Y01), the rows of the derived digit 2 of both (WY2). The
+// The key rows of a mask or a seat as the recursion reads them, made once when the set or the seat is: per slot the
+// rows of digits 0 and 1 side by side (2n words), then the row of the derived digit 2 (n words, exact gadget only).
+// The recursion holds c_i = n^-1 R_i, so the inverse transform of a link needs no n^-1:
+//   c_i = (n^-1 a)[tau] S + sum_k (n^-1 W_k)[tau] D_k,   sum_b += sum_k Y_k[tau] D_k,
+// and with the exact gadget (rows folded as fold_gadget3 does), where R_{i+1} = n c_{i+1} takes the third digit's
+// place, W_2 stays and Y_2 is scaled by n. One CTA: the rows' transforms side by side, then the fold. Folded by every
+// respond CTA into its shared memory instead, the rows took 17,800 of the 123,000 cycles of a lone query of gamma 16.
+template <int LOGN, int ROWS>
+__global__ void __launch_bounds__((1 << LOGN) / 4) k_key_rows(CrsDev c, const u64* in, u64* out, KeyScale f) {
+  constexpr int N = 1 << LOGN, NT = N / 4;
+  extern __shared__ __align__(16) u64 sm[];
+  Tw* tw = reinterpret_cast<Tw*>(sm);
+  u64* x = sm + 2 * N;
+  for (int k = threadIdx.x; k < N; k += NT) {
+    tw[k] = c.tw[k];
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) x[r * N + k] = reduce128(in[r * N + k]);
+  }
+  __syncthreads();
+  {
+    u64* bufs_[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) bufs_[r] = x + r * N;
+    u64* const(&bufs)[ROWS] = bufs_;
+    ntt_fwd_r4<LOGN, NT, ROWS>(bufs, tw);
+  }
+  ulonglong2* pairs = reinterpret_cast<ulonglong2*>(out);
+  for (int k = threadIdx.x; k < N; k += NT) {
+    u64 y0 = mulw(x[k], f.digit), y1 = mulw(x[N + k], f.digit);
+    if constexpr (ROWS == 3) {
+      const u64 y2 = x[2 * N + k];
+      y0 += mulw(y2, f.fold0);
+      y1 += mulw(y2, f.fold1);
+      out[2 * N + k] = canon(mulw(y2, f.derived));
+    }
+    pairs[k] = make_ulonglong2(canon(y0), canon(y1));
+  }
+}
+
+// A query's key rows in shared memory: W01 and Y01 the pairs of the mask and the seat, WY2 the third rows of both. The
 // pointwise step gathers them with three 16-byte loads a slot.
 struct KeyRows {
   ulonglong2 *W01, *Y01, *WY2;
 };
-
-// Per-query constants into shared memory: forward ladder and slot tables of the ring (c), the mask
-// rows of the query's parameter set (v) and the seat's key rows (R-form NTT in global memory). The
-// recursion holds c_i = n^-1 R_i, so the inverse transform of a link needs no n^-1:
-//   c_i = (n^-1 a)[tau] S + sum_k (n^-1 W_k)[tau] D_k,   sum_b += sum_k Y_k[tau] D_k,
-// and with the exact gadget (rows folded by fold_gadget3), where R_{i+1} = n c_{i+1} takes the third
-// digit's place, W_2 stays and Y_2 is scaled by n.
-__device__ __forceinline__ void stage_key_rows(const CrsDev& c, const SetView& v, const u64* yR, const KeyRows& K, int n,
-                                               int k, int to) {
-  u64 w[3] = {v.wmask_R[k], v.wmask_R[n + k], 0}, y[3] = {yR[k], yR[n + k], 0};
-  if (v.approx == 0) {
-    fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, v.wmask_R + k, w, n, 1);
-    fold_gadget3(v.ld_inv_R, v.ld_c0_R, v.ld_c1_R, yR + k, y, n, 1);
-  }
-  K.W01[to] = make_ulonglong2(canon(mulw(w[0], c.s_ninv_rinv)), canon(mulw(w[1], c.s_ninv_rinv)));
-  K.Y01[to] = make_ulonglong2(canon(mulw(y[0], c.s_rinv)), canon(mulw(y[1], c.s_rinv)));
-  K.WY2[to] = make_ulonglong2(canon(mulw(w[2], c.s_rinv)), canon(mulw(y[2], c.s_n_rinv)));
+__device__ __forceinline__ void stage_key_rows(const SetView& v, const u64* seat, const KeyRows& K, int n, int k, int to) {
+  const u64* w = v.mask;
+  const ulonglong2 w01 = reinterpret_cast<const ulonglong2*>(w)[k], y01 = reinterpret_cast<const ulonglong2*>(seat)[k];
+  const bool exact = v.approx == 0;
+  const ulonglong2 wy2 = make_ulonglong2(exact ? w[2 * n + k] : 0, exact ? seat[2 * n + k] : 0);
+  K.W01[to] = w01;
+  K.Y01[to] = y01;
+  K.WY2[to] = wy2;
 }
 // The pointwise step of one slot at the gathered position tb: adds sum_k Y_k D_k to sb and returns
 // c_i. d0, d1 at most 15q, cur at most 1+: sb takes at most 31 q^2 < 2^125 a call.
@@ -1252,7 +1281,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
   for (int k = tid; k < N; k += NT) {
     tw[tw8<LOGN>(k)] = c.tw[k];
     s_tab[k] = (uint16_t)slot8<LOGN>(c.exp_slot[k]);
-    stage_key_rows(c, ps, qd.seat_R, K, N, k, slot8<LOGN>(k));
+    stage_key_rows(ps, qd.seat, K, N, k, slot8<LOGN>(k));
   }
   expand_a<N, NT>(qd, D + N, status, qi, force_serial);  // ends with a barrier
   {
@@ -1552,7 +1581,7 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   for (int k = tid; k < N; k += NT) {
     tw[k] = c.tw[k];
     s_tab[k] = (uint16_t)slot2<LOGN>(c.exp_slot[k]);
-    stage_key_rows(c, ps, qd.seat_R, KR, N, k, slot2<LOGN>(k));
+    stage_key_rows(ps, qd.seat, KR, N, k, slot2<LOGN>(k));
   }
   // The query's a: expanded and transformed in the exchange buffers' place, kept at its slots' positions.
   static_assert(4 * P >= N, "a fits the buffers");
@@ -2304,6 +2333,18 @@ cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t
   const u32 total = count * 2 * c.n;
   if (total == 0) return cudaSuccess;
   k_fold_gadget_keys<<<(total + 255) / 256, 256, 0, s>>>(c, keys, count);
+  return cudaGetLastError();
+}
+
+cudaError_t key_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, const KeyScale& f, cudaStream_t s) {
+  if (rows != 2 && rows != 3) return cudaErrorInvalidValue;
+  const size_t smem = (2 + rows) * (size_t)c.n * 8;
+  IG_DISPATCH_LOGN(c.logn, {
+    auto k = rows == 3 ? k_key_rows<L, 3> : k_key_rows<L, 2>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<1, (1 << L) / 4, smem, s>>>(c, in, out, f);
+  });
   return cudaGetLastError();
 }
 

@@ -19,9 +19,8 @@ enum DeviceStatus : u32 {
 struct CrsDev {
   u32 n, logn, gamma, rows, approx;
   const Tw* tw;           // forward ladder psi^brv(m), index m in [1, n)
-  // Scalars: n^-1; n^-1 2^-64, 2^-64 and n 2^-64, which take the recursion's R-form operands to
-  // the scaled standard form its links use (stage_constants).
-  Tw ninv, s_ninv_rinv, s_rinv, s_n_rinv;
+  // Scalars: n^-1; n^-1 2^-64 and 2^-64, which take R-form operands to the (scaled) standard form of the links.
+  Tw ninv, s_ninv_rinv, s_rinv;
   const uint16_t* slot_exp;  // odd exponent e_t of slot t's root relative to slot 0's
   const uint16_t* exp_slot;  // slot holding exponent e, indexed e/2
   const u32* gpow;           // g^i mod 2n, i < gamma
@@ -30,9 +29,9 @@ struct CrsDev {
   const Tw* pow_root;        // w0^e for e < 2n (w0 = slot 0's root)
   const Tw* zeta;            // zeta^j for j < gamma / 2, zeta = w0^(2n/gamma)
   Tw inv_gamma_R;            // gamma^-1 * 2^64 mod q
-  const u64* wmask_R;        // rows x n: NTT of the kept mask rows, R-form
+  const u64* mask;           // the kept mask rows as key rows (key_rows), rows x n words
   // The last exact-gadget digit's factors (D2 = base^-2 (R - D0 - base D1)) in R-form:
-  // base^-2, -base^-2 and -base^-1, by which the key rows are folded (fold_gadget3).
+  // base^-2, -base^-2 and -base^-1, by which the Galois keys are folded (fold_gadget3).
   u64 ld_inv_R, ld_c0_R, ld_c1_R;
   // Galois keys of the automorphism tree (OnePacking), null when the CRS carries none:
   // key i (t = n / 2^i + 1) as 3 rows of (a, b), each n words, standard-form NTT, folded and
@@ -46,7 +45,7 @@ struct QueryDev {
   u32 fold_off;       // first of the query's gamma words in the launch's b_fold
   const u32* seed;    // 8 ChaCha20 key words of the query's `a` seed
   const u64* b;       // coefficient-form b of the query (n words)
-  const u64* seat_R;  // rows x n key body in R-form NTT (the packing-key seat)
+  const u64* seat;    // the packing-key seat's key rows (key_rows), rows x n words
   const u64* a;       // explicit coefficient-form `a` (unseeded query), or null
   // The query's parameter set (a device copy of its CrsDev), or null for the launch's. Every
   // set of one launch shares the ring: n, q, the transform ladders and the slot tables;
@@ -61,15 +60,12 @@ struct QueryDev {
 struct SetView {
   u32 gamma, rows, approx;
   const u32* gpow;
-  const u64* wmask_R;
-  u64 ld_inv_R, ld_c0_R, ld_c1_R;
+  const u64* mask;
 };
 
 __device__ __forceinline__ SetView set_view(const CrsDev& c, const CrsDev* own) {
-  if (own)
-    return SetView{own->gamma, own->rows, own->approx, own->gpow, own->wmask_R, own->ld_inv_R, own->ld_c0_R,
-                   own->ld_c1_R};
-  return SetView{c.gamma, c.rows, c.approx, c.gpow, c.wmask_R, c.ld_inv_R, c.ld_c0_R, c.ld_c1_R};
+  if (own) return SetView{own->gamma, own->rows, own->approx, own->gpow, own->mask};
+  return SetView{c.gamma, c.rows, c.approx, c.gpow, c.mask};
 }
 
 // The client's Gaussian sampler (math/gaussian.rs:95-224): acceptance thresholds (f64 bit
@@ -103,6 +99,13 @@ using namespace ig;
 // that take the node in place of the derived third digit, and brought to the standard form
 // and the scale of the tree's nodes (n^-1 times their values).
 cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t s);
+// The factors that make a mask's or a seat's transforms key rows: of the digits' rows, of the third row where it is folded
+// into them, and of the third row itself.
+struct KeyScale {
+  Tw digit, fold0, fold1, derived;
+};
+// Key rows (k_key_rows) of a mask or a seat: 2 or 3 polynomials in, as many times n words out.
+cudaError_t key_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, const KeyScale& f, cudaStream_t s);
 // Forward NTT of `rows` polynomials: out[r] = scale * NTT(in[r] mod q), canonical (scale = 1 for
 // standard form, 2^64 mod q for R-form).
 cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, cudaStream_t s);

@@ -113,12 +113,20 @@ struct DevBuf {
 
 struct CrsObj {
   u32 n = 0, logn = 0, gamma = 0, rows = 0, approx = 0;
+  igk::KeyScale seat_scale;  // of the seats served under the set
   u64 p = 0;
   CrsDev dev{};
   CrsDev* d_self = nullptr;  // device copy of `dev`, named by the queries of mixed launches
   std::vector<void*> allocs;
   size_t bytes = 0;
 };
+
+// The factors of key rows scaled by `digit`, the derived third row's by `third` (k_key_rows).
+igk::KeyScale key_scale(u64 digit, u64 third) {
+  const u64 inv2 = invmod(1ULL << 40), inv1 = mulmod(inv2, 1ULL << 20);  // base^-2, base^-1
+  return igk::KeyScale{make_tw(digit), make_tw(negq(mulmod(digit, inv2))), make_tw(negq(mulmod(digit, inv1))),
+                       make_tw(mulmod(third, inv2))};
+}
 
 struct ShardSlot {
   u64* cols = nullptr;
@@ -145,7 +153,7 @@ struct DbObj {
 struct SeatObj {
   u64 crs = 0;
   u32 n = 0, rows = 0, num_to_pack = 0;
-  u64* yR = nullptr;
+  u64* rows_dev = nullptr;  // key rows (igk::key_rows)
 };
 
 struct StoreObj {
@@ -840,7 +848,7 @@ void ig_ctx_destroy(ig_ctx* c) {
     cudaFree(kv.second.d_table);
   }
   for (auto& kv : c->stores)
-    for (auto& s : kv.second.seats) cudaFree(s.second.yR);
+    for (auto& s : kv.second.seats) cudaFree(s.second.rows_dev);
   for (auto& kv : c->clients)
     for (void* p : kv.second.allocs) cudaFree(p);
   for (auto& kv : c->scratch) cudaFree(kv.second.p);
@@ -970,15 +978,15 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   d.ninv = make_tw(ninv);
   d.s_ninv_rinv = make_tw(mulmod(ninv, rinv));
   d.s_rinv = make_tw(rinv);
-  d.s_n_rinv = make_tw(mulmod(n, rinv));
   d.inv_gamma_R = make_tw(mulmod(invmod(gamma), R_MOD_Q));
-  // Last exact digit: base^-2 (R - D0 - base D1) (inspiring2.rs:1094-1161). The kernels
-  // fold these three factors into the key rows (fold_gadget3) rather than form the digit.
+  // Last exact digit: base^-2 (R - D0 - base D1) (inspiring2.rs:1094-1161). These three
+  // factors are folded into the key rows (key_scale) and Galois keys rather than form the digit.
   const u64 inv = invmod(1ULL << 40);
   d.ld_inv_R = mulmod(inv, R_MOD_Q);
   d.ld_c0_R = mulmod(negq(inv), R_MOD_Q);
   d.ld_c1_R = mulmod(negq(mulmod(inv, 1ULL << 20)), R_MOD_Q);
-  // Mask rows -> NTT, R-form.
+  o.seat_scale = key_scale(1, n);
+  // Mask rows -> key rows.
   void* mraw = nullptr;
   void* wm = nullptr;
   rc = scratch(c, "mask_raw", mask.size() * 8, &mraw);
@@ -990,9 +998,9 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   }
   o.allocs.push_back(wm);
   IG_CUDA(c, cudaMemcpyAsync(mraw, mask.data(), mask.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  IG_CUDA(c, igk::ntt_rows(d, (const u64*)mraw, (u64*)wm, o.rows, R_MOD_Q, c->stream));
+  IG_CUDA(c, igk::key_rows(d, (const u64*)mraw, (u64*)wm, o.rows, key_scale(ninv, 1), c->stream));
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
-  d.wmask_R = (const u64*)wm;
+  d.mask = (const u64*)wm;
   if ((rc = sync_crs_self(c, o))) {
     for (void* p2 : o.allocs) cudaFree(p2);
     c->obj_bytes -= o.bytes;
@@ -1250,7 +1258,7 @@ int ig_session_store_destroy(ig_ctx* c, uint64_t st) {
   auto it = c->stores.find(st);
   if (it == c->stores.end()) return fail(c, IG_ERR_HANDLE, "unknown session store %llu", (unsigned long long)st);
   cudaStreamSynchronize(c->stream);
-  for (auto& s : it->second.seats) dfree(c, s.second.yR, (size_t)s.second.rows * s.second.n * 8);
+  for (auto& s : it->second.seats) dfree(c, s.second.rows_dev, (size_t)s.second.rows * s.second.n * 8);
   c->stores.erase(it);
   return IG_OK;
 }
@@ -1278,7 +1286,7 @@ static int make_seat(ig_ctx* c, CrsObj& o, const uint64_t* y_body, uint32_t rows
     IG_CUDA(c, cudaMemcpyAsync(raw, y_body, (size_t)rows * o.n * 8, cudaMemcpyHostToDevice, c->stream));
     src = (const u64*)raw;
   }
-  IG_CUDA(c, igk::ntt_rows(o.dev, src, dst, rows, R_MOD_Q, c->stream));
+  IG_CUDA(c, igk::key_rows(o.dev, src, dst, rows, o.seat_scale, c->stream));
   return IG_OK;
 }
 
@@ -1297,19 +1305,19 @@ int ig_session_register(ig_ctx* c, uint64_t st, uint64_t crs, const uint64_t* y_
   seat.rows = rows;
   seat.num_to_pack = num_to_pack;
   if (rows == o->rows) {
-    int rc = dalloc(c, (void**)&seat.yR, (size_t)rows * o->n * 8, nullptr);
+    int rc = dalloc(c, (void**)&seat.rows_dev, (size_t)rows * o->n * 8, nullptr);
     if (rc) return rc;
   }
-  int rc = make_seat(c, *o, y_body, rows, num_to_pack, seat.yR, false);
+  int rc = make_seat(c, *o, y_body, rows, num_to_pack, seat.rows_dev, false);
   if (rc) {
-    dfree(c, seat.yR, (size_t)rows * o->n * 8);
+    dfree(c, seat.rows_dev, (size_t)rows * o->n * 8);
     return rc;
   }
   IG_CUDA(c, cudaStreamSynchronize(c->stream));
   u64 h = g_next_handle.load();
   do {
     if (h == ~0ULL) {
-      dfree(c, seat.yR, (size_t)rows * o->n * 8);
+      dfree(c, seat.rows_dev, (size_t)rows * o->n * 8);
       return fail(c, IG_ERR_EXHAUSTED,
                   "ServerSessionStore handle space exhausted at %llu; refusing the session handshake because "
                   "handle reuse could resolve stale clients to another client's packing keys",
@@ -1330,7 +1338,7 @@ int ig_session_remove(ig_ctx* c, uint64_t st, uint64_t handle, int* removed) {
   *removed = s != it->second.seats.end();
   if (*removed) {
     cudaStreamSynchronize(c->stream);
-    dfree(c, s->second.yR, (size_t)s->second.rows * s->second.n * 8);
+    dfree(c, s->second.rows_dev, (size_t)s->second.rows * s->second.n * 8);
     it->second.seats.erase(s);
   }
   return IG_OK;
@@ -1389,7 +1397,7 @@ static int resolve_seat(ig_ctx* c, CrsObj& o, uint64_t st, uint64_t handle, cons
     return fail(c, IG_ERR_WIDTH,
                 "packing-key width mismatch: client keys declare gamma = %u, server pack params use gamma = %u.",
                 seat.num_to_pack, o.gamma);
-  *seat_out = seat.yR;
+  *seat_out = seat.rows_dev;
   return IG_OK;
 }
 
@@ -1409,7 +1417,7 @@ static int resolve_seat_for_db(ig_ctx* c, CrsObj& db_set, uint64_t st, uint64_t 
       CrsObj* own = get_crs(c, sit->second.crs);
       if (own && own != &db_set && own->n == db_set.n && own->gamma == db_set.gamma &&
           sit->second.rows == own->rows && sit->second.num_to_pack == own->gamma) {
-        *seat_out = sit->second.yR;
+        *seat_out = sit->second.rows_dev;
         *set_out = own;
         return IG_OK;
       }
@@ -1515,7 +1523,7 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
     qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
     qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
     qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
-    qs[i].seat_R = seat;
+    qs[i].seat = seat;
     qs[i].ms = ms_target;
     qs[i].row = i;
   }
@@ -1634,7 +1642,7 @@ int ig_respond_nopacking_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const ui
     qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
     qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
     qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
-    qs[i].seat_R = nullptr;
+    qs[i].seat = nullptr;
   }
   cudaStream_t s = igint::host_call_stream(c, hc), copy = igint::host_call_copy_stream(c, hc);
   if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
@@ -1995,7 +2003,7 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     qs[i].seed = as ? nullptr : (const u32*)(io.dev + io.seeds + (size_t)i * 32);
     qs[i].a = as ? (const u64*)(io.dev + io.seeds) + (size_t)i * n : nullptr;
     qs[i].b = (const u64*)(io.dev + io.bs) + (size_t)i * n;
-    qs[i].seat_R = nullptr;
+    qs[i].seat = nullptr;
     qs[i].fold_off = i * o.gamma;
     qs[i].row = i;
   }
@@ -2057,7 +2065,7 @@ int ig_respond_seeded_batch_device(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_
     qs[i].fold_off = i * (u32)g;
     qs[i].seed = (const u32*)(d_seeds + (size_t)i * 32);
     qs[i].b = d_bs + (size_t)i * n;
-    qs[i].seat_R = seat;
+    qs[i].seat = seat;
     qs[i].ms = ms_target;
     qs[i].row = i;
   }
@@ -2136,7 +2144,7 @@ static int plan_mixed(ig_ctx* c, u32 count, const uint64_t* dbs, const uint64_t*
     QueryDev& q = P.qs[i];
     q = QueryDev{};
     q.shard = it->second;
-    q.seat_R = seat;
+    q.seat = seat;
     q.crs = o.d_self;
     q.ms = ms;
     q.row = i;
@@ -3057,7 +3065,7 @@ int ig_respond_seeded_batch_noalloc(ig_ctx* c, uint64_t dbh, uint64_t st, uint64
     qs[i].fold_off = i * (u32)g;
     qs[i].seed = (const u32*)(d_seeds + (size_t)i * 32);
     qs[i].b = d_bs + (size_t)i * n;
-    qs[i].seat_R = seat;
+    qs[i].seat = seat;
     qs[i].ms = ms_target;
     qs[i].row = i;
   }

@@ -377,7 +377,7 @@ int form_batch(ig_serve* s, CrsDev* ring_out) {
     q.fold_off = (u32)fold_off;
     q.seed = (const u32*)(d + sl.L.seeds + (size_t)i * 32);
     q.b = (const u64*)(d + sl.L.bs) + (size_t)i * n;
-    q.seat_R = r->v.seat;
+    q.seat = r->v.seat;
     q.crs = r->v.crs_dev;
     q.ms = r->ms;
     q.row = i;
