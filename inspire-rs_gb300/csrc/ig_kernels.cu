@@ -1269,6 +1269,8 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
   const KeyRows K{rows, rows + N, rows + 2 * N};
   uint16_t* s_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);  // position of the slot of exponent 2e + 1
 
+  // The launch of a batch's tail may follow as SMs come free (it waits for this one's end at its own: scan_done).
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x;
   const QueryDev qd = queries[blockIdx.x];
   const u32 qi = qd.row;  // output and status row
@@ -1278,10 +1280,12 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
   const bool exact = ps.approx == 0;
   const int l0 = 8 * tid;
 
+#pragma unroll 4
+  for (int k = tid; k < N; k += NT) stage_key_rows(ps, qd.seat, K, N, k, slot8<LOGN>(k));
+#pragma unroll 8
   for (int k = tid; k < N; k += NT) {
     tw[tw8<LOGN>(k)] = c.tw[k];
     s_tab[k] = (uint16_t)slot8<LOGN>(c.exp_slot[k]);
-    stage_key_rows(ps, qd.seat, K, N, k, slot8<LOGN>(k));
   }
   expand_a<N, NT>(qd, D + N, status, qi, force_serial);  // ends with a barrier
   {
@@ -1363,7 +1367,14 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 //      cycles); the digits' words go back to their owners the same way.
 //   4. local forward of both digits, the inverse's passes backwards with a unit of one digit a thread, ending with
 //      both digits of the thread's own pair.
-//   5. the pointwise step. The online sum is off the chain, so its products run while the cross words travel.
+//   5. the pointwise step. The online sum is off the chain, so its products run while the cross words travel, and
+//      the products of a, S and c_{i+1} while the digits do: 64 queries of gamma 256 1.27 -> 1.16 ms, 33 of gamma
+//      1024 2.97 -> 2.84 ms.
+// Setup: each CTA transforms its part of a and sends the slots to every CTA (each transforming all of it, and staging
+// one load a thread at a time: 30,700 -> 14,800 cycles, a lone query of gamma 16 122 -> 112 us with the end below).
+// A link of four CTAs now takes 5,000 cycles: inverse 1,600, its exchange 610, cross 820, the digits' 220, forward
+// 1,180, pointwise 570. Two CTAs an SM (the seat's rows from L2, half the shared memory) ran 64 queries no faster
+// than clusters of two: both share the multiply pipe.
 // The data's own arrivals order every buffer's reuse. A CTA sends a link's cross words after its forward of the
 // link before, which took digits from every peer, and a peer sends those after reading its cross words; it sends
 // digits after taking cross words from every peer, and a peer's threads send those after reading their
@@ -1379,16 +1390,24 @@ struct Part {
   static __host__ __device__ constexpr int bits(int b) { return b + 1 < LP ? 2 : 1; }  // of the pass from bit b (odd)
 };
 
+// A part's ladders: level m' (entries m' + i, i < m') holds the ring's level m' R at the entries of the part's blocks
+// for the forward, at those of the mirrored part's for the inverse.
+template <int R>
+__device__ __forceinline__ int part_ladder(int k, int part) {
+  const int m = 1 << (31 - __clz(k));
+  return m * (R + part) + (k - m);
+}
+
 // Local inverse stages from bit B up, on the part's words X (2+ in and out); put(e, word) takes the last
-// pass's words instead of X. `base`: the part's first index.
+// pass's words instead of X. tw: the mirrored part's ladder.
 template <int LOGN, int R, int B, class Put>
-__device__ __forceinline__ void part_inverse(u64* X, int base, const Tw* tw, Put put) {
+__device__ __forceinline__ void part_inverse(u64* X, const Tw* tw, Put put) {
   using G = Part<LOGN, R>;
   if constexpr (B < G::LP) {
-    constexpr int n = G::bits(B), t = 1 << B, M = G::N >> (B + 1);
+    constexpr int n = G::bits(B), t = 1 << B, M = G::P >> (B + 1);
     constexpr bool last = B + n == G::LP;
     if ((int)threadIdx.x < (G::P >> n)) {
-      const int e = G::unit(threadIdx.x, B, n), i = (base + e) >> (B + 1);
+      const int e = G::unit(threadIdx.x, B, n), i = e >> (B + 1);
       u64 x[1 << n];
 #pragma unroll
       for (int k = 0; k < 1 << n; k++) x[k] = X[G::sw(e + k * t)];
@@ -1412,26 +1431,26 @@ __device__ __forceinline__ void part_inverse(u64* X, int base, const Tw* tw, Put
       else
         __syncwarp();
     }
-    part_inverse<LOGN, R, B + n>(X, base, tw, put);
+    part_inverse<LOGN, R, B + n>(X, tw, put);
   }
 }
 
 // Local forward stages from the pass at bit B down to bit 1, both digits in place (D[0..P), D[P..2P)), words
-// up to W in and part_bound out. Ends with a CTA barrier.
+// up to W in and part_bound out. tw: the part's ladder. Ends with a CTA barrier.
 __host__ __device__ constexpr int part_bound(int lp, int b, int w) {
   for (; b >= 1; b -= 2) w = b + 1 < lp ? (w > FWD_FREE ? 1 : w) + 6 : (w > 12 ? 1 : w) + 3;
   return w;
 }
 template <int LOGN, int R, int B, int W>
-__device__ __forceinline__ void part_forward(u64* D, int base, const Tw* tw) {
+__device__ __forceinline__ void part_forward(u64* D, const Tw* tw) {
   using G = Part<LOGN, R>;
   if constexpr (B >= 1) {
-    constexpr int n = G::bits(B), t = 1 << B, m = G::N >> (B + n);
+    constexpr int n = G::bits(B), t = 1 << B, m = G::P >> (B + n);
     constexpr bool RED = n == 2 ? W > FWD_FREE : W > 12;
     if constexpr (n == 2) {  // a unit of one digit a thread
       const int u = threadIdx.x & (G::P / 4 - 1);
       u64* x = D + ((int)threadIdx.x < G::P / 4 ? 0 : G::P);
-      const int e = G::unit(u, B, 2), i = (base + e) >> (B + 2);
+      const int e = G::unit(u, B, 2), i = e >> (B + 2);
       const int i0 = G::sw(e), i1 = G::sw(e + t), i2 = G::sw(e + 2 * t), i3 = G::sw(e + 3 * t);
       u64 a0 = x[i0], a1 = x[i1], a2 = x[i2], a3 = x[i3];
       fwd_unit<RED>(a0, a1, a2, a3, tw[m + i], tw[2 * m + 2 * i], tw[2 * m + 2 * i + 1]);
@@ -1441,7 +1460,7 @@ __device__ __forceinline__ void part_forward(u64* D, int base, const Tw* tw) {
       x[i3] = a3;
     } else {  // a pair of each digit a thread
       const int e = G::unit(threadIdx.x, B, 1), i0 = G::sw(e), i1 = G::sw(e + t);
-      const Tw w = tw[m + ((base + e) >> (B + 1))];
+      const Tw w = tw[m + (e >> (B + 1))];
 #pragma unroll
       for (int d = 0; d < 2; d++) {
         u64* x = D + d * G::P;
@@ -1456,7 +1475,7 @@ __device__ __forceinline__ void part_forward(u64* D, int base, const Tw* tw) {
       __syncthreads();
     else
       __syncwarp();
-    part_forward<LOGN, R, B - 2, (RED ? 1 : W) + 3 * n>(D, base, tw);
+    part_forward<LOGN, R, B - 2, (RED ? 1 : W) + 3 * n>(D, tw);
   }
 }
 
@@ -1513,6 +1532,11 @@ __device__ __forceinline__ void send_word(u32 to, u64 v, u32 bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to), "l"(v), "r"(bar)
                : "memory");
 }
+__device__ __forceinline__ void store_remote(u32 to, u64 v) {
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(to), "l"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void inbox_init(u32 bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
 }
@@ -1549,8 +1573,9 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   u64* D = XB + P;        // [2][P] this part of digits 0 and 1
   u64* X = D + 2 * P;     // [P] the local inverse
   u64* a_ntt = X + P;
-  Tw* tw = reinterpret_cast<Tw*>(a_ntt + N);
-  ulonglong2* rows = reinterpret_cast<ulonglong2*>(tw + N);  // room for three key rows, as in k_respond
+  Tw* fl = reinterpret_cast<Tw*>(a_ntt + N);  // the part's forward ladder
+  Tw* il = fl + P;                            // the mirrored part's, for the inverse
+  ulonglong2* rows = reinterpret_cast<ulonglong2*>(il + P);  // room for three key rows, as in k_respond
   const KeyRows KR{rows, rows + N, rows + 2 * N};
   uint16_t* s_tab = reinterpret_cast<uint16_t*>(rows + 3 * N);  // position of the slot of exponent 2e + 1
 
@@ -1578,22 +1603,66 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   const SetView ps = set_view(c, qd.crs);
   const u32 gamma = ps.gamma;
 
-  for (int k = tid; k < N; k += NT) {
-    tw[k] = c.tw[k];
-    s_tab[k] = (uint16_t)slot2<LOGN>(c.exp_slot[k]);
-    stage_key_rows(ps, qd.seat, KR, N, k, slot2<LOGN>(k));
+  cluster_arrive();
+  {
+#pragma unroll 4
+    for (int k = tid; k < N; k += NT) stage_key_rows(ps, qd.seat, KR, N, k, slot2<LOGN>(k));
+#pragma unroll 8
+    for (int k = tid; k < N; k += NT) s_tab[k] = (uint16_t)slot2<LOGN>(c.exp_slot[k]);
+    Tw f[2], i[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int k = max(tid + j * NT, 1);
+      f[j] = c.tw[part_ladder<R>(k, rank)];
+      i[j] = c.tw[part_ladder<R>(k, R - 1 - rank)];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      fl[tid + j * NT] = f[j];
+      il[tid + j * NT] = i[j];
+    }
   }
-  // The query's a: expanded and transformed in the exchange buffers' place, kept at its slots' positions.
+  const Tw w1 = c.tw[1], w2 = R == 4 ? c.tw[2] : w1, w3 = R == 4 ? c.tw[3] : w1;
+  const int base = rank * P, l0 = base + 2 * tid;  // this thread's slots: l0, l0 + 1
+  const u32 et[2] = {c.slot_exp[l0], c.slot_exp[l0 + 1]};
+  // The query's a, expanded in the exchange buffers' place by every CTA, each transforming its part: the first log R
+  // stages of the part's words, its local stages as one digit's. The slots go to every CTA's a_ntt.
   static_assert(4 * P >= N, "a fits the buffers");
   expand_a<N, NT>(qd, sm, status, qi, force_serial);  // ends with a barrier
   {
-    u64* const bufs[1] = {sm};
-    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
+    u64 y[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const u64* x = sm + tid + j * NT;
+      u64 u = x[0], v;
+      if constexpr (R == 2) {
+        v = mulw(x[P], w1);
+      } else {
+        const u64 t0 = mulw(x[2 * P], w1), t1 = mulw(x[3 * P], w1);
+        u += rank < 2 ? t0 : 3 * Q - t0;
+        v = mulw(rank < 2 ? x[P] + t1 : x[P] + 3 * Q - t1, rank < 2 ? w2 : w3);
+      }
+      y[j] = u + (rank & 1 ? 3 * Q - v : v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; j++) D[G::sw(tid + j * NT)] = y[j];
+    __syncthreads();
+    part_forward<LOGN, R, TOP, 7>(D, fl);  // the second buffer's words go along unused
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(D + G::sw(2 * tid));
+    u64 a0 = part_bound(LP, TOP, 7) > 12 ? red60(v.x) : v.x, a1 = v.y;
+    bf_fwd(a0, a1, fl[P / 2 + tid]);
+    a0 = canon(mulw(a0, c.s_ninv_rinv));
+    a1 = canon(mulw(a1, c.s_ninv_rinv));
+    cluster_wait();  // every CTA runs
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const u32 to = peer[k] + (u32)((uint8_t*)a_ntt - (uint8_t*)sm);
+      store_remote(to + 8 * slot2<LOGN>(l0), a0);
+      store_remote(to + 8 * slot2<LOGN>(l0 + 1), a1);
+    }
   }
-  for (int k = tid; k < N; k += NT) a_ntt[slot2<LOGN>(k)] = canon(mulw(sm[k], c.s_ninv_rinv));
-  const int base = rank * P, l0 = base + 2 * tid;  // this thread's slots: l0, l0 + 1
-  const u32 et[2] = {c.slot_exp[l0], c.slot_exp[l0 + 1]};
-  __syncthreads();
+  cluster.sync();  // every CTA has its a, and is past its use of the exchange buffers
   u64 cur[2];
   Acc sb[2];
   {
@@ -1604,24 +1673,23 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
       sb[k] = Acc{0, 0, 0, 0};
     }
   }
-  const Tw w1 = tw[1], w2 = R == 4 ? tw[2] : w1, w3 = R == 4 ? tw[3] : w1;
   // This thread's cross word and, with four CTAs, its digit.
   const int q = tid & (C - 1), dg = tid / C;
-  cluster.sync();  // every CTA is past its use of the exchange buffers
-
   // Twiddles of the thread's own pair: stage 0 of the inverse, the last of the forward.
-  const Tw wi0 = tw[N - 1 - (l0 >> 1)], wf0 = tw[N / 2 + (l0 >> 1)];
-  // The thread's pair through the local inverse, its words to the CTAs that cross them.
-  auto inverse_to_cross = [&](u64 x0, u64 x1) {
+  const Tw wi0 = il[P - 1 - tid], wf0 = fl[P / 2 + tid];
+  // The thread's pair through the local inverse, its words to the CTAs that cross them (their words buffer, or with
+  // `second` their digits').
+  auto inverse_to_cross = [&](u64 x0, u64 x1, u32 second) {
+    const u32 off = second * 8 * P, box = second * 8;
     bf_inv<2>(x0, x1, wi0);
     *reinterpret_cast<ulonglong2*>(X + G::sw(2 * tid)) = make_ulonglong2(x0, x1);
     __syncthreads();
-    part_inverse<LOGN, R, 1>(X, base, tw, [&](int e, int k, u64 x) {
-      const u32 at = 8 * (rank * C + (e & (C - 1)));
+    part_inverse<LOGN, R, 1>(X, il, [&](int e, int k, u64 x) {
+      const u32 at = off + 8 * (rank * C + (e & (C - 1)));
       if constexpr (G::bits(LP & 1 ? LP - 2 : LP - 1) == G::LR) {  // the pass holds the bits of the crossing CTA
-        send_word(peer[k] + at, x, peer_words[k]);
+        send_word(peer[k] + at, x, peer_words[k] + box);
       } else {
-        send_word(cluster_addr(smem_addr(sm) + at, e / C), x, cluster_addr(in_words, e / C));
+        send_word(cluster_addr(smem_addr(sm) + at, e / C), x, cluster_addr(in_words + box, e / C));
       }
     });
   };
@@ -1657,7 +1725,7 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
         inbox_expect(in_words, P * 8);
         inbox_expect(in_digits, 2 * P * 8);
       }
-      inverse_to_cross(cur[0], cur[1]);
+      inverse_to_cross(cur[0], cur[1], 0);
       online(i);
       await(in_words);
       {
@@ -1686,9 +1754,22 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
           for (int k = 0; k < R; k++) send_word(peer[k] + to, y[k], peer_digits[k]);
         }
       }
+      // What the pointwise step has without the digits, while they travel.
+      Acc r[2];
+      ulonglong2 w[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
+        w[k] = KR.W01[tb];
+        r[k] = Acc{0, 0, 0, 0};
+        mac(r[k], a_ntt[tb], k ? sv.y : sv.x);
+        if constexpr (EXACT) mac(r[k], cur[k], KR.WY2[tb].x);
+        pc[k] = cur[k];
+        pt[k] = tb;
+      }
       await(in_digits);
       parity ^= 1;
-      part_forward<LOGN, R, TOP, 3 * G::LR>(D, base, tw);
+      part_forward<LOGN, R, TOP, 3 * G::LR>(D, fl);
       u64 d[2][2];
 #pragma unroll
       for (int n = 0; n < 2; n++) {
@@ -1699,18 +1780,11 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
       }
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        const u32 tb = s_tab[((gp * et[k]) & M2N) >> 1];
-        const ulonglong2 w = KR.W01[tb];
-        Acc r{0, 0, 0, 0};
-        mac(r, a_ntt[tb], k ? sv.y : sv.x);
-        if constexpr (EXACT) mac(r, cur[k], KR.WY2[tb].x);
-        mac(r, d[0][k], w.x);
-        mac(r, d[1][k], w.y);
+        mac(r[k], d[0][k], w[k].x);
+        mac(r[k], d[1][k], w[k].y);
         pd0[k] = d[0][k];
         pd1[k] = d[1][k];
-        pc[k] = cur[k];
-        pt[k] = tb;
-        cur[k] = acc_fold(r);
+        cur[k] = acc_fold(r[k]);
       }
     }
     online(0);
@@ -1719,21 +1793,19 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
     links(std::true_type{});
   else
     links(std::false_type{});
-  // Final inverse transforms of c_0 (to a) and of the online sum (to b): local stages, then the cross.
+  // Final inverse transforms of c_0 (to a) and of the online sum (to b): local stages, then the cross. With four CTAs
+  // the sum's words go to the digits' buffer (a peer that sent its first words has read its last digits) and the two
+  // crosses run side by side, on half the threads each (12,200 -> 8,800 cycles after the links); with two every
+  // thread crosses, one transform after the other.
   scan_done();
-#pragma unroll 1
-  for (int n = 0; n < 2; n++) {
-    if (tid == 0 && alive) inbox_expect(in_words, P * 8);
-    inverse_to_cross(n ? acc_fold(sb[0]) : cur[0], n ? acc_fold(sb[1]) : cur[1]);
-    await(in_words);
-    parity ^= 1;
+  constexpr bool SIDE = R == 4;
+  auto cross = [&](int n, auto read) {
     u64 x[R], cf[R];
 #pragma unroll
-    for (int k = 0; k < R; k++) x[k] = XB[k * C + q];
-    cluster.sync();  // the words are read before the next are pushed, and before a CTA ends
+    for (int k = 0; k < R; k++) x[k] = XB[(SIDE ? n * P : 0) + k * C + q];
+    read();
     // Unscaled residues: finish_a takes the coefficient as it is, finish_b times n^-1.
     cross_inverse<R>(x, cf, w1, w2, w3);
-    if (dg) continue;
 #pragma unroll
     for (int k = 0; k < R; k++) {
       const int t = k * P + rank * C + q;
@@ -1742,6 +1814,21 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
       else
         b_out[(size_t)qi * N + t] = finish_b(c, cf[k], t, gamma, b_fold + qd.fold_off, qd.ms);
     }
+  };
+#pragma unroll 1
+  for (int n = 0; n < 2; n++) {
+    const u32 second = SIDE ? n : 0, box = in_words + 8 * second;
+    if (tid == 0 && alive) inbox_expect(box, P * 8);
+    inverse_to_cross(n ? acc_fold(sb[0]) : cur[0], n ? acc_fold(sb[1]) : cur[1], second);
+    await(box);
+    if constexpr (!SIDE) {
+      parity ^= 1;
+      cross(n, [&] { cluster.sync(); });  // the words are read before the next are sent, and before a CTA ends
+    }
+  }
+  if constexpr (SIDE) {
+    cross(dg, [] {});
+    cluster.sync();  // no CTA ends with words on their way to a peer
   }
 }
 
@@ -2574,7 +2661,7 @@ size_t respond_smem_bytes(const CrsDev& c, int ctas) {
   // Transform buffers (2n words, or four parts of n / ctas), a_ntt and the ladder, three key rows of W and Y, the
   // u16 slot table.
   const size_t n = c.n;
-  const size_t words = (ctas == 1 ? 2 * n : 4 * n / ctas) + 3 * n + 6 * n;
+  const size_t words = ctas == 1 ? 2 * n + 3 * n + 6 * n : 4 * n / ctas + n + 4 * n / ctas + 6 * n;
   return words * 8 + n * 2;
 }
 
