@@ -1433,6 +1433,26 @@ static bool env_profile() {
   return on;
 }
 
+// The respond launches of `count` queries of one width. A batch larger than the GPU runs one CTA a query for its whole
+// waves; what is left takes the shape of a batch of its size, on the SMs as the last wave leaves them (one CTA a
+// query would hold a third of them for a whole wave: 509 queries of gamma 256 6.78 -> 6.15 ms). Lanes fill such a tail
+// with the next batch instead.
+static cudaError_t respond_waves(ig_ctx* c, const CrsDev& dev, const QueryDev* q, const ShardDev* table, u32 count,
+                                 const u64* fold, u64* a, u64* b, u32* status, cudaStream_t s) {
+  u32 head = 0;
+  if (c->lanes <= 1 && !c->force_ctas && count > c->sms) {
+    const u32 rest = count % c->sms;
+    if (rest && igint::launch_ctas(c, dev.n, dev.gamma, rest, rest) > 1) head = count - rest;
+  }
+  if (head) {
+    cudaError_t e = igk::respond(dev, q, table, head, fold, a, b, status, c->force_serial, 1, s);
+    if (e != cudaSuccess) return e;
+  }
+  const u32 rest = count - head;
+  return igk::respond(dev, q + head, table, rest, fold, a, b, status, c->force_serial,
+                      igint::launch_ctas(c, dev.n, dev.gamma, rest, rest * c->lanes), s);
+}
+
 static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, const uint64_t* inline_y,
                         uint32_t inline_rows, uint32_t inline_ntp, uint32_t count, const uint32_t* shard_ids,
                         const uint8_t* seeds, const uint64_t* as, const uint64_t* bs, uint64_t ms_target,
@@ -1444,7 +1464,7 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
   // are copied out; the context lock is held only while the call validates and launches.
   igint::HostCall hc;
   igint::host_call_begin(c, hc);
-  const u32 lanes = c->lanes, k = hc.k;
+  const u32 k = hc.k;
   std::unique_lock<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   DbObj* db = get_db(c, dbh);
@@ -1542,8 +1562,8 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
   prof_end(c, pk, s);
   if (env_prof) cudaEventRecord(env_ev[1], s);
   pk = prof_begin(c, REGION_RESPOND, s);
-  IG_CUDA(c, igk::respond(o.dev, d_q, d_table, count, (const u64*)d_fold, (u64*)(io.dev + io.a), (u64*)(io.dev + io.b),
-                          d_status, c->force_serial, igint::launch_ctas(c, (u32)n, (u32)g, count, count * lanes), s));
+  IG_CUDA(c, respond_waves(c, o.dev, d_q, d_table, count, (const u64*)d_fold, (u64*)(io.dev + io.a),
+                           (u64*)(io.dev + io.b), d_status, s));
   prof_end(c, pk, s);
   if (env_prof) {
     cudaEventRecord(env_ev[2], s);
@@ -2076,10 +2096,9 @@ int ig_respond_seeded_batch_device(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_
   IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, db->d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
   prof_end(c, pk, s);
   // Several CTAs per query only while every lane's batch still leaves SMs for them.
-  const int ctas = igint::launch_ctas(c, (u32)n, (u32)g, count, count * c->lanes);
   pk = prof_begin(c, REGION_RESPOND, s);
-  IG_CUDA(c, igk::respond(o.dev, (const QueryDev*)d_q, db->d_table, count, (const u64*)d_fold, d_a, d_b, d_status,
-                          c->force_serial, ctas, s));
+  IG_CUDA(c, respond_waves(c, o.dev, (const QueryDev*)d_q, db->d_table, count, (const u64*)d_fold, d_a, d_b, d_status,
+                           s));
   prof_end(c, pk, s);
   return igint::lane_release(c, lane);
 }
@@ -2177,7 +2196,7 @@ struct ShapeRun {
 // Shapes of a mixed launch of several widths, whose queries need not share one: under a bound T on a query's own
 // time each query takes the fewest CTAs that keep it (four where none does), and T is the one whose launch
 // ends first when the queries start longest first as SMs come free. Times are the tuned table's for one query,
-// else 6.65, 4.62 and 2.76 us a link (measured at gamma 256 under one, two and four CTAs). 128 queries over gamma
+// else 6.95, 4.15 and 2.62 us a link (measured at gamma 1024 under one, two and four CTAs). 128 queries over gamma
 // 16, 256 and 1024 in equal parts took one CTA each: 7.65 ms, the time of the 43 longest, with most SMs
 // idle after 2 ms. Lanes share the SMs. More queries than four an SM fill the GPU in any order: one CTA each.
 static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u32 count) {
@@ -2189,7 +2208,7 @@ static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u
   std::vector<double> bounds;
   for (u32 g : P.gammas)
     if (!times.count(g)) {
-      std::array<double, 3> t{6.65 * g, 4.62 * g, 2.76 * g};
+      std::array<double, 3> t{6.95 * g, 4.15 * g, 2.62 * g};
       if (c->tune.count({n, g}))  // milliseconds, of this width only
         for (int k = 0; k < 3; k++) t[k] = 1e3 * (*igint::tuned_row(c, n, g, 1))[k];
       times[g] = t;
@@ -3074,9 +3093,7 @@ int ig_respond_seeded_batch_noalloc(ig_ctx* c, uint64_t dbh, uint64_t st, uint64
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
   IG_CUDA(c, igk::shard_scan(o.dev, d_q, db->d_table, count, nullptr, 0, d_fold, d_status, s));
   // The launch shape of ig_respond_seeded_batch_device for the same batch and lane count.
-  IG_CUDA(c, igk::respond(o.dev, d_q, db->d_table, count, d_fold, d_a, d_b, d_status, c->force_serial,
-                          igint::launch_ctas(c, (u32)n, (u32)g, count, count * c->lanes),
-                          s));
+  IG_CUDA(c, respond_waves(c, o.dev, d_q, db->d_table, count, d_fold, d_a, d_b, d_status, s));
   c->launches += 2;
   u32 status[NOALLOC_MAX_QUERIES];
   IG_CUDA(c, cudaMemcpyAsync(status, d_status, count * 4, cudaMemcpyDeviceToHost, s));
