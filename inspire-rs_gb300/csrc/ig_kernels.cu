@@ -206,9 +206,11 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_ntt_rows(CrsDev c, const u6
 // The sum lands at S_i[t'] with table_i[t'] = t, i.e. t' = slot of exponent c_i * e_t,
 // scaled by gamma^-1 and stored in R-form.
 //
-// One launch folds several shards (blockIdx.y): a shard alone leaves most of the GPU idle. The powers of
-// w0 come from global memory (one gather a word, 64 KB, kept in L1 and L2) and only the DFT's gamma / 2
-// twiddles are staged, where staging every power took 32 KB of loads for a tile of 16 KB.
+// One launch folds several shards (blockIdx.y): a shard alone leaves most of the GPU idle. What bounds it is the LSU
+// path, so its gathers are few: slot t = 8u + k of a unit has e_t = e_8u + brv3(k) 2n/8, so a unit's words share the
+// power w0^(e_8u j), one load for its lanes, and take one of eight multiples of it from shared memory (fold_unit); the slot
+// table is staged; the twiddles of a pass lie side by side; fold_sw spreads the words of every pass over the banks.
+// Powers gathered a word, twiddles a stride apart and divisions by the runtime tile: 61 us for eight shards of gamma 256.
 constexpr int FOLD_TILE = 2048;
 constexpr int FOLD_THREADS = 256;
 
@@ -219,61 +221,92 @@ struct ShardArg {
 };
 __device__ __forceinline__ ShardDev shard_of(const ShardArg& a) { return a.table ? a.table[blockIdx.y] : a.one; }
 
+__device__ __forceinline__ u32 fold_sw(u32 e) { return e ^ (((e >> 4) & 3) * 5); }
+// Twiddles of a fold of length gamma: len entries a pass of two stages.
+__host__ __device__ constexpr u32 fold_twiddles(u32 gamma) {
+  u32 n = 0;
+  for (u32 len = gamma >> 1; len >= 2; len >>= 2) n += len;
+  return n;
+}
+
 template <int LOGN>
-__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, ShardArg shards, u32 SL) {
-  constexpr int N = 1 << LOGN;
+__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, ShardArg shards, u32 lgs) {
+  constexpr int N = 1 << LOGN, BATCH = 4;
   constexpr u32 M2N = 2 * N - 1;
   extern __shared__ __align__(16) u64 sm[];
-  const u32 gamma = c.gamma, half = gamma >> 1;
+  const u32 gamma = c.gamma, half = gamma >> 1, lg = 31 - __clz(gamma), SL = 1u << lgs;
   const u32 tile = SL * gamma, row = gamma + 1;  // SL slots per CTA, tile <= FOLD_TILE words
   Tw* zeta = reinterpret_cast<Tw*>(sm);
-  u64* x = sm + 2 * half;  // [slot][j], a word of padding per slot
-  const u32 t0 = blockIdx.x * SL;
-  const u32 lg = 31 - __clz(gamma);
+  Tw* unit = zeta + fold_twiddles(gamma);
+  uint16_t* slots = reinterpret_cast<uint16_t*>(unit + 8);
+  u64* x = reinterpret_cast<u64*>(slots + N);  // [slot][fold_sw(j)], a word of padding per slot
+  const u32 t0 = blockIdx.x * SL, tid = threadIdx.x;
   H += (size_t)blockIdx.y * gamma * N;
   u64* sums = const_cast<u64*>(shard_of(shards).sums_R);
-  for (u32 k = threadIdx.x; k < half; k += FOLD_THREADS) zeta[k] = c.zeta[k];
-  for (u32 idx = threadIdx.x; idx < tile; idx += FOLD_THREADS) {
-    const u32 j = idx / SL, s = idx % SL;
-    const u32 t = t0 + s;
-    x[s * row + j] = mulw(H[(size_t)j * N + t], c.pow_root[(c.slot_exp[t] * j) & M2N]);
+  for (u32 k = tid; k < N / 8; k += FOLD_THREADS)
+    reinterpret_cast<uint4*>(slots)[k] = reinterpret_cast<const uint4*>(c.exp_slot)[k];
+  if (tid < 8) unit[tid] = c.fold_unit[tid];
+  for (u32 len = half, at = 0; len >= 2; at += len, len >>= 2)
+    for (u32 k = tid; k < len; k += FOLD_THREADS) zeta[at + k] = c.zeta[k * (half / len)];
+  __syncthreads();
+  for (u32 i0 = tid; i0 < tile; i0 += BATCH * FOLD_THREADS) {
+    u64 h[BATCH];
+    Tw w[BATCH];
+#pragma unroll
+    for (int r = 0; r < BATCH; r++) {
+      const u32 idx = i0 + r * FOLD_THREADS, j = idx >> lgs, t = t0 + (idx & (SL - 1));
+      if (idx >= tile) break;
+      h[r] = H[(size_t)j * N + t];
+      w[r] = c.pow_root[(c.slot_exp[t & ~7u] * j) & M2N];
+    }
+#pragma unroll
+    for (int r = 0; r < BATCH; r++) {
+      const u32 idx = i0 + r * FOLD_THREADS, j = idx >> lgs, s = idx & (SL - 1);
+      if (idx >= tile) break;
+      const u32 k = (__brev((t0 + s) & 7) >> 29) * j & 7;
+      x[s * row + fold_sw(j)] = mulw(mulw(h[r], w[r]), unit[k]);
+    }
   }
   __syncthreads();
   // Gentleman-Sande DFT of length gamma per slot, bit-reversed output, two stages a pass on words up to
   // 2+ (sums up to 8+ and 4+ reduced, products 2+), a last stage alone when log gamma is odd.
+  const Tw* z = zeta;
   u32 len = half;
-  for (; len >= 2; len >>= 2) {
-    const u32 q = len >> 1, step = half / len;
-    for (u32 b = threadIdx.x; b < tile / 4; b += FOLD_THREADS) {
-      const u32 s = b / (gamma >> 2), bb = b % (gamma >> 2);
-      const u32 j = bb & (q - 1), i0 = s * row + (bb - j) * 4 + j;
-      u64 a0 = x[i0], a1 = x[i0 + q], a2 = x[i0 + len], a3 = x[i0 + len + q];
+  for (; len >= 2; z += len, len >>= 2) {
+    const u32 q = len >> 1;
+    for (u32 b = tid; b < tile / 4; b += FOLD_THREADS) {
+      const u32 s = b >> (lg - 2), bb = b & ((gamma >> 2) - 1);
+      const u32 j = bb & (q - 1), i0 = (bb - j) * 4 + j;
+      u64* y = x + s * row;
+      const u32 e0 = fold_sw(i0), e1 = fold_sw(i0 + q), e2 = fold_sw(i0 + len), e3 = fold_sw(i0 + len + q);
+      u64 a0 = y[e0], a1 = y[e1], a2 = y[e2], a3 = y[e3];
       const u64 s0 = a0 + a2, s1 = a1 + a3;
-      const u64 d0 = mulw(a0 - a2 + 3 * Q, zeta[j * step]), d1 = mulw(a1 - a3 + 3 * Q, zeta[(j + q) * step]);
-      const Tw w = zeta[2 * j * step];
-      x[i0] = red60(s0 + s1);
-      x[i0 + q] = mulw(s0 - s1 + 5 * Q, w);
-      x[i0 + len] = red60(d0 + d1);
-      x[i0 + len + q] = mulw(d0 - d1 + 3 * Q, w);
+      const u64 d0 = mulw(a0 - a2 + 3 * Q, z[j]), d1 = mulw(a1 - a3 + 3 * Q, z[j + q]);
+      const Tw w = z[2 * j];
+      y[e0] = red60(s0 + s1);
+      y[e1] = mulw(s0 - s1 + 5 * Q, w);
+      y[e2] = red60(d0 + d1);
+      y[e3] = mulw(d0 - d1 + 3 * Q, w);
     }
     __syncthreads();
   }
   if (len == 1) {
-    for (u32 b = threadIdx.x; b < tile / 2; b += FOLD_THREADS) {
-      const u32 s = b / half, i0 = s * row + 2 * (b % half);
-      const u64 u = x[i0], v = x[i0 + 1];
-      x[i0] = u + v;
-      x[i0 + 1] = u - v + 3 * Q;
+    for (u32 b = tid; b < tile / 2; b += FOLD_THREADS) {
+      u64* y = x + (b >> (lg - 1)) * row;
+      const u32 i0 = 2 * (b & (half - 1)), e0 = fold_sw(i0), e1 = fold_sw(i0 + 1);
+      const u64 u = y[e0], v = y[e1];
+      y[e0] = u + v;
+      y[e1] = u - v + 3 * Q;
     }
     __syncthreads();
   }
-  for (u32 idx = threadIdx.x; idx < tile; idx += FOLD_THREADS) {
-    const u32 i = idx / SL, s = idx % SL;
+  for (u32 idx = tid; idx < tile; idx += FOLD_THREADS) {
+    const u32 i = idx >> lgs, s = idx & (SL - 1);
     const u32 e = c.slot_exp[t0 + s];
     const u32 k = (e * c.m_of_i[i]) & (gamma - 1);
     const u32 kr = lg ? (__brev(k) >> (32 - lg)) : 0;
-    const u32 tp = c.exp_slot[((c.cpow[i] * e) & M2N) >> 1];
-    sums[(size_t)i * N + tp] = canon(mulw(x[s * row + kr], c.inv_gamma_R));
+    const u32 tp = slots[((c.cpow[i] * e) & M2N) >> 1];
+    sums[(size_t)i * N + tp] = canon(x[s * row + fold_sw(kr)]);
   }
 }
 
@@ -2454,7 +2487,8 @@ static cudaError_t store_sums(const CrsDev& c, const ShardArg& shards, u32 count
   if (SL > c.n) SL = c.n;
   if (c.n % SL) return cudaErrorInvalidValue;
   const size_t smem_ntt = 3 * (size_t)c.n * 8;
-  const size_t smem_fold = (c.gamma / 2) * sizeof(Tw) + (size_t)SL * (c.gamma + 1) * 8;
+  const u32 lgs = 31 - __builtin_clz(SL);
+  const size_t smem_fold = (fold_twiddles(c.gamma) + 8) * sizeof(Tw) + c.n * 2 + (size_t)SL * (c.gamma + 1) * 8;
   IG_DISPATCH_LOGN(c.logn, {
     auto kn = k_store_ntt<L>;
     auto kf = k_store_fold<L>;
@@ -2462,7 +2496,7 @@ static cudaError_t store_sums(const CrsDev& c, const ShardArg& shards, u32 count
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fold);
     if (e != cudaSuccess) return e;
     kn<<<dim3((c.gamma + STORE_ROWS - 1) / STORE_ROWS, count), (1 << L) / 8, smem_ntt, s>>>(c, shards, H);
-    kf<<<dim3(c.n / SL, count), FOLD_THREADS, smem_fold, s>>>(c, H, shards, SL);
+    kf<<<dim3(c.n / SL, count), FOLD_THREADS, smem_fold, s>>>(c, H, shards, lgs);
   });
   return cudaGetLastError();
 }

@@ -28,7 +28,7 @@ struct CrsDev {
   const u32* m_of_i;         // (g^-i - 1) / (2n/gamma)
   const Tw* pow_root;        // w0^e for e < 2n (w0 = slot 0's root)
   const Tw* zeta;            // zeta^j for j < gamma / 2, zeta = w0^(2n/gamma)
-  Tw inv_gamma_R;            // gamma^-1 * 2^64 mod q
+  Tw fold_unit[8];           // gamma^-1 2^64 w0^(k n/4): a unit's eight factors in the store fold
   const u64* mask;           // the kept mask rows as key rows (key_rows), rows x n words
   // The last exact-gadget digit's factors (D2 = base^-2 (R - D0 - base D1)) in R-form:
   // base^-2, -base^-2 and -base^-1, by which the Galois keys are folded (fold_gadget3).

@@ -978,7 +978,8 @@ int ig_crs_create(ig_ctx* c, uint32_t n, uint64_t q, uint64_t p, uint64_t gadget
   d.ninv = make_tw(ninv);
   d.s_ninv_rinv = make_tw(mulmod(ninv, rinv));
   d.s_rinv = make_tw(rinv);
-  d.inv_gamma_R = make_tw(mulmod(invmod(gamma), R_MOD_Q));
+  for (u32 k = 0; k < 8; k++)
+    d.fold_unit[k] = make_tw(mulmod(mulmod(invmod(gamma), R_MOD_Q), powmod(w0, (u64)k * (n / 4))));
   // Last exact digit: base^-2 (R - D0 - base D1) (inspiring2.rs:1094-1161). These three
   // factors are folded into the key rows (key_scale) and Galois keys rather than form the digit.
   const u64 inv = invmod(1ULL << 40);
