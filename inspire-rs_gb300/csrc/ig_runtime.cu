@@ -408,9 +408,10 @@ int sync_crs_self(ig_ctx* c, CrsObj& o) {
   return IG_OK;
 }
 
-// Shards of a store build that share a launch: enough column transforms to fill the GPU, their H words
-// (a group's, 32 MB) kept in L2 between the two kernels.
-u32 store_group(const CrsObj& o) { return std::max<u32>(1, (u32)((32u << 20) / ((size_t)o.gamma * o.n * 8))); }
+// Shards of a store build that share a launch: their H words take 128 MB, most of which stays in L2 between the two
+// kernels. A launch's last wave leaves a fifth of the GPU idle at 32 MB: 64 shards of gamma 256 1.95 ms with 32 MB,
+// 1.86 with 64, 1.83 with 128.
+u32 store_group(const CrsObj& o) { return std::max<u32>(1, (u32)((128u << 20) / ((size_t)o.gamma * o.n * 8))); }
 
 // Shards a launch takes at most (a grid's y and z run to 65,535).
 enum : u32 { LAUNCH_SHARDS = 16384 };
@@ -471,9 +472,13 @@ int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
     wide |= !sl.compact;
   }
   if (ready) {
-    const u32 group = std::min(ready, store_group(o));
+    u32 group = std::min(ready, store_group(o));
     void* H;
     int rc = scratch(c, "fold_H", (size_t)group * g * n * 8, &H);
+    if (rc && group > 1) {  // short of memory: a shard at a time
+      group = 1;
+      rc = scratch(c, "fold_H", (size_t)g * n * 8, &H);
+    }
     if (rc) return rc;
     // Tag keys: two words per column word below 2^61 - 1, expanded on the device from OS entropy; they
     // never leave it (shard_store.rs:127-135).
