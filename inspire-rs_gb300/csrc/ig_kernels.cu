@@ -745,19 +745,21 @@ __device__ __forceinline__ void fold_gadget3(u64 ld_inv_R, u64 ld_c0_R, u64 ld_c
   dst[2 * dst_stride] = f2;
 }
 
-// The Galois keys ([key][digit][part][n], R-form NTT) folded in place by fold_gadget3 and brought
-// to standard form. The tree holds n^-1 times each node, so a digit's product is scaled by n^-1
-// and the node's own stays.
-__global__ void k_fold_gadget_keys(CrsDev c, u64* keys, u32 count) {
+// The Galois keys ([key][digit][part][n], R-form NTT) folded by fold_gadget3, brought to standard form and laid out
+// for the tree's threads: the pairs of a row's slots that thread u takes (2j, 2j + 1 of unit u) lie N/8 apart, so a
+// warp's loads are contiguous (a thread's eight words in a row of their own took 16 wavefronts a load). The tree holds
+// n^-1 times each node, so a digit's product is scaled by n^-1 and the node's own stays.
+__global__ void k_fold_gadget_keys(CrsDev c, const u64* keys, u64* out, u32 count) {
   const u32 n = c.n;
   const u32 i = blockIdx.x * blockDim.x + threadIdx.x;  // (key, part, coefficient)
   if (i >= count * 2 * n) return;
-  const u32 key = i / (2 * n), r = i - key * 2 * n;
-  u64* x = keys + (size_t)key * 6 * n + r;
-  fold_gadget3(c.ld_inv_R, c.ld_c0_R, c.ld_c1_R, x, x, (int)(2 * n), (int)(2 * n));
-  x[0] = canon(mulw(x[0], c.s_ninv_rinv));
-  x[2 * n] = canon(mulw(x[2 * n], c.s_ninv_rinv));
-  x[4 * n] = canon(mulw(x[4 * n], c.s_rinv));
+  const u32 key = i / (2 * n), r = i - key * 2 * n, part = r / n, t = r - part * n;
+  u64 x[3];
+  fold_gadget3(c.ld_inv_R, c.ld_c0_R, c.ld_c1_R, keys + (size_t)key * 6 * n + r, x, (int)(2 * n), 1);
+  u64* o = out + (size_t)key * 6 * n + (size_t)part * n + 2 * (((t & 7) >> 1) * (n / 8) + (t >> 3)) + (t & 1);
+  o[0] = canon(mulw(x[0], c.s_ninv_rinv));
+  o[2 * n] = canon(mulw(x[1], c.s_ninv_rinv));
+  o[4 * n] = canon(mulw(x[2], c.s_rinv));
 }
 
 // The key rows of a mask or a seat as the recursion reads them, made once when the set or the seat is: per slot the
@@ -1965,7 +1967,9 @@ __global__ void k_nopack_sum(u32 n, u32 gamma, u64* out) {
 //
 // The walk is the recursion's depth-first order: leaf k of the walk is start = bitrev(k),
 // and a binary-counter carry combines each finished node with its waiting sibling; the
-// waiting nodes sit in a stack of node slots in global memory. The leaves [j n/S, (j+1) n/S) of the walk make up
+// waiting nodes sit in a stack of node slots in global memory. At gamma < n the odd children of the lowest
+// log(n / gamma) levels are all zero: a leaf walks those levels alone, from its registers (three of four nodes at
+// gamma 256; with the keys laid out for their loads 64 queries 4.80 -> 3.63 ms). The leaves [j n/S, (j+1) n/S) of the walk make up
 // the subtree of start bitrev(j) at level log n - log S, so k_tree_part walks S subtrees of a query on as many
 // CTAs and k_tree_top the S - 1 nodes above them: a query alone on one CTA took 11 ms whatever the batch, and
 // 64 left most SMs idle. 103 KB of shared memory a CTA: two on an SM.
@@ -2005,28 +2009,32 @@ __device__ __forceinline__ void node_store(u64* node, const u64 (&a)[8], const u
     p[(k + 4) * NT] = make_ulonglong2(b[2 * k], b[2 * k + 1]);
   }
 }
-// The current node (a, b at the thread's slots) becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell; it is
-// O, zero when odd_zero. Ends with a barrier.
-template <int LOGN>
-__device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S, const u64* E, int ell, bool odd_zero,
+// The current node (a, b at the thread's slots) becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell: it is
+// O and E waits in memory, or with ALONE it is E itself and its odd sibling zero. Ends with a barrier.
+template <int LOGN, bool ALONE>
+__device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S, const u64* E, int ell,
                                              const u32 (&et)[8], u64 (&ca)[8], u64 (&cb)[8]) {
   constexpr int N = 1 << LOGN, NT = N / 8;
   constexpr u32 M2N = 2 * N - 1;
   const u32 sy = (u32)(N >> ell), t = (1u << ell) + 1;
-  u64 ea[8], eb[8];
-  node_load<LOGN>(E, ea, eb);
+  if constexpr (ALONE) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    u64 ya = 0, yb = 0;
-    if (!odd_zero) {
-      const Tw y = c.pow_root[(et[k] * sy) & M2N];
-      ya = canon(mulw(ca[k], y));
-      yb = canon(mulw(cb[k], y));
+    for (int k = 0; k < 8; k++) {
+      S.S1a[k * NT + threadIdx.x] = ca[k];
+      S.S1b[k * NT + threadIdx.x] = cb[k];
     }
-    ca[k] = addq(ea[k], ya);
-    cb[k] = addq(eb[k], yb);
-    S.S1a[k * NT + threadIdx.x] = subq(ea[k], ya);
-    S.S1b[k * NT + threadIdx.x] = subq(eb[k], yb);
+  } else {
+    u64 ea[8], eb[8];
+    node_load<LOGN>(E, ea, eb);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const Tw y = c.pow_root[(et[k] * sy) & M2N];
+      const u64 ya = canon(mulw(ca[k], y)), yb = canon(mulw(cb[k], y));
+      ca[k] = addq(ea[k], ya);
+      cb[k] = addq(eb[k], yb);
+      S.S1a[k * NT + threadIdx.x] = subq(ea[k], ya);
+      S.S1b[k * NT + threadIdx.x] = subq(eb[k], yb);
+    }
   }
   __syncthreads();
   u64 d[2][8];
@@ -2036,20 +2044,26 @@ __device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S,
     for (int k = 0; k < 8; k++) aa[k] = S.S1a[S.s_tab[((t * et[k]) & M2N) >> 1]];
     link_transforms8<LOGN, true>(aa, d, S.D, S.tw);
   }
-  const u64* key = c.galois + (size_t)(LOGN - ell) * 6 * N + 8 * threadIdx.x;
+  const ulonglong2* key = reinterpret_cast<const ulonglong2*>(c.galois + (size_t)(LOGN - ell) * 6 * N) + threadIdx.x;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const u32 at = S.s_tab[((t * et[k]) & M2N) >> 1];
-    const u64 aa = S.S1a[at];
-    Acc na{0, 0, 0, 0}, nb{0, 0, 0, 0};
-    mac(na, d[0][k], key[k]);
-    mac(nb, d[0][k], key[N + k]);
-    mac(na, d[1][k], key[2 * N + k]);
-    mac(nb, d[1][k], key[3 * N + k]);
-    mac(na, aa, key[4 * N + k]);
-    mac(nb, aa, key[5 * N + k]);
-    ca[k] = addq(ca[k], csub(acc_fold(na)));
-    cb[k] = addq(cb[k], addq(S.S1b[at], csub(acc_fold(nb))));
+  for (int k = 0; k < 8; k += 2) {
+    ulonglong2 w[6];
+#pragma unroll
+    for (int r = 0; r < 6; r++) w[r] = key[(r * 4 + k / 2) * NT];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const u32 at = S.s_tab[((t * et[k + j]) & M2N) >> 1];
+      const u64 aa = S.S1a[at];
+      Acc na{0, 0, 0, 0}, nb{0, 0, 0, 0};
+      mac(na, d[0][k + j], j ? w[0].y : w[0].x);
+      mac(nb, d[0][k + j], j ? w[1].y : w[1].x);
+      mac(na, d[1][k + j], j ? w[2].y : w[2].x);
+      mac(nb, d[1][k + j], j ? w[3].y : w[3].x);
+      mac(na, aa, j ? w[4].y : w[4].x);
+      mac(nb, aa, j ? w[5].y : w[5].x);
+      ca[k + j] = addq(ca[k + j], csub(acc_fold(na)));
+      cb[k + j] = addq(cb[k + j], addq(S.S1b[at], csub(acc_fold(nb))));
+    }
   }
   __syncthreads();  // S1 and D are rewritten next
 }
@@ -2075,12 +2089,11 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
   expand_a<N, NT>(qd, S.D + N, status, qi, 0);  // ends with a barrier
   transform_slots8<LOGN>(S.D + N, S.D, S.tw, c.ninv, aR);
   u64 ca[8], cb[8];
-  u32 zero_slots = 0;  // bit L: the waiting node at level L is zero
+  const int zeros = LOGN - (31 - __clz(gamma));  // levels whose odd children are all zero
 #pragma unroll 1
-  for (u32 k = 0; k < (u32)N >> log_parts; k++) {
-    const u32 start = __brev((part << levels) | k) >> (32 - LOGN);
-    bool cur_zero = start >= gamma;
-    if (!cur_zero) {
+  for (u32 m = 0; m < (u32)N >> log_parts >> zeros; m++) {
+    const u32 start = __brev((part << levels) | (m << zeros)) >> (32 - LOGN);
+    {
       // Leaf `start`: the column through the transform times NTT(a).
       __syncthreads();  // every thread is past its last read of D
 #pragma unroll
@@ -2108,18 +2121,12 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
     }
     if (gamma == 1) break;  // a single leaf is the root
     int L = 0;
-    while ((k >> L) & 1) {
-      if ((zero_slots >> L) & 1) {
-        cur_zero = true;  // an even child at or past gamma makes its sibling zero too
-      } else {
-        tree_combine<LOGN>(c, S, stk + (size_t)L * 2 * N, L + 1, cur_zero, et, ca, cb);
-        cur_zero = false;
-      }
-      L++;
-    }
-    if (L == levels) break;  // the subtree's root (start below gamma: never zero)
-    zero_slots = (zero_slots & ~(1u << L)) | (cur_zero ? 1u << L : 0);
-    if (!cur_zero) node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
+#pragma unroll 1
+    for (; L < zeros; L++) tree_combine<LOGN, true>(c, S, nullptr, L + 1, et, ca, cb);
+#pragma unroll 1
+    for (; (m >> (L - zeros)) & 1; L++) tree_combine<LOGN, false>(c, S, stk + (size_t)L * 2 * N, L + 1, et, ca, cb);
+    if (L == levels) break;  // the subtree's root
+    node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
   }
   node_store<LOGN>(roots + (size_t)blockIdx.x * 2 * N, ca, cb);
 }
@@ -2148,7 +2155,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
   for (u32 j = 0; j < 1u << log_parts; j++) {
     node_load<LOGN>(roots + ((size_t)(qi << log_parts) + j) * 2 * N, ca, cb);
     int L = 0;
-    for (; (j >> L) & 1; L++) tree_combine<LOGN>(c, S, stk + (size_t)L * 2 * N, levels + L + 1, false, et, ca, cb);
+    for (; (j >> L) & 1; L++) tree_combine<LOGN, false>(c, S, stk + (size_t)L * 2 * N, levels + L + 1, et, ca, cb);
     if (L < (int)log_parts) node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
   }
   inv_first8<LOGN>(ca, S.D, S.tw);
@@ -2449,10 +2456,10 @@ __global__ void __launch_bounds__(256) k_butterfly_peak(u64* out, int iters, Tw 
     default: return cudaErrorInvalidValue;                 \
   }
 
-cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t s) {
+cudaError_t fold_gadget_keys(const CrsDev& c, const u64* keys, u64* out, u32 count, cudaStream_t s) {
   const u32 total = count * 2 * c.n;
   if (total == 0) return cudaSuccess;
-  k_fold_gadget_keys<<<(total + 255) / 256, 256, 0, s>>>(c, keys, count);
+  k_fold_gadget_keys<<<(total + 255) / 256, 256, 0, s>>>(c, keys, out, count);
   return cudaGetLastError();
 }
 

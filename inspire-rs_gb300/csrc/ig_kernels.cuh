@@ -95,10 +95,10 @@ struct ShardDev {
 namespace igk {
 using namespace ig;
 
-// The Galois keys ([key][3 digits][2 parts][n], R-form NTT) folded in place for consumers
-// that take the node in place of the derived third digit, and brought to the standard form
-// and the scale of the tree's nodes (n^-1 times their values).
-cudaError_t fold_gadget_keys(const CrsDev& c, u64* keys, u32 count, cudaStream_t s);
+// The Galois keys ([key][3 digits][2 parts][n], R-form NTT) folded for consumers that take the node in place of
+// the derived third digit, and brought to the standard form and the scale of the tree's nodes (n^-1 times their
+// values), a row's slots in the order of the tree's loads (k_fold_gadget_keys).
+cudaError_t fold_gadget_keys(const CrsDev& c, const u64* keys, u64* out, u32 count, cudaStream_t s);
 // The factors that make a mask's or a seat's transforms key rows: of the digits' rows, of the third row where it is folded
 // into them, and of the third row itself.
 struct KeyScale {
@@ -106,7 +106,7 @@ struct KeyScale {
 };
 // Key rows (k_key_rows) of a mask or a seat: 2 or 3 polynomials in, as many times n words out.
 cudaError_t key_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, const KeyScale& f, cudaStream_t s);
-// Forward NTT of `rows` polynomials: out[r] = scale * NTT(in[r] mod q), canonical (scale = 1 for
+// Forward NTT of `rows` polynomials (in place where out == in): out[r] = scale * NTT(in[r] mod q), canonical (scale = 1 for
 // standard form, 2^64 mod q for R-form).
 cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, cudaStream_t s);
 
