@@ -211,7 +211,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_ntt_rows(CrsDev c, const u6
 // power w0^(e_8u j), one load for its lanes, and take one of eight multiples of it from shared memory (fold_unit); the slot
 // table is staged; the twiddles of a pass lie side by side; fold_sw spreads the words of every pass over the banks.
 // Powers gathered a word, twiddles a stride apart and divisions by the runtime tile: 61 us for eight shards of gamma 256.
-constexpr int FOLD_TILE = 2048;
+constexpr int FOLD_TILE_LOG = 11, FOLD_TILE = 1 << FOLD_TILE_LOG;
 constexpr int FOLD_THREADS = 256;
 
 // The shard a store kernel works on: entry blockIdx.y of a device table, or the one given.
@@ -229,38 +229,40 @@ __host__ __device__ constexpr u32 fold_twiddles(u32 gamma) {
   return n;
 }
 
-template <int LOGN>
-__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, ShardArg shards, u32 lgs) {
-  constexpr int N = 1 << LOGN, BATCH = 4;
-  constexpr u32 M2N = 2 * N - 1;
+// LG = log gamma; lgs = log SL, which the tile fixes from gamma 8 up.
+template <int LG>
+__global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64* H, ShardArg shards, u32 lgs_) {
+  constexpr u32 gamma = 1u << LG, half = gamma >> 1, row = gamma + 1, BATCH = 4;
+  const u32 lgs = LG >= 3 ? FOLD_TILE_LOG - LG : lgs_, SL = 1u << lgs, n = c.n, m2n = 2 * n - 1;
+  const u32 tile = SL * gamma;  // SL slots per CTA, tile <= FOLD_TILE words
   extern __shared__ __align__(16) u64 sm[];
-  const u32 gamma = c.gamma, half = gamma >> 1, lg = 31 - __clz(gamma), SL = 1u << lgs;
-  const u32 tile = SL * gamma, row = gamma + 1;  // SL slots per CTA, tile <= FOLD_TILE words
   Tw* zeta = reinterpret_cast<Tw*>(sm);
   Tw* unit = zeta + fold_twiddles(gamma);
   uint16_t* slots = reinterpret_cast<uint16_t*>(unit + 8);
-  u64* x = reinterpret_cast<u64*>(slots + N);  // [slot][fold_sw(j)], a word of padding per slot
+  u64* x = reinterpret_cast<u64*>(slots + n);  // [slot][fold_sw(j)], a word of padding per slot
   const u32 t0 = blockIdx.x * SL, tid = threadIdx.x;
-  H += (size_t)blockIdx.y * gamma * N;
+  H += ((size_t)blockIdx.y * gamma << c.logn) + t0;
   u64* sums = const_cast<u64*>(shard_of(shards).sums_R);
-  for (u32 k = tid; k < N / 8; k += FOLD_THREADS)
+  for (u32 k = tid; k < n / 8; k += FOLD_THREADS)
     reinterpret_cast<uint4*>(slots)[k] = reinterpret_cast<const uint4*>(c.exp_slot)[k];
   if (tid < 8) unit[tid] = c.fold_unit[tid];
+#pragma unroll
   for (u32 len = half, at = 0; len >= 2; at += len, len >>= 2)
     for (u32 k = tid; k < len; k += FOLD_THREADS) zeta[at + k] = c.zeta[k * (half / len)];
   __syncthreads();
+#pragma unroll
   for (u32 i0 = tid; i0 < tile; i0 += BATCH * FOLD_THREADS) {
     u64 h[BATCH];
     Tw w[BATCH];
 #pragma unroll
-    for (int r = 0; r < BATCH; r++) {
-      const u32 idx = i0 + r * FOLD_THREADS, j = idx >> lgs, t = t0 + (idx & (SL - 1));
+    for (u32 r = 0; r < BATCH; r++) {
+      const u32 idx = i0 + r * FOLD_THREADS, j = idx >> lgs, s = idx & (SL - 1);
       if (idx >= tile) break;
-      h[r] = H[(size_t)j * N + t];
-      w[r] = c.pow_root[(c.slot_exp[t & ~7u] * j) & M2N];
+      h[r] = H[(j << c.logn) + s];
+      w[r] = c.pow_root[(c.slot_exp[(t0 + s) & ~7u] * j) & m2n];
     }
 #pragma unroll
-    for (int r = 0; r < BATCH; r++) {
+    for (u32 r = 0; r < BATCH; r++) {
       const u32 idx = i0 + r * FOLD_THREADS, j = idx >> lgs, s = idx & (SL - 1);
       if (idx >= tile) break;
       const u32 k = (__brev((t0 + s) & 7) >> 29) * j & 7;
@@ -271,11 +273,12 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64
   // Gentleman-Sande DFT of length gamma per slot, bit-reversed output, two stages a pass on words up to
   // 2+ (sums up to 8+ and 4+ reduced, products 2+), a last stage alone when log gamma is odd.
   const Tw* z = zeta;
-  u32 len = half;
-  for (; len >= 2; z += len, len >>= 2) {
+#pragma unroll
+  for (u32 len = half; len >= 2; z += len, len >>= 2) {
     const u32 q = len >> 1;
+#pragma unroll 2
     for (u32 b = tid; b < tile / 4; b += FOLD_THREADS) {
-      const u32 s = b >> (lg - 2), bb = b & ((gamma >> 2) - 1);
+      const u32 s = b / (gamma / 4 ? gamma / 4 : 1), bb = b & (gamma / 4 - 1);
       const u32 j = bb & (q - 1), i0 = (bb - j) * 4 + j;
       u64* y = x + s * row;
       const u32 e0 = fold_sw(i0), e1 = fold_sw(i0 + q), e2 = fold_sw(i0 + len), e3 = fold_sw(i0 + len + q);
@@ -290,9 +293,9 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64
     }
     __syncthreads();
   }
-  if (len == 1) {
+  if constexpr (LG & 1) {
     for (u32 b = tid; b < tile / 2; b += FOLD_THREADS) {
-      u64* y = x + (b >> (lg - 1)) * row;
+      u64* y = x + b / half * row;
       const u32 i0 = 2 * (b & (half - 1)), e0 = fold_sw(i0), e1 = fold_sw(i0 + 1);
       const u64 u = y[e0], v = y[e1];
       y[e0] = u + v;
@@ -300,13 +303,14 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64
     }
     __syncthreads();
   }
+#pragma unroll 4
   for (u32 idx = tid; idx < tile; idx += FOLD_THREADS) {
     const u32 i = idx >> lgs, s = idx & (SL - 1);
     const u32 e = c.slot_exp[t0 + s];
     const u32 k = (e * c.m_of_i[i]) & (gamma - 1);
-    const u32 kr = lg ? (__brev(k) >> (32 - lg)) : 0;
-    const u32 tp = slots[((c.cpow[i] * e) & M2N) >> 1];
-    sums[(size_t)i * N + tp] = canon(x[s * row + fold_sw(kr)]);
+    const u32 kr = LG ? __brev(k) >> (32 - (LG ? LG : 1)) : 0;
+    const u32 tp = slots[((c.cpow[i] * e) & m2n) >> 1];
+    sums[((size_t)i << c.logn) + tp] = canon(x[s * row + fold_sw(kr)]);
   }
 }
 
@@ -767,38 +771,40 @@ __global__ void k_fold_gadget_keys(CrsDev c, const u64* keys, u64* out, u32 coun
 // The recursion holds c_i = n^-1 R_i, so the inverse transform of a link needs no n^-1:
 //   c_i = (n^-1 a)[tau] S + sum_k (n^-1 W_k)[tau] D_k,   sum_b += sum_k Y_k[tau] D_k,
 // and with the exact gadget (rows folded as fold_gadget3 does), where R_{i+1} = n c_{i+1} takes the third digit's
-// place, W_2 stays and Y_2 is scaled by n. One CTA: the rows' transforms side by side, then the fold. Folded by every
+// place, W_2 stays and Y_2 is scaled by n. A CTA a row, in one cluster: the fold reads the third row's transform from its
+// CTA (13 us with the three transforms in one CTA). Folded by every
 // respond CTA into its shared memory instead, the rows took 17,800 of the 123,000 cycles of a lone query of gamma 16.
 template <int LOGN, int ROWS>
 __global__ void __launch_bounds__((1 << LOGN) / 4) k_key_rows(CrsDev c, const u64* in, u64* out, KeyScale f) {
+  namespace cg = cooperative_groups;
   constexpr int N = 1 << LOGN, NT = N / 4;
   extern __shared__ __align__(16) u64 sm[];
   Tw* tw = reinterpret_cast<Tw*>(sm);
   u64* x = sm + 2 * N;
+  const int r = blockIdx.x;  // the CTA's row, and its rank in the cluster
   for (int k = threadIdx.x; k < N; k += NT) {
     tw[k] = c.tw[k];
-#pragma unroll
-    for (int r = 0; r < ROWS; r++) x[r * N + k] = reduce128(in[r * N + k]);
+    x[k] = reduce128(in[r * N + k]);
   }
   __syncthreads();
   {
-    u64* bufs_[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; r++) bufs_[r] = x + r * N;
-    u64* const(&bufs)[ROWS] = bufs_;
-    ntt_fwd_r4<LOGN, NT, ROWS>(bufs, tw);
+    u64* const bufs[1] = {x};
+    ntt_fwd_r4<LOGN, NT, 1>(bufs, tw);
   }
-  ulonglong2* pairs = reinterpret_cast<ulonglong2*>(out);
+  cg::cluster_group cluster = cg::this_cluster();
+  if constexpr (ROWS == 3) cluster.sync();
+  const u64* third = ROWS == 3 ? cluster.map_shared_rank(x, 2) : x;
+  const Tw fold = r ? f.fold1 : f.fold0;
   for (int k = threadIdx.x; k < N; k += NT) {
-    u64 y0 = mulw(x[k], f.digit), y1 = mulw(x[N + k], f.digit);
-    if constexpr (ROWS == 3) {
-      const u64 y2 = x[2 * N + k];
-      y0 += mulw(y2, f.fold0);
-      y1 += mulw(y2, f.fold1);
-      out[2 * N + k] = canon(mulw(y2, f.derived));
+    if (r == 2) {
+      out[2 * N + k] = canon(mulw(x[k], f.derived));
+    } else {
+      u64 y = mulw(x[k], f.digit);
+      if constexpr (ROWS == 3) y += mulw(third[k], fold);
+      out[2 * k + r] = canon(y);
     }
-    pairs[k] = make_ulonglong2(canon(y0), canon(y1));
   }
+  if constexpr (ROWS == 3) cluster.sync();  // the third row is read before its CTA ends
 }
 
 // A query's key rows in shared memory: W01 and Y01 the pairs of the mask and the seat, WY2 the third rows of both. The
@@ -1203,7 +1209,7 @@ __device__ __forceinline__ void transform_slots8(const u64* src, u64* D, const T
 // 32-bit product.
 constexpr int STORE_ROWS = 4;
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 8) k_store_ntt(CrsDev c, ShardArg shards, u64* H) {
+__global__ void __launch_bounds__((1 << LOGN) / 8, 4) k_store_ntt(CrsDev c, ShardArg shards, u64* H) {
   constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
   extern __shared__ __align__(16) u64 sm[];
   Tw* tw = reinterpret_cast<Tw*>(sm);
@@ -1212,16 +1218,24 @@ __global__ void __launch_bounds__((1 << LOGN) / 8) k_store_ntt(CrsDev c, ShardAr
   for (int k = threadIdx.x; k < N; k += NT) tw[tw8<LOGN>(k)] = c.tw[k];
   __syncthreads();
   H += (size_t)blockIdx.y * c.gamma * N;
+  const u32 end = min(c.gamma, (blockIdx.x + 1) * STORE_ROWS);
+  u32 next[2][4] = {};  // the next compact column's words
+  auto fetch = [&](u32 j) {
+    if (!sh.cols16 || j >= end) return;
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) next[r][k] = sh.cols16[(size_t)j * N + threadIdx.x + r * NT + k * P];
+  };
+  fetch(blockIdx.x * STORE_ROWS);
 #pragma unroll 1
-  for (u32 j = blockIdx.x * STORE_ROWS; j < min(c.gamma, (blockIdx.x + 1) * STORE_ROWS); j++) {
+  for (u32 j = blockIdx.x * STORE_ROWS; j < end; j++) {
 #pragma unroll
     for (int r = 0; r < 2; r++) {
       const int b = threadIdx.x + r * NT;
       u64 x[4];
       if (sh.cols16) {
-        u32 w[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) w[k] = sh.cols16[(size_t)j * N + b + k * P];
+        const u32(&w)[4] = next[r];
         const u64 t2 = mulw_digit(w[2], tw[1]), t3 = mulw_digit(w[3], tw[1]);
         x[0] = w[0] + t2;
         x[1] = w[1] + t3;
@@ -1237,6 +1251,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8) k_store_ntt(CrsDev c, ShardAr
 #pragma unroll
       for (int k = 0; k < 4; k++) D[sw8(b + k * P)] = x[k];
     }
+    fetch(j + 1);  // while this one is transformed
     __syncthreads();
     fwd_middle8<LOGN, 1, 7>(D, tw);
     u64 x[1][8];
@@ -2465,12 +2480,23 @@ cudaError_t fold_gadget_keys(const CrsDev& c, const u64* keys, u64* out, u32 cou
 
 cudaError_t key_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, const KeyScale& f, cudaStream_t s) {
   if (rows != 2 && rows != 3) return cudaErrorInvalidValue;
-  const size_t smem = (2 + rows) * (size_t)c.n * 8;
+  const size_t smem = 3 * (size_t)c.n * 8;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = rows;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(rows);
+  cfg.blockDim = dim3(c.n / 4);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   IG_DISPATCH_LOGN(c.logn, {
     auto k = rows == 3 ? k_key_rows<L, 3> : k_key_rows<L, 2>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k, c, in, out, f);
     if (e != cudaSuccess) return e;
-    k<<<1, (1 << L) / 4, smem, s>>>(c, in, out, f);
   });
   return cudaGetLastError();
 }
@@ -2498,13 +2524,19 @@ static cudaError_t store_sums(const CrsDev& c, const ShardArg& shards, u32 count
   const size_t smem_fold = (fold_twiddles(c.gamma) + 8) * sizeof(Tw) + c.n * 2 + (size_t)SL * (c.gamma + 1) * 8;
   IG_DISPATCH_LOGN(c.logn, {
     auto kn = k_store_ntt<L>;
-    auto kf = k_store_fold<L>;
     cudaError_t e = cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ntt);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fold);
     if (e != cudaSuccess) return e;
     kn<<<dim3((c.gamma + STORE_ROWS - 1) / STORE_ROWS, count), (1 << L) / 8, smem_ntt, s>>>(c, shards, H);
-    kf<<<dim3(c.n / SL, count), FOLD_THREADS, smem_fold, s>>>(c, H, shards, lgs);
   });
+  using Fold = void (*)(CrsDev, const u64*, ShardArg, u32);
+  static constexpr Fold folds[] = {k_store_fold<0>, k_store_fold<1>, k_store_fold<2>, k_store_fold<3>,
+                                   k_store_fold<4>, k_store_fold<5>, k_store_fold<6>, k_store_fold<7>,
+                                   k_store_fold<8>, k_store_fold<9>, k_store_fold<10>};
+  const u32 lg = 31 - __builtin_clz(c.gamma);
+  if (lg >= sizeof folds / sizeof folds[0]) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(folds[lg], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fold);
+  if (e != cudaSuccess) return e;
+  folds[lg]<<<dim3(c.n / SL, count), FOLD_THREADS, smem_fold, s>>>(c, H, shards, lgs);
   return cudaGetLastError();
 }
 cudaError_t store_sums(const CrsDev& c, const ShardDev* table, u32 count, u64* H, cudaStream_t s) {
