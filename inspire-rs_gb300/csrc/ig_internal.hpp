@@ -69,16 +69,18 @@ struct HostCall {
       if (s) cudaStreamSynchronize(s);
   }
 };
-// A host-buffer call's arrays: one device block (scratch of the lane) and its image in the lane's pinned buffer, in this
-// order, so the small arrays cross in one copy each way (a lone query of gamma 16 131 -> 120 us, where seven copies and a
-// memset went around its two launches). Arrays of COPY_DIRECT_BYTES and more are copied straight between the caller's memory and the device where the
-// GPU reads pageable memory through the host's page tables (an MB in 16 us, against 50 in and 71 out through the pinned
-// image; below 256 KB the image's copy is the shorter). A caller's result memory that no one has touched yet costs the
-// direct copy 180 us an MB in faults that the CPU takes in 10: wait() touches it while the device works. 64 queries
-// 1.455 -> 1.285 ms, 128 mixed ones 5.00 -> 4.46 ms, 256 special_modulus ones 4.43 -> 4.07 ms.
+// A host-buffer call's arrays: one device block (scratch of the lane) and its image in the lane's pinned buffer, so the
+// small arrays cross in one copy each way (a lone query of gamma 16 131 -> 120 us, where seven copies and a memset
+// went around its two launches). Arrays of COPY_DIRECT_BYTES and more are copied straight between the caller's memory
+// and the device where the GPU reads pageable memory through the host's page tables (an MB in 16 us, against 50 in and
+// 71 out through the pinned image; below 256 KB the image's copy is the shorter). A caller's result memory that no one
+// has touched yet costs the direct copy 180 us an MB in faults that the CPU takes in 10: wait() touches it while the
+// device works. 64 queries 1.455 -> 1.285 ms, 128 mixed ones 5.00 -> 4.46 ms, 256 special_modulus ones 4.43 -> 4.07 ms.
 constexpr size_t COPY_DIRECT_BYTES = 256 << 10;
 struct HostIO {
-  size_t table, queries, work, seeds, bs, status, a, b, end;  // offsets
+  // Offsets. The arrays below `down` have a place in the image: those up to `up` go to the device, those from the
+  // status words on come back.
+  size_t table, queries, work, seeds, bs, status, a, b, up, down;
   size_t table_bytes, query_bytes, work_bytes, seed_bytes, bs_bytes, status_bytes, a_bytes, b_bytes;
   uint8_t *dev, *pin;
 };

@@ -2738,6 +2738,29 @@ size_t respond_smem_bytes(const CrsDev& c, int ctas) {
   return words * 8 + n * 2;
 }
 
+u32 max_quads() {
+  CrsDev c{};
+  c.n = 2048;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 4;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(4);
+  cfg.blockDim = dim3(c.n / 8);
+  cfg.dynamicSmemBytes = respond_smem_bytes(c, 4);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  auto k = k_respond_cluster<11, 4>;
+  int n = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (u32)n;
+}
+
 cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq,
                     const u64* b_fold, u64* a_out, u64* b_out, u32* status,
                     int force_serial_expand, int ctas, cudaStream_t s) {

@@ -155,6 +155,8 @@ cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* sh
                     int ctas, cudaStream_t s);
 
 size_t respond_smem_bytes(const CrsDev& c, int ctas);
+// Four-CTA clusters of the largest ring that the current device runs at once.
+u32 max_quads();
 
 // NoPacking respond of `nq` queries: prep transforms them into AB_R (nq x 2n words, r_mod_q = 2^64 mod q); cols gives
 // out[q], gamma + 1 ciphertexts of (a, b), n words each in coefficient form, the column sum first (respond.rs:614-643).

@@ -15,6 +15,7 @@
 #include <functional>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <random>
 #include <string>
 #include <unordered_map>
@@ -245,6 +246,9 @@ struct ig_ctx {
     cudaEvent_t copied = nullptr;
     std::vector<cudaEvent_t> parts;  // ends of a batch's parts, each copied out while the next runs
   };
+  // Clusters of four that run at once: a cluster takes its SMs within one GPC, 36 of them where 38 would fill the SMs
+  // (37 queries of gamma 64 375 us as fours, 299 as pairs).
+  u32 quads = 0;
   bool direct_copies = false;  // the GPU reads pageable memory through the host's page tables
   HostLane hlane[IG_MAX_LANES];
   std::atomic<u32> hlane_next{0};
@@ -588,7 +592,7 @@ int launch_ctas(ig_ctx* c, u32 n, u32 gamma, u32 count, u32 in_flight) {
   const std::array<double, 3>* row = tuned_row(c, n, gamma, queries);
   if (!row) {  // the fixed rule: as many CTAs per query as the threshold leaves room for
     const u64 t = c->pair_threshold;
-    return 2 * (u64)queries <= t ? 4 : (u64)queries <= t ? 2 : 1;
+    return 2 * (u64)queries <= t && queries <= c->quads ? 4 : (u64)queries <= t ? 2 : 1;
   }
   const int shapes[3] = {1, 2, 4};
   int best = 1;
@@ -667,20 +671,27 @@ int host_io_open(ig_ctx* c, HostCall& hc, HostIO& io, size_t table, size_t queri
     len = bytes;
     at = (at + bytes + 255) & ~(size_t)255;
   };
+  const bool ds = host_io_direct(c, seeds), db = host_io_direct(c, bs), da = host_io_direct(c, a),
+             dr = host_io_direct(c, b);
   put(table, io.table, io.table_bytes);
   put(queries, io.queries, io.query_bytes);
   put(work, io.work, io.work_bytes);
-  put(seeds, io.seeds, io.seed_bytes);
-  put(bs, io.bs, io.bs_bytes);
+  if (!ds) put(seeds, io.seeds, io.seed_bytes);
+  if (!db) put(bs, io.bs, io.bs_bytes);
   put(count * 4, io.status, io.status_bytes);
-  put(a, io.a, io.a_bytes);
-  put(b, io.b, io.b_bytes);
-  io.end = at;
+  io.up = at;
+  if (!da) put(a, io.a, io.a_bytes);
+  if (!dr) put(b, io.b, io.b_bytes);
+  io.down = at;
+  if (ds) put(seeds, io.seeds, io.seed_bytes);
+  if (db) put(bs, io.bs, io.bs_bytes);
+  if (da) put(a, io.a, io.a_bytes);
+  if (dr) put(b, io.b, io.b_bytes);
   char name[32];
   snprintf(name, sizeof name, "call%u", hc.k);
   void *d, *h;
   int rc = ::scratch(c, name, at, &d);
-  if (!rc) rc = host_call_pinned(c, hc, at, &h);
+  if (!rc) rc = host_call_pinned(c, hc, io.down, &h);
   if (rc) return rc;
   io.dev = (uint8_t*)d;
   io.pin = (uint8_t*)h;
@@ -688,44 +699,34 @@ int host_io_open(ig_ctx* c, HostCall& hc, HostIO& io, size_t table, size_t queri
 }
 int host_io_send(ig_ctx* c, HostCall& hc, HostIO& io, const void* table, const void* queries, const void* work,
                  const void* seeds, const void* bs) {
-  if (io.table_bytes) memcpy(io.pin + io.table, table, io.table_bytes);
-  memcpy(io.pin + io.queries, queries, io.query_bytes);
-  if (io.work_bytes) memcpy(io.pin + io.work, work, io.work_bytes);
-  memset(io.pin + io.status, 0, io.status_bytes);
   // The large inputs go first, on the copy stream: nothing else uses their part of the block, so they need not wait for
   // the context's work.
-  const bool ds = host_io_direct(c, io.seed_bytes), db = host_io_direct(c, io.bs_bytes);
-  cudaStream_t s = host_call_stream(c, hc), copy = nullptr;
-  int rc;
-  if (ds || db) {
-    hc.queued[1] = copy = host_call_copy_stream(c, hc);
-    if (ds) IG_CUDA(c, cudaMemcpyAsync(io.dev + io.seeds, seeds, io.seed_bytes, cudaMemcpyHostToDevice, copy));
-    if (db) IG_CUDA(c, cudaMemcpyAsync(io.dev + io.bs, bs, io.bs_bytes, cudaMemcpyHostToDevice, copy));
-    IG_CUDA(c, cudaEventRecord(c->hlane[hc.k].copied, copy));
-  }
-  if (!ds) memcpy(io.pin + io.seeds, seeds, io.seed_bytes);
-  if (!db) memcpy(io.pin + io.bs, bs, io.bs_bytes);
-  if ((rc = host_call_enter(c, hc))) return rc;
+  cudaStream_t s = host_call_stream(c, hc), copy = host_call_copy_stream(c, hc);
+  auto take = [&](size_t off, size_t bytes, const void* src) {
+    if (off >= io.down) {
+      hc.queued[1] = copy;
+      return cudaMemcpyAsync(io.dev + off, src, bytes, cudaMemcpyHostToDevice, copy);
+    }
+    if (bytes) memcpy(io.pin + off, src, bytes);
+    return cudaSuccess;
+  };
+  IG_CUDA(c, take(io.seeds, io.seed_bytes, seeds));
+  IG_CUDA(c, take(io.bs, io.bs_bytes, bs));
+  if (hc.queued[1]) IG_CUDA(c, cudaEventRecord(c->hlane[hc.k].copied, copy));
+  IG_CUDA(c, take(io.table, io.table_bytes, table));
+  IG_CUDA(c, take(io.queries, io.query_bytes, queries));
+  IG_CUDA(c, take(io.work, io.work_bytes, work));
+  memset(io.pin + io.status, 0, io.status_bytes);
+  int rc = host_call_enter(c, hc);
+  if (rc) return rc;
   hc.queued[0] = s;
-  if (copy) IG_CUDA(c, cudaStreamWaitEvent(s, c->hlane[hc.k].copied, 0));
-  // One copy up to the first array that went by itself, another past the last one.
-  const size_t first = ds ? io.seeds : db ? io.bs : io.a, last = db ? io.status : ds ? io.bs : io.a;
-  if (first) IG_CUDA(c, cudaMemcpyAsync(io.dev, io.pin, first, cudaMemcpyHostToDevice, s));
-  if (last < io.a) IG_CUDA(c, cudaMemcpyAsync(io.dev + last, io.pin + last, io.a - last, cudaMemcpyHostToDevice, s));
+  if (hc.queued[1]) IG_CUDA(c, cudaStreamWaitEvent(s, c->hlane[hc.k].copied, 0));
+  IG_CUDA(c, cudaMemcpyAsync(io.dev, io.pin, io.up, cudaMemcpyHostToDevice, s));
   return IG_OK;
 }
 int host_io_receive(ig_ctx* c, HostCall& hc, HostIO& io) {
-  const size_t last = !host_io_direct(c, io.b_bytes)   ? io.end
-                      : !host_io_direct(c, io.a_bytes) ? io.b
-                                                       : io.a;
-  cudaStream_t s = host_call_stream(c, hc);
-  const size_t first = host_io_direct(c, io.a_bytes) && last == io.end ? io.b : io.a;
-  if (first == io.b) {  // a goes by itself, b through the image
-    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.status, io.dev + io.status, io.a - io.status, cudaMemcpyDeviceToHost, s));
-    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.b, io.dev + io.b, io.end - io.b, cudaMemcpyDeviceToHost, s));
-  } else {
-    IG_CUDA(c, cudaMemcpyAsync(io.pin + io.status, io.dev + io.status, last - io.status, cudaMemcpyDeviceToHost, s));
-  }
+  IG_CUDA(c, cudaMemcpyAsync(io.pin + io.status, io.dev + io.status, io.down - io.status, cudaMemcpyDeviceToHost,
+                             host_call_stream(c, hc)));
   return host_call_launched(c, hc);
 }
 // Faults the pages of a result buffer in without changing a byte of it.
@@ -741,14 +742,14 @@ static void touch_pages(void* p, size_t bytes) {
   }
 }
 int host_io_wait(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out) {
-  if (host_io_direct(c, io.a_bytes)) touch_pages(a_out, io.a_bytes);
-  if (host_io_direct(c, io.b_bytes)) touch_pages(b_out, io.b_bytes);
+  if (io.a >= io.down) touch_pages(a_out, io.a_bytes);
+  if (io.b >= io.down) touch_pages(b_out, io.b_bytes);
   int rc = host_call_wait(c, hc);
   if (!rc) hc.queued[0] = hc.queued[1] = nullptr;
   return rc;
 }
 int host_io_finish(ig_ctx* c, HostCall& hc, HostIO& io, void* a_out, void* b_out) {
-  const bool da = host_io_direct(c, io.a_bytes), db = host_io_direct(c, io.b_bytes);
+  const bool da = io.a >= io.down, db = io.b >= io.down;
   if (!da) memcpy(a_out, io.pin + io.a, io.a_bytes);
   if (!db) memcpy(b_out, io.pin + io.b, io.b_bytes);
   if (!da && !db) return IG_OK;
@@ -802,6 +803,7 @@ int ig_ctx_create(int device, ig_ctx** out) {
   if (cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) != cudaSuccess)
     cudaGetLastError();
   c->direct_copies = tables != 0;
+  c->quads = igk::max_quads();
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       !igint::host_lane_streams(c->hlane[0].copy, c->hlane[0].copied)) {
     delete c;
@@ -2226,8 +2228,10 @@ static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u
   };
   double best = 0, best_bound = 0;
   std::vector<double> busy;
+  const u32 quads = std::max<u32>(1, c->quads / c->lanes);
   for (double bound : bounds) {
     busy.assign(sms, 0.0);  // a heap of the SMs' ends, the earliest first
+    std::priority_queue<double, std::vector<double>, std::greater<double>> fours;  // ends of the clusters of four
     double end = 0;
     for (u32 g : P.gammas) {
       const int k = shape_of(g, bound), r = std::min<int>(1 << k, (int)sms);
@@ -2235,6 +2239,13 @@ static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u
       for (int j = 0; j < r; j++) {
         std::pop_heap(busy.begin(), busy.end() - j, std::greater<double>());
         start = busy[busy.size() - 1 - j];
+      }
+      if (k == 2) {  // no more of them at once than their GPCs hold
+        if (fours.size() >= quads) {
+          start = std::max(start, fours.top());
+          fours.pop();
+        }
+        fours.push(start + times[g][k]);
       }
       for (int j = r - 1; j >= 0; j--) {
         busy[busy.size() - 1 - j] = start + times[g][k];
