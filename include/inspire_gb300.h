@@ -54,8 +54,10 @@ uint64_t ig_ctx_device_bytes(const ig_ctx* ctx);
 /* Launch-shape knob of the fixed rule, used when the context holds no tuned table for the
  * launch's width (ig_tune_launch_shapes): with q the queries expected on the device (the
  * batch times the lanes, or the queries in flight), a launch runs four CTAs per query (a
- * thread-block cluster) while 2q <= max_queries, two while q <= max_queries, else one, so
- * small batches still occupy most SMs. Default: half the device's SM count; 0 runs one CTA
+ * thread-block cluster) while 2q <= max_queries and q such clusters run at once (36: each
+ * takes its SMs within one GPC), two while q <= max_queries, else one, so small batches
+ * still occupy most SMs. A batch of more queries than SMs on one lane runs its whole waves
+ * with one CTA a query and what is left as a batch of that size. Default: half the device's SM count; 0 runs one CTA
  * per query always. Responses are identical under every shape. */
 int ig_ctx_set_pair_threshold(ig_ctx* ctx, uint32_t max_queries);
 /* Launch shapes and their tuner. A respond launch runs 1, 2 or 4 CTAs per query: one CTA

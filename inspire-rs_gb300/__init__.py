@@ -249,8 +249,8 @@ class Context:
 
     def set_pair_threshold(self, max_queries):
         """The fixed launch rule (no tuned table): four CTAs per query while twice the
-        queries expected in flight fit max_queries, two while they fit it, else one
-        (0: one CTA per query always)."""
+        queries expected in flight fit max_queries and as many clusters run at once, two
+        while they fit it, else one (0: one CTA per query always)."""
         self.check(self._lib.ig_ctx_set_pair_threshold(self.h, int(max_queries)))
 
     def response_wire_len(self, ring_dim, retained, modulus):

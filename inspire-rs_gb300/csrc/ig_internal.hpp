@@ -43,8 +43,8 @@ int resolve_request(ig_ctx* c, uint64_t db, uint64_t store, uint64_t handle, uin
 // CTAs per query (1, 2 or 4) for a respond launch of `count` queries of width `gamma` on
 // ring n with `in_flight` queries expected on the device with it (its own included): the
 // forced shape, else the shape the tuned table times fastest at that many queries, else the
-// fixed rule: four CTAs while twice the queries fit the pair threshold, two while they fit
-// it, else one.
+// fixed rule: four CTAs while twice the queries fit the pair threshold and the device runs
+// that many clusters of four at once, two while they fit the threshold, else one.
 int launch_ctas(ig_ctx* c, uint32_t n, uint32_t gamma, uint32_t count, uint32_t in_flight);
 // The launch shape set by ig_ctx_set_launch_shape (0 when the context chooses).
 int forced_ctas(ig_ctx* c);

@@ -1,16 +1,17 @@
 // Kernels of the InspiRING respond path on sm_103a.
 //
 // Work map (reference call sites in src/):
-//   ntt_rows      negacyclic forward NTT of many rows: the seat's key body
-//                 (pir/session.rs:600-625), the offline mask rows
-//                 (inspiring/inspiring2.rs:537-598) and a shard's columns before its
-//                 store is folded (inspiring/shard_store.rs:139-144).
+//   key_rows      the seat's key body (pir/session.rs:600-625) and the offline mask rows
+//                 (inspiring/inspiring2.rs:537-598) transformed, folded and scaled once.
+//   ntt_rows      negacyclic forward NTT of many rows (Galois keys, the client's secret).
+//   store_ntt     a shard's columns transformed before its store is folded
+//                 (inspiring/shard_store.rs:139-144).
 //   store_fold    step 1 of the offline phase folded over one shard's columns
 //                 (inspiring/inspiring2.rs:964-1004 via shard_store.rs:145), computed per
 //                 slot as a length-gamma cyclic DFT instead of gamma^2 monomial products.
 //   shard_scan    the store's column check and b fold (shard_store.rs:197-264): one HBM
 //                 pass over the queried shard's columns per query.
-//   respond       one CTA per query: the query's `a` expansion (math/poly.rs:657-686),
+//   respond       one CTA, or a cluster of two or four, per query: the `a` expansion (math/poly.rs:657-686),
 //                 the store gather (shard_store.rs:282-342), the backward recursion
 //                 (inspiring2.rs:1014-1085) with the online gather fused into each link
 //                 (inspiring2.rs:1393-1485), the final inverse transforms and the 36-bit
@@ -1301,7 +1302,7 @@ __device__ __forceinline__ void respond_links8(u64 (&cur)[8], Acc (&sb)[8], cons
 // with tau_i the slot permutation of the automorphism X -> X^(g^i), S the packing store,
 // W the mask rows and Y the seat. Digits 0 and 1 are transformed; with the exact gadget
 // digit 2's transform is D_2 = base^-2 (R_{i+1} - D_0 - base D_1) (inspiring2.rs:1094-1161),
-// a fixed linear combination, so the key rows are folded at staging (fold_gadget3) and
+// a fixed linear combination, so the key rows hold it folded (k_key_rows) and
 // R_{i+1} takes digit 2's place in the sums.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
@@ -1955,14 +1956,22 @@ __global__ void __launch_bounds__((1 << LOGN) / 4) k_nopack_cols(CrsDev c, const
   }
 }
 
-__global__ void k_nopack_sum(u32 n, u32 gamma, u64* out) {
-  const u32 qi = blockIdx.y;
-  const u32 k = blockIdx.x * blockDim.x + threadIdx.x;  // over 2n words of a ciphertext
-  if (k >= 2 * n) return;
-  u64* base = out + (size_t)qi * (gamma + 1) * 2 * n;
+// A CTA sums 32 words of a query's ciphertexts, a warp every eighth column, eight loads in flight: one thread a word over
+// all the columns waited for 256 loads in turn on 16 CTAs a query (39 us for one query of gamma 256).
+constexpr int SUM_WARPS = 8;
+__global__ void __launch_bounds__(32 * SUM_WARPS) k_nopack_sum(u32 n, u32 gamma, u64* out) {
+  __shared__ u64 part[SUM_WARPS][32];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;  // over 2n words
+  u64* base = out + (size_t)blockIdx.y * (gamma + 1) * 2 * n + k;
   u64 acc = 0;
-  for (u32 j = 1; j <= gamma; j++) acc = addq(acc, base[(size_t)j * 2 * n + k]);
-  base[k] = acc;
+#pragma unroll 8
+  for (u32 j = 1 + w; j <= gamma; j += SUM_WARPS) acc = addq(acc, base[(size_t)j * 2 * n]);
+  part[w][lane] = acc;
+  __syncthreads();
+  if (w) return;
+#pragma unroll
+  for (int r = 1; r < SUM_WARPS; r++) acc = addq(acc, part[r][lane]);
+  base[0] = acc;
 }
 
 // ------------------------------------------------------------------------------------
@@ -2636,7 +2645,7 @@ cudaError_t nopack_cols(const CrsDev& c, const QueryDev* queries, const ShardDev
     if (e != cudaSuccess) return e;
     k<<<dim3(c.gamma, nq), (1 << L) / 4, smem, s>>>(c, queries, shards, AB_R, out);
   });
-  k_nopack_sum<<<dim3((2 * c.n + 255) / 256, nq), 256, 0, s>>>(c.n, c.gamma, out);
+  k_nopack_sum<<<dim3(2 * c.n / 32, nq), 32 * SUM_WARPS, 0, s>>>(c.n, c.gamma, out);
   return cudaGetLastError();
 }
 
@@ -2769,7 +2778,7 @@ cudaError_t respond(const CrsDev& c, const QueryDev* queries, const ShardDev* sh
   const size_t smem = respond_smem_bytes(c, ctas);
   // A cluster a query, and a start beside the scan before it on the stream (the scan lets its successor launch at once,
   // the recursion reads the folds only at its end: scan_done). The recursion's CTAs fill the SMs that the scan's last
-  // wave leaves: a lone query of 1 KB records 142 -> 131 us, 128 mixed queries 5.20 -> 5.00 ms, 64 of one shard
+  // wave leaves: a lone query of gamma 16 142 -> 131 us, 128 mixed queries 5.20 -> 5.00 ms, 64 of one shard
   // 1.47 -> 1.46 ms.
   cudaLaunchAttribute attrs[2]{};
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -1678,9 +1678,9 @@ int ig_respond_nopacking_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const ui
   IG_CUDA(c, igk::nopack_prep(o.dev, (const QueryDev*)(io.dev + io.queries), count, R_MOD_Q, (u64*)d_ab, d_status, s));
   c->launches++;
   // The columns in parts, each copied out while the next runs: the copy (190 GB/s) takes twice the kernels' time, so a
-  // part need only be long enough to hide its launches: 16 MB, two queries of gamma 256 (16 of them 1.07 -> 0.86 ms, of
+  // part need only be long enough to hide its launches: 20 MB, two queries of gamma 256 (16 of them 1.07 -> 0.82 ms, of
   // which the copy is 0.70).
-  const u32 part = (u32)std::min<size_t>(count, std::max<size_t>(1, (16 << 20) / (row_words * 8)));
+  const u32 part = (u32)std::min<size_t>(count, std::max<size_t>(1, (20 << 20) / (row_words * 8)));
   auto& ends = c->hlane[k].parts;
   for (u32 i = 0, p = 0; i < count; i += part, p++) {
     const u32 nq = std::min(part, count - i);
