@@ -79,10 +79,9 @@ def peaks():
 SCAN_TRAFFIC_BYTES = 66_610_944
 # Heavy integer pipe (IMAD, IMAD.WIDE, IMAD.HI) busy cycles of k_respond per query, summed
 # over the four sub-partitions of each SM: sm__pipe_fmaheavy_cycles_active.sum of one
-# 64-query launch of this workload's timed region (1,043,445,848) / 64, from the ncu
-# capture in profiles/k_respond_single_batch64_d2048_g256.md. The pipe offers four such
-# cycles per SM per clock.
-RESPOND_HEAVY_CYCLES_PER_QUERY = 16_303_841
+# 152-query launch of this width and gadget (1,497,124,528) / 152, from the ncu capture in
+# profiles/k_respond_d2048_g256.md. The pipe offers four such cycles per SM per clock.
+RESPOND_HEAVY_CYCLES_PER_QUERY = 9_849_503
 
 
 def shard_seed(rank, s):
@@ -370,7 +369,7 @@ def small_batch_leg(pkg, ctx, crs, db, cache, store, handle, shards, rng, ms, ca
     """Latency of small batches under each launch shape: batches of 7 and 1 through
     respond_seeded_batch (host buffers, one synchronous call at a time), at one, two and four
     CTAs per query, and the shape the context picks for that batch alone. Inside a profiler
-    range, so an ncu --profile-from-start off capture with -k regex:k_respond_quad -c 1 takes
+    range, so an ncu --profile-from-start off capture with -k regex:k_respond_cluster -c 1 takes
     the first four-CTA launch of 7 queries."""
     out = {}
     for count in (7, 1):
@@ -596,10 +595,9 @@ def run_gb300(args, rank, world):
     heavy_achieved = value / world * RESPOND_HEAVY_CYCLES_PER_QUERY / 1e9  # G pipe-cycles/s per GPU
     heavy_peak = sms * 4 * mhz * 1e6 / 1e9
     # Cross-check: modular products per second against a register-only butterfly loop (3
-    # transforms of n/2 log n butterflies per link; per slot 7 pointwise products and 2
-    # Montgomery reductions of 2 products each).
+    # transforms of n/2 log n butterflies per link; per slot 7 pointwise products).
     links = GAMMA - 1
-    modmul_per_query = links * (3 * (N_RING // 2) * 11 + 11 * N_RING) + 3 * (N_RING // 2) * 11
+    modmul_per_query = links * (3 * (N_RING // 2) * 11 + 7 * N_RING) + 3 * (N_RING // 2) * 11
     timed_gmodmul = value / world * modmul_per_query / 1e9
     peak_gmodmul = ctx.butterfly_peak() / 1e9
     return {
@@ -1125,7 +1123,7 @@ def run_cfg4(args, rank, world):
         return max_over_ranks(ev0.elapsed_time(ev1), world), ctx.launch_count - launches0, clk
 
     timed_queries = int(offs[-1] - offs[args.warmup])
-    # The fixed rule first (no table: four CTAs per query while 2 x count x lanes <= SMs / 2, two
+    # The fixed rule first (no table: four CTAs per query while count x lanes <= 36, two
     # while count x lanes <= SMs / 2, else one), then
     # the launch-shape tuner's table for the three widths, then the same launches tuned.
     ms_fixed, _, _ = timed_region()
@@ -1262,7 +1260,7 @@ def run_cfg4(args, rank, world):
                 "d2h_bytes_per_step": int(timed_queries * 2 * N_RING * 8 / args.steps), "callers": lanes,
                 "call": "respond_mixed_batch (one launch per call)"},
         "fixed_rule": {"value": fixed_value, "unit": "queries/s",
-                       "rule": "four CTAs per query while 2 x count x lanes <= SMs / 2, two while "
+                       "rule": "four CTAs per query while count x lanes <= 36, two while "
                                "count x lanes <= SMs / 2, else one"},
         "launch_shapes": {"tuned_ms_per_launch": {str(g): {str(b): {"1": t[0], "2": t[1], "4": t[2]}
                                                            for b, t in rows.items()} for g, rows in tuned.items()},
