@@ -1993,10 +1993,11 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_nopack_sum(u32 n, u32 gamma,
 // and a binary-counter carry combines each finished node with its waiting sibling; the
 // waiting nodes sit in a stack of node slots in global memory. At gamma < n the odd children of the lowest
 // log(n / gamma) levels are all zero: a leaf walks those levels alone, from its registers (three of four nodes at
-// gamma 256; with the keys laid out for their loads 64 queries 4.80 -> 3.63 ms). The leaves [j n/S, (j+1) n/S) of the walk make up
-// the subtree of start bitrev(j) at level log n - log S, so k_tree_part walks S subtrees of a query on as many
-// CTAs and k_tree_top the S - 1 nodes above them: a query alone on one CTA took 11 ms whatever the batch, and
-// 64 left most SMs idle. 103 KB of shared memory a CTA: two on an SM.
+// gamma 256; with the keys laid out for their loads 64 queries 4.80 -> 3.63 ms). The leaves [j n/S, (j+1) n/S) of
+// the walk make up the subtree of start bitrev(j) at level log n - log S, so S CTAs walk a query's subtrees, and of two
+// CTAs whose subtrees are siblings the one that ends last goes on with the node above: log S nodes after the last
+// subtree (one CTA walking all S - 1 of them took 0.2 ms after a batch's subtrees: 64 queries 3.64 -> 3.51 ms, one
+// 0.91 -> 0.37). A query on one CTA took 11 ms whatever the batch, and 64 left most SMs idle. 103 KB of shared memory a CTA: two on an SM.
 struct TreeSmem {
   Tw* tw;
   u64 *S1a, *S1b, *D;  // E - y O of a node, by gather position; the transforms' buffers (2N)
@@ -2019,7 +2020,7 @@ __device__ __forceinline__ void node_load(const u64* node, u64 (&a)[8], u64 (&b)
   const ulonglong2* p = reinterpret_cast<const ulonglong2*>(node) + threadIdx.x;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const ulonglong2 x = p[k * NT], y = p[(k + 4) * NT];
+    const ulonglong2 x = __ldcg(p + k * NT), y = __ldcg(p + (k + 4) * NT);  // another CTA may have written it
     a[2 * k] = x.x, a[2 * k + 1] = x.y, b[2 * k] = y.x, b[2 * k + 1] = y.y;
   }
 }
@@ -2034,14 +2035,14 @@ __device__ __forceinline__ void node_store(u64* node, const u64 (&a)[8], const u
   }
 }
 // The current node (a, b at the thread's slots) becomes (E + y O) + keyswitch(tau_t(E - y O)) at level ell: it is
-// O and E waits in memory, or with ALONE it is E itself and its odd sibling zero. Ends with a barrier.
-template <int LOGN, bool ALONE>
+// O and E waits in memory, or it is E itself, its odd sibling zero (E null). Ends with a barrier.
+template <int LOGN>
 __device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S, const u64* E, int ell,
                                              const u32 (&et)[8], u64 (&ca)[8], u64 (&cb)[8]) {
   constexpr int N = 1 << LOGN, NT = N / 8;
   constexpr u32 M2N = 2 * N - 1;
   const u32 sy = (u32)(N >> ell), t = (1u << ell) + 1;
-  if constexpr (ALONE) {
+  if (!E) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       S.S1a[k * NT + threadIdx.x] = ca[k];
@@ -2094,8 +2095,8 @@ __device__ __forceinline__ void tree_combine(const CrsDev& c, const TreeSmem& S,
 
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
-    k_tree_part(CrsDev c, const QueryDev* queries, const ShardDev* shards, u32 log_parts, u64* stack, u64* roots,
-                u32* status) {
+    k_tree(CrsDev c, const QueryDev* queries, const ShardDev* shards, u32 log_parts, u64 ms_target, u64* stack, u64* roots,
+           u32* arrived, const u64* b_fold, u64* a_out, u64* b_out, u32* status) {
   constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
   extern __shared__ __align__(16) u64 sm[];
   const TreeSmem S = tree_stage<LOGN>(c, sm);
@@ -2105,7 +2106,10 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
   const ShardDev sh = shards[qd.shard];
   const u32 gamma = c.gamma;
   const int levels = LOGN - (int)log_parts;
-  u64* stk = stack + (size_t)blockIdx.x * levels * 2 * N;
+  const int zeros = LOGN - (31 - __clz(gamma));  // levels whose odd children are all zero
+  u64* stk = stack + (size_t)blockIdx.x * (levels - zeros) * 2 * N;
+  u64* slots = roots + ((size_t)qi << log_parts) * 2 * N;
+  __shared__ u32 first;
   u32 et[8];
   u64 aR[8];  // n^-1 NTT(a) at the thread's slots
 #pragma unroll
@@ -2113,9 +2117,8 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
   expand_a<N, NT>(qd, S.D + N, status, qi, 0);  // ends with a barrier
   transform_slots8<LOGN>(S.D + N, S.D, S.tw, c.ninv, aR);
   u64 ca[8], cb[8];
-  const int zeros = LOGN - (31 - __clz(gamma));  // levels whose odd children are all zero
 #pragma unroll 1
-  for (u32 m = 0; m < (u32)N >> log_parts >> zeros; m++) {
+  for (u32 m = 0;; m++) {
     const u32 start = __brev((part << levels) | (m << zeros)) >> (32 - LOGN);
     {
       // Leaf `start`: the column through the transform times NTT(a).
@@ -2144,44 +2147,43 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2)
       }
     }
     if (gamma == 1) break;  // a single leaf is the root
-    int L = 0;
+    bool root = false;
 #pragma unroll 1
-    for (; L < zeros; L++) tree_combine<LOGN, true>(c, S, nullptr, L + 1, et, ca, cb);
-#pragma unroll 1
-    for (; (m >> (L - zeros)) & 1; L++) tree_combine<LOGN, false>(c, S, stk + (size_t)L * 2 * N, L + 1, et, ca, cb);
-    if (L == levels) break;  // the subtree's root
-    node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
+    for (int L = 0;; L++) {
+      const u64* E = nullptr;
+      if (L >= levels) {
+        // Above the subtrees a node waits in the slot of its first subtree; the first of two siblings to arrive leaves,
+        // the other goes on. The even one is E whichever comes last.
+        const u32 up = L - levels, at = part >> up;
+        if (up == log_parts) {
+          root = true;
+          break;
+        }
+        u64 *mine = slots + ((size_t)at << up) * 2 * N, *other = slots + ((size_t)(at ^ 1) << up) * 2 * N;
+        node_store<LOGN>(mine, ca, cb);
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) first = atomicAdd(arrived + (qi << log_parts) + (1u << (log_parts - 1 - up)) + (at >> 1), 1u) == 0;
+        __syncthreads();
+        if (first) return;
+        __threadfence();
+        if (!(at & 1)) node_load<LOGN>(other, ca, cb);
+        E = at & 1 ? other : mine;
+      } else if (L >= zeros) {
+        u64* wait = stk + (size_t)(L - zeros) * 2 * N;
+        if (!((m >> (L - zeros)) & 1)) {
+          node_store<LOGN>(wait, ca, cb);
+          break;
+        }
+        E = wait;
+      }
+      tree_combine<LOGN>(c, S, E, L + 1, et, ca, cb);
+    }
+    if (root) break;
   }
-  node_store<LOGN>(roots + (size_t)blockIdx.x * 2 * N, ca, cb);
-}
-
-// The nodes above the subtrees, then the root to coefficients; b_z += n b-value_z for z < gamma (pack_lwes,
-// automorph_pack.rs 327-338), except for a single input, which pack_lwes returns untouched: no tree and no d
-// scaling.
-template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 8, 2)
-    k_tree_top(CrsDev c, const QueryDev* queries, u32 log_parts, u64 ms_target, u64* stack, const u64* roots,
-               const u64* b_fold, u64* a_out, u64* b_out) {
-  constexpr int N = 1 << LOGN, NT = N / 8, P = N / 4;
-  extern __shared__ __align__(16) u64 sm[];
-  const TreeSmem S = tree_stage<LOGN>(c, sm);
-  const int tid = threadIdx.x, levels = LOGN - (int)log_parts;
-  const u32 qi = blockIdx.x, gamma = c.gamma;
-  // The waiting nodes go where the query's first subtree kept its own; log_parts slots are free there or in
-  // the ones after.
-  u64* stk = stack + (size_t)(qi << log_parts) * levels * 2 * N;
-  u32 et[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) et[k] = c.slot_exp[8 * tid + k];
-  __syncthreads();
-  u64 ca[8], cb[8];
-#pragma unroll 1
-  for (u32 j = 0; j < 1u << log_parts; j++) {
-    node_load<LOGN>(roots + ((size_t)(qi << log_parts) + j) * 2 * N, ca, cb);
-    int L = 0;
-    for (; (j >> L) & 1; L++) tree_combine<LOGN, false>(c, S, stk + (size_t)L * 2 * N, levels + L + 1, et, ca, cb);
-    if (L < (int)log_parts) node_store<LOGN>(stk + (size_t)L * 2 * N, ca, cb);
-  }
+  // The root to coefficients; b_z += n b-value_z for z < gamma (pack_lwes, automorph_pack.rs 327-338), except for a
+  // single input, which pack_lwes returns untouched: no tree and no d scaling.
+  scan_done();
   inv_first8<LOGN>(ca, S.D, S.tw);
   inv_first8<LOGN>(cb, S.D + N, S.tw);
   __syncthreads();
@@ -2696,8 +2698,8 @@ cudaError_t client_extract(const CrsDev& c, u32 count, const u64* s_R, const u64
 // Subtrees of a query (a power of two): the split that takes least by a model in key switches (a leaf counts as
 // one; 10.2 us on an SM alone), with the stacks and roots within 256 MB. A subtree takes its own length on an idle
 // GPU; a full one gets through the batch's work at 1.2 subtrees an SM (two CTAs share it), with half a
-// subtree of idle tail; the nodes above follow. Measured at gamma 256 (ms, 1 / 8 / 32 subtrees): a query alone
-// 13.0 / 1.80 / 0.91, 64 queries 13.1 / 5.42 / 4.99 (16 subtrees 4.89), 152 13.4 / 10.8 / 10.8.
+// subtree of idle tail; log S nodes above follow. Measured at gamma 256 (ms, 4 / 8 / 32 subtrees): a query alone
+// 2.24 / 1.17 / 0.37, 64 queries 3.97 / 3.93 / 3.49 (16 subtrees 3.48), 152 7.76 / 7.82 / 7.87.
 u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms) {
   u64 work = c.gamma, best = ~0ULL;  // leaves and nodes of a whole tree
   for (u32 k = 1; k <= c.logn; k++) work += c.gamma < (c.n >> k) ? c.gamma : c.n >> k;
@@ -2705,30 +2707,43 @@ u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms) {
   for (u32 lp = 0; lp <= 5 && (2u << lp) <= c.gamma; lp++) {
     if (lp && tree_scratch_words(c, nq, lp) * 8 > (256ULL << 20)) break;
     const u64 part = work >> lp, full = nq * work * 10 / (12 * (u64)sms) + part / 2;
-    const u64 cost = (part > full ? part : full) + ((1u << lp) - 1);
+    const u64 cost = (part > full ? part : full) + lp;
     if (cost < best) best = cost, log_best = lp;
   }
   return log_best;
 }
-// Node stacks of the subtrees (and of the nodes above them, in their place), then their roots.
+// Node stacks of the subtrees, then their roots' slots.
+static u64 tree_stack_words(const CrsDev& c, u32 nq, u32 log_parts) {
+  return ((u64)nq << log_parts) * (31 - __builtin_clz(c.gamma) - log_parts) * 2 * c.n;
+}
 u64 tree_scratch_words(const CrsDev& c, u32 nq, u32 log_parts) {
-  return ((u64)nq << log_parts) * (c.logn - log_parts + 1) * 2 * c.n;
+  return tree_stack_words(c, nq, log_parts) + ((u64)nq << log_parts) * 2 * c.n;
 }
 
 cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u32 log_parts, u64 ms_target,
-                 u64* nodes, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
+                 u64* nodes, u32* arrived, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   if (!c.galois || c.gamma > c.n / 2) return cudaErrorInvalidValue;
   const size_t smem = (size_t)6 * c.n * 8 + 2 * (size_t)c.n;
-  u64* roots = nodes + ((u64)nq << log_parts) * (c.logn - log_parts) * 2 * c.n;
+  u64* roots = nodes + tree_stack_words(c, nq, log_parts);
+  // Beside the scan before it: only a query's last CTA takes its folds (scan_done).
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nq << log_parts);
+  cfg.blockDim = dim3(c.n / 8);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   IG_DISPATCH_LOGN(c.logn, {
-    auto part = k_tree_part<L>;
-    auto top = k_tree_top<L>;
-    cudaError_t e = cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto k = k_tree<L>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaLaunchKernelEx(&cfg, k, c, queries, shards, log_parts, ms_target, nodes, roots, arrived, b_fold, a_out, b_out,
+                             status);
     if (e != cudaSuccess) return e;
-    part<<<nq << log_parts, (1 << L) / 8, smem, s>>>(c, queries, shards, log_parts, nodes, roots, status);
-    top<<<nq, (1 << L) / 8, smem, s>>>(c, queries, log_parts, ms_target, nodes, roots, b_fold, a_out, b_out);
   });
   return cudaGetLastError();
 }

@@ -165,13 +165,13 @@ cudaError_t nopack_prep(const CrsDev& c, const QueryDev* queries, u32 nq, u64 r_
 cudaError_t nopack_cols(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u64* AB_R,
                         u64* out, cudaStream_t s);
 
-// OnePacking (respond_one_packing): 2^log_parts CTAs per query walk the automorphism tree's subtrees, one the nodes
-// above them; nodes holds tree_scratch_words, b_fold the scan's b-values. Outputs coefficient-form
-// (a, b), switched to ms_target when nonzero.
+// OnePacking (respond_one_packing): 2^log_parts CTAs per query walk the automorphism tree's subtrees, the last of two
+// siblings the node above them; nodes holds tree_scratch_words, arrived nq << log_parts zeroed words, b_fold the
+// b-values of the scan launched before it. Outputs coefficient-form (a, b), switched to ms_target when nonzero.
 u32 tree_log_parts(const CrsDev& c, u32 nq, u32 sms);
 u64 tree_scratch_words(const CrsDev& c, u32 nq, u32 log_parts);
 cudaError_t tree(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, u32 log_parts, u64 ms_target,
-                 u64* nodes, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s);
+                 u64* nodes, u32* arrived, const u64* b_fold, u64* a_out, u64* b_out, u32* status, cudaStream_t s);
 
 // Client side: the sampler's keystream (ChaCha20 blocks of stream 0), the parallel parse of
 // W stream words from u32 offset `base` of ks into the first S samples (out) and the word

@@ -2017,13 +2017,13 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
   };
   int rc;
   if ((rc = igint::host_io_open(c, hc, io, table.size() * sizeof(ShardDev), count * sizeof(QueryDev), 0,
-                                as ? words : (size_t)count * 32, words, count, words, words)) ||
+                                as ? words : (size_t)count * 32, words, count + ((size_t)count << parts), words, words)) ||
       (rc = lane_scratch("tr_nodes", igk::tree_scratch_words(o.dev, count, parts) * 8, &d_nodes)) ||
       (rc = lane_scratch("tr_fold", (size_t)count * o.gamma * 8, &d_fold)))
     return rc;
   const QueryDev* d_q = (const QueryDev*)(io.dev + io.queries);
   const ShardDev* d_table = (const ShardDev*)(io.dev + io.table);
-  u32* d_status = (u32*)(io.dev + io.status);
+  u32* d_status = (u32*)(io.dev + io.status);  // zeroed with the arrival counts after them
   std::vector<QueryDev> qs(count);
   for (u32 i = 0; i < count; i++) {
     qs[i] = QueryDev{};
@@ -2039,9 +2039,9 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
   if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
     return rc;
   IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
-  IG_CUDA(c, igk::tree(o.dev, d_q, d_table, count, parts, ms_target, (u64*)d_nodes, (const u64*)d_fold,
-                       (u64*)(io.dev + io.a), (u64*)(io.dev + io.b), d_status, s));
-  c->launches += 3;
+  IG_CUDA(c, igk::tree(o.dev, d_q, d_table, count, parts, ms_target, (u64*)d_nodes, d_status + count,
+                       (const u64*)d_fold, (u64*)(io.dev + io.a), (u64*)(io.dev + io.b), d_status, s));
+  c->launches += 2;
   if ((rc = igint::host_io_receive(c, hc, io))) return rc;
   lk.unlock();  // other callers launch while this batch runs
   if ((rc = igint::host_io_wait(c, hc, io, a_out, b_out))) return rc;
