@@ -326,7 +326,8 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_store_fold(CrsDev c, const u64
 // encode), so the tags are recomputed once, at each such change, and compared with the
 // stored ones: a mismatch marks the shard stale, and every later respond on it is refused
 // with the reference's message until the store is rebuilt. The refusal stays at respond
-// time; the tag check leaves the per-query scan.
+// time; the tag check leaves the per-query scan. A launch covers a range of shards, and those of
+// them that hold no store have no tag key and no tags: their CTAs return at once.
 //
 // b fold (k_scan), per query and column j of its shard:
 //   fold_j = sum_k w_k * b_rev[k],  b_rev[0] = b_0, b_rev[k] = -b_{n-k}   (mod q)
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(256) k_column_tags(u32 gamma, const ShardDev* 
   const ShardDev sh = table[blockIdx.y];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const u32 j = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (j >= gamma || sh.cols16) return;
+  if (j >= gamma || sh.cols16 || !sh.tag_key) return;
   const u64* col = sh.columns + (size_t)j * N;
   u128 tag = 0;
 #pragma unroll 4
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_column_tags16(u32 gamma,
   constexpr int N = 1 << LOGN, M = N / 8;
   extern __shared__ __align__(16) uint4 scan_sm[];
   const ShardDev sh = table[blockIdx.y];
-  if (!sh.cols16) return;
+  if (!sh.cols16 || !sh.tag_key) return;
   const u32 j0 = blockIdx.x * SCAN_COLS + (threadIdx.x >> 5) * SCAN_ROWS;
   const int rows = j0 < gamma ? min(SCAN_ROWS, (int)(gamma - j0)) : 0;
   scan_columns16<LOGN>(
