@@ -1437,10 +1437,11 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
 // A link of four CTAs now takes 5,000 cycles: inverse 1,600, its exchange 610, cross 820, the digits' 220, forward
 // 1,180, pointwise 570. Two CTAs an SM (the seat's rows from L2, half the shared memory) ran 64 queries no faster
 // than clusters of two: both share the multiply pipe.
-// The data's own arrivals order every buffer's reuse. A CTA sends a link's cross words after its forward of the
-// link before, which took digits from every peer, and a peer sends those after reading its cross words; it sends
+// The data's own arrivals order the reuse of the exchange buffers. A CTA sends a link's cross words after its forward of
+// the link before, which took digits from every peer, and a peer sends those after reading its cross words; it sends
 // digits after taking cross words from every peer, and a peer's threads send those after reading their
-// digits of the link before.
+// digits of the link before. X is a CTA's own: between two links the forward's last barrier orders its reuse, between
+// the two final transforms a barrier of its own.
 template <int LOGN, int R>
 struct Part {
   static constexpr int N = 1 << LOGN, LR = R == 4 ? 2 : 1, LP = LOGN - LR, P = 1 << LP, NT = P / 2;
@@ -1886,6 +1887,10 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
     if constexpr (!SIDE) {
       parity ^= 1;
       cross(n, [&] { cluster.sync(); });  // the words are read before the next are sent, and before a CTA ends
+    } else if (n == 0) {
+      // Every thread has read X before the next transform rewrites it. The arrivals alone say so only where each thread of
+      // the last local pass sends a word to its own CTA; a pass of one bit (rings 256 and 1024) sends to two CTAs of the four.
+      __syncthreads();
     }
   }
   if constexpr (SIDE) {
