@@ -443,54 +443,71 @@ int fold_store(ig_ctx* c, CrsObj& o, const ShardDev& sh) {
 
 // Stores of shards [first, first + count): keyed tags and step-1 sums, one launch sequence a group of shards
 // and one wait at the end. A shard that cannot be built ends the range: those before it are built, the
-// call then fails.
+// call then fails. A shard counts as stored when `sums` is set, so a failure after that takes the new stores back.
 int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
-  const size_t n = o.n, g = o.gamma;
+  const size_t n = o.n, g = o.gamma, store_bytes = g * n * 8 + 2 * n * 8 + g * 8;
   int failed = IG_OK;
   u32 ready = 0;
   bool wide = false;
+  std::vector<u32> fresh;  // shards whose store this call allocated
+  auto withdraw = [&](int rc) {
+    for (u32 s : fresh) {
+      ShardSlot& sl = db.shards[s];
+      cudaFree(sl.sums);
+      cudaFree(sl.tag_key);
+      cudaFree(sl.tags);
+      sl.sums = sl.tag_key = sl.tags = nullptr;
+    }
+    c->obj_bytes -= fresh.size() * store_bytes;
+    db.bytes -= fresh.size() * store_bytes;
+    sync_table(c, db, first, ready);
+    return rc;
+  };
+  // Room for one shard's transforms before any store, for a group's after the stores: memory that holds a shard at a
+  // time is not refused.
+  void* H = nullptr;
+  if (db.shards[first].cols)
+    if (int rc = scratch(c, "fold_H", g * n * 8, &H)) return rc;
   for (; ready < count; ready++) {
     ShardSlot& sl = db.shards[first + ready];
-    if (!sl.cols) {
-      failed = fail(c, IG_ERR_ARG, "shard %u: no columns uploaded; precompute_packing needs the shard's columns",
-                    first + ready);
-      break;
-    }
+    if (!sl.cols) break;
     if (!sl.sums) {
-      // All three buffers or none: a shard counts as stored when `sums` is set.
       u64 *sums = nullptr, *key = nullptr, *tags = nullptr;
-      size_t got = 0;
-      failed = dalloc(c, (void**)&sums, g * n * 8, &got);
-      if (!failed) failed = dalloc(c, (void**)&key, 2 * n * 8, &got);
-      if (!failed) failed = dalloc(c, (void**)&tags, g * 8, &got);
+      failed = dalloc(c, (void**)&sums, g * n * 8, &db.bytes);
+      if (!failed) failed = dalloc(c, (void**)&key, 2 * n * 8, &db.bytes);
+      if (!failed) failed = dalloc(c, (void**)&tags, g * 8, &db.bytes);
       if (failed) {
-        if (sums) dfree(c, sums, g * n * 8);
-        if (key) dfree(c, key, 2 * n * 8);
+        if (sums) dfree(c, sums, g * n * 8), db.bytes -= g * n * 8;
+        if (key) dfree(c, key, 2 * n * 8), db.bytes -= 2 * n * 8;
         break;
       }
-      db.bytes += got;
       sl.sums = sums;
       sl.tag_key = key;
       sl.tags = tags;
+      fresh.push_back(first + ready);
     }
     wide |= !sl.compact;
   }
-  if (ready) {
-    u32 group = std::min(ready, store_group(o));
-    void* H;
-    int rc = scratch(c, "fold_H", (size_t)group * g * n * 8, &H);
-    if (rc && group > 1) {  // short of memory: a shard at a time
-      group = 1;
-      rc = scratch(c, "fold_H", (size_t)g * n * 8, &H);
-    }
-    if (rc) return rc;
-    // Tag keys: two words per column word below 2^61 - 1, expanded on the device from OS entropy; they
-    // never leave it (shard_store.rs:127-135).
-    std::random_device rd;
-    u32 seed[8];
-    for (auto& w : seed) w = rd();
+  const bool no_columns = ready < count && !failed;
+  auto end = [&]() {
+    return no_columns ? fail(c, IG_ERR_ARG, "shard %u: no columns uploaded; precompute_packing needs the shard's columns",
+                             first + ready)
+                      : failed;
+  };
+  if (!ready) return end();
+  u32 group = std::min(ready, store_group(o));
+  if (group > 1 && scratch(c, "fold_H", (size_t)group * g * n * 8, &H)) {  // short of memory: a shard at a time
+    group = 1;
+    if (int rc = scratch(c, "fold_H", g * n * 8, &H)) return withdraw(rc);
+  }
+  // Tag keys: two words per column word below 2^61 - 1, expanded on the device from OS entropy; they
+  // never leave it (shard_store.rs:127-135).
+  std::random_device rd;
+  u32 seed[8];
+  for (auto& w : seed) w = rd();
+  auto build = [&]() -> int {
     for (u32 k = 0; k < ready; k++) db.shards[first + k].stale = false;
-    rc = sync_table(c, db, first, ready);
+    int rc = sync_table(c, db, first, ready);
     if (rc) return rc;
     const ShardDev* table = db.d_table + first;
     for (u32 k = 0; k < ready; k += LAUNCH_SHARDS) {
@@ -506,8 +523,10 @@ int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
       prof_end(c, p);
     }
     IG_CUDA(c, cudaStreamSynchronize(c->stream));
-  }
-  return failed;
+    return IG_OK;
+  };
+  if (int rc = build()) return withdraw(rc);
+  return end();
 }
 
 // After new columns land in shards [first, first + count), with their table entries written: the columns'
