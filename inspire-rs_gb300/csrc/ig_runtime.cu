@@ -506,7 +506,6 @@ int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
   u32 seed[8];
   for (auto& w : seed) w = rd();
   auto build = [&]() -> int {
-    for (u32 k = 0; k < ready; k++) db.shards[first + k].stale = false;
     int rc = sync_table(c, db, first, ready);
     if (rc) return rc;
     const ShardDev* table = db.d_table + first;
@@ -523,7 +522,13 @@ int build_stores(ig_ctx* c, DbObj& db, CrsObj& o, u32 first, u32 count) {
       prof_end(c, p);
     }
     IG_CUDA(c, cudaStreamSynchronize(c->stream));
-    return IG_OK;
+    // A stale shard is served again only now: a batch queued on a lane reads the table when it runs.
+    bool changed = false;
+    for (u32 k = 0; k < ready; k++) {
+      changed |= db.shards[first + k].stale;
+      db.shards[first + k].stale = false;
+    }
+    return changed ? sync_table(c, db, first, ready) : IG_OK;
   };
   if (int rc = build()) return withdraw(rc);
   return end();
