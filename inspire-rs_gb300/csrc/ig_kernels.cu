@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_column_tags16(u32 gamma,
 
 template <int LOGN>
 __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_scan(CrsDev c, const QueryDev* queries, const ShardDev* shards,
-                                                          const u32* work, u32 chunks, u64* b_fold, u32* status) {
+                                                          const u32* work, u32 chunks, u64* b_fold) {
   constexpr int N = 1 << LOGN, M = N / 8;
   extern __shared__ __align__(16) uint4 scan_sm[];
   u32 qi, chunk;
@@ -578,7 +578,6 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, 2) k_scan(CrsDev c, const Que
   const u32 j0 = chunk * SCAN_COLS + warp * SCAN_ROWS;
   const u64* b = qd.b;
   u64* fold_out = b_fold + qd.fold_off;
-  if (chunk == 0 && threadIdx.x == 0 && sh.stale) atomicOr(status + qd.row, (u32)DEV_TAG_MISMATCH);
   const int rows = j0 < gamma ? min(SCAN_ROWS, (int)(gamma - j0)) : 0;
 
   if (sh.cols16) {
@@ -907,6 +906,12 @@ __device__ __forceinline__ void expand_a(const QueryDev& qd, u64* a, u32* status
 // Waits for the launch's scan, which runs beside the recursion (programmatic launch): called before the first use of
 // a b fold.
 __device__ __forceinline__ void scan_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Refuses a query on a stale shard. The respond kernel itself checks, on the table entry that it takes the store from and
+// before its first use: its scan runs beside it, and a store rebuilt between the two reads would pass for a good one.
+__device__ __forceinline__ void refuse_stale(const ShardDev& sh, u32* status, u32 qi) {
+  if (sh.stale) atomicOr(status + qi, (u32)DEV_TAG_MISMATCH);
+}
 
 // Coefficients of the response from the unscaled inverse transforms of c_0 = n^-1 R_0 (a) and of
 // the online sum (b).
@@ -1341,6 +1346,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 1)
   const u32 gamma = ps.gamma;
   const bool exact = ps.approx == 0;
   const int l0 = 8 * tid;
+  if (tid == 0) refuse_stale(sh, status, qi);
 
 #pragma unroll 4
   for (int k = tid; k < N; k += NT) stage_key_rows(ps, qd.seat, K, N, k, slot8<LOGN>(k));
@@ -1667,6 +1673,7 @@ __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
   const u32 gamma = ps.gamma;
 
   cluster_arrive();
+  if (tid == 0) refuse_stale(sh, status, qi);
   {
 #pragma unroll 4
     for (int k = tid; k < N; k += NT) stage_key_rows(ps, qd.seat, KR, N, k, slot2<LOGN>(k));
@@ -2576,7 +2583,7 @@ cudaError_t store_sums_one(const CrsDev& c, const ShardDev& shard, u64* H, cudaS
 u32 scan_chunks(u32 gamma) { return (gamma + SCAN_COLS - 1) / SCAN_COLS; }
 
 cudaError_t shard_scan(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u32* work,
-                       u32 nwork, u64* b_fold, u32* status, cudaStream_t s) {
+                       u32 nwork, u64* b_fold, cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
   const u32 chunks = scan_chunks(c.gamma);
   const u32 blocks = work ? nwork : nq * chunks;
@@ -2586,7 +2593,7 @@ cudaError_t shard_scan(const CrsDev& c, const QueryDev* queries, const ShardDev*
     auto k = k_scan<L>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<blocks, SCAN_WARPS * 32, smem, s>>>(c, queries, shards, work, chunks, b_fold, status);
+    k<<<blocks, SCAN_WARPS * 32, smem, s>>>(c, queries, shards, work, chunks, b_fold);
   });
   return cudaGetLastError();
 }

@@ -111,13 +111,12 @@ cudaError_t key_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, const K
 cudaError_t ntt_rows(const CrsDev& c, const u64* in, u64* out, u32 rows, u64 scale, cudaStream_t s);
 
 // Shard scan over `nq` queries: for query q and column j < gamma_q,
-// b_fold[fold_off_q + j] = coeff0(b_q * column_j); a query on a stale shard gets
-// DEV_TAG_MISMATCH. The work list (nwork entries, query << 12 | chunk, chunk < scan_chunks
-// of the query's gamma) lets queries of different widths share a launch; without one, every
-// query has c's gamma.
+// b_fold[fold_off_q + j] = coeff0(b_q * column_j). The work list (nwork entries, query << 12 | chunk,
+// chunk < scan_chunks of the query's gamma) lets queries of different widths share a launch; without one,
+// every query has c's gamma.
 u32 scan_chunks(u32 gamma);
 cudaError_t shard_scan(const CrsDev& c, const QueryDev* queries, const ShardDev* shards, u32 nq, const u32* work,
-                       u32 nwork, u64* b_fold, u32* status, cudaStream_t s);
+                       u32 nwork, u64* b_fold, cudaStream_t s);
 
 // Tag keys of `count` shards of a device table (2n words below 2^61 - 1 each) from a 32-byte seed.
 cudaError_t tag_keys(const CrsDev& c, const ShardDev* table, u32 count, const u32 (&seed)[8], u64 stream, cudaStream_t s);

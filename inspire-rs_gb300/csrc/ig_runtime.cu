@@ -1590,7 +1590,7 @@ static int respond_host(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_t handle, c
     for (auto& e : env_ev) cudaEventCreate(&e);
   if (env_prof) cudaEventRecord(env_ev[0], s);
   long pk = prof_begin(c, REGION_SCAN, s);
-  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
+  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, s));
   prof_end(c, pk, s);
   if (env_prof) cudaEventRecord(env_ev[1], s);
   pk = prof_begin(c, REGION_RESPOND, s);
@@ -2027,7 +2027,6 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
     if (!local.count(s)) {
       local[s] = (u32)table.size();
       table.push_back(db->shards[s].dev());
-      table.back().stale = 0;  // the tree reads columns alone: no store to be out of date
     }
   }
   const size_t words = (size_t)count * n * 8;
@@ -2062,7 +2061,7 @@ int ig_respond_one_packing_batch(ig_ctx* c, uint64_t dbh, uint32_t count, const 
   cudaStream_t s = igint::host_call_stream(c, hc);
   if ((rc = igint::host_io_send(c, hc, io, table.data(), qs.data(), nullptr, as ? (const void*)as : (const void*)seeds, bs)))
     return rc;
-  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
+  IG_CUDA(c, igk::shard_scan(o.dev, d_q, d_table, count, nullptr, 0, (u64*)d_fold, s));
   IG_CUDA(c, igk::tree(o.dev, d_q, d_table, count, parts, ms_target, (u64*)d_nodes, d_status + count,
                        (const u64*)d_fold, (u64*)(io.dev + io.a), (u64*)(io.dev + io.b), d_status, s));
   c->launches += 2;
@@ -2125,7 +2124,7 @@ int ig_respond_seeded_batch_device(ig_ctx* c, uint64_t dbh, uint64_t st, uint64_
   if ((rc = igint::lane_enter(c, lane))) return rc;
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
   long pk = prof_begin(c, REGION_SCAN, s);
-  IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, db->d_table, count, nullptr, 0, (u64*)d_fold, d_status, s));
+  IG_CUDA(c, igk::shard_scan(o.dev, (const QueryDev*)d_q, db->d_table, count, nullptr, 0, (u64*)d_fold, s));
   prof_end(c, pk, s);
   // Several CTAs per query only while every lane's batch still leaves SMs for them.
   pk = prof_begin(c, REGION_RESPOND, s);
@@ -2355,7 +2354,7 @@ int ig_respond_mixed_batch_device(ig_ctx* c, uint32_t count, const uint64_t* dbs
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
   long pk = prof_begin(c, REGION_SCAN, s);
   IG_CUDA(c, igk::shard_scan(P.ring, (const QueryDev*)dq, (const ShardDev*)dt, count, (const u32*)dw,
-                             (u32)P.work.size(), (u64*)df, d_status, s));
+                             (u32)P.work.size(), (u64*)df, s));
   prof_end(c, pk, s);
   pk = prof_begin(c, REGION_RESPOND, s);
   if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), lane < 0 ? 0 : (u32)lane, (const QueryDev*)dq,
@@ -2400,7 +2399,7 @@ int ig_respond_mixed_batch(ig_ctx* c, uint32_t count, const uint64_t* dbs, const
   u32* dst = (u32*)(io.dev + io.status);
   cudaStream_t s = igint::host_call_stream(c, hc);
   if ((rc = igint::host_io_send(c, hc, io, P.table.data(), P.qs.data(), P.work.data(), seeds, bs))) return rc;
-  IG_CUDA(c, igk::shard_scan(P.ring, dq, dt, count, (const u32*)(io.dev + io.work), (u32)P.work.size(), (u64*)df, dst, s));
+  IG_CUDA(c, igk::shard_scan(P.ring, dq, dt, count, (const u32*)(io.dev + io.work), (u32)P.work.size(), (u64*)df, s));
   if ((rc = respond_runs(c, P, plan_shapes(c, P, (u32)n, count), k, dq, dt, (const u64*)df, (u64*)(io.dev + io.a),
                          (u64*)(io.dev + io.b), dst, s)))
     return rc;
@@ -3132,7 +3131,7 @@ int ig_respond_seeded_batch_noalloc(ig_ctx* c, uint64_t dbh, uint64_t st, uint64
   cudaStream_t s = c->stream;
   IG_CUDA(c, cudaMemcpyAsync(d_q, qs, count * sizeof(QueryDev), cudaMemcpyHostToDevice, s));
   IG_CUDA(c, cudaMemsetAsync(d_status, 0, count * 4, s));
-  IG_CUDA(c, igk::shard_scan(o.dev, d_q, db->d_table, count, nullptr, 0, d_fold, d_status, s));
+  IG_CUDA(c, igk::shard_scan(o.dev, d_q, db->d_table, count, nullptr, 0, d_fold, s));
   // The launch shape of ig_respond_seeded_batch_device for the same batch and lane count.
   IG_CUDA(c, respond_waves(c, o.dev, d_q, db->d_table, count, d_fold, d_a, d_b, d_status, s));
   c->launches += 2;

@@ -482,7 +482,7 @@ void dispatch_loop(ig_serve* s) {
     if (e == cudaSuccess) e = cudaMemsetAsync(d + L.status, 0, count * 4, st);
     if (e == cudaSuccess)
       e = igk::shard_scan(ring, (const QueryDev*)(d + L.q), (const ShardDev*)(d + L.table), count,
-                          (const u32*)(d + L.work), sl.work_items, (u64*)(d + L.fold), (u32*)(d + L.status), st);
+                          (const u32*)(d + L.work), sl.work_items, (u64*)(d + L.fold), st);
     if (e == cudaSuccess)
       e = igk::respond(ring, (const QueryDev*)(d + L.q), (const ShardDev*)(d + L.table), count,
                        (const u64*)(d + L.fold), (u64*)(d + L.a), (u64*)(d + L.b), (u32*)(d + L.status), 0, ctas, st);
