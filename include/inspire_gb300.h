@@ -57,8 +57,9 @@ uint64_t ig_ctx_device_bytes(const ig_ctx* ctx);
  * thread-block cluster) while 2q <= max_queries and q such clusters run at once (36: each
  * takes its SMs within one GPC), two while q <= max_queries, else one, so small batches
  * still occupy most SMs. A batch of more queries than SMs on one lane runs its whole waves
- * with one CTA a query and what is left as a batch of that size. Default: half the device's SM count; 0 runs one CTA
- * per query always. Responses are identical under every shape. */
+ * with one CTA a query and what is left as a batch of that size; a mixed batch of several
+ * widths gives each width a shape of its own whatever the threshold. Default: half the
+ * device's SM count; 0 runs one CTA per query. Responses are identical under every shape. */
 int ig_ctx_set_pair_threshold(ig_ctx* ctx, uint32_t max_queries);
 /* Launch shapes and their tuner. A respond launch runs 1, 2 or 4 CTAs per query: one CTA
  * per SM is the most work per SM-second; a cluster of 2 or 4 splits each query's
@@ -74,8 +75,9 @@ int ig_ctx_set_pair_threshold(ig_ctx* ctx, uint32_t max_queries);
  * time is least (by at least 2% for more CTAs) in the table's row for the queries expected
  * in flight with it: the smallest tuned batch size at or above that number, the largest
  * beyond the grid. The device path expects count x lanes queries in flight, the serving
- * loop its batch and the CTAs of its batches in flight. Responses are identical under
- * every shape.
+ * loop its batch and the CTAs of its batches in flight. A time that is not above 0 marks a
+ * shape that was not measured: it is not taken. A mixed batch of several widths plans their
+ * shapes from the widths' rows of one query. Responses are identical under every shape.
  * ig_tune_get copies the row of (ring_dim, gamma) for `queries` in flight (ms_out[0..2]: 1,
  * 2, 4 CTAs per query); ig_tune_choose gives the shape a launch of `count` queries with
  * `in_flight` queries expected would take. ig_tune_save writes the table to a text file

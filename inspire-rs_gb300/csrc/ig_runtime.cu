@@ -6,8 +6,8 @@
 
 #include <algorithm>
 #include <array>
-#include <cmath>
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -2225,11 +2225,12 @@ struct ShapeRun {
 };
 
 // Shapes of a mixed launch of several widths, whose queries need not share one: under a bound T on a query's own
-// time each query takes the fewest CTAs that keep it (four where none does), and T is the one whose launch
-// ends first when the queries start longest first as SMs come free. Times are the tuned table's for one query,
-// else 6.95, 4.15 and 2.62 us a link (measured at gamma 1024 under one, two and four CTAs). 128 queries over gamma
-// 16, 256 and 1024 in equal parts took one CTA each: 7.65 ms, the time of the 43 longest, with most SMs
-// idle after 2 ms. Lanes share the SMs. More queries than four an SM fill the GPU in any order: one CTA each.
+// time each query takes the fewest CTAs that keep it (the fastest where none does), and T is the one whose launch
+// ends first when the queries start longest first as SMs come free. Times are those the tuned table holds for one query
+// of the width (a shape that it did not measure is not taken), else 6.95, 4.15 and 2.62 us a link (measured at gamma
+// 1024 under one, two and four CTAs). 128 queries over gamma 16, 256 and 1024 in equal parts took one CTA each: 7.65 ms,
+// the time of the 43 longest, with most SMs idle after 2 ms. Lanes share the SMs. More queries than four an SM fill the
+// GPU in any order: one CTA each.
 static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u32 count) {
   const bool uniform = P.gammas.front() == P.gammas.back();
   const u32 sms = std::max<u32>(1, c->sms / c->lanes);
@@ -2240,14 +2241,21 @@ static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u
   for (u32 g : P.gammas)
     if (!times.count(g)) {
       std::array<double, 3> t{6.95 * g, 4.15 * g, 2.62 * g};
-      if (c->tune.count({n, g}))  // milliseconds, of this width only
-        for (int k = 0; k < 3; k++) t[k] = 1e3 * (*igint::tuned_row(c, n, g, 1))[k];
+      const auto width = c->tune.find({n, g});
+      if (width != c->tune.end() && width->second.count(1)) {
+        const std::array<double, 3>& ms = width->second.at(1);
+        if (ms[0] > 0 || ms[1] > 0 || ms[2] > 0)
+          for (int k = 0; k < 3; k++) t[k] = ms[k] > 0 ? 1e3 * ms[k] : HUGE_VAL;
+      }
       times[g] = t;
-      bounds.insert(bounds.end(), t.begin(), t.end());
+      for (double x : t)
+        if (x < HUGE_VAL) bounds.push_back(x);
     }
   auto shape_of = [&](u32 g, double bound) {
     const std::array<double, 3>& t = times[g];
-    return t[0] <= bound ? 0 : t[1] <= bound ? 1 : 2;
+    for (int k = 0; k < 3; k++)
+      if (t[k] <= bound) return k;
+    return (int)(std::min_element(t.begin(), t.end()) - t.begin());
   };
   double best = 0, best_bound = 0;
   std::vector<double> busy;
