@@ -58,8 +58,8 @@ uint64_t ig_ctx_device_bytes(const ig_ctx* ctx);
  * takes its SMs within one GPC), two while q <= max_queries, else one, so small batches
  * still occupy most SMs. A batch of more queries than SMs on one lane runs its whole waves
  * with one CTA a query and what is left as a batch of that size; a mixed batch of several
- * widths gives each width a shape of its own whatever the threshold. Default: half the
- * device's SM count; 0 runs one CTA per query. Responses are identical under every shape. */
+ * widths gives each width a shape of its own. Default: half the device's SM count; 0 runs
+ * one CTA per query always. Responses are identical under every shape. */
 int ig_ctx_set_pair_threshold(ig_ctx* ctx, uint32_t max_queries);
 /* Launch shapes and their tuner. A respond launch runs 1, 2 or 4 CTAs per query: one CTA
  * per SM is the most work per SM-second; a cluster of 2 or 4 splits each query's

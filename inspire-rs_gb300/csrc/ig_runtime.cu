@@ -2230,11 +2230,12 @@ struct ShapeRun {
 // of the width (a shape that it did not measure is not taken), else 6.95, 4.15 and 2.62 us a link (measured at gamma
 // 1024 under one, two and four CTAs). 128 queries over gamma 16, 256 and 1024 in equal parts took one CTA each: 7.65 ms,
 // the time of the 43 longest, with most SMs idle after 2 ms. Lanes share the SMs. More queries than four an SM fill the
-// GPU in any order: one CTA each.
+// GPU in any order: one CTA each. A pair threshold of 0 asks for one CTA a query always.
 static std::vector<ShapeRun> plan_shapes(ig_ctx* c, const MixedPlan& P, u32 n, u32 count) {
   const bool uniform = P.gammas.front() == P.gammas.back();
+  const bool single = c->pair_threshold == 0 && !igint::tuned_row(c, n, P.max_gamma, count);
   const u32 sms = std::max<u32>(1, c->sms / c->lanes);
-  if (c->force_ctas || uniform || count > 4 * sms)
+  if (c->force_ctas || uniform || single || count > 4 * sms)
     return {{0, count, igint::launch_ctas(c, n, P.max_gamma, count, count * c->lanes)}};
   std::map<u32, std::array<double, 3>> times;  // by gamma: a query under 1, 2, 4 CTAs
   std::vector<double> bounds;

@@ -1,6 +1,6 @@
 """The shapes that a mixed launch of several widths plans, seen in its number of launches (a scan and one a shape): a
 tuned row's times that are not above 0 are shapes that were not measured, not free ones; a row of a larger batch says
-nothing of one query. Responses are the same under every plan."""
+nothing of one query; a pair threshold of 0 keeps one CTA a query. Responses are the same under every plan."""
 import numpy as np
 import pytest
 
@@ -68,3 +68,10 @@ def test_tuned_rows(served, tmp_path, rows, launched):
     ctx, launches = served
     load_rows(ctx, tmp_path, rows)
     assert (launches() > 2) == (launched == "several")
+
+
+def test_pair_threshold(served):
+    ctx, launches = served
+    assert launches() > 2
+    ctx.set_pair_threshold(0)
+    assert launches() == 2
