@@ -412,13 +412,16 @@ int sync_crs_self(ig_ctx* c, CrsObj& o) {
   return IG_OK;
 }
 
+// Shards a launch takes at most (a grid's y and z run to 65,535).
+enum : u32 { LAUNCH_SHARDS = 16384 };
+
 // Shards of a store build that share a launch: their H words take 128 MB, most of which stays in L2 between the two
 // kernels. A launch's last wave leaves a fifth of the GPU idle at 32 MB: 64 shards of gamma 256 1.95 ms with 32 MB,
 // 1.86 with 64, 1.83 with 128.
-u32 store_group(const CrsObj& o) { return std::max<u32>(1, (u32)((128u << 20) / ((size_t)o.gamma * o.n * 8))); }
-
-// Shards a launch takes at most (a grid's y and z run to 65,535).
-enum : u32 { LAUNCH_SHARDS = 16384 };
+u32 store_group(const CrsObj& o) {
+  const size_t fit = (128u << 20) / ((size_t)o.gamma * o.n * 8);
+  return (u32)std::min<size_t>(LAUNCH_SHARDS, std::max<size_t>(1, fit));
+}
 
 // Writes the table entries of shards [first, first + count) on the context stream.
 int sync_table(ig_ctx* c, DbObj& db, u32 first, u32 count) {
