@@ -21,6 +21,7 @@
 
 #include <type_traits>
 
+#include "ig_inbox.cuh"
 #include "ig_kernels.cuh"
 
 namespace igk {
@@ -1591,7 +1592,6 @@ __device__ __forceinline__ int slot2(int t) {
 // on an mbarrier there, so a receiver waits for its data alone. A cluster barrier's release made every
 // thread wait until its remote stores had landed and its loads were back (1,400 cycles of a 6,480-cycle
 // link, twice).
-__device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ u32 cluster_addr(u32 addr, int rank) {
   u32 a;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
@@ -1606,27 +1606,6 @@ __device__ __forceinline__ void store_remote(u32 to, u64 v) {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void inbox_init(u32 bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-}
-// One thread opens a phase of `bytes`; every thread waits for its end.
-__device__ __forceinline__ void inbox_expect(u32 bar, u32 bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Waits for the phase of the given parity, a bounded number of tries (each suspends the thread up to a
-// hardware time limit); false when they ran out.
-constexpr int INBOX_TRIES = 1 << 20;
-__device__ __forceinline__ bool inbox_wait(u32 bar, u32 parity) {
-  for (int k = 0; k < INBOX_TRIES; k++) {
-    u32 done;
-    asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
-                 : "=r"(done)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-    if (done) return true;
-  }
-  return false;
-}
 
 template <int LOGN, int R>
 __global__ void __launch_bounds__((1 << LOGN) / R / 2, 1)
