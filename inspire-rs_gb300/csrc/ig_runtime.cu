@@ -1299,7 +1299,7 @@ int ig_session_store_destroy(ig_ctx* c, uint64_t st) {
 }
 
 // PackingKeySeat::build checks (session.rs:600-625, 661-697, 766-826), then the key
-// body's NTT in R-form on the device.
+// body's key rows (igk::key_rows) on the device.
 static int make_seat(ig_ctx* c, CrsObj& o, const uint64_t* y_body, uint32_t rows, uint32_t num_to_pack, u64* dst,
                      bool y_on_device) {
   if (rows != o.rows)

@@ -45,11 +45,10 @@ struct Prime32 {
   __host__ __device__ __forceinline__ i64 centred(u32 x) const { return x > (m >> 1) ? (i64)x - (i64)m : (i64)x; }
 };
 
-// One transform's constants (arith.rs:131-166): bit-reversed Montgomery-form powers of psi and psi^-1.
+// One transform's constants (arith.rs:131-166): bit-reversed Montgomery-form powers of psi.
 struct Ntt32Dev {
   Prime32 p;
   const u32* fwd;
-  const u32* inv;
   const uint2* fwd_sh;  // the forward ladder in standard form with Shoup companions (w, w')
   u32 n_inv;            // 1/n in Montgomery form
 };

@@ -18,9 +18,8 @@ namespace igsmk {
 using namespace igsm;
 
 // ------------------------------------------------------------------------------------
-// Ntt32 in shared memory, radix-4 (one 4-word unit per thread, N/4 threads). The stage
-// schedule and twiddle indices are those of arith.rs:169-251: forward Cooley-Tukey over
-// fwd[m + i], inverse Gentleman-Sande over inv[h + i] with the last stage carrying 1/n.
+// Forward Ntt32 in shared memory, radix-4 (one 4-word unit per thread, N/4 threads). The stage
+// schedule and twiddle indices are those of arith.rs:169-251: Cooley-Tukey over fwd[m + i].
 template <int LOGN>
 __device__ __forceinline__ void fwd32(u32* x, const Ntt32Dev& T, const u32* tw) {
   constexpr int N = 1 << LOGN, NT = N / 4;

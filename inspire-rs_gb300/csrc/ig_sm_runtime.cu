@@ -53,7 +53,7 @@ struct HostNtt32 {
   u64 m;
   size_t n;
   u32 neg_minv;
-  std::vector<u32> fwd_std, fwd, inv;  // standard-form ladder (host transform), Montgomery ladders
+  std::vector<u32> fwd_std, fwd;  // standard-form ladder (host transform), Montgomery ladder
   u32 n_inv;
   u32 to_mont(u64 x) const { return (u32)(((u128)x << 32) % m); }
   HostNtt32(size_t nn, u64 mm) : m(mm), n(nn) {
@@ -68,24 +68,19 @@ struct HostNtt32 {
         break;
       }
     }
-    const u32 psi_inv = powm(psi, 2 * n - 1, m);
     unsigned bits = 0;
     while ((size_t(1) << bits) < n) bits++;
-    std::vector<u32> pf(n), pi(n);
-    u64 a = 1, b = 1;
+    std::vector<u32> pf(n);
+    u64 a = 1;
     for (size_t k = 0; k < n; k++) {
       pf[k] = (u32)a;
-      pi[k] = (u32)b;
       a = a * psi % m;
-      b = b * psi_inv % m;
     }
     fwd_std.resize(n);
     fwd.resize(n);
-    inv.resize(n);
     for (size_t k = 0; k < n; k++) {
       fwd_std[k] = pf[bitrev(k, bits)];
       fwd[k] = to_mont(pf[bitrev(k, bits)]);
-      inv[k] = to_mont(pi[bitrev(k, bits)]);
     }
     n_inv = to_mont(powm(n, m - 2, m));
   }
@@ -313,8 +308,8 @@ int ig_sm_server_create(ig_ctx* c, uint32_t ring_dim, uint32_t gamma, uint64_t q
   const u32* shq_dev = nullptr;
   const u32* shp_dev = nullptr;
   int rc;
-  if ((rc = up(c, o, hq.fwd, &dv.lq.fwd)) || (rc = up(c, o, hq.inv, &dv.lq.inv)) || (rc = up(c, o, hp.fwd, &dv.lp.fwd)) ||
-      (rc = up(c, o, hp.inv, &dv.lp.inv)) || (rc = up(c, o, shq, &shq_dev)) || (rc = up(c, o, shp, &shp_dev)) ||
+  if ((rc = up(c, o, hq.fwd, &dv.lq.fwd)) || (rc = up(c, o, hp.fwd, &dv.lp.fwd)) ||
+      (rc = up(c, o, shq, &shq_dev)) || (rc = up(c, o, shp, &shp_dev)) ||
       (rc = up(c, o, se, &dv.slot_exp)) || (rc = up(c, o, es, &dv.exp_slot)) ||
       (rc = up(c, o, gpow, &dv.gpow)) || (rc = up(c, o, cpow, &dv.cpow)) || (rc = up(c, o, mi, &dv.m_of_i)) ||
       (rc = up(c, o, pw, &dv.pow_root_R))) {
