@@ -1123,7 +1123,7 @@ def run_cfg4(args, rank, world):
         return max_over_ranks(ev0.elapsed_time(ev1), world), ctx.launch_count - launches0, clk
 
     timed_queries = int(offs[-1] - offs[args.warmup])
-    # The fixed rule first (no table: four CTAs per query while count x lanes <= 36, two
+    # The fixed rule first (no table: four CTAs per query while count x lanes such clusters run at once, two
     # while count x lanes <= SMs / 2, else one), then
     # the launch-shape tuner's table for the three widths, then the same launches tuned.
     ms_fixed, _, _ = timed_region()
@@ -1260,7 +1260,7 @@ def run_cfg4(args, rank, world):
                 "d2h_bytes_per_step": int(timed_queries * 2 * N_RING * 8 / args.steps), "callers": lanes,
                 "call": "respond_mixed_batch (one launch per call)"},
         "fixed_rule": {"value": fixed_value, "unit": "queries/s",
-                       "rule": "four CTAs per query while count x lanes <= 36, two while "
+                       "rule": "four CTAs per query while count x lanes such clusters run at once, two while "
                                "count x lanes <= SMs / 2, else one"},
         "launch_shapes": {"tuned_ms_per_launch": {str(g): {str(b): {"1": t[0], "2": t[1], "4": t[2]}
                                                            for b, t in rows.items()} for g, rows in tuned.items()},

@@ -54,8 +54,8 @@ uint64_t ig_ctx_device_bytes(const ig_ctx* ctx);
 /* Launch-shape knob of the fixed rule, used when the context holds no tuned table for the
  * launch's width (ig_tune_launch_shapes): with q the queries expected on the device (the
  * batch times the lanes, or the queries in flight), a launch runs four CTAs per query (a
- * thread-block cluster) while 2q <= max_queries and q such clusters run at once (36: each
- * takes its SMs within one GPC), two while q <= max_queries, else one, so small batches
+ * thread-block cluster) while 2q <= max_queries and q such clusters run at once (asked of
+ * the device: each takes its SMs within one GPC), two while q <= max_queries, else one, so small batches
  * still occupy most SMs. A batch of more queries than SMs on one lane runs its whole waves
  * with one CTA a query and what is left as a batch of that size; a mixed batch of several
  * widths gives each width a shape of its own. Default: half the device's SM count; 0 runs
